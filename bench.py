@@ -427,7 +427,7 @@ def main():
                       "frac_of_measured_hbm": kbytes[name] / (stage[name] * 1e-6) / 1e9 / hbm}
                for name in stage}
     dominant = max(stage, key=stage.get)
-    kernel_names = {"indexer_scores": "indexer_decode_kernel<64, 16 heads>", "topk_select": "topk_cluster_kernel",
+    kernel_names = {"indexer_scores": "indexer_decode_kernel<64, 16 heads>", "topk_select": "topk_pivot_kernel",
                     "sparse_attn": "sparse_attn_tc_kernel<int8 kv, bf16 q> (splits merged inside a cluster)"}
     # DRAM traffic from ncu captures on the --small case (profiles/), scaled by the units each launch processes:
     # the key scan reads 65.0 B and writes 4.8 B per key row; the attention kernel reads 787 B per gathered row

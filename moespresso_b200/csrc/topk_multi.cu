@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kMThreads) topk_mfilter_kernel(TopkMultiParams
   TRF(0);
   if (tid < 4) s_thr[tid] = 0;
   __syncthreads();
-  row_threshold(p.hist + (int64_t)row * kBigBins, p.k, warp_sums, &s_total, s_thr);
+  row_threshold<kMThreads>(p.hist + (int64_t)row * kBigBins, p.k, warp_sums, &s_total, s_thr);
   TRF(1);
   if (s_thr[0] == 0) return;
   const uint32_t bin = s_thr[1];
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(1024) topk_mfinish_kernel(TopkMultiParams p, i
   if (tid < 4) s_thr[tid] = 0;
   if (tid == 0) s_cnt = 0;
   __syncthreads();
-  row_threshold(p.hist + (int64_t)row * kBigBins, p.k, warp_sums, &s_total, s_thr);
+  row_threshold<1024>(p.hist + (int64_t)row * kBigBins, p.k, warp_sums, &s_total, s_thr);
   const uint32_t k_eff = s_thr[0];
   for (int i = tid + (int)k_eff; i < p.k; i += 1024) out[i] = -1;
   if (k_eff == 0 || n <= 0) return;

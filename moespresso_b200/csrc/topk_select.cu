@@ -6,10 +6,9 @@
 // Selected set: every row with key > T, plus the `need` LOWEST-index rows with
 // key == T, where T is the k-th largest key.  Output ids ascending, -1 padded.
 //
-//  * topk_row_kernel      — one CTA per row, the row's keys resident in shared memory
-//    (rows up to kSmemRowMax); four 8-bit radix passes, then an ordered emission
-//    through a block scan, so the output is ascending without a sort.
-//  * topk_stream_kernel   — rows longer than that (up to 2^31 - 1): one CTA streams the
+//  * topk_pivot_kernel (topk_pivot.cu)  rows of up to 2^21 scores;
+//  * topk_mhist / mfilter / mfinish (topk_multi.cu)  longer rows;
+//  * topk_stream_kernel (here)  the entry point for callers that cannot allocate: one CTA streams the
 //    row twice from L2 (11-bit histogram, then strictly-above ids + the threshold bin's
 //    candidates), resolves the remaining 21 bits and the ties by lowest index among the
 //    candidates, and sorts the selected ids.
@@ -33,92 +32,6 @@ struct TopkParams {
   uint32_t* cand_key;  // [rows][n]
   int32_t* cand_idx;   // [rows][n]
 };
-
-// --------------------------------------------------------------------------
-// one CTA per row, keys in shared memory
-// --------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) topk_row_kernel(TopkParams p) {
-  extern __shared__ uint32_t keys[];  // [n]
-  __shared__ uint32_t hist[256];
-  __shared__ uint32_t warp_sums[32];
-  __shared__ uint32_t s_digit, s_above, s_total, s_total2, s_nvalid;
-
-  const int row = blockIdx.x;
-  const int tid = threadIdx.x;
-  const int64_t base = p.row_start ? p.row_start[row] : (int64_t)row * p.row_stride;
-  int n = (int)(p.row_count ? min((int64_t)p.row_count[row], p.n) : p.n);
-  if (n < 0) n = 0;
-  const float* src = p.scores + base;
-  int32_t* out = p.out_ids + (int64_t)row * p.k;
-
-  if (tid == 0) s_nvalid = 0;
-  __syncthreads();
-  uint32_t nv = 0;
-  for (int i = tid; i < n; i += blockDim.x) {
-    uint32_t key = score_key_full(src[i]);
-    keys[i] = key;
-    nv += key != 0;
-  }
-  nv = __reduce_add_sync(0xffffffffu, nv);
-  if ((tid & 31) == 0 && nv) atomicAdd(&s_nvalid, nv);
-  __syncthreads();
-  const uint32_t k_eff = min((uint32_t)p.k, s_nvalid);
-  for (int i = tid + (int)k_eff; i < p.k; i += blockDim.x) out[i] = -1;
-  if (k_eff == 0) return;
-
-  uint32_t prefix = 0, prefix_mask = 0, want = k_eff;
-  // Scores cluster in a few exponent values, so one shared histogram would serialise almost every
-  // atomic on the same address; each warp counts into its own 256 bins, merged afterwards.
-  uint32_t* whist = keys + p.n;                    // [warps][256]
-  const int nwarps = (int)blockDim.x >> 5;
-  uint32_t* my_hist = whist + (tid >> 5) * 256;
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    for (int i = tid; i < nwarps * 256; i += blockDim.x) whist[i] = 0;
-    __syncthreads();
-    for (int i = tid; i < n; i += blockDim.x) {
-      uint32_t key = keys[i];
-      if (key != 0 && (key & prefix_mask) == prefix) atomicAdd(&my_hist[(key >> shift) & 255u], 1u);
-    }
-    __syncthreads();
-    if (tid < 256) {
-      uint32_t t = 0;
-      for (int w = 0; w < nwarps; ++w) t += whist[w * 256 + tid];
-      hist[tid] = t;
-    }
-    __syncthreads();
-    if (tid < 32) pick_digit_256(hist, want, &s_digit, &s_above);
-    __syncthreads();
-    prefix |= s_digit << shift;
-    prefix_mask |= 255u << shift;
-    want -= s_above;
-    __syncthreads();
-  }
-  const uint32_t thr = prefix;
-  const uint32_t need = want;  // ties to take, >= 1
-
-  // ordered emission: thread t owns the contiguous slice [t*per, (t+1)*per)
-  // (odd slice length: lanes of a warp then walk different shared-memory banks)
-  const int per = ((n + (int)blockDim.x - 1) / (int)blockDim.x) | 1;
-  const int lo = min(tid * per, n), hi = min(lo + per, n);
-  uint32_t ca = 0, ct = 0;
-  for (int i = lo; i < hi; ++i) {
-    uint32_t key = keys[i];
-    ca += key > thr;
-    ct += key == thr;
-  }
-  uint32_t base_a = block_excl_scan(ca, warp_sums, &s_total);
-  uint32_t base_t = block_excl_scan(ct, warp_sums, &s_total2);
-  for (int i = lo; i < hi; ++i) {
-    uint32_t key = keys[i];
-    if (key > thr) {
-      out[base_a + min(base_t, need)] = i;
-      ++base_a;
-    } else if (key == thr) {
-      if (base_t < need) out[base_a + base_t] = i;
-      ++base_t;
-    }
-  }
-}
 
 // --------------------------------------------------------------------------
 // long rows: one CTA per row streams the row twice (the scores were just written by
@@ -306,8 +219,8 @@ __global__ void __launch_bounds__(1024) topk_stream_kernel(TopkParams p, int sor
 
 int64_t topk_multi_workspace(int32_t rows, int64_t n, int32_t k);   // topk_multi.cu
 int launch_topk_multi(const mxb_topk_args* a, cudaStream_t st);
-int topk_cluster_size(int32_t rows, int64_t n);                        // topk_cluster.cu
-int launch_topk_cluster(const mxb_topk_args* a, int cs, cudaStream_t st);
+int topk_pivot_size(int32_t rows, int64_t n);                          // topk_pivot.cu
+int launch_topk_pivot(const mxb_topk_args* a, int cs, cudaStream_t st);
 
 }  // namespace mxb
 
@@ -315,7 +228,7 @@ using namespace mxb;
 
 extern "C" int64_t mxb_topk_workspace_bytes(int32_t rows, int64_t n, int32_t k) {
   if (rows <= 0 || n <= 0 || k <= 0) return 0;
-  if (topk_cluster_size(rows, n) > 0 || n <= kSmemRowMax) return 0;
+  if (topk_pivot_size(rows, n) > 0) return 0;
   return topk_multi_workspace(rows, n, k);
 }
 
@@ -326,24 +239,9 @@ extern "C" int mxb_topk_select(const mxb_topk_args* a, void* stream) {
   MXB_REQUIRE(a->n < ((int64_t)1 << 31), MXB_ERR_INVALID, "topk: row length must be below 2^31");
   MXB_REQUIRE(a->scores && a->out_ids, MXB_ERR_INVALID, "topk: null tensor");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  TopkParams p{};
-  p.scores = a->scores; p.row_stride = a->row_stride; p.row_start = a->row_start; p.row_count = a->row_count;
-  p.out_ids = a->out_ids; p.rows = a->rows; p.n = a->n; p.k = a->k;
-
-  if (const int cs = topk_cluster_size(a->rows, a->n)) return launch_topk_cluster(a, cs, st);
-  // the other kernels count their own first digit: only keep the promise that the counters end up clear
+  // these kernels count for themselves: only keep the promise that the counters end up clear
   if (a->digit_hist) MXB_CUDA_OK(cudaMemsetAsync(a->digit_hist, 0, (size_t)a->rows * kBigBins * sizeof(uint32_t), st));
-  if (a->n <= kSmemRowMax) {
-    int threads = a->n >= 8192 ? 1024 : (a->n >= 2048 ? 512 : 256);
-    size_t smem = (size_t)a->n * 4 + (size_t)(threads / 32) * 256 * 4;   // keys + per-warp histograms
-    if (smem > 48 * 1024)
-      MXB_CUDA_OK(cudaFuncSetAttribute(topk_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    topk_row_kernel<<<a->rows, threads, smem, st>>>(p);
-    note_launch();
-    MXB_CUDA_OK(cudaGetLastError());
-    return MXB_OK;
-  }
-
+  if (const int cs = topk_pivot_size(a->rows, a->n)) return launch_topk_pivot(a, cs, st);
   return launch_topk_multi(a, st);
 }
 

@@ -71,6 +71,41 @@ def test_many_rows_small_clusters(n, k, rows):
     _check(np.round(rng.standard_normal((rows, n)) * 2).astype(np.float32), k)
 
 
+@pytest.mark.parametrize("n,k,rows", [(7901, 512, 2), (8191, 512, 2), (8192, 8192, 1), (8193, 2048, 3), (16384, 2048, 160),
+                                      (16385, 8192, 1), (32767, 16, 33), (131072, 2048, 20), (300001, 8192, 2),
+                                      (1 << 21, 2048, 1), ((1 << 21) + 1, 2048, 1)])
+def test_direct_and_sampled_rows(n, k, rows):
+    """Either side of the direct kernel's sizes, of the cluster sizes and of the longest sampled row; random rows, and
+    rows on which the sample misleads: few large scores packed into one place (the sampled positions miss them), scores
+    of a few distinct values (more keys reach the pivot than the list holds), fewer finite scores than k."""
+    need_gpu()
+    rng = np.random.default_rng(n + k)
+    s = rng.standard_normal((rows, n)).astype(np.float32)
+    _check(s, k)
+    packed = s.copy()
+    packed[:, n // 3:n // 3 + min(k + 5, n // 2)] += 100.0
+    _check(packed, k)
+    _check(np.round(s), k)
+    s[:, n // 7:] = -np.inf
+    _check(s, k)
+
+
+def test_sampled_rows_of_a_ragged_batch():
+    """Rows that start at any offset and range from empty to the longest, on clusters and on one CTA per row."""
+    need_gpu()
+    rng = np.random.default_rng(12)
+    for count in (9, 200):
+        lens = rng.integers(1, 30000, size=count)
+        lens[:6] = [0, 1, 40001, 16383, 2049, 5]
+        start = np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.int64)
+        flat = rng.standard_normal(int(lens.sum()) + 3).astype(np.float32)
+        got = topk_select(dev(flat), 2048, valid=dev(lens.astype(np.int32)), row_start=dev(start),
+                          n=int(lens.max())).cpu().numpy()
+        for b, (s, n) in enumerate(zip(start, lens)):
+            ref = ds4.topk_ids(flat[s:s + n], 2048)[0] if n else np.full(2048, -1)
+            np.testing.assert_array_equal(got[b], ref)
+
+
 def test_long_rows_ties():
     need_gpu()
     rng = np.random.default_rng(4)
@@ -97,8 +132,7 @@ def test_ragged_flat_rows():
 @pytest.mark.parametrize("kind", ["normal", "ties", "specials"])
 def test_selection_from_a_precounted_first_digit(kind):
     """With the rows' first-digit histograms handed in (as the decode scan leaves them) the selection is the same,
-    bit for bit, and the counters are zero afterwards — on the cluster kernel, which uses them, and on the kernels
-    that only clear them."""
+    bit for bit, and the counters are zero afterwards."""
     need_gpu()
     from tests.gpu_util import first_digit_hist
     rng = np.random.default_rng(11)
@@ -119,7 +153,7 @@ def test_selection_from_a_precounted_first_digit(kind):
             ref = ds4.topk_ids(flat[s:s + n], k)[0] if n else np.full(k, -1)
             np.testing.assert_array_equal(got[b], ref)
         assert int(h.abs().sum()) == 0
-    # short rows go to the one-CTA kernel, very long ones to the multi-launch one: both ignore and clear the counters
+    # the selection counts for itself whatever the row length, and clears the counters
     for n in (5000, 400000):
         s2 = rng.standard_normal((2, n)).astype(np.float32)
         h = dev(np.stack([first_digit_hist(r) for r in s2]))
