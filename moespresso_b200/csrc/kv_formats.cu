@@ -12,6 +12,7 @@
 //  * quant_i8_rows_kernel — the per-token int8 quantiser that produces the int8 + fp16-scale cache the
 //    sparse decode kernels read: scale = fp16(amax / 127) (rounded up when the rounding would let a
 //    value exceed 127), q = clamp(rint(x / scale), -127, 127).  No counterpart in the reference.
+//    quant_i8_rows_vec_kernel is the form for rows of whole 16-byte pieces, quant_i8_rows_kernel takes any row.
 #include "common.cuh"
 
 namespace mxb {
@@ -91,6 +92,17 @@ __global__ void __launch_bounds__(128) fp8_kv_rows_kernel(const float* __restric
   for (int j = 0; j < 4; ++j) dst[j] = make_float4(xv[4 * j], xv[4 * j + 1], xv[4 * j + 2], xv[4 * j + 3]);
 }
 
+// fp16 scale of a row whose largest magnitude is amax
+__device__ __forceinline__ __half i8_row_scale(float amax) {
+  __half hs = __float2half_rn(amax / 127.0f);
+  if (__half2float(hs) * 127.0f < amax) hs = __ushort_as_half((unsigned short)(__half_as_ushort(hs) + 1));  // next fp16 up
+  if (__half2float(hs) == 0.0f) hs = __ushort_as_half((unsigned short)1);   // all-zero row: any scale will do
+  return hs;
+}
+__device__ __forceinline__ int8_t i8_quant_exact(float x, float s) {
+  return (int8_t)fminf(fmaxf(rintf(x / s), -127.0f), 127.0f);
+}
+
 template <int XT>
 __global__ void __launch_bounds__(128) quant_i8_rows_kernel(const void* __restrict__ x, int8_t* __restrict__ q,
                                                             __half* __restrict__ scales, int64_t n_rows, int width) {
@@ -101,13 +113,68 @@ __global__ void __launch_bounds__(128) quant_i8_rows_kernel(const void* __restri
   for (int i = lane; i < width; i += 32) amax = fmaxf(amax, fabsf(load_elem<XT>(x, row * width + i)));
 #pragma unroll
   for (int m = 16; m >= 1; m >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
-  __half hs = __float2half_rn(amax / 127.0f);
-  if (__half2float(hs) * 127.0f < amax) hs = __ushort_as_half((unsigned short)(__half_as_ushort(hs) + 1));  // next fp16 up
-  if (__half2float(hs) == 0.0f) hs = __ushort_as_half((unsigned short)1);   // all-zero row: any scale will do
+  const __half hs = i8_row_scale(amax);
   const float s = __half2float(hs);
-  for (int i = lane; i < width; i += 32) {
-    const float v = rintf(load_elem<XT>(x, row * width + i) / s);
-    q[row * width + i] = (int8_t)fminf(fmaxf(v, -127.0f), 127.0f);
+  for (int i = lane; i < width; i += 32) q[row * width + i] = i8_quant_exact(load_elem<XT>(x, row * width + i), s);
+  if (lane == 0) scales[row] = hs;
+}
+
+// One warp per row, the row in registers as NV 16-byte pieces per lane (a piece beyond the row reads as zeros).
+// Bound: HBM (row in, int8 row out).  The elements are read once, and no element is divided: x * (1 / s) differs from
+// x / s by a few units in the last place, so both round to the same integer unless the product lies within 1e-4 of a
+// half-integer (|product| <= 127, an error of 3 * 2^-24 relative is below 3e-5); a lane that holds such an element, or
+// a NaN or an infinity, redoes its piece with the division.  40,001 rows of 576 bf16 values: 30.2 -> 17.0 us
+// (2.3 -> 4.1 TB/s); the scalar form spends 20 instructions on each division and reads every element twice.
+template <int XT, int NV>
+__global__ void __launch_bounds__(128) quant_i8_rows_vec_kernel(const uint4* __restrict__ x, int8_t* __restrict__ q,
+                                                                __half* __restrict__ scales, int64_t n_rows, int width) {
+  constexpr int EPV = XT == MXB_F32 ? 4 : 8;   // elements per piece
+  const int lane = threadIdx.x & 31;
+  const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (row >= n_rows) return;
+  const int pieces = width / EPV;
+  uint4 raw[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v)
+    raw[v] = 32 * v + lane < pieces ? __ldcs(x + row * pieces + 32 * v + lane) : make_uint4(0, 0, 0, 0);
+  float amax = 0.0f;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    float f[EPV];
+    unpack16<XT>(raw[v], f);
+#pragma unroll
+    for (int e = 0; e < EPV; ++e) amax = fmaxf(amax, fabsf(f[e]));
+  }
+  // magnitudes order like their bits
+  amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
+  const __half hs = i8_row_scale(amax);
+  const float s = __half2float(hs), inv = 1.0f / s;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    if (32 * v + lane < pieces) {
+      float f[EPV];
+      unpack16<XT>(raw[v], f);
+      uint32_t b[EPV];
+      bool sure = true;
+#pragma unroll
+      for (int e = 0; e < EPV; ++e) {
+        const float t = f[e] * inv;
+        const float m = t + 12582912.0f;   // 1.5 * 2^23: the rounded integer sits in the low mantissa bits
+        sure = sure && fabsf(t - (m - 12582912.0f)) < 0.4999f;   // false for NaN and infinities
+        b[e] = __float_as_uint(m);
+      }
+      if (!sure) {
+#pragma unroll
+        for (int e = 0; e < EPV; ++e) b[e] = (uint8_t)i8_quant_exact(f[e], s);
+      }
+      uint32_t w[EPV / 4];
+#pragma unroll
+      for (int i = 0; i < EPV / 4; ++i)
+        w[i] = __byte_perm(__byte_perm(b[4 * i], b[4 * i + 1], 0x0040), __byte_perm(b[4 * i + 2], b[4 * i + 3], 0x0040), 0x5410);
+      int8_t* dst = q + row * width + (32 * v + lane) * EPV;
+      if constexpr (EPV == 8) *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+      else *reinterpret_cast<uint32_t*>(dst) = w[0];
+    }
   }
   if (lane == 0) scales[row] = hs;
 }
@@ -141,11 +208,29 @@ extern "C" int mxb_quantize_kv_int8(const mxb_quantize_kv_int8_args* a, void* st
   MXB_REQUIRE(a->x_dtype == MXB_F32 || a->x_dtype == MXB_F16 || a->x_dtype == MXB_BF16, MXB_ERR_INVALID,
               "int8 quantiser rows must be float32, float16, or bfloat16");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  MXB_REQUIRE(ceil_div(a->n_rows, 4) <= 0x7FFFFFFFll, MXB_ERR_INVALID, "int8 quantiser: too many rows");
   const unsigned grid = (unsigned)ceil_div(a->n_rows, 4);
   __half* sc = reinterpret_cast<__half*>(a->scales);
-  if (a->x_dtype == MXB_F32) quant_i8_rows_kernel<MXB_F32><<<grid, 128, 0, st>>>(a->x, a->q, sc, a->n_rows, a->width);
-  else if (a->x_dtype == MXB_F16) quant_i8_rows_kernel<MXB_F16><<<grid, 128, 0, st>>>(a->x, a->q, sc, a->n_rows, a->width);
-  else quant_i8_rows_kernel<MXB_BF16><<<grid, 128, 0, st>>>(a->x, a->q, sc, a->n_rows, a->width);
+  // whole 16-byte pieces on 16-byte boundaries, at most eight per lane
+  const int epv = a->x_dtype == MXB_F32 ? 4 : 8;
+  const int nv = a->width % epv == 0 ? (int)ceil_div(a->width / epv, 32) : 99;
+  if (nv <= 8 && (reinterpret_cast<uintptr_t>(a->x) & 15) == 0 && (reinterpret_cast<uintptr_t>(a->q) & 7) == 0) {
+    const uint4* xv = reinterpret_cast<const uint4*>(a->x);
+#define MXB_QVEC(XT)                                                                                            \
+  if (nv <= 3) quant_i8_rows_vec_kernel<XT, 3><<<grid, 128, 0, st>>>(xv, a->q, sc, a->n_rows, a->width);        \
+  else if (nv <= 5) quant_i8_rows_vec_kernel<XT, 5><<<grid, 128, 0, st>>>(xv, a->q, sc, a->n_rows, a->width);   \
+  else quant_i8_rows_vec_kernel<XT, 8><<<grid, 128, 0, st>>>(xv, a->q, sc, a->n_rows, a->width)
+    if (a->x_dtype == MXB_F32) { MXB_QVEC(MXB_F32); }
+    else if (a->x_dtype == MXB_F16) { MXB_QVEC(MXB_F16); }
+    else { MXB_QVEC(MXB_BF16); }
+#undef MXB_QVEC
+  } else if (a->x_dtype == MXB_F32) {
+    quant_i8_rows_kernel<MXB_F32><<<grid, 128, 0, st>>>(a->x, a->q, sc, a->n_rows, a->width);
+  } else if (a->x_dtype == MXB_F16) {
+    quant_i8_rows_kernel<MXB_F16><<<grid, 128, 0, st>>>(a->x, a->q, sc, a->n_rows, a->width);
+  } else {
+    quant_i8_rows_kernel<MXB_BF16><<<grid, 128, 0, st>>>(a->x, a->q, sc, a->n_rows, a->width);
+  }
   note_launch();
   MXB_CUDA_OK(cudaGetLastError());
   return MXB_OK;

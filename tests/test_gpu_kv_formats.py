@@ -84,6 +84,33 @@ def test_quantize_kv_int8(dtype):
     # the decode operators read this format: a one-row sanity check through sparse attention happens elsewhere
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("width", [1, 8, 20, 256, 576, 768, 1288, 2048, 2056])
+def test_quantize_kv_int8_widths_and_half_integers(dtype, width):
+    """Both forms of the quantiser (rows of whole 16-byte pieces, up to eight per lane, and any other row), bit for bit:
+    quotients exactly between two integers, NaN and infinite elements, rows whose scale overflows or underflows fp16."""
+    need_gpu()
+    rng = np.random.default_rng(width)
+    x = (rng.standard_normal((37, width)) * np.exp(rng.uniform(-12, 8, size=(37, 1)))).astype(np.float32)
+    x[1] = (rng.integers(-127, 127, size=width) + 0.5) * 2.0 ** -5
+    x[1, 0] = 127 * 2.0 ** -5                                        # scale 2^-5: every quotient is a half-integer
+    x[2] = 0
+    x[3, width // 2] = np.inf
+    x[4, width // 2] = np.nan
+    x[5] *= 1e-8
+    if dtype != torch.float16:
+        x[6] *= 1e12
+    t = dev(x).to(dtype)
+    q, s = quantize_kv_int8(t)
+    ok = [r for r in range(37) if r not in (3, 4)]
+    eq, es = ds4.quantize_kv_int8(t.float().cpu().numpy()[ok])
+    finite = np.isfinite(es.astype(np.float32))
+    np.testing.assert_array_equal(s.cpu().numpy()[ok].view(np.uint16), es.view(np.uint16))
+    np.testing.assert_array_equal(q.cpu().numpy()[ok][finite], eq[finite])
+    assert np.isinf(s[3].item()) and int(q[3, width // 2]) == -127 and int(q[3].abs().sum()) == 127
+    assert int(q[4, width // 2]) == -127
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-7), (torch.bfloat16, 0.0), (torch.float16, 0.0)])
 def test_rope_tail_against_reference_vectors(dtype, tol):
     """apply_rope_tail through the CUDA kernel against outputs of the reference's NumPy function."""
