@@ -119,64 +119,82 @@ __global__ void __launch_bounds__(128) quant_i8_rows_kernel(const void* __restri
   if (lane == 0) scales[row] = hs;
 }
 
-// One warp per row, the row in registers as NV 16-byte pieces per lane (a piece beyond the row reads as zeros).
-// Bound: HBM (row in, int8 row out).  The elements are read once, and no element is divided: x * (1 / s) differs from
-// x / s by a few units in the last place, so both round to the same integer unless the product lies within 1e-4 of a
-// half-integer (|product| <= 127, an error of 3 * 2^-24 relative is below 3e-5); a lane that holds such an element, or
-// a NaN or an infinity, redoes its piece with the division.  40,001 rows of 576 bf16 values: 30.2 -> 17.0 us
-// (2.3 -> 4.1 TB/s); the scalar form spends 20 instructions on each division and reads every element twice.
+// max(|a|, |b|, |c|), NaN if one of them is
+__device__ __forceinline__ float max3_nan_abs(float a, float b, float c) {
+  float r;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// One warp per row at a time, the row in registers as NV 16-byte pieces per lane (a piece beyond the row reads as
+// zeros), the next row on its way.  Bound: HBM (row in, int8 row out), with instruction issue close behind: the elements
+// are read once, and no element is divided.  x * (1 / s) differs from x / s by a few units in the last place, so both
+// round to the same integer unless the product lies within 1e-4 of a half-integer (|product| <= 127, a relative error of
+// 2^-23 is below 2e-5); a lane that holds such an element, or a NaN or an infinity, redoes its piece with the division.
+// The multiply-adds are packed in pairs.  40,001 rows of 576 bf16 values: 30.2 -> 14.2 us (2.3 -> 4.9 TB/s); the scalar
+// form spends 20 instructions on each division and reads every element twice, one row per warp without the look-ahead
+// and the pairs took 17.0 us.
 template <int XT, int NV>
-__global__ void __launch_bounds__(128) quant_i8_rows_vec_kernel(const uint4* __restrict__ x, int8_t* __restrict__ q,
+__global__ void __launch_bounds__(256) quant_i8_rows_vec_kernel(const uint4* __restrict__ x, int8_t* __restrict__ q,
                                                                 __half* __restrict__ scales, int64_t n_rows, int width) {
   constexpr int EPV = XT == MXB_F32 ? 4 : 8;   // elements per piece
   const int lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (row >= n_rows) return;
+  const int64_t step = (int64_t)gridDim.x * 8;
+  int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int pieces = width / EPV;
-  uint4 raw[NV];
+  uint4 next[NV];
+  auto fetch = [&](int64_t r) {
 #pragma unroll
-  for (int v = 0; v < NV; ++v)
-    raw[v] = 32 * v + lane < pieces ? __ldcs(x + row * pieces + 32 * v + lane) : make_uint4(0, 0, 0, 0);
-  float amax = 0.0f;
+    for (int v = 0; v < NV; ++v)
+      next[v] = r < n_rows && 32 * v + lane < pieces ? __ldcs(x + r * pieces + 32 * v + lane) : make_uint4(0, 0, 0, 0);
+  };
+  fetch(row);
+  for (; row < n_rows; row += step) {   // the same trip count for the lanes of a warp
+    float f[NV][EPV];
+    float amax = 0.0f;
 #pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    float f[EPV];
-    unpack16<XT>(raw[v], f);
+    for (int v = 0; v < NV; ++v) {
+      unpack16<XT>(next[v], f[v]);
 #pragma unroll
-    for (int e = 0; e < EPV; ++e) amax = fmaxf(amax, fabsf(f[e]));
-  }
-  // magnitudes order like their bits
-  amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
-  const __half hs = i8_row_scale(amax);
-  const float s = __half2float(hs), inv = 1.0f / s;
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    if (32 * v + lane < pieces) {
-      float f[EPV];
-      unpack16<XT>(raw[v], f);
-      uint32_t b[EPV];
-      bool sure = true;
-#pragma unroll
-      for (int e = 0; e < EPV; ++e) {
-        const float t = f[e] * inv;
-        const float m = t + 12582912.0f;   // 1.5 * 2^23: the rounded integer sits in the low mantissa bits
-        sure = sure && fabsf(t - (m - 12582912.0f)) < 0.4999f;   // false for NaN and infinities
-        b[e] = __float_as_uint(m);
-      }
-      if (!sure) {
-#pragma unroll
-        for (int e = 0; e < EPV; ++e) b[e] = (uint8_t)i8_quant_exact(f[e], s);
-      }
-      uint32_t w[EPV / 4];
-#pragma unroll
-      for (int i = 0; i < EPV / 4; ++i)
-        w[i] = __byte_perm(__byte_perm(b[4 * i], b[4 * i + 1], 0x0040), __byte_perm(b[4 * i + 2], b[4 * i + 3], 0x0040), 0x5410);
-      int8_t* dst = q + row * width + (32 * v + lane) * EPV;
-      if constexpr (EPV == 8) *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
-      else *reinterpret_cast<uint32_t*>(dst) = w[0];
+      for (int e = 0; e < EPV; e += 2) amax = fmaxf(fmaxf(amax, fabsf(f[v][e])), fabsf(f[v][e + 1]));
     }
+    fetch(row + step);
+    // magnitudes order like their bits
+    amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
+    const __half hs = i8_row_scale(amax);
+    const float s = __half2float(hs), inv = __frcp_rn(s);
+    const float2 inv2 = make_float2(inv, inv);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      if (32 * v + lane < pieces) {
+        uint32_t b[EPV];
+        float off = 0.0f;   // largest distance from the rounded integer; NaN if one is
+#pragma unroll
+        for (int e = 0; e < EPV; e += 2) {
+          const float2 x2 = make_float2(f[v][e], f[v][e + 1]);
+          // 1.5 * 2^23: the rounded integer sits in the low mantissa bits of the sum
+          const float2 m = __ffma2_rn(x2, inv2, make_float2(12582912.0f, 12582912.0f));
+          const float2 r = __fadd2_rn(m, make_float2(-12582912.0f, -12582912.0f));
+          const float2 d = __ffma2_rn(x2, inv2, make_float2(-r.x, -r.y));
+          off = max3_nan_abs(off, d.x, d.y);
+          b[e] = __float_as_uint(m.x);
+          b[e + 1] = __float_as_uint(m.y);
+        }
+        if (!(off < 0.4999f)) {
+#pragma unroll
+          for (int e = 0; e < EPV; ++e) b[e] = (uint8_t)i8_quant_exact(f[v][e], s);
+        }
+        uint32_t w[EPV / 4];
+#pragma unroll
+        for (int i = 0; i < EPV / 4; ++i)
+          w[i] = __byte_perm(__byte_perm(b[4 * i], b[4 * i + 1], 0x0040), __byte_perm(b[4 * i + 2], b[4 * i + 3], 0x0040), 0x5410);
+        int8_t* dst = q + row * width + (32 * v + lane) * EPV;
+        if constexpr (EPV == 8) *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+        else *reinterpret_cast<uint32_t*>(dst) = w[0];
+      }
+    }
+    if (lane == 0) scales[row] = hs;
   }
-  if (lane == 0) scales[row] = hs;
 }
 
 }  // namespace mxb
@@ -216,10 +234,13 @@ extern "C" int mxb_quantize_kv_int8(const mxb_quantize_kv_int8_args* a, void* st
   const int nv = a->width % epv == 0 ? (int)ceil_div(a->width / epv, 32) : 99;
   if (nv <= 8 && (reinterpret_cast<uintptr_t>(a->x) & 15) == 0 && (reinterpret_cast<uintptr_t>(a->q) & 7) == 0) {
     const uint4* xv = reinterpret_cast<const uint4*>(a->x);
-#define MXB_QVEC(XT)                                                                                            \
-  if (nv <= 3) quant_i8_rows_vec_kernel<XT, 3><<<grid, 128, 0, st>>>(xv, a->q, sc, a->n_rows, a->width);        \
-  else if (nv <= 5) quant_i8_rows_vec_kernel<XT, 5><<<grid, 128, 0, st>>>(xv, a->q, sc, a->n_rows, a->width);   \
-  else quant_i8_rows_vec_kernel<XT, 8><<<grid, 128, 0, st>>>(xv, a->q, sc, a->n_rows, a->width)
+    // one resident wave (three CTAs of 256 threads per SM by registers) whose warps fetch a row ahead
+    const int64_t most = 3 * (int64_t)sm_count();
+    const unsigned vgrid = (unsigned)(ceil_div(a->n_rows, 8) < most ? ceil_div(a->n_rows, 8) : most);
+#define MXB_QVEC(XT)                                                                                             \
+  if (nv <= 3) quant_i8_rows_vec_kernel<XT, 3><<<vgrid, 256, 0, st>>>(xv, a->q, sc, a->n_rows, a->width);        \
+  else if (nv <= 5) quant_i8_rows_vec_kernel<XT, 5><<<vgrid, 256, 0, st>>>(xv, a->q, sc, a->n_rows, a->width);   \
+  else quant_i8_rows_vec_kernel<XT, 8><<<vgrid, 256, 0, st>>>(xv, a->q, sc, a->n_rows, a->width)
     if (a->x_dtype == MXB_F32) { MXB_QVEC(MXB_F32); }
     else if (a->x_dtype == MXB_F16) { MXB_QVEC(MXB_F16); }
     else { MXB_QVEC(MXB_BF16); }
