@@ -42,6 +42,27 @@ def test_matches_oracle(S, past, Hq, Hkv, dt):
     assert max_abs(out_ng, qwen.causal_gqa_prefill(q, k, v, None, scale=1.0 / 16.0, past_len=past)) <= 2e-2
 
 
+@pytest.mark.parametrize("S,past,Hq,Hkv", [
+    (1, 2500, 16, 2),     # one row; the last piece of each item is mostly past the diagonal
+    (64, 3001, 2, 1),     # two items in several pieces each
+    (100, 8000, 16, 2),   # an item spans many stretches
+    (700, 3365, 16, 2),   # stretches that end one item and start the next
+    (1200, 4000, 16, 2),  # more items than SMs: whole items between two pieces
+])
+@pytest.mark.parametrize("dt,gate", [("bf16", True), ("f16", False)])
+def test_items_cut_at_equal_stretches(S, past, Hq, Hkv, dt, gate):
+    need_gpu()
+    rng = np.random.default_rng(S + past)
+    tdt = torch.bfloat16 if dt == "bf16" else torch.float16
+    q, k, v, g = _inputs(rng, S, past, Hq, Hkv, bf16_round if dt == "bf16" else f16_round)
+    q[-1] *= 8.0           # one peaked row: its maximum moves between the pieces
+    out = fa.sdpa_fa_prefill(dev(q, tdt), dev(k, tdt), dev(v, tdt), 1.0 / 16.0, gate=dev(g, tdt) if gate else None,
+                             layout="lhd", check=True)
+    ref = qwen.causal_gqa_prefill(q, k, v, g if gate else None, scale=1.0 / 16.0, past_len=past)
+    # P and the result are 16-bit: half a unit of bf16 (2^-9) for each, relative to the largest |v| a row can average
+    assert max_abs(out, ref) <= 2 * 2.0 ** -9 * float(np.abs(v).max())
+
+
 def test_gate_layout_without_tensor_map():
     """A gate whose row stride is not a multiple of its head stride cannot be described by a tensor map: the drain
     then reads the gate and writes the output with per-thread accesses.  Same result as the tiled drain."""
