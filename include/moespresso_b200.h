@@ -204,6 +204,28 @@ typedef struct {
 int mxb_affine_q8_quantize(const mxb_affine_q8_args* a, void* stream);
 int mxb_affine_q8_dequantize(const mxb_affine_q8_args* a, void* stream);
 
+/* The same for keys and values of all heads of a cache at once (index 0 = keys, 1 = values, equal shapes).
+ *   append: x [heads, n_rows, width] -> rows row0 .. row0 + n_rows of packed / scales / biases [heads, head_rows, ...]
+ *   expand: rows row0 .. row0 + n_rows of the cache -> x rows [0, n_rows); tail [heads, n_tail, width], of x's type, is
+ *           copied to x rows [n_rows, n_rows + n_tail)
+ * Feature strides are 1. */
+typedef struct {
+  const void* x[2];     /* rows; the OUTPUT of mxb_affine_q8_expand */
+  const void* tail[2];  /* expand only (NULL when n_tail is 0) */
+  void* packed[2];
+  void* scales[2];
+  void* biases[2];
+  int32_t x_dtype;
+  int32_t sb_dtype;     /* append: must equal x_dtype */
+  int64_t x_head_stride, x_row_stride, tail_head_stride, tail_row_stride;   /* elements */
+  int64_t head_rows;    /* rows between consecutive heads of the cache (its capacity) */
+  int64_t row0, n_rows, n_tail;
+  int32_t heads, width;
+} mxb_affine_q8_pair_args;
+
+int mxb_affine_q8_append(const mxb_affine_q8_pair_args* a, void* stream);
+int mxb_affine_q8_expand(const mxb_affine_q8_pair_args* a, void* stream);
+
 /* ------------------------------------------------------------------------ *
  * One decode token over the affine-q8 cache, head_dim 256, split over the keys.
  * Replaces  mlx_kquant.sdpa_decode_q8(queries, *q_keys, *q_values, scale, group_size=64, bits=8, splits=128, ...)

@@ -65,6 +65,13 @@ class AffineQ8Args(C.Structure):
                 ("sb_dtype", _i32), ("n_rows", _i64), ("width", _i32)]
 
 
+class AffineQ8PairArgs(C.Structure):
+    _fields_ = [("x", _p * 2), ("tail", _p * 2), ("packed", _p * 2), ("scales", _p * 2), ("biases", _p * 2),
+                ("x_dtype", _i32), ("sb_dtype", _i32), ("x_head_stride", _i64), ("x_row_stride", _i64),
+                ("tail_head_stride", _i64), ("tail_row_stride", _i64), ("head_rows", _i64), ("row0", _i64),
+                ("n_rows", _i64), ("n_tail", _i64), ("heads", _i32), ("width", _i32)]
+
+
 class SdpaDecodeQ8Args(C.Structure):
     _fields_ = [("q", _p), ("q_dtype", _i32), ("k_packed", _p), ("k_scales", _p), ("k_biases", _p),
                 ("v_packed", _p), ("v_scales", _p), ("v_biases", _p), ("sb_dtype", _i32), ("head_stride_rows", _i64),
@@ -136,6 +143,8 @@ EXPORTS = {
     "mxb_rope_tail": (C.c_int, [C.POINTER(RopeTailArgs), _p]),
     "mxb_affine_q8_quantize": (C.c_int, [C.POINTER(AffineQ8Args), _p]),
     "mxb_affine_q8_dequantize": (C.c_int, [C.POINTER(AffineQ8Args), _p]),
+    "mxb_affine_q8_append": (C.c_int, [C.POINTER(AffineQ8PairArgs), _p]),
+    "mxb_affine_q8_expand": (C.c_int, [C.POINTER(AffineQ8PairArgs), _p]),
     "mxb_sdpa_decode_q8": (C.c_int, [C.POINTER(SdpaDecodeQ8Args), _p]),
     "mxb_range_candidates": (C.c_int, [C.POINTER(RangeCandidatesArgs), _p]),
     "mxb_range_local_ids": (C.c_int, [C.POINTER(RangeLocalIdsArgs), _p]),

@@ -8,9 +8,9 @@
 // bias = beta; element = round((w - bias) / scale) in [0, 255]; w ~= element * scale + bias.  Four elements per
 // uint32 word, lowest byte first; scales and biases in the row's floating type.
 //
-//  * affine_q8_quantize_kernel / affine_q8_dequantize_kernel — the format, one warp per row (any width that is
-//    a multiple of 64); the dequantiser writes with a caller-chosen row stride so that a past can be expanded
-//    straight into the front of a [past + chunk] operand of the flash prefill kernel.
+//  * affine_q8_quantize_kernel / affine_q8_dequantize_kernel — the format, for any width that is a multiple of 64
+//    and any row and head strides: keys and values of all heads are appended to a cache in one launch, and a past
+//    and the chunk behind it become one [past + chunk] operand of the flash prefill kernel in one launch.
 //  * q8_decode_kernel — one query token over a q8 cache, split over the keys: a CTA owns (split, KV head), its four
 //    warps take 16 keys at a time and run both contractions on the warp-level tensor cores straight from the packed
 //    rows (see the comment at the kernel); every split writes (o, m, l) partials for the log-sum-exp merge kernel
@@ -21,19 +21,72 @@ namespace mxb {
 
 constexpr int Q8_GROUP = 64;
 
-template <int XT>
-__global__ void __launch_bounds__(128) affine_q8_quantize_kernel(const void* __restrict__ x, int64_t x_row_stride,
-                                                                 uint32_t* __restrict__ packed, void* __restrict__ scales,
-                                                                 void* __restrict__ biases, int64_t n_rows, int width) {
+// Rows of up to two tensors (a cache append: keys and values), each [heads, rows, width] with free head and row
+// strides on the floating side; the packed side is [heads, head_rows, ...], written from row `row0` on.
+struct Q8Rows {
+  const void* x[2];        // floating rows (written by the dequantiser)
+  const void* tail[2];     // dequantiser: rows n_rows .. n_rows + n_tail of the output, copied as they are (or null)
+  uint32_t* packed[2];
+  void* scales[2];
+  void* biases[2];
+  int64_t x_head_stride, x_row_stride, tail_head_stride, tail_row_stride;   // elements
+  int64_t head_rows, row0;
+  int64_t n_rows, n_tail;
+  int32_t heads, width;
+};
+
+// Eight consecutive elements: one 16-byte access (two for float) where base and strides allow it.
+template <int DT, bool VEC>
+__device__ __forceinline__ void load8(const void* p, int64_t i, float (&v)[8]) {
+  if constexpr (VEC && DT == MXB_F32) {
+    const float4* q = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + i);
+    const float4 a = __ldg(q), b = __ldg(q + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else if constexpr (VEC) {
+    unpack16<DT>(__ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p) + i)), v);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = load_elem<DT>(p, i + e);
+  }
+}
+template <int DT, bool VEC>
+__device__ __forceinline__ void store8(void* p, int64_t i, const float (&v)[8]) {
+  if constexpr (VEC && DT == MXB_F32) {
+    float4* q = reinterpret_cast<float4*>(reinterpret_cast<float*>(p) + i);
+    q[0] = make_float4(v[0], v[1], v[2], v[3]);
+    q[1] = make_float4(v[4], v[5], v[6], v[7]);
+  } else if constexpr (VEC) {
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if constexpr (DT == MXB_F16) {
+        const __half2 h = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
+        w[e] = *reinterpret_cast<const uint32_t*>(&h);
+      } else {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+        w[e] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+    }
+    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p) + i) = make_uint4(w[0], w[1], w[2], w[3]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) store_elem<DT>(p, i + e, v[e]);
+  }
+}
+
+// One warp per row; grid.y = tensor * heads + head.
+template <int XT, bool VEC>
+__global__ void __launch_bounds__(128) affine_q8_quantize_kernel(const __grid_constant__ Q8Rows p) {
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (row >= n_rows) return;
+  if (row >= p.n_rows) return;
+  const int which = (int)blockIdx.y / p.heads, head = (int)blockIdx.y % p.heads;
+  const int64_t xo = head * p.x_head_stride + row * p.x_row_stride, po = head * p.head_rows + p.row0 + row;
   // 8 lanes share a group of 64 features: lane l of a 256-feature span holds features 8 l .. 8 l + 7
-  for (int f0 = 0; f0 < width; f0 += 256) {
+  for (int f0 = 0; f0 < p.width; f0 += 256) {
     const int f = f0 + lane * 8;
-    float v[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = f < width ? load_elem<XT>(x, row * x_row_stride + f + e) : 0.f;
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (f < p.width) load8<XT, VEC>(p.x[which], xo + f, v);
     float lo = v[0], hi = v[0];
 #pragma unroll
     for (int e = 1; e < 8; ++e) {
@@ -45,7 +98,7 @@ __global__ void __launch_bounds__(128) affine_q8_quantize_kernel(const void* __r
       lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, m));
       hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, m));
     }
-    if (f >= width) continue;
+    if (f >= p.width) continue;
     // scale and bias are stored in the row's type; the elements are taken against the STORED values
     // (every step is a single correctly rounded float32 operation, no contraction: the packed words are compared
     // bit for bit with the CPU restatement)
@@ -64,31 +117,54 @@ __global__ void __launch_bounds__(128) affine_q8_quantize_kernel(const void* __r
       const float q = fminf(fmaxf(floorf(__fadd_rn(__fmul_rn(__fsub_rn(v[e], bias), inv), 0.5f)), 0.f), 255.f);
       w[e >> 2] |= (uint32_t)q << (8 * (e & 3));
     }
-    *reinterpret_cast<uint2*>(packed + row * (width / 4) + f / 4) = make_uint2(w[0], w[1]);
+    *reinterpret_cast<uint2*>(p.packed[which] + po * (p.width / 4) + f / 4) = make_uint2(w[0], w[1]);
     if ((lane & 7) == 0) {
-      const int64_t g = row * (width / Q8_GROUP) + f / Q8_GROUP;
-      store_elem<XT>(scales, g, scale);
-      store_elem<XT>(biases, g, bias);
+      const int64_t g = po * (p.width / Q8_GROUP) + f / Q8_GROUP;
+      store_elem<XT>(p.scales[which], g, scale);
+      store_elem<XT>(p.biases[which], g, bias);
     }
   }
 }
 
-template <int ST, int OT>
-__global__ void __launch_bounds__(128) affine_q8_dequantize_kernel(const uint32_t* __restrict__ packed,
-                                                                   const void* __restrict__ scales,
-                                                                   const void* __restrict__ biases, void* __restrict__ out,
-                                                                   int64_t out_row_stride, int64_t n_rows, int width) {
+// One warp per four rows, all of whose loads are issued before the first is used; grid.y = tensor * heads + head.
+// Rows behind the packed ones (n_tail) are copied: a past and the chunk behind it become one operand in one launch.
+// HBM-bound.  Keys and values of 2 heads, 30,720 rows and 2,048 behind them: 29 us (3.4 TB/s); one launch per head
+// and tensor with two-byte stores, and copies for the rows behind, took 108 us.
+constexpr int kDqRows = 4;
+template <int ST, int OT, bool VEC>
+__global__ void __launch_bounds__(128) affine_q8_dequantize_kernel(const __grid_constant__ Q8Rows p) {
   const int lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (row >= n_rows) return;
-  for (int f = lane * 8; f < width; f += 256) {
-    const uint2 w = *reinterpret_cast<const uint2*>(packed + row * (width / 4) + f / 4);
-    const int64_t g = row * (width / Q8_GROUP) + f / Q8_GROUP;
-    const float scale = load_elem<ST>(scales, g), bias = load_elem<ST>(biases, g);
-    const uint32_t ww[2] = {w.x, w.y};
+  const int64_t row_lo = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * kDqRows;
+  const int which = (int)blockIdx.y / p.heads, head = (int)blockIdx.y % p.heads;
+  void* out = const_cast<void*>(p.x[which]);
+  const int64_t oo = head * p.x_head_stride, n_all = p.n_rows + p.n_tail;
+  for (int f = lane * 8; f < p.width; f += 256) {
+    uint2 w[kDqRows];
+    float scale[kDqRows], bias[kDqRows];
 #pragma unroll
-    for (int e = 0; e < 8; ++e)
-      store_elem<OT>(out, row * out_row_stride + f + e, fmaf((float)((ww[e >> 2] >> (8 * (e & 3))) & 0xffu), scale, bias));
+    for (int u = 0; u < kDqRows; ++u) {
+      const int64_t row = row_lo + u;
+      if (row < p.n_rows) {
+        const int64_t po = head * p.head_rows + p.row0 + row;
+        w[u] = __ldg(reinterpret_cast<const uint2*>(p.packed[which] + po * (p.width / 4) + f / 4));
+        const int64_t g = po * (p.width / Q8_GROUP) + f / Q8_GROUP;
+        scale[u] = load_elem<ST>(p.scales[which], g);
+        bias[u] = load_elem<ST>(p.biases[which], g);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kDqRows; ++u) {
+      const int64_t row = row_lo + u;
+      float v[8];
+      if (row < p.n_rows) {
+        const uint32_t ww[2] = {w[u].x, w[u].y};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = fmaf((float)((ww[e >> 2] >> (8 * (e & 3))) & 0xffu), scale[u], bias[u]);
+      } else if (row < n_all) {
+        load8<OT, VEC>(p.tail[which], head * p.tail_head_stride + (row - p.n_rows) * p.tail_row_stride + f, v);
+      }
+      if (row < n_all) store8<OT, VEC>(out, oo + row * p.x_row_stride + f, v);
+    }
   }
 }
 
@@ -457,34 +533,38 @@ static int q8_check(const mxb_affine_q8_args* a, const char* what) {
   return MXB_OK;
 }
 
-extern "C" int mxb_affine_q8_quantize(const mxb_affine_q8_args* a, void* stream) {
-  int rc = q8_check(a, "affine q8 quantise");
-  if (rc != MXB_OK) return rc;
-  MXB_REQUIRE(a->sb_dtype == a->x_dtype, MXB_ERR_INVALID, "affine q8 quantise: scales and biases take the rows' type");
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const unsigned grid = (unsigned)ceil_div(a->n_rows, 4);
-  uint32_t* pk = reinterpret_cast<uint32_t*>(a->packed);
-#define MXB_Q(XT) affine_q8_quantize_kernel<XT><<<grid, 128, 0, st>>>(a->x, a->x_row_stride, pk, a->scales, a->biases, a->n_rows, a->width)
-  if (a->x_dtype == MXB_F32) MXB_Q(MXB_F32);
-  else if (a->x_dtype == MXB_F16) MXB_Q(MXB_F16);
-  else MXB_Q(MXB_BF16);
+static bool vec16(const void* p, int dt, int64_t stride_a, int64_t stride_b) {
+  return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)(stride_a * dtype_bytes(dt)) | (uintptr_t)(stride_b * dtype_bytes(dt))) & 15) == 0;
+}
+
+// x_dtype: the floating rows' type (tails have it too)
+static int launch_quantize(const Q8Rows& p, int tensors, int x_dtype, cudaStream_t st) {
+  bool vec = true;
+  for (int i = 0; i < tensors; ++i) vec = vec && vec16(p.x[i], x_dtype, p.x_head_stride, p.x_row_stride);
+  const dim3 grid((unsigned)ceil_div(p.n_rows, 4), (unsigned)(tensors * p.heads));
+#define MXB_Q(XT)                                                    \
+  if (x_dtype == XT) {                                               \
+    if (vec) affine_q8_quantize_kernel<XT, true><<<grid, 128, 0, st>>>(p);  \
+    else affine_q8_quantize_kernel<XT, false><<<grid, 128, 0, st>>>(p);     \
+  }
+  MXB_Q(MXB_F32) else MXB_Q(MXB_F16) else MXB_Q(MXB_BF16)
 #undef MXB_Q
   note_launch();
   MXB_CUDA_OK(cudaGetLastError());
   return MXB_OK;
 }
 
-extern "C" int mxb_affine_q8_dequantize(const mxb_affine_q8_args* a, void* stream) {
-  int rc = q8_check(a, "affine q8 dequantise");
-  if (rc != MXB_OK) return rc;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const unsigned grid = (unsigned)ceil_div(a->n_rows, 4);
-  const uint32_t* pk = reinterpret_cast<const uint32_t*>(a->packed);
-  void* out = const_cast<void*>(a->x);
-#define MXB_DQ(ST, OT) \
-  if (a->sb_dtype == ST && a->x_dtype == OT)                                                                          \
-    affine_q8_dequantize_kernel<ST, OT><<<grid, 128, 0, st>>>(pk, a->scales, a->biases, out, a->x_row_stride, a->n_rows, a->width); \
-  else
+static int launch_dequantize(const Q8Rows& p, int tensors, int sb_dtype, int x_dtype, cudaStream_t st) {
+  bool vec = true;
+  for (int i = 0; i < tensors; ++i)
+    vec = vec && vec16(p.x[i], x_dtype, p.x_head_stride, p.x_row_stride) &&
+          (p.n_tail == 0 || vec16(p.tail[i], x_dtype, p.tail_head_stride, p.tail_row_stride));
+  const dim3 grid((unsigned)ceil_div(p.n_rows + p.n_tail, 4 * kDqRows), (unsigned)(tensors * p.heads));
+#define MXB_DQ(ST, OT)                                                              \
+  if (sb_dtype == ST && x_dtype == OT) {                                            \
+    if (vec) affine_q8_dequantize_kernel<ST, OT, true><<<grid, 128, 0, st>>>(p);    \
+    else affine_q8_dequantize_kernel<ST, OT, false><<<grid, 128, 0, st>>>(p);       \
+  } else
   MXB_DQ(MXB_F32, MXB_F32) MXB_DQ(MXB_F32, MXB_F16) MXB_DQ(MXB_F32, MXB_BF16)
   MXB_DQ(MXB_F16, MXB_F32) MXB_DQ(MXB_F16, MXB_F16) MXB_DQ(MXB_F16, MXB_BF16)
   MXB_DQ(MXB_BF16, MXB_F32) MXB_DQ(MXB_BF16, MXB_F16) MXB_DQ(MXB_BF16, MXB_BF16)
@@ -493,6 +573,78 @@ extern "C" int mxb_affine_q8_dequantize(const mxb_affine_q8_args* a, void* strea
   note_launch();
   MXB_CUDA_OK(cudaGetLastError());
   return MXB_OK;
+}
+
+static Q8Rows one_tensor(const mxb_affine_q8_args* a) {
+  Q8Rows p{};
+  p.x[0] = a->x;
+  p.packed[0] = reinterpret_cast<uint32_t*>(a->packed);
+  p.scales[0] = a->scales;
+  p.biases[0] = a->biases;
+  p.x_row_stride = a->x_row_stride;
+  p.n_rows = a->n_rows;
+  p.heads = 1;
+  p.width = a->width;
+  return p;
+}
+
+extern "C" int mxb_affine_q8_quantize(const mxb_affine_q8_args* a, void* stream) {
+  int rc = q8_check(a, "affine q8 quantise");
+  if (rc != MXB_OK) return rc;
+  MXB_REQUIRE(a->sb_dtype == a->x_dtype, MXB_ERR_INVALID, "affine q8 quantise: scales and biases take the rows' type");
+  return launch_quantize(one_tensor(a), 1, a->x_dtype, reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" int mxb_affine_q8_dequantize(const mxb_affine_q8_args* a, void* stream) {
+  int rc = q8_check(a, "affine q8 dequantise");
+  if (rc != MXB_OK) return rc;
+  return launch_dequantize(one_tensor(a), 1, a->sb_dtype, a->x_dtype, reinterpret_cast<cudaStream_t>(stream));
+}
+
+static int q8_pair_check(const mxb_affine_q8_pair_args* a, const char* what) {
+  MXB_REQUIRE(a != nullptr, MXB_ERR_INVALID, "%s: null args", what);
+  MXB_REQUIRE(a->heads > 0 && a->heads <= 32767 && a->width > 0 && a->width % Q8_GROUP == 0 && a->n_rows >= 0 &&
+                  a->n_tail >= 0 && a->n_rows + a->n_tail > 0 && a->row0 >= 0 && a->row0 + a->n_rows <= a->head_rows,
+              MXB_ERR_INVALID, "%s: rows must be non-empty, lie within the cache, and have a width that is a multiple of 64", what);
+  MXB_REQUIRE(a->x_dtype == MXB_F32 || a->x_dtype == MXB_F16 || a->x_dtype == MXB_BF16, MXB_ERR_INVALID,
+              "%s: rows must be float32, float16 or bfloat16", what);
+  for (int i = 0; i < 2; ++i) {
+    MXB_REQUIRE(a->x[i] && a->packed[i] && a->scales[i] && a->biases[i] && (a->n_tail == 0 || a->tail[i]), MXB_ERR_INVALID,
+                "%s: null tensor", what);
+    MXB_REQUIRE((reinterpret_cast<uintptr_t>(a->packed[i]) & 7) == 0, MXB_ERR_INVALID, "%s: packed words must be 8-byte aligned", what);
+  }
+  return MXB_OK;
+}
+
+static Q8Rows two_tensors(const mxb_affine_q8_pair_args* a) {
+  Q8Rows p{};
+  for (int i = 0; i < 2; ++i) {
+    p.x[i] = a->x[i];
+    p.tail[i] = a->tail[i];
+    p.packed[i] = reinterpret_cast<uint32_t*>(a->packed[i]);
+    p.scales[i] = a->scales[i];
+    p.biases[i] = a->biases[i];
+  }
+  p.x_head_stride = a->x_head_stride; p.x_row_stride = a->x_row_stride;
+  p.tail_head_stride = a->tail_head_stride; p.tail_row_stride = a->tail_row_stride;
+  p.head_rows = a->head_rows; p.row0 = a->row0;
+  p.n_rows = a->n_rows; p.n_tail = a->n_tail;
+  p.heads = a->heads; p.width = a->width;
+  return p;
+}
+
+extern "C" int mxb_affine_q8_append(const mxb_affine_q8_pair_args* a, void* stream) {
+  int rc = q8_pair_check(a, "affine q8 append");
+  if (rc != MXB_OK) return rc;
+  MXB_REQUIRE(a->sb_dtype == a->x_dtype, MXB_ERR_INVALID, "affine q8 append: scales and biases take the rows' type");
+  MXB_REQUIRE(a->n_rows > 0 && a->n_tail == 0, MXB_ERR_INVALID, "affine q8 append: rows without a tail");
+  return launch_quantize(two_tensors(a), 2, a->x_dtype, reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" int mxb_affine_q8_expand(const mxb_affine_q8_pair_args* a, void* stream) {
+  int rc = q8_pair_check(a, "affine q8 expand");
+  if (rc != MXB_OK) return rc;
+  return launch_dequantize(two_tensors(a), 2, a->sb_dtype, a->x_dtype, reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" int mxb_sdpa_decode_q8(const mxb_sdpa_decode_q8_args* a, void* stream) {

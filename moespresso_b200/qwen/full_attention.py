@@ -133,6 +133,35 @@ def _q8_call(name, rows, row_stride, packed, scales, biases, n, D):
     _abi.check(_t.launch(name, getattr(_abi.load(), "mxb_" + name), a))
 
 
+def _q8_head_rows(tensors) -> int:
+    """Rows between consecutive heads of (packed, scales, biases) x (keys, values), all row-contiguous views
+    ``[1, Hkv, P, w]`` of one capacity with scales of one type; 0 when they are not."""
+    heads, n = (int(x) for x in tensors[0].shape[1:3])
+    if any(t.stride(3) != 1 or t.stride(2) != t.shape[3] or tuple(t.shape[1:3]) != (heads, n) for t in tensors):
+        return 0
+    if len({t.dtype for t in tensors[1:3] + tensors[4:6]}) != 1 or tensors[0].shape[3] != tensors[3].shape[3]:
+        return 0
+    if heads == 1:
+        return n
+    rows = {divmod(int(t.stride(1)), int(t.shape[3])) for t in tensors}
+    return max(0, rows.pop()[0]) if len(rows) == 1 and next(iter(rows))[1] == 0 else 0
+
+
+def _q8_pair(name, rows, head_stride, row_stride, k_store, v_store, head_rows, row0, n_rows, tails=None):
+    """Keys and values of all heads in one launch (``mxb_affine_q8_append`` / ``mxb_affine_q8_expand``)."""
+    a = _abi.AffineQ8PairArgs()
+    for i, store in enumerate((k_store, v_store)):
+        a.x[i], a.packed[i], a.scales[i], a.biases[i] = ptr(rows[i]), *(ptr(t) for t in store)
+        if tails is not None:
+            a.tail[i] = ptr(tails[i])
+    if tails is not None:
+        a.tail_head_stride, a.tail_row_stride, a.n_tail = tails[0].stride(-3), tails[0].stride(-2), int(tails[0].shape[-2])
+    a.x_dtype, a.sb_dtype = dtype_code(rows[0]), dtype_code(k_store[1])
+    a.x_head_stride, a.x_row_stride, a.head_rows, a.row0, a.n_rows = head_stride, row_stride, head_rows, row0, n_rows
+    a.heads, a.width = int(k_store[0].shape[1]), int(k_store[0].shape[3]) * 4
+    _abi.check(_t.launch(name, getattr(_abi.load(), "mxb_" + name), a))
+
+
 class QuantizedKVCache:
     """Pre-allocated affine-q8 KV cache with the surface of mlx-lm's ``QuantizedKVCache`` that the reference relies
     on (qwen/full_attention.py:200-236, 313-382): ``bits`` 8, ``group_size`` 64, ``offset``, ``keys`` / ``values``
@@ -148,7 +177,7 @@ class QuantizedKVCache:
         self.values = (mk(head_dim // 4, torch.int32), mk(head_dim // Q8_GROUP, dtype), mk(head_dim // Q8_GROUP, dtype))
 
     def _prefix(self, n):
-        return tuple(t[:, :, :n] for t in self.keys), tuple(t[:, :, :n] for t in self.values)
+        return tuple(t.narrow(2, 0, n) for t in self.keys), tuple(t.narrow(2, 0, n) for t in self.values)
 
     @property
     def state(self):
@@ -160,10 +189,19 @@ class QuantizedKVCache:
         L = int(keys.shape[2])
         if self.offset + L > self.capacity:
             raise ValueError("QuantizedKVCache capacity exceeded")
-        for store, x in ((self.keys, keys), (self.values, values)):
-            q = quantize_affine_q8(x.to(store[1].dtype))
-            for dst, src in zip(store, q):
-                dst[:, :, self.offset:self.offset + L].copy_(src)
+        dt = self.keys[1].dtype
+        keys, values = keys.to(dt), values.to(dt)
+        shape = (1, int(self.keys[0].shape[1]), L, 4 * int(self.keys[0].shape[3]))
+        if L and tuple(keys.shape) == shape and tuple(values.shape) == shape:
+            if keys.stride() != values.stride() or keys.stride(3) != 1:
+                keys, values = keys.contiguous(), values.contiguous()
+            require_cuda(keys, values, self.keys[0])
+            _q8_pair("affine_q8_append", (keys, values), keys.stride(1), keys.stride(2), self.keys, self.values,
+                     self.capacity, self.offset, L)
+        else:                                  # shapes that broadcast into the cache
+            for store, x in ((self.keys, keys), (self.values, values)):
+                for dst, src in zip(store, quantize_affine_q8(x)):
+                    dst[:, :, self.offset:self.offset + L].copy_(src)
         self.offset += L
         return self._prefix(self.offset)
 
@@ -203,12 +241,22 @@ def sdpa_fa_prefill_q8(queries, k_packed, k_scales, k_biases, v_packed, v_scales
     op = self_k.dtype if self_k.dtype in (torch.bfloat16, torch.float16) else torch.bfloat16
     kfull = torch.empty((Hkv, P + L, D), dtype=op, device=dev)
     vfull = torch.empty_like(kfull)
-    for h in range(Hkv):
-        if P:
-            dequantize_affine_q8(k_packed[0, h], k_scales[0, h], k_biases[0, h], out=kfull[h, :P])
-            dequantize_affine_q8(v_packed[0, h], v_scales[0, h], v_biases[0, h], out=vfull[h, :P])
-    kfull[:, P:].copy_(self_k[0])
-    vfull[:, P:].copy_(self_v[0])
+    self_k, self_v = self_k[0].to(op), self_v[0].to(op)
+    if self_k.stride() != self_v.stride() or self_k.stride(-1) != 1:
+        self_k, self_v = self_k.contiguous(), self_v.contiguous()
+    past = (k_packed, k_scales, k_biases, v_packed, v_scales, v_biases)
+    require_cuda(queries, self_k, self_v, *past)
+    head_rows = _q8_head_rows(past) if P else 0
+    same = tuple(self_k.shape) == tuple(self_v.shape) == (Hkv, L, D)
+    if head_rows and same:
+        _q8_pair("affine_q8_expand", (kfull, vfull), (P + L) * D, D, past[:3], past[3:], head_rows, 0, P, (self_k, self_v))
+    else:
+        for h in range(Hkv):
+            if P:
+                dequantize_affine_q8(k_packed[0, h], k_scales[0, h], k_biases[0, h], out=kfull[h, :P])
+                dequantize_affine_q8(v_packed[0, h], v_scales[0, h], v_biases[0, h], out=vfull[h, :P])
+        kfull[:, P:].copy_(self_k)
+        vfull[:, P:].copy_(self_v)
     q = queries[0].to(op).permute(1, 0, 2)                       # [L, Hq, D]
     g = None if gate is None else gate.reshape(L, Hq, D).to(op)
     out = sdpa_fa_prefill(q, kfull.permute(1, 0, 2), vfull.permute(1, 0, 2), scale, gate=g, layout="lhd", check=check)

@@ -124,3 +124,38 @@ def test_wrapper_routes_q8_prefill_and_decode():
     # decode below the long-context threshold goes to the stock path
     attn(x[:, :1], mask=None, cache=cache)
     assert inner.stock_calls == 2 and attn.decode_calls == 0
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("Hkv,L,P", [(1, 1, 1), (2, 7, 33), (3, 64, 5)])
+def test_append_and_expand_of_both_tensors_at_once(dt, Hkv, L, P):
+    """Rows of every stride and alignment against the oracle's format: one row, remainders of the four rows a warp
+    expands, keys and values of different layouts, and a base that is not 16-byte aligned."""
+    need_gpu()
+    D, cap = 256, P + L + 3
+    g = torch.Generator(device="cuda").manual_seed(L * 100 + P)
+    mk = lambda n: torch.randn(1, n, Hkv, D, generator=g, device="cuda").to(dt)
+    cache = fa.QuantizedKVCache(Hkv, D, cap, dtype=dt)
+    kp, vp = mk(P), mk(P)
+    cache.update_and_fetch(kp.transpose(1, 2), vp.transpose(1, 2))              # rows outside heads
+    def odd(rows):
+        t = torch.empty(Hkv * L * (D + 1) + 1, dtype=dt, device="cuda")[1:].as_strided((1, Hkv, L, D), (1, L * (D + 1), D + 1, 1))
+        return t.copy_(rows)
+    kn = odd(mk(L).transpose(1, 2))
+    vn = mk(L).transpose(1, 2) if L == 7 else odd(mk(L).transpose(1, 2))
+    past_k, past_v = cache.state
+    qk, qv = cache.update_and_fetch(kn, vn)
+    kind = {torch.bfloat16: "bf16", torch.float16: "f16", torch.float32: "f32"}[dt]
+    for got, rows in ((qk, torch.cat([kp.transpose(1, 2), kn], 2)), (qv, torch.cat([vp.transpose(1, 2), vn], 2))):
+        want = qwen.affine_q8_quantize(rows[0].float().cpu().numpy(), kind)
+        np.testing.assert_array_equal(got[0][0].cpu().numpy().view(np.uint32), want[0])
+        for i in (1, 2):
+            np.testing.assert_array_equal(got[i][0].float().cpu().numpy(), want[i])
+    assert all(int(t[:, :, P + L:].abs().max()) == 0 for t in cache.keys + cache.values)   # nothing behind the rows
+    if dt != torch.float32:
+        full = [torch.empty(Hkv, P + L, D, dtype=dt, device="cuda") for _ in range(2)]
+        tails = [t[0].contiguous() for t in (kn, vn)]
+        fa._q8_pair("affine_q8_expand", full, (P + L) * D, D, past_k, past_v, fa._q8_head_rows(past_k + past_v), 0, P, tails)
+        for out, q8, tail in zip(full, (past_k, past_v), tails):
+            assert torch.equal(out[:, :P], fa.dequantize_affine_q8(*(t[0].contiguous() for t in q8)))
+            assert torch.equal(out[:, P:], tail)
