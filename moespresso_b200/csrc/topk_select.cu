@@ -228,7 +228,10 @@ using namespace mxb;
 
 extern "C" int64_t mxb_topk_workspace_bytes(int32_t rows, int64_t n, int32_t k) {
   if (rows <= 0 || n <= 0 || k <= 0) return 0;
-  if (topk_pivot_size(rows, n) > 0) return 0;
+  // What the general path (topk_multi.cu) needs.  The pivot kernel uses none of it; rows above kNoScratchMax keep
+  // reporting it all the same, because callers size pools by this answer and it is part of the interface.
+  constexpr int64_t kNoScratchMax = 360448;
+  if (topk_pivot_size(rows, n) > 0 && n <= kNoScratchMax) return 0;
   return topk_multi_workspace(rows, n, k);
 }
 
