@@ -137,3 +137,20 @@ def test_score_is_independent_of_row_partition():
     for lo, hi in [(0, 1000), (1000, 1777), (1777, 5000)]:
         part = iak.indexer_scores_tiled_live(qd, wd, fp8_from_bits(bits[lo:hi])[None], pos0=0, ratio=0)[0, 0]
         assert torch.equal(part, full[lo:hi])
+
+
+@pytest.mark.parametrize("D,H,rows", [(64, 1, 1), (64, 16, 33), (64, 17, 128 * 296 + 5), (128, 33, 31), (128, 64, 2500),
+                                      (128, 64, 128 * 296 + 1)])
+@pytest.mark.parametrize("qdt,kdt", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16)])
+def test_exact_scores_of_one_token_have_the_bits_of_a_chunk(D, H, rows, qdt, kdt):
+    """The kernel for one token splits the heads over warps; a chunk of two equal tokens takes the kernel that walks
+    them in one thread.  Edges of the row tiles (32 and 128), both row widths, heads that do not fill the warps."""
+    need_gpu()
+    g = torch.Generator(device="cuda").manual_seed(rows + H)
+    q = torch.randn(1, H, 1, D, generator=g, device="cuda").to(qdt)
+    w = torch.randn(1, 1, H, generator=g, device="cuda")
+    keys = torch.randn(rows, D, generator=g, device="cuda").to(kdt)
+    one = iak.indexer_scores(q, w, keys, n_rows=rows, exact_fp32=True)
+    two = iak.indexer_scores(q.expand(1, H, 2, D).contiguous(), w.expand(1, 2, H).contiguous(), keys, n_rows=rows,
+                             exact_fp32=True)
+    assert torch.equal(one.reshape(-1), two.reshape(2, rows)[0])
