@@ -454,6 +454,57 @@ typedef struct {
 int64_t mxb_flash_prefill_workspace_bytes(const mxb_flash_prefill_args* a);
 int mxb_flash_prefill(const mxb_flash_prefill_args* a, void* stream);
 
+/* ------------------------------------------------------------------------ *
+ * The fused decode operators of one ratio-4 token (batch 1).
+ * Replaces  fused_decode_prep / fused_decode_sdpa
+ *           src/moespresso/runtime/deepseek_v4/decode_attention_kernel.py:669-786
+ *   prep: sel = ids of the topk largest scores (ascending), row = the prepared KV row, scores over the pool
+ *   sdpa: attention over the window (row params[1] of it replaced by `row`) and the selected pool rows
+ * params = [position, write index] on the device; all tensors contiguous; the workspace 256-byte aligned.
+ * ------------------------------------------------------------------------ */
+typedef struct {
+  const void* q_idx;        /* [n_heads, 128] */
+  int32_t q_dtype;          /* MXB_F32 | MXB_F16 | MXB_BF16 */
+  const float* pooled_qat;  /* [n_rows, 128] */
+  const float* weights;     /* [n_heads] */
+  const void* kv_row;       /* fp16 [512] */
+  const float* inv_freq;    /* [32] */
+  const void* params;
+  int32_t params_int64;     /* params are int64 (else int32) */
+  float scale;
+  int32_t n_heads, topk;
+  int64_t n_rows;
+  int32_t* sel;             /* [topk] */
+  void* row;                /* fp16 [512] */
+  float* scores;            /* [n_rows] */
+  void* workspace;
+  int64_t workspace_bytes;
+} mxb_fused_decode_prep_args;
+
+int64_t mxb_fused_decode_prep_workspace_bytes(const mxb_fused_decode_prep_args* a);
+int mxb_fused_decode_prep(const mxb_fused_decode_prep_args* a, void* stream);
+
+typedef struct {
+  const void* q;            /* fp16 [n_heads, 512] */
+  const void* window;       /* fp16 [window_rows, 512] */
+  const void* row;          /* fp16 [512] */
+  const void* pooled;       /* fp16 [n_rows, 512] */
+  const int32_t* sel;       /* [topk] */
+  const void* sinks;        /* fp16 [n_heads] */
+  const float* inv_freq;    /* [32] */
+  const void* params;
+  int32_t params_int64;
+  float scale;
+  int32_t n_heads, window_rows, topk;
+  int64_t n_rows;
+  void* out;                /* fp16 [n_heads, 512] */
+  void* workspace;
+  int64_t workspace_bytes;
+} mxb_fused_decode_sdpa_args;
+
+int64_t mxb_fused_decode_sdpa_workspace_bytes(const mxb_fused_decode_sdpa_args* a);
+int mxb_fused_decode_sdpa(const mxb_fused_decode_sdpa_args* a, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

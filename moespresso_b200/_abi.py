@@ -121,6 +121,18 @@ class FlashPrefillArgs(C.Structure):
     ]
 
 
+class FusedDecodePrepArgs(C.Structure):
+    _fields_ = [("q_idx", _p), ("q_dtype", _i32), ("pooled_qat", _p), ("weights", _p), ("kv_row", _p), ("inv_freq", _p),
+                ("params", _p), ("params_int64", _i32), ("scale", _f32), ("n_heads", _i32), ("topk", _i32),
+                ("n_rows", _i64), ("sel", _p), ("row", _p), ("scores", _p), ("workspace", _p), ("workspace_bytes", _i64)]
+
+
+class FusedDecodeSdpaArgs(C.Structure):
+    _fields_ = [("q", _p), ("window", _p), ("row", _p), ("pooled", _p), ("sel", _p), ("sinks", _p), ("inv_freq", _p),
+                ("params", _p), ("params_int64", _i32), ("scale", _f32), ("n_heads", _i32), ("window_rows", _i32),
+                ("topk", _i32), ("n_rows", _i64), ("out", _p), ("workspace", _p), ("workspace_bytes", _i64)]
+
+
 class RangeCandidatesArgs(C.Structure):
     _fields_ = [("scores", _p), ("ids", _p), ("out_scores", _p), ("out_ids", _p), ("k", _i32), ("row_lo", _i64)]
 
@@ -154,6 +166,10 @@ EXPORTS = {
     "mxb_sparse_attn_workspace_bytes": (_i64, [C.POINTER(SparseAttnArgs)]),
     "mxb_sparse_attn": (C.c_int, [C.POINTER(SparseAttnArgs), _p]),
     "mxb_merge_partials": (C.c_int, [C.POINTER(MergeArgs), _p]),
+    "mxb_fused_decode_prep_workspace_bytes": (_i64, [C.POINTER(FusedDecodePrepArgs)]),
+    "mxb_fused_decode_prep": (C.c_int, [C.POINTER(FusedDecodePrepArgs), _p]),
+    "mxb_fused_decode_sdpa_workspace_bytes": (_i64, [C.POINTER(FusedDecodeSdpaArgs)]),
+    "mxb_fused_decode_sdpa": (C.c_int, [C.POINTER(FusedDecodeSdpaArgs), _p]),
     "mxb_flash_prefill_workspace_bytes": (_i64, [C.POINTER(FlashPrefillArgs)]),
     "mxb_flash_prefill": (C.c_int, [C.POINTER(FlashPrefillArgs), _p]),
 }

@@ -15,7 +15,7 @@
 //    xor-butterfly over the 32 partials, invalid tail = +inf, result negated
 //    (src/moespresso/runtime/deepseek_v4/indexer_score_kernel.py:472-490).  One thread per
 //    column evaluates the same expression tree, so consecutive threads read consecutive columns.
-#include "common.cuh"
+#include "decode_rows.cuh"
 
 namespace mxb {
 
@@ -24,23 +24,6 @@ struct QatParams {
   float* out;
   int64_t n_rows;
 };
-
-__device__ __forceinline__ float lattice_snap(float n) {
-  // nearest of the eight e2m1 magnitudes; the first (lower) value wins a tie
-  const float values[8] = {0.0f, 0.5f, 1.0f, 1.5f, 2.0f, 3.0f, 4.0f, 6.0f};
-  const float absn = fabsf(n);
-  float best = fabsf(__fsub_rn(absn, values[0]));
-  float dq = values[0];
-#pragma unroll
-  for (int k = 1; k < 8; ++k) {
-    const float d = fabsf(__fsub_rn(absn, values[k]));
-    if (d < best) {
-      best = d;
-      dq = values[k];
-    }
-  }
-  return n < 0.0f ? -dq : dq;
-}
 
 template <int XT>
 __global__ void __launch_bounds__(128) indexer_qat_kernel(QatParams p) {
@@ -51,45 +34,11 @@ __global__ void __launch_bounds__(128) indexer_qat_kernel(QatParams p) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) v[j] = load_elem<XT>(p.x, row * 128 + 4 * lane + j);
 
-  // strides 1 and 2 inside the lane
-  const float a0 = __fadd_rn(v[0], v[1]), a1 = __fsub_rn(v[0], v[1]);
-  const float a2 = __fadd_rn(v[2], v[3]), a3 = __fsub_rn(v[2], v[3]);
-  float x[4] = {__fadd_rn(a0, a2), __fadd_rn(a1, a3), __fsub_rn(a0, a2), __fsub_rn(a1, a3)};
-  // strides 4 .. 64 pair lanes
-#pragma unroll
-  for (int m = 1; m <= 16; m <<= 1) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float other = __shfl_xor_sync(0xffffffffu, x[j], m);
-      x[j] = (lane & m) ? __fsub_rn(other, x[j]) : __fadd_rn(x[j], other);
-    }
-  }
-  const float kHadamardScale = 0.08838834764831845f;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) x[j] = __fmul_rn(x[j], kHadamardScale);
-
-  // e2m1 round trip over groups of 32 elements = 8 lanes
-  // the maximum skips NaN elements (fmax), as the reference kernel's does; a group of nothing but NaN keeps NaN
-  float amax = fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3])));
-#pragma unroll
-  for (int m = 1; m <= 4; m <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
-  const float kAmaxFloor = 7.052966104933725e-38f;
-  if (!isnan(amax) && !(amax > kAmaxFloor)) amax = kAmaxFloor;
-  const float kLn2 = 0.6931471805599453f;           // ln 2 rounded to float32, as the float32 chain sees it
-  const float ratio = __fdiv_rn(amax, 6.0f);
-  const float lg = (float)log((double)ratio);        // correctly rounded float32 log
-  const float log2_scale = __fdiv_rn(lg, kLn2);
-  const float arg = __fmul_rn(ceilf(log2_scale), kLn2);
-  const float scale = (float)exp((double)arg);       // correctly rounded float32 exp
-
+  float r[4];
+  indexer_qat_row(v, lane, r);
   float* o = p.out + row * 128 + 4 * lane;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    float n = __fdiv_rn(x[j], scale);
-    n = (isnan(n) || n > -6.0f) ? n : -6.0f;
-    n = (isnan(n) || n < 6.0f) ? n : 6.0f;
-    o[j] = __fmul_rn(lattice_snap(n), scale);
-  }
+  for (int j = 0; j < 4; ++j) o[j] = r[j];
 }
 
 struct TailParams {

@@ -13,38 +13,10 @@
 //    sparse decode kernels read: scale = fp16(amax / 127) (rounded up when the rounding would let a
 //    value exceed 127), q = clamp(rint(x / scale), -127, 127).  No counterpart in the reference.
 //    quant_i8_rows_vec_kernel is the form for rows of whole 16-byte pieces, quant_i8_rows_kernel takes any row.
-#include "common.cuh"
+#include "decode_rows.cuh"
 
 namespace mxb {
 
-__device__ __forceinline__ float e4m3_nearest_lower_tie(float absn) {
-  // absn in [0, 448]
-  float step;
-  if (absn < 0.015625f) {
-    step = 0.001953125f;   // subnormal spacing 2^-9
-  } else {
-    const int e = (int)((__float_as_uint(absn) >> 23) & 0xff) - 127;   // floor(log2(absn)), -6 .. 8
-    step = __uint_as_float((uint32_t)(e - 3 + 127) << 23);
-  }
-  const float t = __fdiv_rn(absn, step);             // exact: step is a power of two
-  return __fmul_rn(fabsf(ceilf(__fsub_rn(t, 0.5f))), step);  // exact; a tie (t = k + 1/2) goes to k; fabsf: ceil(-0.3) = -0
-}
-
-// nearest E4M3FN magnitude with ties to the even code: within a binade the code's parity is the parity of the
-// grid multiple, so this is round-half-even on t
-__device__ __forceinline__ float e4m3_nearest_even_tie(float absn) {
-  float step;
-  if (absn < 0.015625f) {
-    step = 0.001953125f;
-  } else {
-    const int e = (int)((__float_as_uint(absn) >> 23) & 0xff) - 127;
-    step = __uint_as_float((uint32_t)(e - 3 + 127) << 23);
-  }
-  return __fmul_rn(rintf(__fdiv_rn(absn, step)), step);
-}
-
-// REPLAY = false: the served transcription; true: the reference's NumPy replay form (exact power-of-two scale,
-// ties to the even code)
 template <bool REPLAY>
 __global__ void __launch_bounds__(128) fp8_kv_rows_kernel(const float* __restrict__ x, float* __restrict__ out,
                                                           int64_t n_rows) {
@@ -59,35 +31,7 @@ __global__ void __launch_bounds__(128) fp8_kv_rows_kernel(const float* __restric
     const float4 v = src[j];
     xv[4 * j] = v.x; xv[4 * j + 1] = v.y; xv[4 * j + 2] = v.z; xv[4 * j + 3] = v.w;
   }
-  // lanes 28 .. 31 hold the rotary tail: they take part in the shuffles and store their input back
-  float amax = 0.0f;   // the maximum skips NaN elements (fmax), as the reference kernel's does
-#pragma unroll
-  for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(xv[j]));
-#pragma unroll
-  for (int m = 1; m <= 2; m <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
-  if (lane < 28) {
-    if (!(amax > 1.0e-4f)) amax = 1.0e-4f;
-    float scale;
-    if (REPLAY) {
-      int e;
-      const double m = frexp((double)amax / 448.0, &e);   // amax / 448 = m * 2^e, m in [0.5, 1)
-      scale = ldexpf(1.0f, m == 0.5 ? e - 1 : e);         // 2^ceil(log2(amax / 448)), exactly
-    } else {
-      const float kLn2 = 0.6931471805599453f;
-      const float lg = (float)log((double)__fdiv_rn(amax, 448.0f));   // correctly rounded float32 log
-      const float arg = __fmul_rn(ceilf(__fdiv_rn(lg, kLn2)), kLn2);
-      scale = (float)exp((double)arg);                                // correctly rounded float32 exp
-    }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      float n = __fdiv_rn(xv[j], scale);
-      n = (isnan(n) || n > -448.0f) ? n : -448.0f;
-      n = (isnan(n) || n < 448.0f) ? n : 448.0f;
-      const float qv = isnan(n) ? 0.0f : (REPLAY ? e4m3_nearest_even_tie(fabsf(n)) : e4m3_nearest_lower_tie(fabsf(n)));
-      const float sign = n < 0.0f ? -1.0f : (n > 0.0f ? 1.0f : 0.0f);
-      xv[j] = __fmul_rn(__fmul_rn(sign, qv), scale);
-    }
-  }
+  fp8_kv_row<REPLAY>(xv, lane);   // lanes 28 .. 31 hold the rotary tail and store their input back
 #pragma unroll
   for (int j = 0; j < 4; ++j) dst[j] = make_float4(xv[4 * j], xv[4 * j + 1], xv[4 * j + 2], xv[4 * j + 3]);
 }
@@ -284,21 +228,11 @@ __global__ void __launch_bounds__(128) rope_tail_kernel(const void* __restrict__
   const double pos = (double)positions[row % seq_len];
   if constexpr (XT == MXB_F16) {
     if (half_chain) {
-      // the fused decode kernels' float16 form: float32 angle, cos / sin rounded to float16, every product and
-      // sum rounded to float16 (decode_attention_kernel.py:120-147, 398-422)
       const int64_t ipos = positions[row % seq_len];
-      for (int pr = lane; pr < rope_dim / 2; pr += 32) {
-        const float theta = __fmul_rn((float)ipos, (float)inv_freq[pr]);
-        const __half c = __float2half_rn((float)cos((double)theta));
-        __half s = __float2half_rn((float)sin((double)theta));
-        if (inverse) s = __hneg(s);
-        const __half x0 = reinterpret_cast<const __half*>(x)[base + lead + 2 * pr];
-        const __half x1 = reinterpret_cast<const __half*>(x)[base + lead + 2 * pr + 1];
-        // the _rn forms are never contracted into a fused multiply-add: every product is rounded on its own
-        const __half m0 = __hmul_rn(x0, c), m1 = __hmul_rn(x1, s), m2 = __hmul_rn(x0, s), m3 = __hmul_rn(x1, c);
-        reinterpret_cast<__half*>(out)[base + lead + 2 * pr] = __hsub_rn(m0, m1);
-        reinterpret_cast<__half*>(out)[base + lead + 2 * pr + 1] = __hadd_rn(m2, m3);
-      }
+      const __half* xh = reinterpret_cast<const __half*>(x) + base + lead;
+      __half* oh = reinterpret_cast<__half*>(out) + base + lead;
+      for (int pr = lane; pr < rope_dim / 2; pr += 32)
+        rope_half_pair(xh[2 * pr], xh[2 * pr + 1], ipos, (float)inv_freq[pr], inverse != 0, oh[2 * pr], oh[2 * pr + 1]);
       return;
     }
   }

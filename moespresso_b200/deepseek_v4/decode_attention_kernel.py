@@ -7,10 +7,12 @@
 ``fused_decode_sdpa``    rope on q, attention over the window (with the prepared row) and the selected rows, sink,
                          inverse rope (:733-786)
 
-The two fused operators are compositions of this package's kernels (the reference runs each as one Metal launch);
+Each fused operator is one call of the library and a few launches (the reference runs each as one Metal launch);
 ``params`` is read on the device, so neither synchronises with the host and both can be captured in a CUDA graph.
 """
 from __future__ import annotations
+
+import ctypes as C
 
 import torch
 
@@ -46,9 +48,15 @@ _MAX_HEADS = 64
 _ROPE_DIM = 64
 
 
-def _position(params):
-    """The token position as a one-element int64 device tensor (no host round trip)."""
-    return params.reshape(-1)[0:1].to(torch.int64)
+def _token_operands(inv_freq, params, need):
+    """inv_freq float32 [32] and params int32 / int64 [>= need], contiguous, with the int64 flag."""
+    if int(inv_freq.numel()) != _ROPE_DIM // 2:
+        raise ValueError("inv_freq must hold rope_dim / 2 values")
+    if int(params.numel()) < need:
+        raise ValueError("params must hold the token position and the write index")
+    if params.dtype not in (torch.int32, torch.int64):
+        params = params.to(torch.int64)
+    return inv_freq.contiguous(), params.contiguous(), 1 if params.dtype == torch.int64 else 0
 
 
 def fused_decode_prep(q_idx, pooled_qat, weights, kv_row, inv_freq, params, *, scale, topk):
@@ -60,9 +68,7 @@ def fused_decode_prep(q_idx, pooled_qat, weights, kv_row, inv_freq, params, *, s
     Returns ``(sel int32 [topk], row float16 [512], scores float32 [n_rows])``: the selected pool rows (the exact
     top-k with ties to the lower row; ids ASCENDING here, where the reference emits the strictly-above rows first
     and the boundary ties after them — the same set), the roped and FP8-rounded KV row, and the scores.
-    Composed of the QAT, score, top-k, FP8 round-trip and rope operators of this package (five launches)."""
-    from .attention import apply_rope_tail, topk_select
-    from .indexer_score_kernel import fused_qat_indexer_scores
+    Three launches: everything that precedes the scan, the exact fp32 scores, the top-k."""
     if q_idx.ndim != 2 or int(q_idx.shape[1]) != _INDEX_HEAD_DIM:
         raise ValueError("q_idx must have shape [n_heads, 128]")
     n_heads = int(q_idx.shape[0])
@@ -82,14 +88,20 @@ def fused_decode_prep(q_idx, pooled_qat, weights, kv_row, inv_freq, params, *, s
         raise ValueError("kv_row must be float16 [512]")
     if int(inv_freq.shape[-1]) != _ROPE_DIM // 2 or inv_freq.dtype != torch.float32:
         raise ValueError("inv_freq must be float32 [32]")
-    require_cuda(q_idx, pooled_qat, weights, kv_row, inv_freq, params)
-    scores = fused_qat_indexer_scores(q_idx.reshape(1, n_heads, 1, _INDEX_HEAD_DIM), pooled_qat[None],
-                                      weights.reshape(1, 1, n_heads), scale)
-    sel = topk_select(scores[None], topk)[0]
-    # the round trip touches dims [0, 448), the rope dims [448, 512): they commute
-    row = fp8_kv_prefix_rows(kv_row.float()[None])[0].to(torch.float16)
-    roped = apply_rope_tail(kv_row.reshape(1, 1, _HEAD_DIM), _position(params), inv_freq=inv_freq, half_chain=True)
-    row[_HEAD_DIM - _ROPE_DIM:] = roped.reshape(-1)[_HEAD_DIM - _ROPE_DIM:]
+    dev = require_cuda(q_idx, pooled_qat, weights, kv_row, inv_freq, params)
+    inv_freq, params, wide = _token_operands(inv_freq, params, 1)
+    q_idx, pooled_qat, weights, kv_row = (t.contiguous() for t in (q_idx, pooled_qat, weights, kv_row))
+    lib = _abi.load()
+    a = _abi.FusedDecodePrepArgs()
+    a.q_idx, a.q_dtype, a.pooled_qat, a.weights = ptr(q_idx), _t.dtype_code(q_idx), ptr(pooled_qat), ptr(weights)
+    a.kv_row, a.inv_freq, a.params, a.params_int64 = ptr(kv_row), ptr(inv_freq), ptr(params), wide
+    a.scale, a.n_heads, a.topk, a.n_rows = float(scale), n_heads, topk, n_rows
+    sel = torch.empty((topk,), dtype=torch.int32, device=dev)
+    row = torch.empty((_HEAD_DIM,), dtype=torch.float16, device=dev)
+    scores = torch.empty((n_rows,), dtype=torch.float32, device=dev)
+    ws = _t.workspace(lib.mxb_fused_decode_prep_workspace_bytes(C.byref(a)), dev)
+    a.sel, a.row, a.scores, a.workspace, a.workspace_bytes = ptr(sel), ptr(row), ptr(scores), ptr(ws), ws.numel()
+    _abi.check(_t.launch("fused_decode_prep", lib.mxb_fused_decode_prep, a))
     return sel, row, scores
 
 
@@ -101,9 +113,7 @@ def fused_decode_sdpa(q, window, row, pooled, sel, sinks, inv_freq, params, *, s
     sel int32 ``[topk]``, sinks float16 ``[n_heads]``, inv_freq float32 ``[32]``, params int32
     ``[position, write_idx]``.  Every window row and every selected row is a key and a value; the sink joins the
     maximum and the denominator once.  Returns float16 ``[n_heads, 512]`` after the inverse rope.
-    Composed of the rope and sparse-attention operators of this package."""
-    from .attention import apply_rope_tail
-    from .indexed_attention_kernel import sparse_attention
+    Launches: the operands (rope, window, sinks), the attention (and its merge), the inverse rope."""
     if q.ndim != 2 or int(q.shape[1]) != _HEAD_DIM or q.dtype != torch.float16:
         raise ValueError("q must be float16 [n_heads, 512]")
     n_heads = int(q.shape[0])
@@ -121,19 +131,16 @@ def fused_decode_sdpa(q, window, row, pooled, sel, sinks, inv_freq, params, *, s
         raise ValueError("sinks must be float16 [n_heads]")
     if int(inv_freq.shape[-1]) != _ROPE_DIM // 2 or inv_freq.dtype != torch.float32:
         raise ValueError("inv_freq must be float32 [32]")
-    require_cuda(q, window, row, pooled, sel, sinks, inv_freq, params)
-    pos = _position(params)
-    write_idx = params.reshape(-1)[1:2].to(torch.int64)
-    window_rows = int(window.shape[0])
-    qr = apply_rope_tail(q.reshape(1, n_heads, _HEAD_DIM).transpose(0, 1).contiguous(), pos, inv_freq=inv_freq,
-                         half_chain=True)                                   # [H, 1, 512]
-    # the prepared row replaces window[write_idx] (an index outside the window replaces nothing), on the device
-    slot = torch.arange(window_rows, device=window.device, dtype=torch.int64)[:, None] == write_idx
-    win = torch.where(slot, row[None], window)
-    # all window rows are keys: place the window so that its last row is the newest position and nothing is clipped
-    pos0 = torch.clamp(pos, min=window_rows - 1)
-    out = sparse_attention(qr.reshape(1, n_heads, 1, _HEAD_DIM), pooled, sel.reshape(1, 1, -1), sinks.float(),
-                           pos0=0, pos0_dev=pos0, window=0, ratio=0, raw_kv=win[None], raw_start=0,
-                           scale=float(scale), d_v=_HEAD_DIM, out_dtype=torch.float16)
-    out = out.reshape(n_heads, 1, _HEAD_DIM)
-    return apply_rope_tail(out, pos, inv_freq=inv_freq, inverse=True, half_chain=True).reshape(n_heads, _HEAD_DIM)
+    dev = require_cuda(q, window, row, pooled, sel, sinks, inv_freq, params)
+    inv_freq, params, wide = _token_operands(inv_freq, params, 2)
+    q, window, row, pooled, sel, sinks = (t.contiguous() for t in (q, window, row, pooled, sel, sinks))
+    lib = _abi.load()
+    a = _abi.FusedDecodeSdpaArgs()
+    a.q, a.window, a.row, a.pooled, a.sel, a.sinks = ptr(q), ptr(window), ptr(row), ptr(pooled), ptr(sel), ptr(sinks)
+    a.inv_freq, a.params, a.params_int64, a.scale = ptr(inv_freq), ptr(params), wide, float(scale)
+    a.n_heads, a.window_rows, a.topk, a.n_rows = n_heads, int(window.shape[0]), int(sel.shape[0]), int(pooled.shape[0])
+    out = torch.empty((n_heads, _HEAD_DIM), dtype=torch.float16, device=dev)
+    ws = _t.workspace(lib.mxb_fused_decode_sdpa_workspace_bytes(C.byref(a)), dev)
+    a.out, a.workspace, a.workspace_bytes = ptr(out), ptr(ws), ws.numel()
+    _abi.check(_t.launch("fused_decode_sdpa", lib.mxb_fused_decode_sdpa, a))
+    return out

@@ -99,3 +99,16 @@ def test_synth_rounding_helpers():
     c = synth.config3(seed=1, lens=[10, 20])
     assert c["kv"].shape == (30, 576) and c["kv"].dtype == np.int8 and c["kv_scales"].dtype == np.float16
     assert float(c["kv_scales"].min()) >= 9e-4 and float(c["kv_scales"].max()) <= 1.01e-1
+
+
+def test_operator_pair_and_fused_struct_layouts_match_c(tmp_path):
+    from moespresso_b200 import _abi
+    pairs = [("mxb_affine_q8_pair_args", _abi.AffineQ8PairArgs), ("mxb_fused_decode_prep_args", _abi.FusedDecodePrepArgs),
+             ("mxb_fused_decode_sdpa_args", _abi.FusedDecodeSdpaArgs)]
+    body = "".join(f'printf("%zu ", sizeof({c}));' + "".join(f'printf("%zu ", offsetof({c}, {f[0]}));' for f in cls._fields_)
+                   for c, cls in pairs)
+    src, exe = tmp_path / "layout.c", tmp_path / "layout"
+    src.write_text(f'#include <stdio.h>\n#include <stddef.h>\n#include "{HEADER}"\nint main(void){{{body}return 0;}}')
+    subprocess.run(["gcc", str(src), "-o", str(exe)], check=True)
+    got = [int(x) for x in subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()]
+    assert got == [n for _, cls in pairs for n in [C.sizeof(cls)] + [getattr(cls, f[0]).offset for f in cls._fields_]]

@@ -75,3 +75,46 @@ def test_fused_decode_rejects_bad_inputs():
         fused_decode_sdpa(z(8, 512), z(128, 512, dt=torch.float16), z(512, dt=torch.float16),
                           z(16, 512, dt=torch.float16), torch.zeros(4, dtype=torch.int32, device="cuda"),
                           z(8, dt=torch.float16), z(32), params, scale=0.1)
+
+
+@pytest.mark.parametrize("n_heads,window_rows,n_rows,topk,pos,write_idx,pdtype", [
+    (64, 128, 961, 512, 3843, 3, torch.int32),     # replaced row inside the window
+    (1, 1, 5, 4, 0, 0, torch.int64),               # the smallest of everything; the window is older than the position
+    (7, 127, 300, 64, 60, 127, torch.int32),       # position before the window's end, write index outside it
+    (64, 0, 961, 512, 3843, 0, torch.int32),       # no window
+])
+def test_fused_operators_equal_the_single_operators(n_heads, window_rows, n_rows, topk, pos, write_idx, pdtype):
+    """Bit for bit what the QAT, score, top-k, FP8 round-trip, rope and attention operators give one by one; operands
+    that are views of larger tensors, bases that are not 16-byte aligned included."""
+    need_gpu()
+    from moespresso_b200.deepseek_v4.decode_attention_kernel import fp8_kv_prefix_rows
+    from moespresso_b200.deepseek_v4.indexed_attention_kernel import sparse_attention
+    from moespresso_b200.deepseek_v4.indexer_score_kernel import fused_qat_indexer_scores
+    g = torch.Generator(device="cuda").manual_seed(n_rows + pos)
+    mk = lambda *s, dt=torch.float16: torch.randn(s, generator=g, device="cuda").to(dt)  # noqa: E731
+    h16 = torch.float16
+    inv = dev(_inv_freq())
+    params = torch.tensor([pos, write_idx], dtype=pdtype, device="cuda")
+    q_idx, weights = mk(n_heads, 2, 128)[:, 0], mk(n_heads, dt=torch.float32)
+    pooled_qat, kv_row = mk(n_rows, 128, dt=torch.float32), mk(513)[1:]
+    sel, row, scores = fused_decode_prep(q_idx, pooled_qat, weights, kv_row, inv, params, scale=0.09, topk=topk)
+    ref_scores = fused_qat_indexer_scores(q_idx.reshape(1, n_heads, 1, 128), pooled_qat[None],
+                                          weights.reshape(1, 1, n_heads), 0.09)
+    p64 = params[0:1].to(torch.int64)
+    rope = lambda x, **kw: att.apply_rope_tail(x, p64, inv_freq=inv, half_chain=True, **kw)  # noqa: E731
+    ref_row = fp8_kv_prefix_rows(kv_row.float()[None])[0].to(h16)
+    ref_row[448:] = rope(kv_row.reshape(1, 1, 512)).reshape(-1)[448:]
+    assert torch.equal(scores, ref_scores) and torch.equal(sel, att.topk_select(ref_scores[None], topk)[0])
+    assert torch.equal(row.view(torch.int16), ref_row.view(torch.int16))
+
+    q, sinks = mk(n_heads * 512 + 1)[1:].reshape(n_heads, 512), mk(n_heads)
+    window, pooled = mk(window_rows, 512), mk(n_rows, 512)
+    got = fused_decode_sdpa(q, window, row, pooled, sel, sinks, inv, params, scale=512 ** -0.5)
+    win = window.clone()
+    if write_idx < window_rows:
+        win[write_idx] = row
+    out = sparse_attention(rope(q.reshape(n_heads, 1, 512)).reshape(1, n_heads, 1, 512), pooled, sel.reshape(1, 1, -1),
+                           sinks.float(), pos0=max(pos, window_rows - 1), window=0, ratio=0,
+                           raw_kv=win[None] if window_rows else None, scale=512 ** -0.5, d_v=512, out_dtype=h16)
+    ref = rope(out.reshape(n_heads, 1, 512), inverse=True).reshape(n_heads, 512)
+    assert torch.equal(got.view(torch.int16), ref.view(torch.int16))
