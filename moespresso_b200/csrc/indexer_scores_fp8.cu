@@ -1,6 +1,6 @@
 // Indexer score over FP8-E4M3 key tables: a warp-specialised streaming pipeline.
 //
-//   warp roles      drain warps (2 sets x 4, thread = key row = TMEM lane)
+//   warp roles      drain warps (2 or 4 sets x 4, thread = key row = TMEM lane)
 //                   1 MMA-issue warp, 1 TMA-producer warp, [NA widening warps]
 //
 // Two operand modes.
@@ -52,6 +52,7 @@ struct Fp8Params {
   int64_t pos0;
   int32_t ratio;
   int32_t t_tile;        // tokens per CTA
+  int32_t t_first;       // first token of this launch
   int32_t N;             // MMA N
   int32_t acc_stride;    // TMEM columns per accumulator (N rounded up to 32)
   int32_t n_acc;         // accumulators in the TMEM ring
@@ -70,11 +71,13 @@ struct Fp8Cfg {
   // 16-bit operand buffers (WIDEN: one per widening warp; KEYS16: the TMA ring itself)
   static constexpr int kNA = MODE == kDirect ? 0 : (MODE == kWiden ? (D == 64 ? 4 : 2) : (D == 64 ? 4 : 3));
   static constexpr int kConv = MODE == kWiden ? kNA : 0;                            // widening warps
-  // drain warps: kTileGroups tiles drained concurrently, each by kColSplit groups of 4 warps that share
-  // the tile's columns (the wide prefill tiles of KEYS16 need more drain threads per tile)
-  static constexpr int kTileGroups = 2;
-  static constexpr int kColSplit = MODE == kKeys16 ? 2 : 1;
-  static constexpr int kDrainWarps = 4 * kTileGroups * kColSplit;
+  // Columns of a tile = (tokens x heads).  KEYS16, where the drain sets the pace: 128 columns, so that TMEM holds four
+  // accumulators and each of the four groups of drain warps has one of its own; with 256 columns and two accumulators a
+  // tile's MMAs had to wait for the drain of the tile before last and the drain for them (with the packed multiply-adds of
+  // the drain: 333 tokens x 5,003 rows 27.4 -> 14.7 us, 4,096 x 32,768 in seven launches 648 -> 595 us).
+  static constexpr int kCols = MODE == kKeys16 ? 128 : 256;
+  static constexpr int kTileGroups = MODE == kKeys16 ? 4 : 2;   // tiles drained concurrently, four warps each
+  static constexpr int kDrainWarps = 4 * kTileGroups;
   static constexpr int kMmaWarp = kDrainWarps;
   static constexpr int kTmaWarp = kDrainWarps + kMmaWarps;
   static constexpr int kConvWarp0 = kTmaWarp + 1;
@@ -106,8 +109,8 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
   uint8_t* raw_buf = smem + C::raw_off;
   uint8_t* a16_buf = smem + C::a16_off;
   uint8_t* b_buf = smem + C::b_off;
-  float* w_s = reinterpret_cast<float*>(b_buf + p.b_bytes);              // [<= 256]
-  int32_t* vis_s = reinterpret_cast<int32_t*>(w_s + 256);                // [<= 256] rows visible to each token
+  float* w_s = reinterpret_cast<float*>(b_buf + p.b_bytes);              // [<= 512]: see pair_index
+  int32_t* vis_s = reinterpret_cast<int32_t*>(w_s + 512);                // [<= 256] rows visible to each token
   uint64_t* raw_full = reinterpret_cast<uint64_t*>(vis_s + 256);         // [8]
   uint64_t* raw_empty = raw_full + 8;                                    // [8]
   uint64_t* a_full = raw_empty + 8;                                      // [4]
@@ -119,7 +122,7 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int b = blockIdx.z;
-  const int t0 = blockIdx.y * p.t_tile;
+  const int t0 = p.t_first + blockIdx.y * p.t_tile;
   const int64_t count = p.row_count ? (int64_t)p.row_count[b] : p.n_rows;
   const int64_t rbase = p.row_start ? p.row_start[b] : (int64_t)b * p.n_rows;
   const int64_t row0 = (int64_t)blockIdx.x * p.rows_per_cta;
@@ -146,7 +149,7 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
     }
     for (int a = 0; a < n_acc; ++a) {
       ptx::mbar_init(&acc_full[a], 1);
-      ptx::mbar_init(&acc_empty[a], 128 * C::kColSplit);
+      ptx::mbar_init(&acc_empty[a], 128);
     }
     *abort_flag = 0;
     ptx::mbar_fence_init();
@@ -157,6 +160,9 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
     ptx::tmem_alloc(tmem_slot, (uint32_t)p.tmem_cols);
     ptx::tmem_relinquish();
   }
+
+  // head weights of tokens 2 i and 2 i + 1 side by side, as the drain multiplies them
+  auto pair_index = [&](int t, int h) { return ((t >> 1) * H + h) * 2 + (t & 1); };
 
   // ---- query -> B operand.
   // 16-bit keys: q has the keys' type and is used as it is, so the operand is a plain copy, one 16-byte chunk
@@ -177,7 +183,7 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
     }
     for (int n = tid; n < p.t_tile * H; n += C::kThreads) {
       const int t = n / H, h = n % H;
-      w_s[n] = (t < nt) ? p.weights[((int64_t)b * p.T + t0 + t) * H + h] : 0.f;
+      w_s[pair_index(t, h)] = (t < nt) ? p.weights[((int64_t)b * p.T + t0 + t) * H + h] : 0.f;
     }
   }
   // Otherwise one warp per (token, head) row; lane owns D/32 features.
@@ -236,7 +242,7 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
         reinterpret_cast<uint16_t*>(b_buf + (size_t)kb * N * 128 + (size_t)n * 128 + ((c ^ (n & 7)) << 4))[within] = bits;
       }
     }
-    if (lane == 0) w_s[r] = (t < nt) ? ldexpf(p.weights[((int64_t)b * p.T + t0 + t) * H + h], -a) : 0.f;
+    if (lane == 0) w_s[pair_index(t, h)] = (t < nt) ? ldexpf(p.weights[((int64_t)b * p.T + t0 + t) * H + h], -a) : 0.f;
   }
   // rows a token may see (causal mask over compressed rows), once per token instead of once per score
   for (int t = tid; t < nt; t += C::kThreads) {
@@ -385,12 +391,9 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
   } else {
     // ------------------------------------------------------------ drain: thread = key row
     const int set = warp >> 2, quad = warp & 3;
-    const int tg = set / C::kColSplit, ch = set % C::kColSplit;   // tile group, share of the tile's tokens
-    const int t_per = (p.t_tile + C::kColSplit - 1) / C::kColSplit;
-    const int t_lo = min(ch * t_per, nt), t_hi = min(t_lo + t_per, nt);
     const int rloc = quad * 32 + lane;
     const int64_t sbase = (p.row_start ? p.row_start[b] : 0) + (int64_t)b * p.s_sb;
-    for (int i = tg; i < ntiles; i += C::kTileGroups) {
+    for (int i = set; i < ntiles; i += C::kTileGroups) {
       const int a = i % n_acc;
       ptx::mbar_wait(&acc_full[a], (uint32_t)((i / n_acc) & 1), abort_flag);
       ptx::tc_fence_after_sync();
@@ -398,7 +401,7 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
       const int64_t r = row0 + (int64_t)i * 128 + rloc;
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * p.acc_stride);
       const bool r_ok = r < count;
-      float* sp = p.scores + sbase + (int64_t)(t0 + t_lo) * p.s_st + r;
+      float* sp = p.scores + sbase + (int64_t)t0 * p.s_st + r;
       // two tokens per step: their TMEM loads travel together and their two head sums (each in head order) are
       // independent chains, so the loop is no longer one load latency plus one dependent chain per token
       auto load_tok = [&](int t, int c0, uint32_t* v) {
@@ -413,49 +416,38 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
           ptx::tmem_ld16(taddr + (uint32_t)(t * H + c0), v);
         }
       };
-      int t = t_lo;
-      for (; t + 1 < t_hi; t += 2, sp += 2 * p.s_st) {
-        float sum0 = 0.f, sum1 = 0.f;
+      int t = 0;
+      for (; t + 1 < nt; t += 2, sp += 2 * p.s_st) {
+        float2 sum = make_float2(0.f, 0.f);   // tokens t and t + 1: one packed multiply-add per head
         for (int c0 = 0; c0 < H; c0 += 16) {
           uint32_t va[16], vb[16];
           load_tok(t, c0, va);
           load_tok(t + 1, c0, vb);
           ptx::tmem_ld_wait();
-          const float4* wa = reinterpret_cast<const float4*>(w_s + t * H + c0);   // H is a multiple of 16
-          const float4* wb = reinterpret_cast<const float4*>(w_s + (t + 1) * H + c0);
+          const float4* w = reinterpret_cast<const float4*>(w_s + (t * H + 2 * c0));   // H is a multiple of 16
 #pragma unroll
-          for (int j4 = 0; j4 < 4; ++j4) {
-            const float4 x = wa[j4], y = wb[j4];
-            sum0 = fmaf(x.x, fmaxf(__uint_as_float(va[4 * j4 + 0]), 0.f), sum0);
-            sum1 = fmaf(y.x, fmaxf(__uint_as_float(vb[4 * j4 + 0]), 0.f), sum1);
-            sum0 = fmaf(x.y, fmaxf(__uint_as_float(va[4 * j4 + 1]), 0.f), sum0);
-            sum1 = fmaf(y.y, fmaxf(__uint_as_float(vb[4 * j4 + 1]), 0.f), sum1);
-            sum0 = fmaf(x.z, fmaxf(__uint_as_float(va[4 * j4 + 2]), 0.f), sum0);
-            sum1 = fmaf(y.z, fmaxf(__uint_as_float(vb[4 * j4 + 2]), 0.f), sum1);
-            sum0 = fmaf(x.w, fmaxf(__uint_as_float(va[4 * j4 + 3]), 0.f), sum0);
-            sum1 = fmaf(y.w, fmaxf(__uint_as_float(vb[4 * j4 + 3]), 0.f), sum1);
+          for (int j = 0; j < 8; ++j) {
+            const float4 x = w[j];   // heads c0 + 2 j and + 1, tokens t and t + 1 of each
+            sum = __ffma2_rn(make_float2(x.x, x.y), make_float2(fmaxf(__uint_as_float(va[2 * j]), 0.f),
+                                                                fmaxf(__uint_as_float(vb[2 * j]), 0.f)), sum);
+            sum = __ffma2_rn(make_float2(x.z, x.w), make_float2(fmaxf(__uint_as_float(va[2 * j + 1]), 0.f),
+                                                                fmaxf(__uint_as_float(vb[2 * j + 1]), 0.f)), sum);
           }
         }
         if (r_ok) {
-          sp[0] = r < (int64_t)vis_s[t] ? sum0 : -INFINITY;
-          sp[p.s_st] = r < (int64_t)vis_s[t + 1] ? sum1 : -INFINITY;
+          sp[0] = r < (int64_t)vis_s[t] ? sum.x : -INFINITY;
+          sp[p.s_st] = r < (int64_t)vis_s[t + 1] ? sum.y : -INFINITY;
         }
       }
-      if (t < t_hi) {
+      if (t < nt) {
         float sum = 0.f;
         for (int c0 = 0; c0 < H; c0 += 16) {
           uint32_t v1[16];
           load_tok(t, c0, v1);
           ptx::tmem_ld_wait();
-          const float4* w4 = reinterpret_cast<const float4*>(w_s + t * H + c0);
+          const float* w = w_s + (t * H + 2 * c0);   // (every second entry: the pair's other token is not there)
 #pragma unroll
-          for (int j4 = 0; j4 < 4; ++j4) {
-            const float4 w = w4[j4];
-            sum = fmaf(w.x, fmaxf(__uint_as_float(v1[4 * j4 + 0]), 0.f), sum);
-            sum = fmaf(w.y, fmaxf(__uint_as_float(v1[4 * j4 + 1]), 0.f), sum);
-            sum = fmaf(w.z, fmaxf(__uint_as_float(v1[4 * j4 + 2]), 0.f), sum);
-            sum = fmaf(w.w, fmaxf(__uint_as_float(v1[4 * j4 + 3]), 0.f), sum);
-          }
+          for (int j = 0; j < 16; ++j) sum = fmaf(w[2 * j], fmaxf(__uint_as_float(v1[j]), 0.f), sum);
         }
         if (r_ok) *sp = r < (int64_t)vis_s[t] ? sum : -INFINITY;
       }
@@ -478,7 +470,7 @@ static int launch_fp8_d(Fp8Params& p, const mxb_indexer_scores_args* a, cudaStre
   constexpr bool DIRECT = MODE == kDirect;
   constexpr bool K16 = MODE == kKeys16;
   const int cols_per_token = (DIRECT ? 2 : 1) * p.H;
-  int t_tile = 256 / cols_per_token;
+  int t_tile = C::kCols / cols_per_token;
   if (t_tile > p.T) t_tile = p.T;
   p.t_tile = t_tile;
   p.N = t_tile * cols_per_token;
@@ -493,7 +485,7 @@ static int launch_fp8_d(Fp8Params& p, const mxb_indexer_scores_args* a, cudaStre
   p.b_bytes = (int)round_up((int64_t)p.N * D * (DIRECT ? 1 : 2), 1024);
   const int64_t t_tiles = ceil_div(p.T, t_tile);
   const int64_t tiles = ceil_div(p.n_rows, 128);
-  const int smem = C::b_off + p.b_bytes + 256 * 4 + 256 * 4 + 56 * 8 + 64 + 1024;
+  const int smem = C::b_off + p.b_bytes + 512 * 4 + 256 * 4 + 56 * 8 + 64 + 1024;
   const int ctas_per_sm = smem <= 113 * 1024 ? 2 : 1;
   // static chunks of rows per CTA, several per resident slot so that ragged sequences balance
   int64_t want_ctas = (int64_t)sm_count() * ctas_per_sm * 6;
@@ -530,10 +522,13 @@ static int launch_fp8_d(Fp8Params& p, const mxb_indexer_scores_args* a, cudaStre
   if (rc != MXB_OK) return rc;
   auto kern = indexer_fp8_kernel<D, MODE>;
   MXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  dim3 grid((unsigned)ceil_div(p.n_rows, p.rows_per_cta), (unsigned)t_tiles, (unsigned)p.B);
-  kern<<<grid, C::kThreads, smem, st>>>(tmap, p);
-  note_launch();
-  MXB_CUDA_OK(cudaGetLastError());
+  for (int64_t y = 0; y < t_tiles; y += 65535) {   // (a grid holds that many token tiles)
+    p.t_first = (int32_t)(y * t_tile);
+    const dim3 grid((unsigned)ceil_div(p.n_rows, p.rows_per_cta), (unsigned)(t_tiles - y < 65535 ? t_tiles - y : 65535), (unsigned)p.B);
+    kern<<<grid, C::kThreads, smem, st>>>(tmap, p);
+    note_launch();
+    MXB_CUDA_OK(cudaGetLastError());
+  }
   return MXB_OK;
 }
 
