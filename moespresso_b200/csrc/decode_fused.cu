@@ -4,7 +4,7 @@
 // (src/moespresso/runtime/deepseek_v4/decode_attention_kernel.py:669-786).  A token is all latency: the arithmetic of
 // the small kernels is nothing, so what counts is how many of them there are.  decode_prep_kernel does everything that
 // precedes the score scan and decode_sdpa_prep_kernel everything that precedes the attention, whatever the row type;
-// the scan, the selection and the attention are the package's kernels.  At 2,500 rows a token takes 67 us (46 us of it
+// the scan, the selection and the attention are the package's kernels.  At 2,500 rows a token takes 57 us (44 us of it
 // in eight kernels); as some twenty single operators it took 378 us, 104 of them in kernels.
 #include "decode_rows.cuh"
 
@@ -20,6 +20,16 @@ struct TokenParams {     // int32 or int64 [position, write index]
   }
 };
 
+// Rotates the last 64 channels of a row, a pair per lane; the other channels stay where they are.
+__device__ __forceinline__ void rope_row(__half* dst, const __half* src, int64_t pos, const float* inv_freq, bool inverse,
+                                         int lane) {
+  const int i = kRowDim - kRopeDim + 2 * lane;
+  __half y0, y1;
+  rope_half_pair(src[i], src[i + 1], pos, inv_freq[lane], inverse, y0, y1);
+  dst[i] = y0;
+  dst[i + 1] = y1;
+}
+
 struct DecodePrepParams {
   const void* q;          // [H, 128]
   const float* weights;   // [H]
@@ -33,8 +43,8 @@ struct DecodePrepParams {
   __half* row;            // [512]
 };
 
-// Warp w: QAT of head w; warp H: the KV row (E4M3FN round trip of dims [0, 448), rope of the other 64); warp H + 1:
-// the score scale folded into the head weights.
+// Warp w: QAT of head w; warp H: E4M3FN round trip of dims [0, 448) of the KV row; warp H + 1: rope of its other 64, a
+// pair per lane (cos and sin are the longest chain here); warp H + 2: the score scale folded into the head weights.
 template <int QT>
 __global__ void __launch_bounds__(128) decode_prep_kernel(DecodePrepParams p) {
   const int lane = threadIdx.x & 31, w = (int)blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -45,30 +55,17 @@ __global__ void __launch_bounds__(128) decode_prep_kernel(DecodePrepParams p) {
     indexer_qat_row(v, lane, o);
     *reinterpret_cast<float4*>(p.q_qat + w * kIdxDim + 4 * lane) = make_float4(o[0], o[1], o[2], o[3]);
   } else if (w == p.H) {
-    __half x[16];
     float xv[16];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      x[j] = p.kv_row[16 * lane + j];
-      xv[j] = __half2float(x[j]);
-    }
+    for (int j = 0; j < 16; ++j) xv[j] = __half2float(p.kv_row[16 * lane + j]);
     fp8_kv_row<false>(xv, lane);
     if (lane < 28) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) x[j] = __float2half_rn(xv[j]);
-    } else {
-      const int64_t pos = p.token.at(0);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        __half y0, y1;
-        rope_half_pair(x[2 * j], x[2 * j + 1], pos, p.inv_freq[(lane - 28) * 8 + j], false, y0, y1);
-        x[2 * j] = y0;
-        x[2 * j + 1] = y1;
-      }
+      for (int j = 0; j < 16; ++j) p.row[16 * lane + j] = __float2half_rn(xv[j]);
     }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) p.row[16 * lane + j] = x[j];
   } else if (w == p.H + 1) {
+    rope_row(p.row, p.kv_row, p.token.at(0), p.inv_freq, false, lane);
+  } else if (w == p.H + 2) {
     for (int h = lane; h < p.H; h += 32) p.w_scaled[h] = __fmul_rn(p.weights[h], p.scale);
   }
 }
@@ -97,16 +94,6 @@ __device__ __forceinline__ void copy_row(__half* dst, const __half* src, int lan
   } else {
     for (int i = lane; i < kRowDim; i += 32) dst[i] = src[i];
   }
-}
-
-// Rotates the last 64 channels of a row, a pair per lane; the other channels stay where they are.
-__device__ __forceinline__ void rope_row(__half* dst, const __half* src, int64_t pos, const float* inv_freq, bool inverse,
-                                         int lane) {
-  const int i = kRowDim - kRopeDim + 2 * lane;
-  __half y0, y1;
-  rope_half_pair(src[i], src[i + 1], pos, inv_freq[lane], inverse, y0, y1);
-  dst[i] = y0;
-  dst[i + 1] = y1;
 }
 
 // Warp w: head w of q, then row w - H of the window; warp H + W: the sinks and the position.
@@ -188,7 +175,7 @@ extern "C" int mxb_fused_decode_prep(const mxb_fused_decode_prep_args* a, void* 
   p.row = reinterpret_cast<__half*>(a->row);
   const int64_t topk_bytes = mxb_topk_workspace_bytes(1, a->n_rows, a->topk);
   void* topk_ws = ws.take(topk_bytes);
-  const unsigned grid = (unsigned)ceil_div(a->n_heads + 2, 4);
+  const unsigned grid = (unsigned)ceil_div(a->n_heads + 3, 4);
   if (a->q_dtype == MXB_F32) decode_prep_kernel<MXB_F32><<<grid, 128, 0, st>>>(p);
   else if (a->q_dtype == MXB_F16) decode_prep_kernel<MXB_F16><<<grid, 128, 0, st>>>(p);
   else decode_prep_kernel<MXB_BF16><<<grid, 128, 0, st>>>(p);
