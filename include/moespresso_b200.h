@@ -55,6 +55,15 @@ int64_t mxb_kernel_launches(void);
  * side stream without a CUDA binding of their own (the decode plan copies q this way while the selection runs). */
 int mxb_copy_h2d_async(void* dst_device, const void* src_host, int64_t bytes, void* stream);
 
+/* Device-to-device copies of up to four buffers in one launch (the inputs of a captured step). */
+typedef struct {
+  void* dst[4];
+  const void* src[4];
+  int64_t bytes[4];     /* 0: nothing to copy */
+} mxb_copy_buffers_args;
+
+int mxb_copy_buffers(const mxb_copy_buffers_args* a, void* stream);
+
 /* ------------------------------------------------------------------------ *
  * Indexer score.
  * Replaces  indexer_scores_tiled_live(q, weights, index_comp, *, pos0, ratio)

@@ -133,6 +133,10 @@ class FusedDecodeSdpaArgs(C.Structure):
                 ("topk", _i32), ("n_rows", _i64), ("out", _p), ("workspace", _p), ("workspace_bytes", _i64)]
 
 
+class CopyBuffersArgs(C.Structure):
+    _fields_ = [("dst", _p * 4), ("src", _p * 4), ("bytes", _i64 * 4)]
+
+
 class RangeCandidatesArgs(C.Structure):
     _fields_ = [("scores", _p), ("ids", _p), ("out_scores", _p), ("out_ids", _p), ("k", _i32), ("row_lo", _i64)]
 
@@ -147,6 +151,7 @@ EXPORTS = {
     "mxb_last_error": (C.c_char_p, []),
     "mxb_kernel_launches": (C.c_int64, []),
     "mxb_copy_h2d_async": (C.c_int, [_p, _p, _i64, _p]),
+    "mxb_copy_buffers": (C.c_int, [C.POINTER(CopyBuffersArgs), _p]),
     "mxb_indexer_scores": (C.c_int, [C.POINTER(IndexerScoresArgs), _p]),
     "mxb_indexer_qat": (C.c_int, [C.POINTER(IndexerQatArgs), _p]),
     "mxb_score_tail": (C.c_int, [C.POINTER(ScoreTailArgs), _p]),

@@ -94,6 +94,41 @@ extern "C" int mxb_copy_h2d_async(void* dst_device, const void* src_host, int64_
 }
 
 namespace mxb {
+// One CTA column per buffer; 16-byte pieces where both sides allow it.  A decode step's three inputs (a few KB to a few
+// MB) are three launches as single copies, and a launch is what each of them costs.
+__global__ void __launch_bounds__(256) copy_buffers_kernel(mxb_copy_buffers_args a) {
+  const int i = blockIdx.y;
+  const int64_t n = a.bytes[i], step = (int64_t)gridDim.x * 256, at = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  uint8_t* dst = reinterpret_cast<uint8_t*>(a.dst[i]);
+  const uint8_t* src = reinterpret_cast<const uint8_t*>(a.src[i]);
+  int64_t done = 0;
+  if (((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0) {
+    const int64_t pieces = n / 16;
+#pragma unroll 4
+    for (int64_t j = at; j < pieces; j += step) reinterpret_cast<uint4*>(dst)[j] = __ldg(reinterpret_cast<const uint4*>(src) + j);
+    done = pieces * 16;
+  }
+  for (int64_t j = done + at; j < n; j += step) dst[j] = src[j];
+}
+}  // namespace mxb
+
+extern "C" int mxb_copy_buffers(const mxb_copy_buffers_args* a, void* stream) {
+  MXB_REQUIRE(a != nullptr, MXB_ERR_INVALID, "copy buffers: null args");
+  int64_t longest = 0;
+  for (int i = 0; i < 4; ++i) {
+    MXB_REQUIRE(a->bytes[i] >= 0 && (a->bytes[i] == 0 || (a->dst[i] && a->src[i])), MXB_ERR_INVALID,
+                "copy buffers: null pointer or negative size");
+    if (a->bytes[i] > longest) longest = a->bytes[i];
+  }
+  if (longest == 0) return MXB_OK;
+  const int64_t want = mxb::ceil_div(longest, 256 * 16 * 2), most = 2 * (int64_t)mxb::sm_count();
+  mxb::copy_buffers_kernel<<<dim3((unsigned)(want < most ? want : most), 4), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(*a);
+  mxb::note_launch();
+  MXB_CUDA_OK(cudaGetLastError());
+  return MXB_OK;
+}
+
+namespace mxb {
 __global__ void range_candidates_kernel(mxb_range_candidates_args a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.k) return;

@@ -204,6 +204,17 @@ class SparseDecodePlan:
 
     def load_inputs(self, q, idx_q, idx_w) -> None:
         """Copy one step's inputs (device or pinned-host tensors) into the plan's buffers."""
+        pairs = ((self.q, q), (self.idx_q, idx_q), (self.idx_w, idx_w))
+        if torch.cuda.current_device() == self.q.device.index and all(
+               isinstance(s, torch.Tensor) and s.device == d.device and s.dtype == d.dtype and s.shape == d.shape
+               and s.is_contiguous() for d, s in pairs):
+            from .. import _abi
+            from .. import _torchabi as _t
+            a = _abi.CopyBuffersArgs()
+            for i, (d, s) in enumerate(pairs):
+                a.dst[i], a.src[i], a.bytes[i] = d.data_ptr(), s.data_ptr(), self._sizes[i]
+            _abi.check(_t.launch("copy_buffers", _abi.load().mxb_copy_buffers, a))
+            return
         self.q.copy_(q, non_blocking=True)
         self.idx_q.copy_(idx_q, non_blocking=True)
         self.idx_w.copy_(idx_w, non_blocking=True)

@@ -127,3 +127,39 @@ def test_plan_with_16bit_cache():
         ref = ds4.indexed_mixed_attention_decode(c["q"][b], None, kv[s:s + n], ids[b], None, pos0=0, window=0, ratio=0,
                                                  scale=c["scale"], d_v=c["d_v"])
         assert max_abs(eager[b], ref) <= tol
+
+
+@pytest.mark.parametrize("sizes", [(0, 1, 15), (16, 17, 4097), (8192, 8191, (3 << 20) + 5)])
+@pytest.mark.parametrize("offset", [0, 2])
+def test_copy_buffers(sizes, offset):
+    """Bytes on and off 16-byte boundaries, nothing copied behind them."""
+    need_gpu()
+    from moespresso_b200 import _abi
+    from moespresso_b200 import _torchabi as _t
+    a = _abi.CopyBuffersArgs()
+    src = [torch.randint(1, 256, (n + 32,), dtype=torch.uint8, device="cuda") for n in sizes]
+    dst = [torch.zeros(n + 32, dtype=torch.uint8, device="cuda") for n in sizes]
+    for i, n in enumerate(sizes):
+        a.dst[i], a.src[i], a.bytes[i] = dst[i].data_ptr() + offset, src[i].data_ptr() + 16, n
+    _abi.check(_t.launch("copy_buffers", _abi.load().mxb_copy_buffers, a))
+    for i, n in enumerate(sizes):
+        assert torch.equal(dst[i][offset:offset + n], src[i][16:16 + n])
+        assert int(dst[i].sum()) == int(src[i][16:16 + n].sum())
+
+
+def test_plan_takes_inputs_of_every_layout():
+    """Contiguous device inputs are copied together, strided or otherwise typed ones one by one: the same step."""
+    need_gpu()
+    from moespresso_b200.deepseek_v4.decode_step import SparseDecodePlan
+    g = torch.Generator(device="cuda").manual_seed(3)
+    mk = lambda *s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
+    lens = [1500, 1100]
+    cache = LatentCache(kv=mk(2600, 576).bfloat16(), kv_scales=None, idx_keys=mk(2600, 64).to(torch.float8_e4m3fn),
+                        row_start=torch.tensor([0, 1500], device="cuda"),
+                        row_count=torch.tensor(lens, dtype=torch.int32, device="cuda"), max_rows=1500)
+    plan = SparseDecodePlan(cache, heads=64, d_qk=576, idx_heads=16, idx_dim=64, k=256, scale=576 ** -0.5, d_v=512)
+    q, iq, iw = mk(2, 64, 576).bfloat16(), mk(2, 16, 64).bfloat16(), mk(2, 16)
+    want = plan.run(q, iq, iw).clone()
+    for args in ((q.float(), iq, iw), (q.transpose(1, 2).contiguous().transpose(1, 2), iq, iw), (q.cpu(), iq, iw.cpu())):
+        plan.packed.zero_()
+        assert torch.equal(plan.run(*args), want)
