@@ -484,3 +484,33 @@ def test_tensor_core_kernel_prefill_form():
         ref = ds4.indexed_mixed_attention_prefill(q[b].transpose(1, 0, 2), None, comp[b], ids[b], sinks, pos0=pos0,
                                                   ratio=4, d_v=Dv)
         assert max_abs(out[b].permute(1, 0, 2), ref) <= TOL_16
+
+
+@pytest.mark.parametrize("extra,k,window", [(1, 512, 0), (37, 300, 100), (74, 512, 128), (75, 512, 0), (40, 100, 0)])
+@pytest.mark.parametrize("kind", ["bf16", "f16", "i8"])
+def test_last_wave_of_a_chunk(extra, k, window, kind):
+    """One token per SM and ``extra`` more: up to half a wave of them runs as split clusters (too many for four, three
+    or two splits, and lists too short to split, among the cases), against the fp32 CUDA-core kernel on the same
+    tables."""
+    need_gpu()
+    T, H, D, Dv, R = torch.cuda.get_device_properties(0).multi_processor_count + extra, 64, 576, 512, 1500
+    g = torch.Generator(device="cuda").manual_seed(extra + k)
+    mk = lambda *s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
+    dt = torch.float16 if kind == "f16" else torch.bfloat16
+    comp, raw = mk(R, D), mk(1, T + window, D)
+    scales = raw_scales = None
+    if kind == "i8":
+        scales, raw_scales = (0.01 + 0.02 * torch.rand(n, generator=g, device="cuda") for n in (R, T + window))
+        comp, raw = (x.mul(40).clamp(-127, 127).to(torch.int8) for x in (comp, raw))
+        scales, raw_scales = scales.half(), raw_scales.half()
+    else:
+        comp, raw = comp.to(dt), raw.to(dt)
+    ids = torch.sort(torch.rand(T, R, generator=g, device="cuda").topk(k).indices, dim=1).values.int()
+    q = mk(1, H, T, D).to(dt)
+    kw = dict(pos0=4 * R, window=window, ratio=4, raw_kv=raw if window else None, raw_scales=raw_scales if window else None,
+              kv_scales=scales, scale=D ** -0.5, d_v=Dv, n_comp=R, out_layout="bthd")
+    sinks = mk(H)
+    got = iak.sparse_attention(q, comp, ids[None], sinks, check=True, **kw)
+    want = iak.sparse_attention(q, comp, ids[None], sinks, exact_fp32=True, **kw)
+    # P and its operands are 16-bit (bf16: 2^-9 each), averaged over many rows; the largest |v| is about 4
+    assert max_abs(got, want.cpu().numpy()) <= (2e-3 if kind == "f16" else 2e-2)
