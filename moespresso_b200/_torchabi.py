@@ -47,7 +47,8 @@ def ptr(t) -> int | None:
 
 
 def stream_ptr() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current device's current stream (the raw handle: a ``torch.cuda.Stream`` object per launch is 4 us)."""
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def workspace(nbytes: int, device) -> torch.Tensor | None:

@@ -16,7 +16,7 @@ from .. import _torchabi as _t
 from .._torchabi import ptr, require_cuda, stream_ptr, workspace
 
 
-def topk_select(scores, k: int, *, valid=None, row_start=None, n=None, order: str = "index", digit_hist=None):
+def topk_select(scores, k: int, *, valid=None, row_start=None, n=None, order: str = "index", digit_hist=None, out=None):
     """Ids of the k largest finite scores of every row; ties to the lower id;
     -inf / NaN never selected; -1 in unused slots.
 
@@ -26,7 +26,7 @@ def topk_select(scores, k: int, *, valid=None, row_start=None, n=None, order: st
     attention kernels walk); ``order="score"``: descending score, ties by ascending id
     (the order of the NumPy contract).  Returns int32 ``[..., k]``.  ``digit_hist``: int32 ``[rows, 2048]`` as
     ``indexer_scores(..., digit_hist=)`` left it for exactly these scores; the selection skips its first pass and
-    leaves the counters at zero for the next step.
+    leaves the counters at zero for the next step.  ``out``: contiguous int32 ``[rows, k]`` to write the ids to.
     """
     dev = require_cuda(scores)
     if scores.dtype != torch.float32:
@@ -47,7 +47,10 @@ def topk_select(scores, k: int, *, valid=None, row_start=None, n=None, order: st
         rows = lead[0]
         n_ = int(n)
         row_stride = 0
-    out = torch.empty((rows, int(k)), dtype=torch.int32, device=dev)
+    if out is None:
+        out = torch.empty((rows, int(k)), dtype=torch.int32, device=dev)
+    elif out.dtype != torch.int32 or out.device != dev or out.numel() != rows * int(k) or not out.is_contiguous():
+        raise ValueError("out must be a contiguous int32 [rows, k] tensor on the scores' device")
     if rows == 0:
         return out.reshape(*lead, int(k))
     if valid is not None:

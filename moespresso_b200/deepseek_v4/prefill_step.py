@@ -47,7 +47,7 @@ def sparse_prefill_step(q, comp_kv, idx_q, idx_keys, idx_w, *, pos0: int, ratio:
             n = min(chunk, T - t0)
             scores = indexer_scores_tiled_live(iq[:, :, t0:t0 + n], idx_w[None, t0:t0 + n].contiguous(),
                                                idx_keys[None], pos0=pos0 + t0, ratio=ratio, out=buf[:, :n])
-            ids[t0:t0 + n] = topk_select(scores[0, :n], kk)
+            topk_select(scores[0, :n], kk, out=ids[t0:t0 + n])
     out = sparse_attention(q.permute(1, 0, 2)[None], comp_kv, ids[None], sinks, pos0=pos0, window=window,
                            ratio=ratio, raw_kv=None if raw_kv is None else raw_kv[None], raw_start=raw_start,
                            scale=scale, d_v=d_v, n_comp=R, out_layout="bthd")[0]
