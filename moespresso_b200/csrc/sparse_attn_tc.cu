@@ -548,9 +548,13 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
       // later ones travel); a thread owns (slab, group of four rows) pairs; rows without data are fetched from
       // row -1 (zeros).
       uint8_t* rb = smem + (I8 ? (kb0 + (buf) * kb_st) : (ub0 + (buf) * ub_st));
-      if (pt == 0)
+      if (pt == 0) {
+        // a slab's barrier takes this unit's bytes only once it has counted those of the unit before in this buffer: an
+        // arrival on a phase that still waits for bytes would be one too many
+        if (!I8 && v >= 2) ptx::mbar_wait(&mi->s_ready[buf], sphase(v - 2), abort_flag);
         for (int sl = 0; sl < nrs; ++sl)
           ptx::mbar_expect_tx(&mi->full[buf][sl], (uint32_t)((I8 && sl == L.n128) ? WS_UNIT * 64 : WS_SLAB));
+      }
       // (One TMA operation per instruction, a lane at a time, was measured three times slower: the operations of
       // one warp-wide instruction pipeline, separate instructions of a warp do not.)
       for (int i = pt; i < 16 * nrs; i += NG * 32) {
