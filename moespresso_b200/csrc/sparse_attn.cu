@@ -384,8 +384,9 @@ __global__ void __launch_bounds__(256) merge_kernel(MergeParams p) {
   }
 }
 
-// Many splits of few rows (a decode token split 128 ways): one CTA per row, the splits spread over the CTA so that a
-// thread's chain of dependent loads is P / lanes long instead of P.  Weights exp(m_s - m) are computed once into
+// Many splits of few rows (a decode token split 128 ways): a few CTAs per row (gridDim.y slices of its
+// features; 16 rows alone would leave nine SMs in ten idle), the splits spread over the CTA so that a thread's chain of
+// dependent loads is P / lanes long instead of P.  Weights exp(m_s - m) are computed once into
 // shared memory; thread (lane, vec) sums the splits lane, lane + L, ... in ascending order and the L partial sums
 // are added in lane order: the same order on every run.
 constexpr int kMergeRowsMaxP = 1024;
@@ -428,8 +429,8 @@ __global__ void __launch_bounds__(256) merge_rows_kernel(MergeParams p) {
   }
   float l = red[0];
   if (m > -INFINITY && sink > -INFINITY) l += expf(sink - m);
-  // features: nvec = Dv / 4 vectors, L = 256 / nvec lanes of splits
-  const int nvec = p.Dv / 4, L = 256 / nvec;
+  // features: this slice's nvec vectors from vec0 on, L = 256 / nvec lanes of splits
+  const int nvec = p.Dv / 4 / (int)gridDim.y, L = 256 / nvec, vec0 = (int)blockIdx.y * nvec;
   const int vec = tid % nvec, lane = tid / nvec;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   if (lane < L) {
@@ -439,7 +440,7 @@ __global__ void __launch_bounds__(256) merge_rows_kernel(MergeParams p) {
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
         const int s = s0 + u * L;
-        v[u] = s < p.P ? __ldg(reinterpret_cast<const float4*>(p.o_parts + ((int64_t)s * N + n) * p.Dv) + vec)
+        v[u] = s < p.P ? __ldg(reinterpret_cast<const float4*>(p.o_parts + ((int64_t)s * N + n) * p.Dv) + vec0 + vec)
                        : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
@@ -459,7 +460,7 @@ __global__ void __launch_bounds__(256) merge_rows_kernel(MergeParams p) {
       const float4 x = part[q * nvec + tid];
       r.x += x.x; r.y += x.y; r.z += x.z; r.w += x.w;
     }
-    const int64_t ob = (int64_t)b * p.o_sb + (int64_t)h * p.o_sh + (int64_t)t * p.o_st + 4 * tid;
+    const int64_t ob = (int64_t)b * p.o_sb + (int64_t)h * p.o_sh + (int64_t)t * p.o_st + 4 * (vec0 + tid);
     const float inv = (p.finalize ? (l > 0.f ? 1.f / l : 0.f) : 1.f);
     const float o4[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
@@ -467,7 +468,7 @@ __global__ void __launch_bounds__(256) merge_rows_kernel(MergeParams p) {
       if (p.finalize) store_elem<OT>(p.out, ob + j, o4[j] * inv);
       else reinterpret_cast<float*>(p.out)[ob + j] = o4[j];
     }
-    if (!p.finalize && tid == 0) {
+    if (!p.finalize && tid == 0 && blockIdx.y == 0) {
       p.out_ml[n * 2 + 0] = m;
       p.out_ml[n * 2 + 1] = l;
     }
@@ -481,9 +482,10 @@ static int launch_merge(const MergeParams& mp, int out_dtype, cudaStream_t st) {
   const int64_t items = N * (vec ? mp.Dv / 4 : mp.Dv);
   // few rows, many splits: spread the splits over a CTA per row instead of one thread walking them all
   if (vec && mp.P > 16 && mp.P <= kMergeRowsMaxP && mp.Dv / 4 <= 256 && 256 % (mp.Dv / 4) == 0 && items < 148 * 2 * 256) {
-    if (out_dtype == MXB_F32) merge_rows_kernel<MXB_F32><<<(unsigned)N, 256, 0, st>>>(mp);
-    else if (out_dtype == MXB_BF16) merge_rows_kernel<MXB_BF16><<<(unsigned)N, 256, 0, st>>>(mp);
-    else merge_rows_kernel<MXB_F16><<<(unsigned)N, 256, 0, st>>>(mp);
+    const dim3 rows((unsigned)N, mp.Dv >= 64 && 4 * N <= sm_count() ? 4u : 1u);
+    if (out_dtype == MXB_F32) merge_rows_kernel<MXB_F32><<<rows, 256, 0, st>>>(mp);
+    else if (out_dtype == MXB_BF16) merge_rows_kernel<MXB_BF16><<<rows, 256, 0, st>>>(mp);
+    else merge_rows_kernel<MXB_F16><<<rows, 256, 0, st>>>(mp);
     note_launch();
     MXB_CUDA_OK(cudaGetLastError());
     return MXB_OK;

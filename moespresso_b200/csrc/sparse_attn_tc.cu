@@ -138,6 +138,8 @@ struct WsMisc {
   uint64_t full[2][WS_MAX_SLABS];  // a slab of the unit in row buffer b has landed
   uint64_t v_full[4];              // int8 tables: a 128-feature block of the value buffer has been widened
   uint64_t k_free[2];              // int8 tables: the widening warps have read row buffer b
+  uint64_t tok_ready[2], tok_free[2];   // TOKENS: a token's list has been scanned; its slot may be reused
+  int tok_units[2], tok_keff[2];
   uint64_t meta_ready;             // int8 tables: the scales of units 0 and 1 have been published
   uint64_t s_ready[2], s_free[2], p_ready[2];
   uint64_t p_summed;               // int8 tables: the widening warps have added a unit's P^T to the row sums
@@ -229,12 +231,21 @@ __device__ __forceinline__ bool __syncthreads_or_256(bool pred) {
   return r != 0;
 }
 
-template <int KVT, int QT, int OT>
+// TOKENS: the CTA works through the tokens blockIdx.x, + gridDim.x, ... of the launch (16-bit tables, one split, final
+// output, q by TMA).  What a token costs beyond its units (list scan and first gathers ~10 K cycles, output ~10 K) then
+// overlaps its neighbours' units: the gather warps scan the next token's list and fetch its first units while the
+// softmax warps finish and write the last one (4,096 tokens x 2,048 bf16 rows: 2,599 us as 28 one-wave launches, 2,375 so;
+// 296 tokens of up to 640 rows: 77 -> 71).  Units are counted through (`ub` + u), so that buffers, phases and
+// the metadata ring run on across tokens; the gather warps announce every token's number of units (tok_ready), its
+// readers give the slot back, the softmax warps behind the output (tok_free); the first logit issuer fetches q as soon
+// as the last logit MMA of the token before has read its own.
+template <int KVT, int QT, int OT, bool TOKENS = false>
 __global__ void __launch_bounds__(WS_THREADS, 1)
 sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_comp,
                       const __grid_constant__ CUtensorMap tm_raw, const __grid_constant__ CUtensorMap tm_comp_tail,
                       const __grid_constant__ CUtensorMap tm_raw_tail, const __grid_constant__ CUtensorMap tm_q) {
   constexpr bool I8 = (KVT == MXB_I8);
+  static_assert(!TOKENS || !I8, "int8 tables take one token per CTA");
   constexpr bool BF16 = (KVT == MXB_BF16);       // type of the 16-bit operands: bf16 for bf16 tables, fp16 otherwise
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -249,9 +260,10 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned cta = blockIdx.x + (unsigned)p.cta_base;
-  const int bt = (int)(cta / (unsigned)p.nsplit);
+  int bt = (int)(cta / (unsigned)p.nsplit);
   const int split = (int)(cta - (unsigned)bt * (unsigned)p.nsplit);
-  const int b = bt / p.T, t = bt % p.T;
+  const int bt_end = TOKENS ? p.cta_base + p.n_tok : bt + 1;
+  int b = bt / p.T, t = bt % p.T;
   const int nslab = L.nslab;
   const int n_mt = p.Dv / 128;
   // Row buffers and S^T alternate with the unit's parity.  The value operand (and P^T) of a unit: 16-bit tables
@@ -275,30 +287,38 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
     else wait_pv_all(u);
   };
 
-  const int64_t pos_b = p.pos0_dev ? p.pos0_dev[b] : p.pos0;
-  const int64_t qpos = pos_b + t;
-  const int64_t last_pos = pos_b + p.T - 1;
-  const int64_t count = p.comp_row_count ? (int64_t)p.comp_row_count[b] : p.n_comp;
-  const int64_t cbase = p.comp_row_start ? p.comp_row_start[b] : (int64_t)b * p.n_comp;
-  int64_t visible = count;
-  if (p.ratio > 0) {
-    visible = (qpos + 1) / p.ratio;
-    if (visible > count) visible = count;
-  }
-  int64_t first_raw_pos = 0, first = 0;
-  int n_raw = 0;
-  if (p.raw_cap > 0) {
-    first_raw_pos = last_pos + 1 - p.raw_cap;
-    const int64_t window_first = (p.window != 0 && qpos + 1 > p.window) ? qpos + 1 - p.window : 0;
-    first = first_raw_pos > window_first ? first_raw_pos : window_first;
-    if (first < 0) first = 0;
-    const int64_t last = qpos < last_pos ? qpos : last_pos;
-    n_raw = last >= first ? (int)(last - first + 1) : 0;
-  }
-  // The list of entries: raw rows, padding up to a multiple of four (a TMA gather fetches four rows of ONE
-  // table), then the selected compressed rows.
-  const int n_raw_pad = (n_raw + 3) & ~3;
-  const int32_t* ids = p.topk + (int64_t)bt * p.k;
+  // what token (b, t) sees
+  int64_t visible, cbase, first_raw_pos, first;
+  int n_raw, n_raw_pad;
+  const int32_t* ids;
+  auto look_at_token = [&]() {
+    const int64_t pos_b = p.pos0_dev ? p.pos0_dev[b] : p.pos0;
+    const int64_t qpos = pos_b + t;
+    const int64_t last_pos = pos_b + p.T - 1;
+    const int64_t count = p.comp_row_count ? (int64_t)p.comp_row_count[b] : p.n_comp;
+    cbase = p.comp_row_start ? p.comp_row_start[b] : (int64_t)b * p.n_comp;
+    visible = count;
+    if (p.ratio > 0) {
+      visible = (qpos + 1) / p.ratio;
+      if (visible > count) visible = count;
+    }
+    first_raw_pos = 0;
+    first = 0;
+    n_raw = 0;
+    if (p.raw_cap > 0) {
+      first_raw_pos = last_pos + 1 - p.raw_cap;
+      const int64_t window_first = (p.window != 0 && qpos + 1 > p.window) ? qpos + 1 - p.window : 0;
+      first = first_raw_pos > window_first ? first_raw_pos : window_first;
+      if (first < 0) first = 0;
+      const int64_t last = qpos < last_pos ? qpos : last_pos;
+      n_raw = last >= first ? (int)(last - first + 1) : 0;
+    }
+    // The list of entries: raw rows, padding up to a multiple of four (a TMA gather fetches four rows of ONE
+    // table), then the selected compressed rows.
+    n_raw_pad = (n_raw + 3) & ~3;
+    ids = p.topk + (int64_t)bt * p.k;
+  };
+  look_at_token();
 #ifdef MXB_TRACE_SP
   long long* tr = reinterpret_cast<long long*>(p.status);
   const bool tr_on = p.status && blockIdx.x == 0 && (lane == 0);
@@ -320,6 +340,10 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
     ptx::mbar_init(&mi->k_free[1], 4);
     ptx::mbar_init(&mi->meta_ready, (uint32_t)WS_UNIT);
     ptx::mbar_init(&mi->p_summed, 4);
+    for (int i = 0; i < 2; ++i) {
+      ptx::mbar_init(&mi->tok_ready[i], 1);
+      ptx::mbar_init(&mi->tok_free[i], 256u + 2u + (n_mt > 2 ? 2u : 1u));   // softmax threads, logit and value issuers
+    }
     mi->abort_flag = 0;
     mi->keff = p.k;
     ptx::mbar_fence_init();
@@ -354,15 +378,16 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
   // H arrive as zeros): in place as the B operand for 16-bit tables, in a scratch region (the value buffer) for
   // int8 tables, where it is turned into digit planes.  Otherwise q goes through registers.
   uint8_t* q_land = I8 ? smem + (L.qtmp_off >= 0 ? L.qtmp_off : 0) : q_s;
-  if (p.q_tma) {
-    if (tid == 256) {
-      ptx::tma_prefetch_desc(&tm_q);
-      ptx::mbar_expect_tx(&mi->q_full, (uint32_t)(nslab * WS_SLAB));
-      int32_t c[3];
+  auto load_q = [&]() {
+    ptx::mbar_expect_tx(&mi->q_full, (uint32_t)(nslab * WS_SLAB));
+    int32_t c[3];
 #pragma unroll
-      for (int i = 0; i < 3; ++i) c[i] = p.q_axis[i] == 0 ? 0 : (p.q_axis[i] == 1 ? t : b);
-      for (int kb = 0; kb < nslab; ++kb) ptx::tma_load_4d(q_land + kb * WS_SLAB, &tm_q, &mi->q_full, kb * 64, c[0], c[1], c[2]);
-    }
+    for (int i = 0; i < 3; ++i) c[i] = p.q_axis[i] == 0 ? 0 : (p.q_axis[i] == 1 ? t : b);
+    for (int kb = 0; kb < nslab; ++kb) ptx::tma_load_4d(q_land + kb * WS_SLAB, &tm_q, &mi->q_full, kb * 64, c[0], c[1], c[2]);
+  };
+  if (p.q_tma && tid == 256) {
+    ptx::tma_prefetch_desc(&tm_q);
+    if constexpr (!TOKENS) load_q();
   }
   const bool q_vec = ((reinterpret_cast<uintptr_t>(p.q) & 15) == 0) && (p.q_sb % 8 == 0) && (p.q_sh % 8 == 0) &&
                      (p.q_st % 8 == 0);
@@ -395,22 +420,47 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
       }
     }
   };
-  {  // first list entry that ends the walk
+  // first list entry that ends the walk, by `n` threads
+  auto scan_list = [&](int me, int n, int* keff) {
     int mine = p.k;
 #pragma unroll 4
-    for (int j = tid; j < p.k; j += WS_THREADS) {   // no early exit: the loads stay independent
+    for (int j = me; j < p.k; j += n) {   // no early exit: the loads stay independent
       const int64_t v = ids[j];
       if (v >= visible && j < mine) mine = j;
     }
-    if (mine < p.k) atomicMin(&mi->keff, mine);
+    if (mine < p.k) atomicMin(keff, mine);
+  };
+  int e_lo = 0, e_hi = 0, nunits = 0;   // this CTA's entries and units of the token
+  auto cut_list = [&](int keff) {
+    const int total = n_raw_pad + keff;
+    int per = (total + p.nsplit - 1) / p.nsplit;
+    per = ((per + WS_UNIT - 1) / WS_UNIT) * WS_UNIT;
+    e_lo = min(split * per, total);
+    e_hi = min(e_lo + per, total);
+    nunits = (e_hi - e_lo + WS_UNIT - 1) / WS_UNIT;
+  };
+  if constexpr (!TOKENS) {
+    scan_list(tid, WS_THREADS, &mi->keff);
+    __syncthreads();
+    cut_list(mi->keff);
   }
-  __syncthreads();
-
-  const int total = n_raw_pad + mi->keff;
-  int per = (total + p.nsplit - 1) / p.nsplit;
-  per = ((per + WS_UNIT - 1) / WS_UNIT) * WS_UNIT;
-  const int e_lo = min(split * per, total), e_hi = min(e_lo + per, total);
-  const int nunits = (e_hi - e_lo + WS_UNIT - 1) / WS_UNIT;
+  // the next token of this CTA, for a role that only counts its units
+  int ub = 0, it = 0;   // units and tokens before this one
+  auto await_token = [&]() {
+    if constexpr (TOKENS) {
+      ptx::mbar_wait(&mi->tok_ready[it & 1], (uint32_t)((it >> 1) & 1), abort_flag);
+      nunits = mi->tok_units[it & 1];
+      b = bt / p.T;
+      t = bt % p.T;
+    }
+  };
+  auto next_token = [&]() -> bool {
+    if constexpr (!TOKENS) return false;
+    ub += nunits;
+    ++it;
+    bt += (int)gridDim.x;
+    return bt < bt_end;
+  };
   if (tid == 0) TRS(11, 1);
 
   constexpr uint32_t fmt = BF16 ? ptx::kFmtBF16 : ptx::kFmtF16;
@@ -475,6 +525,100 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
     }
   }
 
+  // The softmax warps' output of a token.  Three ways out: one split -> final or external-partial output straight from
+  // TMEM; splits in a cluster -> merged through shared memory further down; otherwise (o, m, l) partials for the merge
+  // kernel.
+  const bool cmerge = !TOKENS && p.cluster_merge != 0;
+  const int n_slots = cmerge ? (n_mt + p.nsplit - 1) / p.nsplit : 0;   // value blocks a CTA merges: mt = rank + slot * nsplit
+  float* recv = reinterpret_cast<float*>(smem);   // cluster merge: [slot][source split][16 head groups][128 features][4 heads]
+  auto emit = [&]() {
+    const int wq = warp & 3, cset = warp >> 2;
+    const uint32_t lane_off = (uint32_t)(wq * 32) << 16;
+    const int64_t N = (int64_t)p.B * p.T * p.H;
+    const bool direct = TOKENS || p.nsplit == 1;
+    const bool finalize = TOKENS || (direct && !p.partial_ml);
+    const bool have_o = nunits > 0;
+    if (tid < WS_HEADS) {
+      // per-head factor applied to O^T: 1 for partial output; otherwise this split's weight over the denominator
+      // of the whole token, exp2(m - m*) / (sum over splits of l exp2(m_s - m*) + sink), the sink joining once
+      float fac = 1.f;
+      if (finalize || cmerge) {
+        const float m = mi->m_ref[tid];
+        const float sink2 = (p.sinks && tid < p.H) ? p.sinks[tid] * 1.4426950408889634f : -INFINITY;
+        float m2v = fmaxf(m, sink2);
+        if (cmerge)
+          for (int r = 0; r < p.nsplit; ++r) m2v = fmaxf(m2v, mi->xm[r][tid]);
+        float w = 0.f, den = 0.f;
+        if (m2v > -INFINITY) {
+          w = (m == -INFINITY) ? 0.f : exp2f(m - m2v);
+          if (cmerge) {
+            for (int r = 0; r < p.nsplit; ++r)   // split order: the same sum in every CTA and on every run
+              if (mi->xm[r][tid] > -INFINITY) den = fmaf(mi->xl[r][tid], exp2f(mi->xm[r][tid] - m2v), den);
+          } else {
+            den = __fmul_rn(mi->l_tot[tid], w);   // (never contracted with the sink: the same bits from every instance)
+          }
+          den += (sink2 == -INFINITY) ? 0.f : exp2f(sink2 - m2v);
+        }
+        fac = den > 0.f ? w / den : 0.f;
+      }
+      mi->factor[tid] = fac;
+    }
+    group_sync(4, 256);
+    // warp -> (lane quarter of TMEM = 32 features, two of the four 128-feature blocks); columns = heads
+    const int64_t gbase = direct ? (int64_t)b * p.o_sb + (int64_t)t * p.o_st : ((int64_t)split * N + (int64_t)bt * p.H) * p.Dv;
+    const int64_t ostep = direct ? p.o_sh : (int64_t)p.Dv;
+    for (int m2 = 0; m2 < 2; ++m2) {
+      const int mt = cset * 2 + m2;
+      if (mt >= n_mt) continue;
+      const int d = mt * 128 + wq * 32 + lane;
+      // cluster merge: block mt belongs to split mt % nsplit; this thread's feature row of it goes there, four
+      // heads per 16-byte store, consecutive features in consecutive lanes
+      const uint32_t owner = (uint32_t)(mt % p.nsplit);
+      const uint32_t dst0 = cmerge ? ptx::cluster_map(ptx::smem_u32(recv) + (uint32_t)((((mt / p.nsplit) * p.nsplit + split) * 16) * 128 + wq * 32 + lane) * 16u, owner) : 0u;
+#pragma unroll 1
+      for (int hh = 0; hh < 2; ++hh) {
+        uint32_t ov[32];
+        if (have_o) {
+          ptx::tmem_ld32(tmem_o + lane_off + (uint32_t)(mt * WS_HEADS + hh * 32), ov);
+          ptx::tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) ov[c] = 0u;
+        }
+        if (cmerge) {
+#pragma unroll
+          for (int c = 0; c < 32; c += 4) {
+            float o4[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int h = hh * 32 + c + e;
+              o4[e] = have_o ? (__uint_as_float(ov[c + e]) - mi->v_bias[h]) * mi->factor[h] : 0.f;
+            }
+            ptx::st_cluster_v4(dst0 + (uint32_t)((hh * 8 + (c >> 2)) * 128) * 16u, o4[0], o4[1], o4[2], o4[3]);
+          }
+          continue;
+        }
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+          const int h = hh * 32 + c;
+          if (h >= p.H) continue;
+          const float o = (__uint_as_float(ov[c]) - mi->v_bias[h]) * mi->factor[h];
+          if (finalize) store_elem<OT>(p.out, gbase + d + h * ostep, o);
+          else if (direct) reinterpret_cast<float*>(p.out)[gbase + d + h * ostep] = o;
+          else p.ws_o[gbase + d + h * ostep] = o;
+        }
+      }
+    }
+    if (!cmerge && tid < p.H && (!direct || p.partial_ml)) {
+      // (m, l) in natural-log units for the merge kernel
+      const float m_nat = mi->m_ref[tid] == -INFINITY ? -INFINITY : mi->m_ref[tid] * 0.6931471805599453f;
+      float* ml = direct ? p.partial_ml + ((int64_t)bt * p.H + tid) * 2
+                         : p.ws_ml + ((int64_t)split * N + (int64_t)bt * p.H + tid) * 2;
+      ml[0] = m_nat;
+      ml[1] = mi->l_tot[tid];
+    }
+  };
+
   constexpr int NG = I8 ? 4 : 8;   // gather warps (int8 tables: the other four producer warps widen the values)
   if (warp >= 12 && warp < 12 + NG) {
     // ================================================================ row gathers
@@ -513,84 +657,102 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
       if (I8) rs = fmaxf(__half2float(raw ? p.raw_scales[ridx] : p.comp_scales[ridx]), 5.9604645e-8f);
     };
     auto publish_ref = [&](int U, uint32_t ref) {
-      if (resolver && U < nunits) mi->row_ref[U & (kRing - 1)][pt] = ref;
+      if (resolver && U < nunits) mi->row_ref[(ub + U) & (kRing - 1)][pt] = ref;
     };
     auto publish_scale = [&](int U, float rs) {
       if (I8 && resolver && U < nunits) mi->row_scale[U & (kRing - 1)][pt] = rs;
     };
-    int32_t id_a = -1;          // stage A result: list id of this thread's entry of unit v + 3
-    uint32_t src_b = kNoRow;    // stage B result: row and scale of this thread's entry of unit v + 2
-    float rs_b = 1.f;
-    float rs0 = 1.f, rs1 = 1.f;   // scales of units 0 and 1: published behind the first gathers
-    if (pt == 0) TRS(14, 0);
-    if (nunits > 0) {
-      const int32_t i0 = fetch_id(0), i1 = fetch_id(1), i2 = fetch_id(2);
-      id_a = fetch_id(3);
-      uint32_t s0, s1;
-      fetch_row(0, i0, s0, rs0);
-      fetch_row(1, i1, s1, rs1);
-      fetch_row(2, i2, src_b, rs_b);
-      publish_ref(0, s0);
-      publish_ref(1, s1);
-    }
-    group_sync(5, NG * 32);
-    if (pt == 0) TRS(14, 3);
-    for (int v = 0; v < nunits; ++v) {
-      const int buf = v & 1, slot = v & (kRing - 1);
-      if (pt == 0) TRS(0, v);
-      if (I8 && v >= 2) {
-        // row buffer `buf` is free once the widening warps and the logit MMAs of unit v - 2 have read it
-        ptx::mbar_wait(&mi->k_free[buf], sphase(v - 2), abort_flag);
-        ptx::mbar_wait(&mi->s_ready[buf], sphase(v - 2), abort_flag);
-      }
-      if (pt == 0) TRS(1, v);
-      // Unit v into row buffer v & 1, slab by slab (so that the logit MMAs of the first slabs can start while the
-      // later ones travel); a thread owns (slab, group of four rows) pairs; rows without data are fetched from
-      // row -1 (zeros).
-      uint8_t* rb = smem + (I8 ? (kb0 + (buf) * kb_st) : (ub0 + (buf) * ub_st));
-      if (pt == 0) {
-        // a slab's barrier takes this unit's bytes only once it has counted those of the unit before in this buffer: an
-        // arrival on a phase that still waits for bytes would be one too many
-        if (!I8 && v >= 2) ptx::mbar_wait(&mi->s_ready[buf], sphase(v - 2), abort_flag);
-        for (int sl = 0; sl < nrs; ++sl)
-          ptx::mbar_expect_tx(&mi->full[buf][sl], (uint32_t)((I8 && sl == L.n128) ? WS_UNIT * 64 : WS_SLAB));
-      }
-      // (One TMA operation per instruction, a lane at a time, was measured three times slower: the operations of
-      // one warp-wide instruction pipeline, separate instructions of a warp do not.)
-      for (int i = pt; i < 16 * nrs; i += NG * 32) {
-        const int sl = i >> 4, r0 = (i & 15) * 4;
-        if (!I8 && v >= 2) wait_pv_slab(v - 2, sl);   // this slab has been multiplied by P V of unit v - 2
-        uint32_t ref[4];
-        bool from_raw = false;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          ref[j] = mi->row_ref[slot][r0 + j];
-          if (ref[j] != kNoRow && (ref[j] >> 31)) from_raw = true;
+    do {
+      if constexpr (TOKENS) {
+        const int ts = it & 1;
+        b = bt / p.T;
+        t = bt % p.T;
+        look_at_token();
+        if (it >= 2) ptx::mbar_wait(&mi->tok_free[ts], (uint32_t)(((it >> 1) - 1) & 1), abort_flag);
+        if (pt == 0) mi->tok_keff[ts] = p.k;
+        group_sync(5, NG * 32);
+        scan_list(pt, NG * 32, &mi->tok_keff[ts]);
+        group_sync(5, NG * 32);
+        cut_list(mi->tok_keff[ts]);
+        if (pt == 0) {
+          mi->tok_units[ts] = nunits;
+          ptx::mbar_arrive(&mi->tok_ready[ts]);
         }
-        int32_t y[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) y[j] = ref[j] != kNoRow ? (int32_t)(ref[j] & 0x7FFFFFFFu) : -1;
-        if (I8 && sl == L.n128)
-          ptx::tma_gather4_2d(rb + (size_t)sl * WS_SLAB + (size_t)r0 * 64, from_raw ? &tm_raw_tail : &tm_comp_tail,
-                              &mi->full[buf][sl], sl * 128, y[0], y[1], y[2], y[3]);
-        else
-          ptx::tma_gather4_2d(rb + (size_t)sl * WS_SLAB + (size_t)r0 * 128, from_raw ? &tm_raw : &tm_comp,
-                              &mi->full[buf][sl], I8 ? sl * 128 : sl * 64, y[0], y[1], y[2], y[3]);
       }
-      if (pt == 0) TRS(2, v);
-      if (I8 && v == 0 && resolver) {
-        publish_scale(0, rs0);
-        publish_scale(1, rs1);
-        ptx::mbar_arrive(&mi->meta_ready);
+      int32_t id_a = -1;          // stage A result: list id of this thread's entry of unit v + 3
+      uint32_t src_b = kNoRow;    // stage B result: row and scale of this thread's entry of unit v + 2
+      float rs_b = 1.f;
+      float rs0 = 1.f, rs1 = 1.f;   // scales of units 0 and 1: published behind the first gathers
+      if (pt == 0) TRS(14, 0);
+      if (nunits > 0) {
+        const int32_t i0 = fetch_id(0), i1 = fetch_id(1), i2 = fetch_id(2);
+        id_a = fetch_id(3);
+        uint32_t s0, s1;
+        fetch_row(0, i0, s0, rs0);
+        fetch_row(1, i1, s1, rs1);
+        fetch_row(2, i2, src_b, rs_b);
+        publish_ref(0, s0);
+        publish_ref(1, s1);
       }
-      // a metadata slot is rewritten six units after its unit: that unit's softmax is long over, because the
-      // buffer wait above implies that the softmax of unit v - 4 has started
-      publish_ref(v + 2, src_b);
-      publish_scale(v + 2, rs_b);
-      fetch_row(v + 3, id_a, src_b, rs_b);
-      id_a = fetch_id(v + 4);
       group_sync(5, NG * 32);
-    }
+      if (pt == 0) TRS(14, 3);
+      for (int v = 0; v < nunits; ++v) {
+        const int buf = (ub + v) & 1, slot = (ub + v) & (kRing - 1);
+        if (pt == 0) TRS(0, v);
+        if (I8 && v >= 2) {
+          // row buffer `buf` is free once the widening warps and the logit MMAs of unit v - 2 have read it
+          ptx::mbar_wait(&mi->k_free[buf], sphase(v - 2), abort_flag);
+          ptx::mbar_wait(&mi->s_ready[buf], sphase(v - 2), abort_flag);
+        }
+        if (pt == 0) TRS(1, v);
+        // Unit v into row buffer v & 1, slab by slab (so that the logit MMAs of the first slabs can start while the
+        // later ones travel); a thread owns (slab, group of four rows) pairs; rows without data are fetched from
+        // row -1 (zeros).
+        uint8_t* rb = smem + (I8 ? (kb0 + (buf) * kb_st) : (ub0 + (buf) * ub_st));
+        if (pt == 0) {
+          // a slab's barrier takes the next unit's bytes only once it has counted those of the unit before in this buffer:
+          // an arrival on a phase that still waits for bytes would be one too many
+          if (!I8 && ub + v >= 2) ptx::mbar_wait(&mi->s_ready[buf], sphase(ub + v - 2), abort_flag);
+          for (int sl = 0; sl < nrs; ++sl)
+            ptx::mbar_expect_tx(&mi->full[buf][sl], (uint32_t)((I8 && sl == L.n128) ? WS_UNIT * 64 : WS_SLAB));
+        }
+        // (One TMA operation per instruction, a lane at a time, was measured three times slower: the operations of
+        // one warp-wide instruction pipeline, separate instructions of a warp do not.)
+        for (int i = pt; i < 16 * nrs; i += NG * 32) {
+          const int sl = i >> 4, r0 = (i & 15) * 4;
+          if (!I8 && ub + v >= 2) wait_pv_slab(ub + v - 2, sl);   // this slab has been multiplied by P V of unit v - 2
+          uint32_t ref[4];
+          bool from_raw = false;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            ref[j] = mi->row_ref[slot][r0 + j];
+            if (ref[j] != kNoRow && (ref[j] >> 31)) from_raw = true;
+          }
+          int32_t y[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) y[j] = ref[j] != kNoRow ? (int32_t)(ref[j] & 0x7FFFFFFFu) : -1;
+          if (I8 && sl == L.n128)
+            ptx::tma_gather4_2d(rb + (size_t)sl * WS_SLAB + (size_t)r0 * 64, from_raw ? &tm_raw_tail : &tm_comp_tail,
+                                &mi->full[buf][sl], sl * 128, y[0], y[1], y[2], y[3]);
+          else
+            ptx::tma_gather4_2d(rb + (size_t)sl * WS_SLAB + (size_t)r0 * 128, from_raw ? &tm_raw : &tm_comp,
+                                &mi->full[buf][sl], I8 ? sl * 128 : sl * 64, y[0], y[1], y[2], y[3]);
+        }
+        if (pt == 0) TRS(2, v);
+        if (I8 && v == 0 && resolver) {
+          publish_scale(0, rs0);
+          publish_scale(1, rs1);
+          ptx::mbar_arrive(&mi->meta_ready);
+        }
+        // a metadata slot is rewritten six units after its unit: that unit's softmax is long over, because the
+        // buffer wait above implies that the softmax of unit v - 4 has started
+        publish_ref(v + 2, src_b);
+        publish_scale(v + 2, rs_b);
+        fetch_row(v + 3, id_a, src_b, rs_b);
+        id_a = fetch_id(v + 4);
+        group_sync(5, NG * 32);
+      }
+    } while (next_token());
   } else if (warp >= 12 + NG) {
     // ================================================================ widening (warps 16-19, int8 tables)
     // The int8 rows land in operand layout and feed the logit MMAs as they are; only the values need 16-bit
@@ -695,7 +857,7 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
     // ================================================================ S^T = Kunit . Q^T issuers
     if (lane == 0) {
       const int j = warp - 8;
-      ptx::mbar_wait(&mi->q_ready, 0, abort_flag);   // also when there is no unit: q has landed before the CTA exits
+      if constexpr (!TOKENS) ptx::mbar_wait(&mi->q_ready, 0, abort_flag);   // also when there is no unit: q has landed before the CTA exits
       if constexpr (I8) {
         // int8 x int8 -> int32, K = 32 per instruction, N = 128 = the hi and lo planes of q.  Issuer j takes the
         // units of parity j, whole.
@@ -725,23 +887,36 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
         const int kb_lo = slab_lo(j), kb_hi = slab_lo(j + 1);
         const uint32_t idesc_s = ptx::idesc_f16(fmt, fmt, WS_UNIT, WS_HEADS, 0, 0);
         const uint64_t q_desc = ptx::smem_desc_sw128(ptx::smem_u32(q_s), 16, 1024);
-        for (int u = 0; u < nunits; ++u) {
-          const int buf = sbuf(u);
-          const uint64_t k_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + (ub0 + (buf) * ub_st)), 16, 1024);
-          const uint32_t d = tmem_base + (uint32_t)(buf * 128 + j * WS_HEADS);
-          if (u >= 2) ptx::mbar_wait(&mi->s_free[buf], sphase(u - 2), abort_flag);   // S^T(u - 2) has been read
-          for (int kb = kb_lo; kb < kb_hi; ++kb) {
-            ptx::mbar_wait(&mi->full[buf][kb], sphase(u), abort_flag);   // each slab as soon as it has landed
-            ptx::tc_fence_after_sync();
-            if (kb == kb_lo && j == 0) TRS(3, u);
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks)
-              ptx::mma_f16_ss(d, ptx::desc_advance(k_desc, kb * WS_SLAB + ks * 32),
-                              ptx::desc_advance(q_desc, kb * WS_SLAB + ks * 32), idesc_s, (kb > kb_lo || ks) ? 1u : 0u);
+        uint32_t q_phase = 0;
+        do {
+          await_token();
+          if constexpr (TOKENS) ptx::mbar_arrive(&mi->tok_free[it & 1]);   // (the number of units is all that is read of it)
+          if (TOKENS && nunits > 0) {
+            if (j == 0) {
+              if (ub > 0) ptx::mbar_wait(&mi->s_ready[sbuf(ub - 1)], sphase(ub - 1), abort_flag);   // nothing reads the last q any more
+              load_q();
+            }
+            ptx::mbar_wait(&mi->q_full, q_phase, abort_flag);
+            q_phase ^= 1u;
           }
-          ptx::mma_commit(&mi->s_ready[buf]);
-          if (j == 0) TRS(4, u);
-        }
+          for (int u = ub; u < ub + nunits; ++u) {
+            const int buf = sbuf(u);
+            const uint64_t k_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + (ub0 + (buf) * ub_st)), 16, 1024);
+            const uint32_t d = tmem_base + (uint32_t)(buf * 128 + j * WS_HEADS);
+            if (u >= 2) ptx::mbar_wait(&mi->s_free[buf], sphase(u - 2), abort_flag);   // S^T(u - 2) has been read
+            for (int kb = kb_lo; kb < kb_hi; ++kb) {
+              ptx::mbar_wait(&mi->full[buf][kb], sphase(u), abort_flag);   // each slab as soon as it has landed
+              ptx::tc_fence_after_sync();
+              if (kb == kb_lo && j == 0) TRS(3, u);
+#pragma unroll
+              for (int ks = 0; ks < 4; ++ks)
+                ptx::mma_f16_ss(d, ptx::desc_advance(k_desc, kb * WS_SLAB + ks * 32),
+                                ptx::desc_advance(q_desc, kb * WS_SLAB + ks * 32), idesc_s, (kb > kb_lo || ks) ? 1u : 0u);
+            }
+            ptx::mma_commit(&mi->s_ready[buf]);
+            if (j == 0) TRS(4, u);
+          }
+        } while (next_token());
       }
     }
   } else if (warp == 10 || warp == 11) {
@@ -749,27 +924,31 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
     const int mt0 = (warp - 10) * 2;
     if (lane == 0 && mt0 < n_mt) {
       const uint32_t idesc_o = ptx::idesc_f16(fmt, fmt, 128, WS_HEADS, 1, 0);   // A read MN-major
-      for (int u = 0; u < nunits; ++u) {
-        const int buf = pbuf(u);
-        // A, MN-major: 64-feature blocks 8 KB apart (LBO), 8-row groups 1 KB apart (SBO); 16 rows per K step
-        const uint64_t v_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + (ub0 + (buf) * ub_st)), WS_SLAB, 1024);
-        const uint64_t pt_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + (pt0 + (buf) * pt_st)), 16, 1024);
-        ptx::mbar_wait(&mi->p_ready[buf], pphase(u), abort_flag);
-        ptx::tc_fence_after_sync();
-        if (warp == 10) TRS(9, u);
-        for (int mt = mt0; mt < mt0 + 2 && mt < n_mt; ++mt) {
-          if (I8) {
-            ptx::mbar_wait(&mi->v_full[mt], (uint32_t)(u & 1), abort_flag);   // this block has been widened
-            ptx::tc_fence_after_sync();
-          }
+      do {
+        await_token();
+        if constexpr (TOKENS) ptx::mbar_arrive(&mi->tok_free[it & 1]);
+        for (int u = ub; u < ub + nunits; ++u) {
+          const int buf = pbuf(u);
+          // A, MN-major: 64-feature blocks 8 KB apart (LBO), 8-row groups 1 KB apart (SBO); 16 rows per K step
+          const uint64_t v_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + (ub0 + (buf) * ub_st)), WS_SLAB, 1024);
+          const uint64_t pt_desc = ptx::smem_desc_sw128(ptx::smem_u32(smem + (pt0 + (buf) * pt_st)), 16, 1024);
+          ptx::mbar_wait(&mi->p_ready[buf], pphase(u), abort_flag);
+          ptx::tc_fence_after_sync();
+          if (warp == 10) TRS(9, u);
+          for (int mt = mt0; mt < mt0 + 2 && mt < n_mt; ++mt) {
+            if (I8) {
+              ptx::mbar_wait(&mi->v_full[mt], (uint32_t)(u & 1), abort_flag);   // this block has been widened
+              ptx::tc_fence_after_sync();
+            }
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            ptx::mma_f16_ss(tmem_o + (uint32_t)(mt * WS_HEADS), ptx::desc_advance(v_desc, (2 * mt) * WS_SLAB + ks * 2048),
-                            ptx::desc_advance(pt_desc, ks * 32), idesc_o, (u > 0 || ks > 0) ? 1u : 0u);
-          ptx::mma_commit(&mi->pv_blk[buf][mt]);
+            for (int ks = 0; ks < 4; ++ks)
+              ptx::mma_f16_ss(tmem_o + (uint32_t)(mt * WS_HEADS), ptx::desc_advance(v_desc, (2 * mt) * WS_SLAB + ks * 2048),
+                              ptx::desc_advance(pt_desc, ks * 32), idesc_o, (u > ub || ks > 0) ? 1u : 0u);
+            ptx::mma_commit(&mi->pv_blk[buf][mt]);
+          }
+          if (warp == 10) TRS(10, u);
         }
-        if (warp == 10) TRS(10, u);
-      }
+      } while (next_token());
     }
   } else {
     // ================================================================ softmax (warps 0-7), one unit at a time
@@ -783,7 +962,9 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
     const uint32_t lane_off = (uint32_t)(wq * 32) << 16;
 
     // ---- q: finish the operand
-    if (p.q_tma) ptx::mbar_wait(&mi->q_full, 0, abort_flag);
+    if (TOKENS) {
+      // (by TMA in place; the logit issuers wait for it)
+    } else if (p.q_tma) ptx::mbar_wait(&mi->q_full, 0, abort_flag);
     if constexpr (I8) {
       // the digit planes were written before the roles parted
     } else if (!p.q_tma) {
@@ -802,7 +983,8 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
             make_uint4(w[0], w[1], w[2], w[3]);
       }
     }
-    if constexpr (!I8) {
+    if constexpr (TOKENS) {
+    } else if constexpr (!I8) {
       ptx::fence_proxy_async_smem();
       ptx::mbar_arrive(&mi->q_ready);
     } else {
@@ -811,290 +993,212 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
 
     // 16-bit tables: l1 = the sum of the softmax weights of head col0 + li over this warp's rows of all units (the
     // denominator).  Int8 tables: the widening warps keep both sums (see add_unit).
-    float l1 = 0.f;
-    for (int u = 0; u < nunits; ++u) {
-      const int sb_i = sbuf(u), pb_i = pbuf(u), slot = u & (kRing - 1);
-      ptx::mbar_wait(&mi->s_ready[sb_i], sphase(u), abort_flag);
-      ptx::tc_fence_after_sync();
-      if (warp == 0) TRS(5, u);
-      uint32_t sv[16];
-      {
-        // two accumulators per unit: the halves of the feature slabs (16-bit tables), or the digit planes of q
-        const uint32_t sa = tmem_base + lane_off + (uint32_t)(sb_i * 128 + cset * 32);
-        uint32_t sb[16];
-        ptx::tmem_ld_16x32bx2_x16(sa, sv);
-        ptx::tmem_ld_16x32bx2_x16(sa + (uint32_t)WS_HEADS, sb);
-        ptx::tmem_ld_wait();
-#pragma unroll
-        for (int c = 0; c < 16; c += 4) {
-          if constexpr (I8) {
-            const float4 qs = *reinterpret_cast<const float4*>(&mi->q_step[col0 + c]);   // the heads' fixed-point steps
-            sv[c] = __float_as_uint(fmaf((float)(int)sv[c], 256.f, (float)(int)sb[c]) * qs.x);
-            sv[c + 1] = __float_as_uint(fmaf((float)(int)sv[c + 1], 256.f, (float)(int)sb[c + 1]) * qs.y);
-            sv[c + 2] = __float_as_uint(fmaf((float)(int)sv[c + 2], 256.f, (float)(int)sb[c + 2]) * qs.z);
-            sv[c + 3] = __float_as_uint(fmaf((float)(int)sv[c + 3], 256.f, (float)(int)sb[c + 3]) * qs.w);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) sv[c + e] = __float_as_uint(__uint_as_float(sv[c + e]) + __uint_as_float(sb[c + e]));
-          }
-        }
-      }
-      ptx::tc_fence_before_sync();
-      ptx::mbar_arrive(&mi->s_free[sb_i]);
-      if (I8 && u == 0) ptx::mbar_wait(&mi->meta_ready, 0, abort_flag);   // the first scales are published behind the gathers
-      const bool ok = mi->row_ref[slot][row] != kNoRow;
-      const float rs = I8 ? mi->row_scale[slot][row] : 1.f;
-      const float mul = scale_log2 * rs;
-      // Int8 tables: the operand weight of a row is its softmax weight times the row's dequantisation scale, and
-      // that product is what has to fit fp16.  So the references follow the maxima of logit + log2(scale): the
-      // largest operand weight of a head is 1 (2^-headroom) when its reference moves, whatever the scales are.
-      const float lrs = (I8 && ok) ? log2f(rs) : 0.f;
-      const float gap = BF16 ? kRescaleGapBF16 : kRescaleGapF16;
-      bool grow = false;
-#pragma unroll
-      for (int c = 0; c < 16; c += 4) {
-        const float4 mr = *reinterpret_cast<const float4*>(&mi->m_ref[col0 + c]);   // the heads' reference maxima
-        const float mrv[4] = {mr.x, mr.y, mr.z, mr.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float x = ok ? fmaf(__uint_as_float(sv[c + e]), mul, lrs) : -INFINITY;
-          sv[c + e] = __float_as_uint(x);
-          grow |= x > mrv[e] + gap;
-        }
-      }
-      if (warp == 0) TRS(6, u);
-      bool grown = false;
-      if (__syncthreads_or_256(grow)) {
-        // exact column maxima of this unit (xor shuffles of 8, 4, 2, 1 stay inside a half warp = one head range)
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          int o = float_order(__uint_as_float(sv[c]));
-          o = max(o, __shfl_xor_sync(0xffffffffu, o, 8));
-          o = max(o, __shfl_xor_sync(0xffffffffu, o, 4));
-          o = max(o, __shfl_xor_sync(0xffffffffu, o, 2));
-          o = max(o, __shfl_xor_sync(0xffffffffu, o, 1));
-          if (li == c) mi->colmax[wq][col0 + c] = order_float(o);
-        }
-        // O^T belongs to the old reference: it is final for the units so far once the previous P V is done (and
-        // the row sums have taken the previous factor, if any, before this one replaces it)
-        if (warp == 0) TRS(29, u);
-        if (u >= 1) wait_pv_all(u - 1);
-        if (I8 && u >= 1) ptx::mbar_wait(&mi->p_summed, (uint32_t)((u - 1) & 1), abort_flag);
-        if (warp == 0) TRS(30, u);
+    do {
+      await_token();
+      float l1 = 0.f;
+      if (TOKENS && it > 0) {
+        group_sync(4, 256);   // the last token's output has been written
+        if (tid < WS_HEADS) mi->m_ref[tid] = -INFINITY;
         group_sync(4, 256);
-        if (tid < WS_HEADS) {
-          const float old = mi->m_ref[tid];
-          float mx = fmaxf(fmaxf(mi->colmax[0][tid], mi->colmax[1][tid]), fmaxf(mi->colmax[2][tid], mi->colmax[3][tid]));
-          mx = mx > old ? mx + (BF16 ? 0.f : kRescaleHeadroom) : old;
-          mi->factor[tid] = (old == -INFINITY) ? 0.f : exp2f(old - mx);
-          mi->m_ref[tid] = mx;
-        }
-        group_sync(4, 256);
+      }
+      for (int u = ub; u < ub + nunits; ++u) {
+        const int sb_i = sbuf(u), pb_i = pbuf(u), slot = u & (kRing - 1);
+        ptx::mbar_wait(&mi->s_ready[sb_i], sphase(u), abort_flag);
         ptx::tc_fence_after_sync();
-        if constexpr (!I8) l1 *= mi->factor[col0 + li];
-        grown = true;
-        if (u >= 1) {
-          // warp -> (lane quarter of TMEM = 32 features, two of the four 128-feature blocks); columns = heads
-          for (int m2 = 0; m2 < 2; ++m2) {
-            const int mt = cset * 2 + m2;
-            if (mt < n_mt) {
-#pragma unroll 1
-              for (int hh = 0; hh < 2; ++hh) {
-                uint32_t ov[32];
-                const uint32_t ta = tmem_o + lane_off + (uint32_t)(mt * WS_HEADS + hh * 32);
-                ptx::tmem_ld32(ta, ov);
-                ptx::tmem_ld_wait();
+        if (warp == 0) TRS(5, u);
+        uint32_t sv[16];
+        {
+          // two accumulators per unit: the halves of the feature slabs (16-bit tables), or the digit planes of q
+          const uint32_t sa = tmem_base + lane_off + (uint32_t)(sb_i * 128 + cset * 32);
+          uint32_t sb[16];
+          ptx::tmem_ld_16x32bx2_x16(sa, sv);
+          ptx::tmem_ld_16x32bx2_x16(sa + (uint32_t)WS_HEADS, sb);
+          ptx::tmem_ld_wait();
 #pragma unroll
-                for (int c = 0; c < 32; ++c) ov[c] = __float_as_uint(__uint_as_float(ov[c]) * mi->factor[hh * 32 + c]);
-                ptx::tmem_st32(ta, ov);
-              }
+          for (int c = 0; c < 16; c += 4) {
+            if constexpr (I8) {
+              const float4 qs = *reinterpret_cast<const float4*>(&mi->q_step[col0 + c]);   // the heads' fixed-point steps
+              sv[c] = __float_as_uint(fmaf((float)(int)sv[c], 256.f, (float)(int)sb[c]) * qs.x);
+              sv[c + 1] = __float_as_uint(fmaf((float)(int)sv[c + 1], 256.f, (float)(int)sb[c + 1]) * qs.y);
+              sv[c + 2] = __float_as_uint(fmaf((float)(int)sv[c + 2], 256.f, (float)(int)sb[c + 2]) * qs.z);
+              sv[c + 3] = __float_as_uint(fmaf((float)(int)sv[c + 3], 256.f, (float)(int)sb[c + 3]) * qs.w);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) sv[c + e] = __float_as_uint(__uint_as_float(sv[c + e]) + __uint_as_float(sb[c + e]));
             }
           }
-          ptx::tmem_st_wait();
         }
-        if (warp == 0) TRS(28, u);
-      }
-      // ---- P^T (16-bit, K-major, swizzled); the weights join this thread's sums as the operand holds them
-      uint32_t prw[8];
-      {
+        ptx::tc_fence_before_sync();
+        ptx::mbar_arrive(&mi->s_free[sb_i]);
+        if (I8 && u == 0) ptx::mbar_wait(&mi->meta_ready, 0, abort_flag);   // the first scales are published behind the gathers
+        const bool ok = mi->row_ref[slot][row] != kNoRow;
+        const float rs = I8 ? mi->row_scale[slot][row] : 1.f;
+        const float mul = scale_log2 * rs;
+        // Int8 tables: the operand weight of a row is its softmax weight times the row's dequantisation scale, and
+        // that product is what has to fit fp16.  So the references follow the maxima of logit + log2(scale): the
+        // largest operand weight of a head is 1 (2^-headroom) when its reference moves, whatever the scales are.
+        const float lrs = (I8 && ok) ? log2f(rs) : 0.f;
+        const float gap = BF16 ? kRescaleGapBF16 : kRescaleGapF16;
+        bool grow = false;
 #pragma unroll
-        for (int c = 0; c < 16; c += 2) {   // two heads per step: one packed conversion each way
-          const float2 mr = *reinterpret_cast<const float2*>(&mi->m_ref[col0 + c]);   // (moves only in the branch above)
-          const float s0 = __uint_as_float(sv[c]), s1 = __uint_as_float(sv[c + 1]);
-          float p0 = (s0 == -INFINITY) ? 0.f : fast_exp2(s0 - mr.x);
-          float p1 = (s1 == -INFINITY) ? 0.f : fast_exp2(s1 - mr.y);
-          float b0, b1;
-          prw[c >> 1] = pack_op16x2<BF16>(p0, p1, b0, b1);
-          sv[c] = __float_as_uint(b0);   // the weights as the operand holds them
-          sv[c + 1] = __float_as_uint(b1);
+        for (int c = 0; c < 16; c += 4) {
+          const float4 mr = *reinterpret_cast<const float4*>(&mi->m_ref[col0 + c]);   // the heads' reference maxima
+          const float mrv[4] = {mr.x, mr.y, mr.z, mr.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float x = ok ? fmaf(__uint_as_float(sv[c + e]), mul, lrs) : -INFINITY;
+            sv[c + e] = __float_as_uint(x);
+            grow |= x > mrv[e] + gap;
+          }
+        }
+        if (warp == 0) TRS(6, u);
+        bool grown = false;
+        if (__syncthreads_or_256(grow)) {
+          // exact column maxima of this unit (xor shuffles of 8, 4, 2, 1 stay inside a half warp = one head range)
+#pragma unroll
+          for (int c = 0; c < 16; ++c) {
+            int o = float_order(__uint_as_float(sv[c]));
+            o = max(o, __shfl_xor_sync(0xffffffffu, o, 8));
+            o = max(o, __shfl_xor_sync(0xffffffffu, o, 4));
+            o = max(o, __shfl_xor_sync(0xffffffffu, o, 2));
+            o = max(o, __shfl_xor_sync(0xffffffffu, o, 1));
+            if (li == c) mi->colmax[wq][col0 + c] = order_float(o);
+          }
+          // O^T belongs to the old reference: it is final for the units so far once the previous P V is done (and
+          // the row sums have taken the previous factor, if any, before this one replaces it)
+          if (warp == 0) TRS(29, u);
+          if (u > ub) wait_pv_all(u - 1);
+          if (I8 && u >= 1) ptx::mbar_wait(&mi->p_summed, (uint32_t)((u - 1) & 1), abort_flag);
+          if (warp == 0) TRS(30, u);
+          group_sync(4, 256);
+          if (tid < WS_HEADS) {
+            const float old = mi->m_ref[tid];
+            float mx = fmaxf(fmaxf(mi->colmax[0][tid], mi->colmax[1][tid]), fmaxf(mi->colmax[2][tid], mi->colmax[3][tid]));
+            mx = mx > old ? mx + (BF16 ? 0.f : kRescaleHeadroom) : old;
+            mi->factor[tid] = (old == -INFINITY) ? 0.f : exp2f(old - mx);
+            mi->m_ref[tid] = mx;
+          }
+          group_sync(4, 256);
+          ptx::tc_fence_after_sync();
+          if constexpr (!I8) l1 *= mi->factor[col0 + li];
+          grown = true;
+          if (u > ub) {
+            // warp -> (lane quarter of TMEM = 32 features, two of the four 128-feature blocks); columns = heads
+            for (int m2 = 0; m2 < 2; ++m2) {
+              const int mt = cset * 2 + m2;
+              if (mt < n_mt) {
+#pragma unroll 1
+                for (int hh = 0; hh < 2; ++hh) {
+                  uint32_t ov[32];
+                  const uint32_t ta = tmem_o + lane_off + (uint32_t)(mt * WS_HEADS + hh * 32);
+                  ptx::tmem_ld32(ta, ov);
+                  ptx::tmem_ld_wait();
+#pragma unroll
+                  for (int c = 0; c < 32; ++c) ov[c] = __float_as_uint(__uint_as_float(ov[c]) * mi->factor[hh * 32 + c]);
+                  ptx::tmem_st32(ta, ov);
+                }
+              }
+            }
+            ptx::tmem_st_wait();
+          }
+          if (warp == 0) TRS(28, u);
+        }
+        // ---- P^T (16-bit, K-major, swizzled); the weights join this thread's sums as the operand holds them
+        uint32_t prw[8];
+        {
+#pragma unroll
+          for (int c = 0; c < 16; c += 2) {   // two heads per step: one packed conversion each way
+            const float2 mr = *reinterpret_cast<const float2*>(&mi->m_ref[col0 + c]);   // (moves only in the branch above)
+            const float s0 = __uint_as_float(sv[c]), s1 = __uint_as_float(sv[c + 1]);
+            float p0 = (s0 == -INFINITY) ? 0.f : fast_exp2(s0 - mr.x);
+            float p1 = (s1 == -INFINITY) ? 0.f : fast_exp2(s1 - mr.y);
+            float b0, b1;
+            prw[c >> 1] = pack_op16x2<BF16>(p0, p1, b0, b1);
+            sv[c] = __float_as_uint(b0);   // the weights as the operand holds them
+            sv[c + 1] = __float_as_uint(b1);
+          }
+        }
+        if (warp == 0) TRS(7, u);
+        if (I8 && u >= 1) {   // the one P^T buffer has been read by the previous unit's P V and by the row sums
+          wait_pv_all(u - 1);
+          ptx::mbar_wait(&mi->p_summed, (uint32_t)((u - 1) & 1), abort_flag);
+        }
+        if constexpr (I8) {
+          if (cset == 0 && ch == 0) mi->row_inv[u & 1][row] = ok ? __frcp_rn(rs) : 0.f;
+          if (tid == 0) mi->grew[u & 1] = grown ? 1 : 0;
+        }
+        {
+          uint8_t* pbase = smem + (pt0 + (pb_i) * pt_st) + (row & 7) * 2;
+          const int cj = row >> 3;
+#pragma unroll
+          for (int c = 0; c < 16; c += 2) {
+            const int h = col0 + c;
+            *reinterpret_cast<uint16_t*>(pbase + (size_t)h * 128 + ((cj ^ (h & 7)) << 4)) = (uint16_t)(prw[c >> 1] & 0xffffu);
+            *reinterpret_cast<uint16_t*>(pbase + (size_t)(h + 1) * 128 + ((cj ^ ((h + 1) & 7)) << 4)) = (uint16_t)(prw[c >> 1] >> 16);
+          }
+        }
+        if (warp == 0) TRS(12, u);
+        ptx::fence_proxy_async_smem();
+        ptx::tc_fence_before_sync();
+        ptx::mbar_arrive(&mi->p_ready[pb_i]);
+        if (warp == 0) TRS(8, u);
+        // 16-bit tables: the sums over the 16 rows of this half warp, behind the hand-off (int8 tables: the widening
+        // warps sum P^T from shared memory)
+        if constexpr (!I8) {
+          float a[16];
+#pragma unroll
+          for (int c = 0; c < 16; ++c) a[c] = __uint_as_float(sv[c]);
+          l1 += half_warp_column_sum(a, li);
         }
       }
-      if (warp == 0) TRS(7, u);
-      if (I8 && u >= 1) {   // the one P^T buffer has been read by the previous unit's P V and by the row sums
-        wait_pv_all(u - 1);
-        ptx::mbar_wait(&mi->p_summed, (uint32_t)((u - 1) & 1), abort_flag);
-      }
-      if constexpr (I8) {
-        if (cset == 0 && ch == 0) mi->row_inv[u & 1][row] = ok ? __frcp_rn(rs) : 0.f;
-        if (tid == 0) mi->grew[u & 1] = grown ? 1 : 0;
-      }
-      {
-        uint8_t* pbase = smem + (pt0 + (pb_i) * pt_st) + (row & 7) * 2;
-        const int cj = row >> 3;
-#pragma unroll
-        for (int c = 0; c < 16; c += 2) {
-          const int h = col0 + c;
-          *reinterpret_cast<uint16_t*>(pbase + (size_t)h * 128 + ((cj ^ (h & 7)) << 4)) = (uint16_t)(prw[c >> 1] & 0xffffu);
-          *reinterpret_cast<uint16_t*>(pbase + (size_t)(h + 1) * 128 + ((cj ^ ((h + 1) & 7)) << 4)) = (uint16_t)(prw[c >> 1] >> 16);
-        }
-      }
-      if (warp == 0) TRS(12, u);
-      ptx::fence_proxy_async_smem();
-      ptx::tc_fence_before_sync();
-      ptx::mbar_arrive(&mi->p_ready[pb_i]);
-      if (warp == 0) TRS(8, u);
-      // 16-bit tables: the sums over the 16 rows of this half warp, behind the hand-off (int8 tables: the widening
-      // warps sum P^T from shared memory)
-      if constexpr (!I8) {
-        float a[16];
-#pragma unroll
-        for (int c = 0; c < 16; ++c) a[c] = __uint_as_float(sv[c]);
-        l1 += half_warp_column_sum(a, li);
-      }
-    }
 
-    // ------------------------------------------------------------------ row sums over all units
-    if (tid == 0) TRS(11, 2);
-    group_sync(4, 256);   // nobody reads the column maxima or the row ring any more
-    if constexpr (!I8) mi->colmax[wq][col0 + li] = l1;
-    if (I8 && nunits >= 1) ptx::mbar_wait(&mi->p_summed, (uint32_t)((nunits - 1) & 1), abort_flag);   // the totals are in
-    if (nunits >= 1) wait_pv_all(nunits - 1);
-    if (!I8 && nunits >= 2) wait_pv_all(nunits - 2);
-    ptx::tc_fence_after_sync();
-    group_sync(4, 256);
-    if (tid == 0) TRS(11, 3);
+      // ------------------------------------------------------------------ row sums over all units
+      if (tid == 0) TRS(11, 2);
+      group_sync(4, 256);   // nobody reads the column maxima or the row ring any more
+      if constexpr (!I8) mi->colmax[wq][col0 + li] = l1;
+      if (I8 && nunits >= 1) ptx::mbar_wait(&mi->p_summed, (uint32_t)((nunits - 1) & 1), abort_flag);   // the totals are in
+      if (nunits >= 1) wait_pv_all(ub + nunits - 1);
+      if (!I8 && nunits >= 2) wait_pv_all(ub + nunits - 2);
+      ptx::tc_fence_after_sync();
+      group_sync(4, 256);
+      if (tid == 0) TRS(11, 3);
 
-    // ------------------------------------------------------------------ per-head sums of this split
-    if (tid < WS_HEADS) {
-      float l, vb = 0.f;
-      if constexpr (I8) {   // rows 0-1: the denominator's two halves, rows 2-3: the operand weights' (widening warps)
-        l = nunits >= 1 ? mi->colmax[0][tid] + mi->colmax[1][tid] : 0.f;
-        vb = nunits >= 1 ? kValueBias * (mi->colmax[2][tid] + mi->colmax[3][tid]) : 0.f;
-      } else {
-        l = (mi->colmax[0][tid] + mi->colmax[1][tid]) + (mi->colmax[2][tid] + mi->colmax[3][tid]);
-      }
-      mi->l_tot[tid] = l;
-      mi->v_bias[tid] = vb;
-      if (p.cluster_merge) {   // tell every split of this token (this one included) where this one stands
-        const uint32_t am = ptx::smem_u32(&mi->xm[split][tid]), al = ptx::smem_u32(&mi->xl[split][tid]);
-        for (int r = 0; r < p.nsplit; ++r) {
-          ptx::st_cluster_f32(ptx::cluster_map(am, (uint32_t)r), mi->m_ref[tid]);
-          ptx::st_cluster_f32(ptx::cluster_map(al, (uint32_t)r), l);
+      // ------------------------------------------------------------------ per-head sums of this split
+      if (tid < WS_HEADS) {
+        float l, vb = 0.f;
+        if constexpr (I8) {   // rows 0-1: the denominator's two halves, rows 2-3: the operand weights' (widening warps)
+          l = nunits >= 1 ? mi->colmax[0][tid] + mi->colmax[1][tid] : 0.f;
+          vb = nunits >= 1 ? kValueBias * (mi->colmax[2][tid] + mi->colmax[3][tid]) : 0.f;
+        } else {
+          l = (mi->colmax[0][tid] + mi->colmax[1][tid]) + (mi->colmax[2][tid] + mi->colmax[3][tid]);
+        }
+        mi->l_tot[tid] = l;
+        mi->v_bias[tid] = vb;
+        if (p.cluster_merge) {   // tell every split of this token (this one included) where this one stands
+          const uint32_t am = ptx::smem_u32(&mi->xm[split][tid]), al = ptx::smem_u32(&mi->xl[split][tid]);
+          for (int r = 0; r < p.nsplit; ++r) {
+            ptx::st_cluster_f32(ptx::cluster_map(am, (uint32_t)r), mi->m_ref[tid]);
+            ptx::st_cluster_f32(ptx::cluster_map(al, (uint32_t)r), l);
+          }
         }
       }
-    }
+      if constexpr (TOKENS) {
+        emit();
+        ptx::tc_fence_before_sync();
+        ptx::mbar_arrive(&mi->tok_free[it & 1]);
+      }
+    } while (next_token());
   }
 
   // ====================================================================== output
   // Every role is done with this CTA's operand buffers (the softmax warps arrive here only after the last P V).
-  // Three ways out: one split -> final or external-partial output straight from TMEM; splits in a cluster ->
-  // merged through shared memory below; otherwise (o, m, l) partials for the merge kernel.
-  const bool cmerge = p.cluster_merge != 0;
   if (cmerge) {
     __syncwarp();
     ptx::cluster_arrive();   // (1) every split's (m, l) is in place and every CTA's buffers are idle
     ptx::cluster_wait();
     if (tid == 0) TRS(11, 5);
   }
-  const int n_slots = cmerge ? (n_mt + p.nsplit - 1) / p.nsplit : 0;   // value blocks a CTA merges: mt = rank + slot * nsplit
-  float* recv = reinterpret_cast<float*>(smem);   // cluster merge: [slot][source split][16 head groups][128 features][4 heads]
-  if (warp < 8) {
-    const int wq = warp & 3, cset = warp >> 2;
-    const uint32_t lane_off = (uint32_t)(wq * 32) << 16;
-    const int64_t N = (int64_t)p.B * p.T * p.H;
-    const bool direct = p.nsplit == 1;
-    const bool finalize = direct && !p.partial_ml;
-    const bool have_o = nunits > 0;
-    if (tid < WS_HEADS) {
-      // per-head factor applied to O^T: 1 for partial output; otherwise this split's weight over the denominator
-      // of the whole token, exp2(m - m*) / (sum over splits of l exp2(m_s - m*) + sink), the sink joining once
-      float fac = 1.f;
-      if (finalize || cmerge) {
-        const float m = mi->m_ref[tid];
-        const float sink2 = (p.sinks && tid < p.H) ? p.sinks[tid] * 1.4426950408889634f : -INFINITY;
-        float m2v = fmaxf(m, sink2);
-        if (cmerge)
-          for (int r = 0; r < p.nsplit; ++r) m2v = fmaxf(m2v, mi->xm[r][tid]);
-        float w = 0.f, den = 0.f;
-        if (m2v > -INFINITY) {
-          w = (m == -INFINITY) ? 0.f : exp2f(m - m2v);
-          if (cmerge) {
-            for (int r = 0; r < p.nsplit; ++r)   // split order: the same sum in every CTA and on every run
-              if (mi->xm[r][tid] > -INFINITY) den = fmaf(mi->xl[r][tid], exp2f(mi->xm[r][tid] - m2v), den);
-          } else {
-            den = mi->l_tot[tid] * w;
-          }
-          den += (sink2 == -INFINITY) ? 0.f : exp2f(sink2 - m2v);
-        }
-        fac = den > 0.f ? w / den : 0.f;
-      }
-      mi->factor[tid] = fac;
-    }
-    group_sync(4, 256);
-    // warp -> (lane quarter of TMEM = 32 features, two of the four 128-feature blocks); columns = heads
-    const int64_t gbase = direct ? (int64_t)b * p.o_sb + (int64_t)t * p.o_st : ((int64_t)split * N + (int64_t)bt * p.H) * p.Dv;
-    const int64_t ostep = direct ? p.o_sh : (int64_t)p.Dv;
-    for (int m2 = 0; m2 < 2; ++m2) {
-      const int mt = cset * 2 + m2;
-      if (mt >= n_mt) continue;
-      const int d = mt * 128 + wq * 32 + lane;
-      // cluster merge: block mt belongs to split mt % nsplit; this thread's feature row of it goes there, four
-      // heads per 16-byte store, consecutive features in consecutive lanes
-      const uint32_t owner = (uint32_t)(mt % p.nsplit);
-      const uint32_t dst0 = cmerge ? ptx::cluster_map(ptx::smem_u32(recv) + (uint32_t)((((mt / p.nsplit) * p.nsplit + split) * 16) * 128 + wq * 32 + lane) * 16u, owner) : 0u;
-#pragma unroll 1
-      for (int hh = 0; hh < 2; ++hh) {
-        uint32_t ov[32];
-        if (have_o) {
-          ptx::tmem_ld32(tmem_o + lane_off + (uint32_t)(mt * WS_HEADS + hh * 32), ov);
-          ptx::tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int c = 0; c < 32; ++c) ov[c] = 0u;
-        }
-        if (cmerge) {
-#pragma unroll
-          for (int c = 0; c < 32; c += 4) {
-            float o4[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int h = hh * 32 + c + e;
-              o4[e] = have_o ? (__uint_as_float(ov[c + e]) - mi->v_bias[h]) * mi->factor[h] : 0.f;
-            }
-            ptx::st_cluster_v4(dst0 + (uint32_t)((hh * 8 + (c >> 2)) * 128) * 16u, o4[0], o4[1], o4[2], o4[3]);
-          }
-          continue;
-        }
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const int h = hh * 32 + c;
-          if (h >= p.H) continue;
-          const float o = (__uint_as_float(ov[c]) - mi->v_bias[h]) * mi->factor[h];
-          if (finalize) store_elem<OT>(p.out, gbase + d + h * ostep, o);
-          else if (direct) reinterpret_cast<float*>(p.out)[gbase + d + h * ostep] = o;
-          else p.ws_o[gbase + d + h * ostep] = o;
-        }
-      }
-    }
-    if (!cmerge && tid < p.H && (!direct || p.partial_ml)) {
-      // (m, l) in natural-log units for the merge kernel
-      const float m_nat = mi->m_ref[tid] == -INFINITY ? -INFINITY : mi->m_ref[tid] * 0.6931471805599453f;
-      float* ml = direct ? p.partial_ml + ((int64_t)bt * p.H + tid) * 2
-                         : p.ws_ml + ((int64_t)split * N + (int64_t)bt * p.H + tid) * 2;
-      ml[0] = m_nat;
-      ml[1] = mi->l_tot[tid];
-    }
-  }
+  if (!TOKENS && warp < 8) emit();
   if (cmerge) {
     if (tid == 0) TRS(11, 6);
     __syncwarp();
@@ -1314,8 +1418,24 @@ static int launch_tc_typed(SparseParams& p, int out_dtype, cudaStream_t st) {
   // left have failed ("unspecified launch failure": always for 160 split CTAs, rarely for 4,096 one-split CTAs) and
   // launches of at most one CTA per SM never have; the cause is not known.  Between launches nothing of the previous
   // wave is in flight.
+  int64_t done = 0;
   const int64_t wave = (int64_t)(sm_count() / p.nsplit) * p.nsplit > 0 ? (int64_t)(sm_count() / p.nsplit) * p.nsplit : p.nsplit;
-  for (int64_t base = 0; base < ctas; base += wave) {
+  // Several whole waves of a final output from a 16-bit table: one launch of one CTA per SM that works through them.
+  if constexpr (!I8) {
+    if (p.nsplit == 1 && !p.partial_ml && p.q_tma && ctas >= 2 * wave) {
+      const Kern walk = final_kernel == 0   ? (Kern)sparse_attn_tc_kernel<KVT, QT, MXB_F32, true>
+                        : final_kernel == 1 ? (Kern)sparse_attn_tc_kernel<KVT, QT, MXB_F16, true>
+                                            : (Kern)sparse_attn_tc_kernel<KVT, QT, MXB_BF16, true>;
+      MXB_CUDA_OK(cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      SparseParams c = p;
+      c.cta_base = 0;
+      c.n_tok = (int32_t)(done = ctas / wave * wave);
+      walk<<<dim3((unsigned)wave), WS_THREADS, smem, st>>>(c, tm_comp, tm_raw, tm_comp_tail, tm_raw_tail, tm_q);
+      note_launch();
+      MXB_CUDA_OK(cudaGetLastError());
+    }
+  }
+  for (int64_t base = done; base < ctas; base += wave) {
     const int64_t n = ctas - base < wave ? ctas - base : wave;
     // A last wave that leaves half of the SMs idle runs its tokens as split clusters instead, at least two units per
     // split (333 tokens of up to 640 rows on 148 SMs: 116 -> 104 us).

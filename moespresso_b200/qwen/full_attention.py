@@ -296,7 +296,8 @@ def sdpa_decode_q8(queries, k_packed, k_scales, k_biases, v_packed, v_scales, v_
     a.P, a.Hq, a.Hkv, a.D, a.scale, a.n_splits = P, Hq, Hkv, D, float(scale), splits
     a.o_parts, a.ml_parts = ptr(o_parts), ptr(ml_parts)
     _abi.check(_t.launch("sdpa_decode_q8", _abi.load().mxb_sdpa_decode_q8, a))
-    out = merge_partials(o_parts, ml_parts, None)                # [1, 1, Hq, D]
+    typed = queries.dtype in (torch.float32, torch.float16, torch.bfloat16)
+    out = merge_partials(o_parts, ml_parts, None, out_dtype=queries.dtype if typed else torch.float32)   # [1, 1, Hq, D]
     return out.reshape(1, Hq, 1, D).to(queries.dtype)
 
 

@@ -514,3 +514,32 @@ def test_last_wave_of_a_chunk(extra, k, window, kind):
     want = iak.sparse_attention(q, comp, ids[None], sinks, exact_fp32=True, **kw)
     # P and its operands are 16-bit (bf16: 2^-9 each), averaged over many rows; the largest |v| is about 4
     assert max_abs(got, want.cpu().numpy()) <= (2e-3 if kind == "f16" else 2e-2)
+
+
+@pytest.mark.parametrize("waves,extra,k,pos0,window,ratio", [
+    (2, 0, 200, 0, 0, 4),        # a chunk's first tokens: no visible row, one row, ... several units
+    (3, 5, 512, 4000, 100, 4),   # whole lists behind a raw window, a ragged last wave
+    (2, 1, 64, 4000, 0, 0),      # one unit per token
+    (2, 3, 130, 4000, 7, 4),     # three units, the last of two entries
+])
+@pytest.mark.parametrize("kind,out_dtype", [("bf16", torch.float32), ("f16", torch.float16)])
+def test_ctas_that_work_through_several_tokens(waves, extra, k, pos0, window, ratio, kind, out_dtype):
+    """Two or more whole waves of tokens run as one launch whose CTAs go from token to token: bit for bit what the
+    tokens give in calls of at most one wave."""
+    need_gpu()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    T, H, D, Dv, R = waves * sms + extra, 64, 576, 512, 700
+    g = torch.Generator(device="cuda").manual_seed(T + k)
+    dt = torch.bfloat16 if kind == "bf16" else torch.float16
+    mk = lambda *s: torch.randn(s, generator=g, device="cuda").to(dt)  # noqa: E731
+    comp, raw, q = mk(R, D), mk(1, T + window, D), mk(1, H, T, D)
+    sinks = torch.randn(H, generator=g, device="cuda")
+    ids = torch.sort(torch.rand(T, R, generator=g, device="cuda").topk(k).indices, dim=1).values.int()
+    kw = dict(window=window, ratio=ratio, scale=D ** -0.5, d_v=Dv, n_comp=R, out_layout="bthd", out_dtype=out_dtype,
+              n_splits=1, check=True)
+    got = iak.sparse_attention(q, comp, ids[None], sinks, pos0=pos0, raw_kv=raw if window else None, **kw)
+    for lo in range(0, T, sms):
+        hi = min(lo + sms, T)
+        part = iak.sparse_attention(q[:, :, lo:hi], comp, ids[None, lo:hi], sinks, pos0=pos0 + lo,
+                                    raw_kv=raw[:, :hi + window].contiguous() if window else None, **kw)
+        assert torch.equal(got[:, lo:hi], part), (lo, hi)
