@@ -192,13 +192,13 @@ class QuantizedKVCache:
         dt = self.keys[1].dtype
         keys, values = keys.to(dt), values.to(dt)
         shape = (1, int(self.keys[0].shape[1]), L, 4 * int(self.keys[0].shape[3]))
-        if L and tuple(keys.shape) == shape and tuple(values.shape) == shape:
+        if L and tuple(keys.shape) == shape and tuple(values.shape) == shape and keys.device == self.keys[0].device:
             if keys.stride() != values.stride() or keys.stride(3) != 1:
                 keys, values = keys.contiguous(), values.contiguous()
             require_cuda(keys, values, self.keys[0])
             _q8_pair("affine_q8_append", (keys, values), keys.stride(1), keys.stride(2), self.keys, self.values,
                      self.capacity, self.offset, L)
-        else:                                  # shapes that broadcast into the cache
+        else:                                  # shapes that broadcast into the cache, rows of another device
             for store, x in ((self.keys, keys), (self.values, values)):
                 for dst, src in zip(store, quantize_affine_q8(x)):
                     dst[:, :, self.offset:self.offset + L].copy_(src)
