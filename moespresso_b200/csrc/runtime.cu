@@ -94,35 +94,48 @@ extern "C" int mxb_copy_h2d_async(void* dst_device, const void* src_host, int64_
 }
 
 namespace mxb {
-// One CTA column per buffer; 16-byte pieces where both sides allow it.  A decode step's three inputs (a few KB to a few
-// MB) are three launches as single copies, and a launch is what each of them costs.
-__global__ void __launch_bounds__(256) copy_buffers_kernel(mxb_copy_buffers_args a) {
-  const int i = blockIdx.y;
-  const int64_t n = a.bytes[i], step = (int64_t)gridDim.x * 256, at = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  uint8_t* dst = reinterpret_cast<uint8_t*>(a.dst[i]);
-  const uint8_t* src = reinterpret_cast<const uint8_t*>(a.src[i]);
-  int64_t done = 0;
+// A CTA copies 16 KB of one buffer, four 16-byte pieces per thread in flight where both sides are aligned.  A decode step's
+// three inputs (a few KB to a few MB) are three launches as single copies, and a launch is what each of them costs.
+constexpr int64_t kCopyBytes = 16384;
+__global__ void __launch_bounds__(256) copy_buffers_kernel(const __grid_constant__ mxb_copy_buffers_args a) {
+  int64_t chunk = blockIdx.x;
+  int i = 0;
+  while (chunk >= (a.bytes[i] + kCopyBytes - 1) / kCopyBytes) chunk -= (a.bytes[i++] + kCopyBytes - 1) / kCopyBytes;
+  const int64_t lo = chunk * kCopyBytes;
+  const int n = (int)(a.bytes[i] - lo < kCopyBytes ? a.bytes[i] - lo : kCopyBytes);
+  uint8_t* dst = reinterpret_cast<uint8_t*>(a.dst[i]) + lo;
+  const uint8_t* src = reinterpret_cast<const uint8_t*>(a.src[i]) + lo;
+  int done = 0;
   if (((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0) {
-    const int64_t pieces = n / 16;
-#pragma unroll 4
-    for (int64_t j = at; j < pieces; j += step) reinterpret_cast<uint4*>(dst)[j] = __ldg(reinterpret_cast<const uint4*>(src) + j);
+    const int pieces = n / 16;
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = u * 256 + (int)threadIdx.x;
+      if (j < pieces) v[u] = __ldg(reinterpret_cast<const uint4*>(src) + j);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = u * 256 + (int)threadIdx.x;
+      if (j < pieces) reinterpret_cast<uint4*>(dst)[j] = v[u];
+    }
     done = pieces * 16;
   }
-  for (int64_t j = done + at; j < n; j += step) dst[j] = src[j];
+  for (int j = done + (int)threadIdx.x; j < n; j += 256) dst[j] = src[j];
 }
 }  // namespace mxb
 
 extern "C" int mxb_copy_buffers(const mxb_copy_buffers_args* a, void* stream) {
   MXB_REQUIRE(a != nullptr, MXB_ERR_INVALID, "copy buffers: null args");
-  int64_t longest = 0;
+  int64_t chunks = 0;
   for (int i = 0; i < 4; ++i) {
     MXB_REQUIRE(a->bytes[i] >= 0 && (a->bytes[i] == 0 || (a->dst[i] && a->src[i])), MXB_ERR_INVALID,
                 "copy buffers: null pointer or negative size");
-    if (a->bytes[i] > longest) longest = a->bytes[i];
+    chunks += mxb::ceil_div(a->bytes[i], mxb::kCopyBytes);
   }
-  if (longest == 0) return MXB_OK;
-  const int64_t want = mxb::ceil_div(longest, 256 * 16 * 2), most = 2 * (int64_t)mxb::sm_count();
-  mxb::copy_buffers_kernel<<<dim3((unsigned)(want < most ? want : most), 4), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(*a);
+  MXB_REQUIRE(chunks <= 0x7FFFFFFFll, MXB_ERR_INVALID, "copy buffers: too many bytes");
+  if (chunks == 0) return MXB_OK;
+  mxb::copy_buffers_kernel<<<(unsigned)chunks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(*a);
   mxb::note_launch();
   MXB_CUDA_OK(cudaGetLastError());
   return MXB_OK;
