@@ -413,6 +413,9 @@ typedef struct {
   int32_t* status;
 } mxb_sparse_attn_args;
 
+/* The caller's promise that mxb_topk_select, writing `topk`, is the last launch on this stream, and that everything else
+ * the call reads was complete before that: the attention may start while the selection finishes. */
+#define MXB_SPARSE_AFTER_SELECT 2
 #define MXB_SPARSE_EXACT_FP32 1 /* CUDA-core fp32 kernel even where the tensor-core kernel applies */
 
 int64_t mxb_sparse_attn_workspace_bytes(const mxb_sparse_attn_args* a);

@@ -591,6 +591,7 @@ extern "C" int mxb_sparse_attn(const mxb_sparse_attn_args* a, void* stream) {
   p.pos0 = a->pos0; p.pos0_dev = a->pos0_dev; p.window = a->window; p.ratio = a->ratio;
   p.nsplit = choose_splits(a);
   p.may_split = a->n_splits <= 0;
+  p.after_select = (a->flags & MXB_SPARSE_AFTER_SELECT) != 0;
   p.status = a->status;
 
   const int64_t N = (int64_t)a->B * a->T * a->H;

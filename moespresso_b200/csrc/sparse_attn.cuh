@@ -33,6 +33,7 @@ struct SparseParams {
   int32_t* status;
   int32_t q_tma;      // q reaches shared memory by TMA (tensor map beside these parameters) instead of registers
   int32_t q_axis[3];  // which of (0 = head, 1 = token, 2 = batch) lies on dimensions 1..3 of that map
+  int32_t after_select;    // launched right behind the selection that writes the list, maybe before it has finished
   int32_t may_split;       // the caller left the number of splits open
   int32_t n_tok;           // set by the tensor-core launcher: tokens of a launch whose CTAs work through several
   int32_t cta_base;        // set by the tensor-core launcher: (token, split) index of this launch's CTA 0

@@ -138,7 +138,7 @@ struct WsMisc {
   uint64_t full[2][WS_MAX_SLABS];  // a slab of the unit in row buffer b has landed
   uint64_t v_full[4];              // int8 tables: a 128-feature block of the value buffer has been widened
   uint64_t k_free[2];              // int8 tables: the widening warps have read row buffer b
-  uint64_t tok_ready[2], tok_free[2];   // TOKENS: a token's list has been scanned; its slot may be reused
+  uint64_t tok_ready[2], tok_free[2];   // a token's list has been scanned; TOKENS: its slot may be reused
   int tok_units[2], tok_keff[2];
   uint64_t meta_ready;             // int8 tables: the scales of units 0 and 1 have been published
   uint64_t s_ready[2], s_free[2], p_ready[2];
@@ -148,7 +148,6 @@ struct WsMisc {
   uint64_t pv_blk[2][4];           // P V of one 128-feature block of the unit in buffer b has completed: its two slabs are free
   uint32_t tmem_slot;
   int abort_flag;
-  int keff;
 };
 static_assert(sizeof(WsMisc) <= kWsMiscBytes, "WsMisc must fit the bytes the layout reserves for it");
 
@@ -345,7 +344,6 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
       ptx::mbar_init(&mi->tok_free[i], 256u + 2u + (n_mt > 2 ? 2u : 1u));   // softmax threads, logit and value issuers
     }
     mi->abort_flag = 0;
-    mi->keff = p.k;
     ptx::mbar_fence_init();
   }
   if (tid == 384) {   // the row tables' descriptors are on their way while the barriers and TMEM are set up
@@ -423,10 +421,13 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
   // first list entry that ends the walk, by `n` threads
   auto scan_list = [&](int me, int n, int* keff) {
     int mine = p.k;
-#pragma unroll 4
-    for (int j = me; j < p.k; j += n) {   // no early exit: the loads stay independent
-      const int64_t v = ids[j];
-      if (v >= visible && j < mine) mine = j;
+    for (int j0 = me; j0 < p.k; j0 += 16 * n) {   // sixteen ids in flight
+      int32_t v[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) v[u] = j0 + u * n < p.k ? ids[j0 + u * n] : -1;
+#pragma unroll
+      for (int u = 15; u >= 0; --u)
+        if ((int64_t)v[u] >= visible && j0 + u * n < mine) mine = j0 + u * n;
     }
     if (mine < p.k) atomicMin(keff, mine);
   };
@@ -439,17 +440,12 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
     e_hi = min(e_lo + per, total);
     nunits = (e_hi - e_lo + WS_UNIT - 1) / WS_UNIT;
   };
-  if constexpr (!TOKENS) {
-    scan_list(tid, WS_THREADS, &mi->keff);
-    __syncthreads();
-    cut_list(mi->keff);
-  }
-  // the next token of this CTA, for a role that only counts its units
+  // The gather warps scan the list; a role that only counts the token's units waits for their number.
   int ub = 0, it = 0;   // units and tokens before this one
   auto await_token = [&]() {
+    ptx::mbar_wait(&mi->tok_ready[it & 1], (uint32_t)((it >> 1) & 1), abort_flag);
+    nunits = mi->tok_units[it & 1];
     if constexpr (TOKENS) {
-      ptx::mbar_wait(&mi->tok_ready[it & 1], (uint32_t)((it >> 1) & 1), abort_flag);
-      nunits = mi->tok_units[it & 1];
       b = bt / p.T;
       t = bt % p.T;
     }
@@ -663,21 +659,24 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
       if (I8 && resolver && U < nunits) mi->row_scale[U & (kRing - 1)][pt] = rs;
     };
     do {
+      const int ts = it & 1;
       if constexpr (TOKENS) {
-        const int ts = it & 1;
         b = bt / p.T;
         t = bt % p.T;
         look_at_token();
         if (it >= 2) ptx::mbar_wait(&mi->tok_free[ts], (uint32_t)(((it >> 1) - 1) & 1), abort_flag);
-        if (pt == 0) mi->tok_keff[ts] = p.k;
-        group_sync(5, NG * 32);
-        scan_list(pt, NG * 32, &mi->tok_keff[ts]);
-        group_sync(5, NG * 32);
-        cut_list(mi->tok_keff[ts]);
-        if (pt == 0) {
-          mi->tok_units[ts] = nunits;
-          ptx::mbar_arrive(&mi->tok_ready[ts]);
-        }
+      }
+      if (pt == 0) mi->tok_keff[ts] = p.k;
+      group_sync(5, NG * 32);
+      // The list is all that the selection right before this launch writes: it may still be running while the other
+      // warps set up and turn q into digit planes (see launch_tc_typed).
+      if (p.after_select) ptx::grid_dependency_wait();
+      scan_list(pt, NG * 32, &mi->tok_keff[ts]);
+      group_sync(5, NG * 32);
+      cut_list(mi->tok_keff[ts]);
+      if (pt == 0) {
+        mi->tok_units[ts] = nunits;
+        ptx::mbar_arrive(&mi->tok_ready[ts]);
       }
       int32_t id_a = -1;          // stage A result: list id of this thread's entry of unit v + 3
       uint32_t src_b = kNoRow;    // stage B result: row and scale of this thread's entry of unit v + 2
@@ -805,6 +804,7 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&mi->p_summed);
       };
+      await_token();
       ptx::mbar_wait(&mi->q_ready, 0, abort_flag);   // q's scratch copy (in the value buffer) has been consumed
       for (int u = 0; u < nunits; ++u) {
         const int buf = u & 1;
@@ -864,6 +864,7 @@ sparse_attn_tc_kernel(SparseParams p, const __grid_constant__ CUtensorMap tm_com
         const uint32_t idesc_s = ptx::idesc_i8(WS_UNIT, 2 * WS_HEADS, 1, 1);
         const uint32_t q_addr = ptx::smem_u32(q_s), k_addr = ptx::smem_u32(smem + (kb0 + (j) * kb_st));
         const uint32_t d = tmem_base + (uint32_t)(j * 128);
+        await_token();
         for (int u = j; u < nunits; u += 2) {
           if (u >= 2) ptx::mbar_wait(&mi->s_free[j], sphase(u - 2), abort_flag);   // S^T(u - 2) has been read
           for (int sl = 0; sl < nrs; ++sl) {
@@ -1366,6 +1367,13 @@ static int launch_tc_typed(SparseParams& p, int out_dtype, cudaStream_t st) {
   for (const int i : {kernel_of, final_kernel})
     MXB_CUDA_OK(cudaFuncSetAttribute(kerns[i], cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
 
+  // Behind a selection (MXB_SPARSE_AFTER_SELECT) the first launch may start before that has finished: on SMs that the
+  // selection leaves idle (a few rows) the CTAs set up and prepare q meanwhile, elsewhere the launch itself is hidden.
+  // Decode steps, with the list scan in the gather warps: batch 3 37.7 -> 35.5 us, 32 110.0 -> 103.2, one row of 2^20 69.0 -> 64.3.
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+
   // `nsplit` splits of each of `tokens` tokens from `first` on as thread-block clusters that merge through shared memory:
   // when a final output is wanted, the blocks to merge fit the (then idle) operand buffers, and every cluster is
   // resident at once (a cluster needs nsplit whole SMs of one GPC; a second wave of clusters would cost more than it
@@ -1379,11 +1387,12 @@ static int launch_tc_typed(SparseParams& p, int out_dtype, cudaStream_t st) {
     cfg.blockDim = dim3(WS_THREADS);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)nsplit;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1] = early;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     static int resident_cache[3][16][kMaxClusterMerge + 1];   // per kernel, device and cluster size; 0 = not asked yet
@@ -1403,6 +1412,8 @@ static int launch_tc_typed(SparseParams& p, int out_dtype, cudaStream_t st) {
     c.nsplit = nsplit;
     c.cluster_merge = 1;
     c.cta_base = (int32_t)(first * nsplit);
+    c.after_select = p.after_select && first == 0;
+    cfg.numAttrs = c.after_select ? 2 : 1;
     MXB_CUDA_OK(cudaLaunchKernelEx(&cfg, kerns[final_kernel], c, tm_comp, tm_raw, tm_comp_tail, tm_raw_tail, tm_q));
     note_launch();
     return MXB_OK;
@@ -1429,6 +1440,7 @@ static int launch_tc_typed(SparseParams& p, int out_dtype, cudaStream_t st) {
       MXB_CUDA_OK(cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       SparseParams c = p;
       c.cta_base = 0;
+      c.after_select = 0;
       c.n_tok = (int32_t)(done = ctas / wave * wave);
       walk<<<dim3((unsigned)wave), WS_THREADS, smem, st>>>(c, tm_comp, tm_raw, tm_comp_tail, tm_raw_tail, tm_q);
       note_launch();
@@ -1450,7 +1462,15 @@ static int launch_tc_typed(SparseParams& p, int out_dtype, cudaStream_t st) {
     }
     SparseParams c = p;
     c.cta_base = (int32_t)base;
-    kerns[kernel_of]<<<dim3((unsigned)n), WS_THREADS, smem, st>>>(c, tm_comp, tm_raw, tm_comp_tail, tm_raw_tail, tm_q);
+    c.after_select = p.after_select && base == 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)n);
+    cfg.blockDim = dim3(WS_THREADS);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cfg.attrs = &early;
+    cfg.numAttrs = c.after_select ? 1 : 0;
+    MXB_CUDA_OK(cudaLaunchKernelEx(&cfg, kerns[kernel_of], c, tm_comp, tm_raw, tm_comp_tail, tm_raw_tail, tm_q));
     note_launch();
     MXB_CUDA_OK(cudaGetLastError());
   }

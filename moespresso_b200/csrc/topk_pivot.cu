@@ -31,6 +31,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "ptx_sm100.cuh"
 #include "topk_common.cuh"
 
 namespace cg = cooperative_groups;
@@ -151,6 +152,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) topk_direct_kernel(TopkPivotPar
   __shared__ uint32_t hist_a[kBigBins], hist_b[kBigBins];
   __shared__ uint32_t w_gt[kWords], w_eq[kWords], w_at[kWords];
   __shared__ TopkShared s;
+  ptx::grid_launch_dependents();   // the attention may set up on idle SMs; it waits for this grid before it reads ids
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int64_t n64;
   const float* src = row_scores(p, row, &n64);
@@ -250,6 +252,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkP
   __shared__ uint32_t s_sum[2], s_top;
   __shared__ uint32_t cl_count[kPMaxCluster], cl_gt[kPMaxCluster], cl_eq[kPMaxCluster];
 
+  ptx::grid_launch_dependents();   // as above
   cg::cluster_group cluster = cg::this_cluster();
   const int cs = CLUSTER ? (int)cluster.num_blocks() : 1;
   const int rank = CLUSTER ? (int)cluster.block_rank() : 0;

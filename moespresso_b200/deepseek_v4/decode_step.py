@@ -80,7 +80,8 @@ def sparse_decode_step(q, idx_q, idx_w, cache: LatentCache, *, k: int, scale: fl
     res = sparse_attention(q[:, :, None, :], cache.kv, ids[:, None, :], sinks, pos0=0, window=0, ratio=0,
                            scale=scale, d_v=d_v, kv_scales=cache.kv_scales, comp_row_start=cache.row_start,
                            comp_row_count=cache.row_count, n_comp=cache.max_rows, out_dtype=out_dtype,
-                           partial=partial)
+                           partial=partial, after_select=q.stride(-1) == 1 and cache.kv.is_contiguous() and (
+                               sinks is None or (sinks.dtype == torch.float32 and sinks.is_contiguous())))
     if partial:
         out, ml = res
         out = (out[:, :, 0, :], ml[:, 0])

@@ -43,7 +43,8 @@ def check_status(status: torch.Tensor, what: str) -> None:
 def sparse_attention(q4, comp_kv, topk3, sinks, *, pos0, window, ratio, raw_kv=None, raw_start=0,
                      scale=None, d_v=None, kv_scales=None, raw_scales=None, comp_row_start=None,
                      comp_row_count=None, n_comp=None, pos0_dev=None, out=None, out_dtype=torch.float32,
-                     out_layout="bhtd", partial=False, n_splits=0, exact_fp32=False, check=False, status=None):
+                     out_layout="bhtd", partial=False, n_splits=0, exact_fp32=False, check=False, status=None,
+                     after_select=False):
     """Launch the sparse attention kernel.
 
     q4 [B,H,T,Dqk] (any strides on the first three axes); comp_kv a flat
@@ -54,7 +55,9 @@ def sparse_attention(q4, comp_kv, topk3, sinks, *, pos0, window, ratio, raw_kv=N
     tables with up to 64 heads run on the tensor-core kernel; ``exact_fp32=True`` forces
     the fp32 CUDA-core kernel (always used for float32 tables).  ``status``: a caller-owned int64 device
     buffer to use in place of the library's status word (``moespresso_b200.cycle_trace`` passes a larger one:
-    an instrumented build writes its cycle stamps there).
+    an instrumented build writes its cycle stamps there).  ``after_select``: the caller's promise that the ``topk_select``
+    which wrote ``topk3`` is the last launch on the stream and that nothing else read here was written since: the
+    attention may then start while the selection finishes.
     """
     dev = require_cuda(q4, comp_kv, topk3)
     lib = _abi.load()
@@ -99,7 +102,7 @@ def sparse_attention(q4, comp_kv, topk3, sinks, *, pos0, window, ratio, raw_kv=N
     a.scale = float(Dqk) ** -0.5 if scale is None else float(scale)
     a.pos0 = int(pos0); a.pos0_dev = ptr(pos0_dev); a.window = int(window); a.ratio = int(ratio)
     a.n_splits = int(n_splits)
-    a.flags = _abi.SPARSE_EXACT_FP32 if exact_fp32 else 0
+    a.flags = (_abi.SPARSE_EXACT_FP32 if exact_fp32 else 0) | (_abi.SPARSE_AFTER_SELECT if after_select else 0)
     ws = workspace(lib.mxb_sparse_attn_workspace_bytes(C.byref(a)), dev)
     a.workspace = ptr(ws); a.workspace_bytes = 0 if ws is None else ws.numel()
     own_status = status is None
