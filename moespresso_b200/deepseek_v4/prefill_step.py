@@ -9,11 +9,11 @@ than ``k`` rows every row is selected (:1393-1395).  Projections, RoPE and the Q
 are outside this operator.
 
 The [tokens x rows] fp32 score matrix is never materialised: tokens are processed in
-chunks whose scores (``token_chunk`` x rows x 4 bytes) are written to one reused buffer that
-stays in the 126 MB L2 between the score kernel and the selection kernel.  The default chunk
-is four tokens per SM (592 on a B200: 78 MB of scores at 32768 rows), which fills whole waves
-of both kernels; measured per 4096-token chunk: 128 -> 7.5 ms, 256 -> 5.5, 592 -> 5.0,
-1024 -> 5.0, 4096 (537 MB of scores) -> 4.9.
+chunks whose scores (``token_chunk`` x rows x 4 bytes) are written to one reused buffer that mostly
+stays in the 126 MB L2 between the score kernel and the selection kernel.  The default chunk is eight
+tokens per SM (1184 on a B200: 155 MB of scores at 32768 rows; four per SM over longer pools), which fills
+whole waves of both kernels; measured per 4096-token chunk over 32768 rows: 296 -> 3343 us, 444 -> 3444,
+592 -> 3259, 888 -> 3364, 1184 -> 3201, 2072 -> 3264, 4096 (537 MB of scores) -> 3195.
 """
 from __future__ import annotations
 
@@ -39,7 +39,7 @@ def sparse_prefill_step(q, comp_kv, idx_q, idx_keys, idx_w, *, pos0: int, ratio:
     else:
         ids = torch.empty((T, kk), dtype=torch.int32, device=dev)
         if token_chunk is None:
-            token_chunk = 4 * torch.cuda.get_device_properties(dev).multi_processor_count
+            token_chunk = (8 if R <= 32768 else 4) * torch.cuda.get_device_properties(dev).multi_processor_count
         chunk = max(1, min(int(token_chunk), T))
         buf = torch.empty((1, chunk, R), dtype=torch.float32, device=dev)
         iq = idx_q.permute(1, 0, 2)[None]            # [1,Hi,T,Di]
