@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(384, 1) flash_prefill_kernel(const __grid_cons
     }
   } else if (warp == 8 || warp == 11) {
     // ------------------------------------------------------------ S = Q K^T issuers
-    // Warp 4 accumulates feature slabs 0-1 into S(s)a, warp 7 slabs 2-3 into S(s)b; P V (4 MMAs) is a third
+    // Warp 8 accumulates feature slabs 0-1 into S(s)a, warp 11 slabs 2-3 into S(s)b; P V (4 MMAs) is a third
     // issuer.  All write different TMEM columns, so none waits for another.
     if (lane == 0) {
       const int half = warp == 8 ? 0 : 1;
@@ -645,7 +645,10 @@ using namespace mxb;
 // How the items are dealt out.  Costs are in tiles (0.9 to 1.05 us each on a B200): a segment costs its tiles and
 // kSegCost for its Q load, first scores and drain; cutting costs kCutCost (partials out, merge launch, partials in), and
 // tiles take a tenth longer when every SM streams K and V at once.  Stretches of less than kMinShare are not worth an
-// SM of their own.
+// SM of their own.  Measured (16 query / 2 KV heads, bf16, gated; tokens over past, us, one CTA per item against equal
+// stretches): 64 over 3,000 51.1 / 27.6, 64 over 30,000 404 / 74.4, 100 over 8,000 122 / 33.7, 1,200 over 4,000 132 / 105,
+// 1,500 over 7,000 221 / 183, 2,048 over 30,720 1,091 / 1,001; on the other side of the rule 700 over 1,365 39.8 / 44.2,
+// 1,000 over 1,000 40.5 / 47.5, 2,048 over 5,000 182 / 192.
 constexpr int kSegCost = 4, kCutCost = 16, kMinShare = 12;
 
 // Fills p.n_bins / p.bin_start (n_bins = 0: one CTA per item) and returns the bytes of partials the plan needs.
