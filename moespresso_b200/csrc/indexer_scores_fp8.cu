@@ -138,6 +138,11 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
   if (tr_on && tid == 0) tr[6 * 64] = clock64();
 #endif
 
+  // 16 heads and eight tokens per tile: every group of drain warps keeps the weights of two tokens in registers and drains
+  // those two of every tile, instead of all tokens of every fourth tile with the weights read again for each.  The reads
+  // of accumulators, MMA operands and weights share one data path, 0.89 full with the weights on it (4,096 tokens x
+  // 32,768 rows, 1,184 tokens a launch: 590 -> 405 us; 333 x 5,003: 14.5 -> 12.3).
+  const bool pairs = K16 && H == 16 && p.t_tile == 2 * C::kTileGroups;
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
       ptx::mbar_init(&raw_full[s], 1);
@@ -149,7 +154,7 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
     }
     for (int a = 0; a < n_acc; ++a) {
       ptx::mbar_init(&acc_full[a], 1);
-      ptx::mbar_init(&acc_empty[a], 128);
+      ptx::mbar_init(&acc_empty[a], pairs ? 128u * C::kTileGroups : 128u);
     }
     *abort_flag = 0;
     ptx::mbar_fence_init();
@@ -393,7 +398,40 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
     const int set = warp >> 2, quad = warp & 3;
     const int rloc = quad * 32 + lane;
     const int64_t sbase = (p.row_start ? p.row_start[b] : 0) + (int64_t)b * p.s_sb;
-    for (int i = set; i < ntiles; i += C::kTileGroups) {
+    if (pairs) {
+      const int t = 2 * set;
+      float2 w[16];
+#pragma unroll
+      for (int h = 0; h < 16; ++h) w[h] = reinterpret_cast<const float2*>(w_s)[set * 16 + h];
+      const int64_t vis0 = t < nt ? (int64_t)vis_s[t] : 0, vis1 = t + 1 < nt ? (int64_t)vis_s[t + 1] : 0;
+      float* sp = p.scores + sbase + (int64_t)(t0 + t) * p.s_st + row0 + rloc;
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(set * 32);
+      int a = 0;
+      uint32_t ph = 0;
+      for (int i = 0; i < ntiles; ++i, sp += 128) {
+        ptx::mbar_wait(&acc_full[a], ph, abort_flag);
+        ptx::tc_fence_after_sync();
+        uint32_t v[32];   // 16 heads of token t, then of token t + 1
+        ptx::tmem_ld32(taddr + (uint32_t)(a * p.acc_stride), v);
+        ptx::tmem_ld_wait();
+        ptx::tc_fence_before_sync();
+        ptx::mbar_arrive(&acc_empty[a]);
+        if (++a == n_acc) {
+          a = 0;
+          ph ^= 1u;
+        }
+        float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int h = 0; h < 16; ++h)
+          sum = __ffma2_rn(w[h], make_float2(fmaxf(__uint_as_float(v[h]), 0.f), fmaxf(__uint_as_float(v[16 + h]), 0.f)), sum);
+        const int64_t r = row0 + (int64_t)i * 128 + rloc;
+        if (r < count) {
+          if (t < nt) sp[0] = r < vis0 ? sum.x : -INFINITY;
+          if (t + 1 < nt) sp[p.s_st] = r < vis1 ? sum.y : -INFINITY;
+        }
+      }
+    }
+    for (int i = set; i < ntiles && !pairs; i += C::kTileGroups) {
       const int a = i % n_acc;
       ptx::mbar_wait(&acc_full[a], (uint32_t)((i / n_acc) & 1), abort_flag);
       ptx::tc_fence_after_sync();
