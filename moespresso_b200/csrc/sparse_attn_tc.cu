@@ -1427,8 +1427,8 @@ static int launch_tc_typed(SparseParams& p, int out_dtype, cudaStream_t st) {
   }
   // One wave per launch.  Launches of this kernel that put a second CTA on an SM which a CTA of the same launch had just
   // left have failed ("unspecified launch failure": always for 160 split CTAs, rarely for 4,096 one-split CTAs) and
-  // launches of at most one CTA per SM never have; the cause is not known.  Between launches nothing of the previous
-  // wave is in flight.
+  // launches of at most one CTA per SM never have; the cause is not proven (the wait before the slab barriers take a
+  // unit's bytes was missing then).  Between launches nothing of the previous wave is in flight.
   int64_t done = 0;
   const int64_t wave = (int64_t)(sm_count() / p.nsplit) * p.nsplit > 0 ? (int64_t)(sm_count() / p.nsplit) * p.nsplit : p.nsplit;
   // Several whole waves of a final output from a 16-bit table: one launch of one CTA per SM that works through them.
