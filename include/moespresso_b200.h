@@ -308,9 +308,9 @@ typedef struct {
   int32_t k;                /* 1 <= k <= 8192 */
   void* workspace;
   int64_t workspace_bytes;
-  uint32_t* digit_hist;     /* NULL, or [rows, 2048]: the first-digit histogram of exactly the scores of each row,
-                               as mxb_indexer_scores leaves it.  The selection then starts at its threshold step,
-                               and the counters are zero again when the call has run (ready for the next step). */
+  uint32_t* digit_hist;     /* NULL, or [rows, 2048]: the first-digit histogram of the scores of each row, as
+                               mxb_indexer_scores leaves it.  The selection does not need it any more; the counters
+                               are zero again when the call has run (ready for the next step). */
 } mxb_topk_args;
 
 int64_t mxb_topk_workspace_bytes(int32_t rows, int64_t n, int32_t k);

@@ -120,9 +120,8 @@ class SparseDecodePlan:
         self._dtypes = (q_dtype, q_dtype, torch.float32)
         self.packed = torch.zeros(self._offs[2] + (nw + 255) // 256 * 256, dtype=torch.uint8, device=dev)
         self.q, self.idx_q, self.idx_w = self._views(self.packed)
-        # Optional: the scan counts the selection's first radix digit (scratch, zero between steps).  Off by
-        # default: on a B200 the scan is co-limited by instruction issue, and the extra key + shared-memory atomic
-        # per score cost it more (37.8 -> 42.2 us at batch 32 x 82 K rows) than the selection saved (20.5 -> 19.3 us).
+        # Optional: the scan counts the scores' first radix digit (scratch, zero between steps).  The selection takes
+        # the counters and clears them, but has no use for them: off by default.
         self.digit_hist = None
         if count_digits_in_scan and scan_counts_digits(self.idx_q[:, :, None, :], cache.idx_keys, n_tokens=1, ratio=0):
             self.digit_hist = torch.zeros((B, DIGIT_BINS), dtype=torch.int32, device=dev)
