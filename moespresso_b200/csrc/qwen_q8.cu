@@ -644,6 +644,9 @@ extern "C" int mxb_affine_q8_append(const mxb_affine_q8_pair_args* a, void* stre
 extern "C" int mxb_affine_q8_expand(const mxb_affine_q8_pair_args* a, void* stream) {
   int rc = q8_pair_check(a, "affine q8 expand");
   if (rc != MXB_OK) return rc;
+  // rows that overlap would be written by several warps
+  MXB_REQUIRE((a->n_rows + a->n_tail == 1 || a->x_row_stride >= a->width) && (a->heads == 1 || a->x_head_stride >= a->width),
+              MXB_ERR_INVALID, "affine q8 expand: output rows must not overlap (strides of at least the width)");
   return launch_dequantize(two_tensors(a), 2, a->sb_dtype, a->x_dtype, reinterpret_cast<cudaStream_t>(stream));
 }
 

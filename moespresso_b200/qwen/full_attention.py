@@ -112,6 +112,8 @@ def dequantize_affine_q8(packed, scales, biases, *, dtype=None, out=None):
     D = int(packed.shape[-1]) * 4
     n = int(packed.numel() // (D // 4))
     lead = tuple(packed.shape[:-1])
+    if any(t.numel() * Q8_GROUP != n * D for t in (scales, biases)):
+        raise ValueError("scales and biases must hold one value per group of 64 features of every packed row")
     if out is None:
         out = torch.empty((n, D), dtype=dtype or scales.dtype, device=dev)
         ret = out.reshape(*lead, D)
@@ -135,16 +137,24 @@ def _q8_call(name, rows, row_stride, packed, scales, biases, n, D):
 
 def _q8_head_rows(tensors) -> int:
     """Rows between consecutive heads of (packed, scales, biases) x (keys, values), all row-contiguous views
-    ``[1, Hkv, P, w]`` of one capacity with scales of one type; 0 when they are not."""
-    heads, n = (int(x) for x in tensors[0].shape[1:3])
-    if any(t.stride(3) != 1 or t.stride(2) != t.shape[3] or tuple(t.shape[1:3]) != (heads, n) for t in tensors):
+    ``[1, Hkv, P, w]`` of one capacity and one row width, with scales of one type; 0 when they are not (the paired
+    kernels take the widths and the rows of a head on trust)."""
+    _, heads, n, words = (int(x) for x in tensors[0].shape)
+    if words * 4 % Q8_GROUP:
         return 0
-    if len({t.dtype for t in tensors[1:3] + tensors[4:6]}) != 1 or tensors[0].shape[3] != tensors[3].shape[3]:
+    rows = set()
+    for i, t in enumerate(tensors):
+        w = words * 4 // Q8_GROUP if i % 3 else words
+        _, st_head, st_row, st = t.stride()
+        if st != 1 or st_row != w or t.shape[1:] != (heads, n, w) or (i % 3 == 0 and t.element_size() != 4):
+            return 0
+        rows.add(divmod(st_head, w))
+    if len({t.dtype for t in tensors[1:3] + tensors[4:6]}) != 1:
         return 0
     if heads == 1:
         return n
-    rows = {divmod(int(t.stride(1)), int(t.shape[3])) for t in tensors}
-    return max(0, rows.pop()[0]) if len(rows) == 1 and next(iter(rows))[1] == 0 else 0
+    head_rows, rest = rows.pop()
+    return head_rows if not rows and rest == 0 and head_rows >= n else 0
 
 
 def _q8_pair(name, rows, head_stride, row_stride, k_store, v_store, head_rows, row0, n_rows, tails=None):
@@ -246,7 +256,7 @@ def sdpa_fa_prefill_q8(queries, k_packed, k_scales, k_biases, v_packed, v_scales
         self_k, self_v = self_k.contiguous(), self_v.contiguous()
     past = (k_packed, k_scales, k_biases, v_packed, v_scales, v_biases)
     require_cuda(queries, self_k, self_v, *past)
-    head_rows = _q8_head_rows(past) if P else 0
+    head_rows = _q8_head_rows(past) if P and 4 * int(k_packed.shape[3]) == D else 0
     same = tuple(self_k.shape) == tuple(self_v.shape) == (Hkv, L, D)
     if head_rows and same:
         _q8_pair("affine_q8_expand", (kfull, vfull), (P + L) * D, D, past[:3], past[3:], head_rows, 0, P, (self_k, self_v))
