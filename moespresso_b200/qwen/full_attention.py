@@ -251,16 +251,17 @@ def sdpa_fa_prefill_q8(queries, k_packed, k_scales, k_biases, v_packed, v_scales
     op = self_k.dtype if self_k.dtype in (torch.bfloat16, torch.float16) else torch.bfloat16
     kfull = torch.empty((Hkv, P + L, D), dtype=op, device=dev)
     vfull = torch.empty_like(kfull)
-    self_k, self_v = self_k[0].to(op), self_v[0].to(op)
-    if self_k.stride() != self_v.stride() or self_k.stride(-1) != 1:
-        self_k, self_v = self_k.contiguous(), self_v.contiguous()
+    self_k, self_v = self_k[0], self_v[0]
     past = (k_packed, k_scales, k_biases, v_packed, v_scales, v_biases)
-    require_cuda(queries, self_k, self_v, *past)
-    head_rows = _q8_head_rows(past) if P and 4 * int(k_packed.shape[3]) == D else 0
-    same = tuple(self_k.shape) == tuple(self_v.shape) == (Hkv, L, D)
-    if head_rows and same:
+    paired = (P and 4 * int(k_packed.shape[3]) == D and tuple(self_k.shape) == tuple(self_v.shape) == (Hkv, L, D) and
+              all(t.device == dev for t in (self_k, self_v, *past)))
+    head_rows = _q8_head_rows(past) if paired else 0
+    if head_rows:
+        self_k, self_v = self_k.to(op), self_v.to(op)
+        if self_k.stride() != self_v.stride() or self_k.stride(-1) != 1:
+            self_k, self_v = self_k.contiguous(), self_v.contiguous()
         _q8_pair("affine_q8_expand", (kfull, vfull), (P + L) * D, D, past[:3], past[3:], head_rows, 0, P, (self_k, self_v))
-    else:
+    else:                                  # no past, layouts of several kinds, a chunk that broadcasts or comes from the host
         for h in range(Hkv):
             if P:
                 dequantize_affine_q8(k_packed[0, h], k_scales[0, h], k_biases[0, h], out=kfull[h, :P])

@@ -31,6 +31,28 @@ def test_past_of_another_width_is_refused(monkeypatch, words, groups):
         fa.sdpa_fa_prefill_q8(torch.zeros(1, 4, 3, 256, dtype=BF), *_past(2, 5, words, groups), chunk, chunk, 1 / 16)
 
 
+@pytest.mark.parametrize("P", [0, 5])
+def test_empty_past_and_chunk_that_broadcasts(monkeypatch, P):
+    """Of an empty past nothing is read, so its tensors may be anywhere ("cpu" stands for the device here, "meta" for
+    another place); values of one head for both are copied like any others."""
+    operand = {}
+    monkeypatch.setattr(fa, "dequantize_affine_q8", lambda *q8, out: out.fill_(7))
+    monkeypatch.setattr(fa, "_q8_pair", lambda *a, **k: pytest.fail("the paired kernel needs whole rows on one device"))
+    monkeypatch.setattr(fa, "sdpa_fa_prefill", lambda q, k, v, scale, **kw: operand.update(k=k, v=v) or q)
+
+    def require(*tensors):
+        assert all(t.device.type == "cpu" for t in tensors)
+        return torch.device("cpu")
+    monkeypatch.setattr(fa, "require_cuda", require)
+    chunk = torch.arange(2 * 3 * 256).reshape(1, 2, 3, 256).remainder(9).to(BF)
+    past = _past(2, P, 64, 4)
+    out = fa.sdpa_fa_prefill_q8(torch.zeros(1, 4, 3, 256, dtype=BF), past[0], *(t if P else t.to("meta") for t in past[1:]),
+                                chunk, chunk[:, :1] if P else chunk, 1 / 16)
+    assert tuple(out.shape) == (1, 4, 3, 256) and tuple(operand["k"].shape) == (P + 3, 2, 256)
+    assert torch.equal(operand["k"][P:], chunk[0].transpose(0, 1)) and bool((operand["k"][:P] == 7).all())
+    assert torch.equal(operand["v"][P:, 1], chunk[0, 0 if P else 1])
+
+
 def test_expansion_refuses_output_rows_that_overlap():
     from moespresso_b200 import _abi
     lib = _abi.load()
