@@ -139,22 +139,20 @@ def _q8_head_rows(tensors) -> int:
     """Rows between consecutive heads of (packed, scales, biases) x (keys, values), all row-contiguous views
     ``[1, Hkv, P, w]`` of one capacity and one row width, with scales of one type; 0 when they are not (the paired
     kernels take the widths and the rows of a head on trust)."""
-    _, heads, n, words = (int(x) for x in tensors[0].shape)
-    if words * 4 % Q8_GROUP:
-        return 0
-    rows = set()
-    for i, t in enumerate(tensors):
-        w = words * 4 // Q8_GROUP if i % 3 else words
-        _, st_head, st_row, st = t.stride()
-        if st != 1 or st_row != w or t.shape[1:] != (heads, n, w) or (i % 3 == 0 and t.element_size() != 4):
-            return 0
-        rows.add(divmod(st_head, w))
-    if len({t.dtype for t in tensors[1:3] + tensors[4:6]}) != 1:
+    kp, ks, kb, vp, vs, vb = tensors
+    _, heads, n, words = shape = kp.shape
+    strides, groups = kp.stride(), words * 4 // Q8_GROUP
+    s_shape, s_strides, dt = ks.shape, ks.stride(), ks.dtype
+    if (words % 16 or vp.shape != shape or s_shape[1:] != (heads, n, groups) or
+            not (kb.shape == vs.shape == vb.shape == s_shape) or
+            strides[2:] != (words, 1) or vp.stride() != strides or
+            s_strides[2:] != (groups, 1) or not (kb.stride() == vs.stride() == vb.stride() == s_strides) or
+            not (kb.dtype == vs.dtype == vb.dtype == dt) or kp.element_size() != 4 or vp.element_size() != 4):
         return 0
     if heads == 1:
         return n
-    head_rows, rest = rows.pop()
-    return head_rows if not rows and rest == 0 and head_rows >= n else 0
+    head_rows, rest = divmod(strides[1], words)
+    return head_rows if rest == 0 and head_rows >= n and s_strides[1] == head_rows * groups else 0
 
 
 def _q8_pair(name, rows, head_stride, row_stride, k_store, v_store, head_rows, row0, n_rows, tails=None):
@@ -199,18 +197,23 @@ class QuantizedKVCache:
         L = int(keys.shape[2])
         if self.offset + L > self.capacity:
             raise ValueError("QuantizedKVCache capacity exceeded")
-        dt = self.keys[1].dtype
-        keys, values = keys.to(dt), values.to(dt)
-        shape = (1, int(self.keys[0].shape[1]), L, 4 * int(self.keys[0].shape[3]))
-        if L and tuple(keys.shape) == shape and tuple(values.shape) == shape and keys.device == self.keys[0].device:
+        stores, words = (*self.keys, *self.values), self.keys[0]
+        dev, shape = words.device, (1, int(words.shape[1]), L, 4 * int(words.shape[3]))
+        # the paired kernel writes whole rows of both tensors by address; the stores are public and may have been replaced
+        paired = (L and 0 <= self.offset <= words.shape[2] - L and words.shape[0] == 1 and
+                  keys.shape == shape and values.shape == shape and all(t.device == dev for t in (keys, values, *stores)))
+        head_rows = _q8_head_rows(stores) if paired else 0
+        if head_rows:
+            dt = stores[1].dtype
+            keys, values = keys.to(dt), values.to(dt)
             if keys.stride() != values.stride() or keys.stride(3) != 1:
                 keys, values = keys.contiguous(), values.contiguous()
-            require_cuda(keys, values, self.keys[0])
+            require_cuda(keys)
             _q8_pair("affine_q8_append", (keys, values), keys.stride(1), keys.stride(2), self.keys, self.values,
-                     self.capacity, self.offset, L)
-        else:                                  # shapes that broadcast into the cache, rows of another device
+                     head_rows, self.offset, L)
+        else:                                  # rows that broadcast into the cache or come from elsewhere, other layouts
             for store, x in ((self.keys, keys), (self.values, values)):
-                for dst, src in zip(store, quantize_affine_q8(x)):
+                for dst, src in zip(store, quantize_affine_q8(x.to(store[1].dtype))):
                     dst[:, :, self.offset:self.offset + L].copy_(src)
         self.offset += L
         return self._prefix(self.offset)

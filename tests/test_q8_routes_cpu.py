@@ -65,3 +65,42 @@ def test_expansion_refuses_output_rows_that_overlap():
     a.x_head_stride, a.x_row_stride = 5 * 256, 256
     assert lib.mxb_affine_q8_expand(C.byref(a), None) == -1
     assert b"must not overlap" in lib.mxb_last_error()
+
+
+def _wide(stores):       # views of the first rows of longer buffers
+    out = []
+    for t in stores:
+        big = torch.zeros(1, t.shape[1], 50, t.shape[3], dtype=t.dtype)
+        out.append(big[:, :, :t.shape[2]])
+    return out
+
+
+@pytest.mark.parametrize("layout,head_rows", [
+    (lambda six: six, 20),                                                           # as allocated
+    (lambda six: _wide(six), 50),
+    (lambda six: [t[:, :, :9].clone() for t in six], 9),                              # compact copies of fewer rows
+    (lambda six: [t.transpose(1, 2).contiguous().transpose(1, 2) for t in six], 0),   # rows outside heads
+    (lambda six: [*six[:3], *_wide(six[3:])], 0),                                    # values laid out unlike the keys
+    (lambda six: [*six[:4], *(t.float() for t in six[4:])], 0),                      # scales of two types
+    (lambda six: [torch.cat([t, t]) for t in six], 0),                               # two batch entries: rows broadcast
+])
+def test_append_follows_the_stores(monkeypatch, layout, head_rows):
+    """``keys`` and ``values`` are public: the paired append must go by what they are, and leave to the copies what it
+    cannot address."""
+    def quantize(x):      # any three values of the right shapes and types
+        return x[..., ::4].to(torch.int32), x[..., ::64], -x[..., ::64]
+    launches = []
+    monkeypatch.setattr(fa, "quantize_affine_q8", quantize)
+    monkeypatch.setattr(fa, "require_cuda", lambda *tensors: torch.device("cpu"))
+    monkeypatch.setattr(fa, "_q8_pair", lambda *a: launches.append(a[6:9]))
+    cache = fa.QuantizedKVCache(2, 256, 20, device="cpu")
+    six = layout([*cache.keys, *cache.values])
+    cache.keys, cache.values, cache.offset = tuple(six[:3]), tuple(six[3:]), 4
+    rows = [torch.randint(1, 100, (1, 2, 5, 256)).float() for _ in range(2)]
+    cache.update_and_fetch(*rows)
+    assert cache.offset == 9 and launches == ([(head_rows, 4, 5)] if head_rows else [])
+    if not head_rows:
+        for store, x in zip((cache.keys, cache.values), rows):
+            for got, want in zip(store, quantize(x.to(store[1].dtype))):
+                assert torch.equal(got[:, :, 4:9], want.expand(got.shape[0], -1, -1, -1))
+                assert not got[:, :, :4].any() and not got[:, :, 9:].any()
