@@ -185,7 +185,7 @@ class QuantizedKVCache:
         self.values = (mk(head_dim // 4, torch.int32), mk(head_dim // Q8_GROUP, dtype), mk(head_dim // Q8_GROUP, dtype))
 
     def _prefix(self, n):
-        return tuple(t.narrow(2, 0, n) for t in self.keys), tuple(t.narrow(2, 0, n) for t in self.values)
+        return tuple(t[:, :, :n] for t in self.keys), tuple(t[:, :, :n] for t in self.values)   # (an offset past the stores clips)
 
     @property
     def state(self):

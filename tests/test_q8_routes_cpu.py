@@ -104,3 +104,11 @@ def test_append_follows_the_stores(monkeypatch, layout, head_rows):
             for got, want in zip(store, quantize(x.to(store[1].dtype))):
                 assert torch.equal(got[:, :, 4:9], want.expand(got.shape[0], -1, -1, -1))
                 assert not got[:, :, :4].any() and not got[:, :, 9:].any()
+
+
+def test_state_of_an_offset_past_the_stores_clips():
+    """A program that trims the stores and keeps counting gets the rows there are, as from any slice."""
+    cache = fa.QuantizedKVCache(2, 256, 20, device="cpu")
+    cache.keys, cache.values = (tuple(t[:, :, :9] for t in six) for six in (cache.keys, cache.values))
+    cache.offset = 12
+    assert all(t.shape[2] == 9 for six in cache.state for t in six)
