@@ -26,7 +26,8 @@ def topk_select(scores, k: int, *, valid=None, row_start=None, n=None, order: st
     attention kernels walk); ``order="score"``: descending score, ties by ascending id
     (the order of the NumPy contract).  Returns int32 ``[..., k]``.  ``digit_hist``: int32 ``[rows, 2048]`` as
     ``indexer_scores(..., digit_hist=)`` left it; the selection does not need it (it did as a radix select) and
-    leaves the counters at zero for the next step.  ``out``: contiguous int32 ``[rows, k]`` to write the ids to.
+    leaves the counters at zero for the next step.  ``out``: contiguous int32 ``[rows, k]`` to write the ids to, in
+    either order.
     """
     dev = require_cuda(scores)
     if scores.dtype != torch.float32:
@@ -74,7 +75,7 @@ def topk_select(scores, k: int, *, valid=None, row_start=None, n=None, order: st
         picked = torch.gather(flat, 1, ids.clamp(min=0))
         picked = torch.where(ids >= 0, picked, torch.full_like(picked, float("-inf")))
         perm = torch.sort(picked, dim=1, descending=True, stable=True).indices
-        out = torch.gather(ids, 1, perm).to(torch.int32).reshape(*lead, int(k))
+        out.copy_(torch.gather(ids, 1, perm).reshape(out.shape))
     elif order != "index":
         raise ValueError("order must be 'index' or 'score'")
     return out
