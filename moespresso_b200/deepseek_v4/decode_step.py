@@ -152,6 +152,7 @@ class SparseDecodePlan:
         self._q_copied = torch.cuda.Event()
         self._attend_done = torch.cuda.Event()
         self._attend_done.record(torch.cuda.current_stream(dev))
+        self._q_on_main = False      # the current stream has written or read q since _attend_done was recorded
 
     def _views(self, buf):
         return tuple(buf[o:o + n].view(dt).view(sh)
@@ -173,6 +174,10 @@ class SparseDecodePlan:
             self.packed.copy_(host_buf, non_blocking=True)
             return self.launch()
         from .. import _abi
+        if self._q_on_main:        # run(), launch() or load_inputs() since the last step fed this way
+            self._copy_stream.wait_event(self._attend_done)
+            self._attend_done.record(main)
+            self._q_on_main = False
         self.packed[nq:].copy_(host_buf[nq:], non_blocking=True)       # selection inputs first: the device starts at once
         self._graph_select.replay()
         self._copy_stream.wait_event(self._attend_done)                # the previous step's attention has read q
@@ -204,6 +209,7 @@ class SparseDecodePlan:
 
     def load_inputs(self, q, idx_q, idx_w) -> None:
         """Copy one step's inputs (device or pinned-host tensors) into the plan's buffers."""
+        self._q_on_main = True
         pairs = ((self.q, q), (self.idx_q, idx_q), (self.idx_w, idx_w))
         if torch.cuda.current_device() == self.q.device.index and all(
                isinstance(s, torch.Tensor) and s.device == d.device and s.dtype == d.dtype and s.shape == d.shape
@@ -221,6 +227,7 @@ class SparseDecodePlan:
 
     def launch(self):
         """Run the step on the inputs currently in the plan's buffers; returns out [B,H,d_v]."""
+        self._q_on_main = True
         if self.graph is not None:
             self.graph.replay()
         else:
