@@ -678,9 +678,12 @@ int topk_pivot_size(int32_t rows, int64_t n) {
 template <bool CLUSTER, int NT, int SAMPLES>
 static int launch_pivot(const TopkPivotParams& p, int rows, int cs, cudaStream_t st) {
   auto kern = topk_pivot_kernel<CLUSTER, NT, SAMPLES>;
+  if (cs > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return MXB_ERR_UNSUPPORTED;
+  }
   const size_t smem = ((size_t)2 * kBigBins + (size_t)p.cap * (CLUSTER ? 3 : 2) + (size_t)2 * (p.part / 32)) * 4;
   MXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  if (cs > 8) MXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((int64_t)rows * cs));
   cfg.blockDim = dim3(NT);
@@ -693,12 +696,20 @@ static int launch_pivot(const TopkPivotParams& p, int rows, int cs, cudaStream_t
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = CLUSTER ? 1 : 0;
+  if (cs > 8) {   // sixteen SMs of one GPC are not there on every device or SM set
+    int resident = 0;
+    if (cudaOccupancyMaxActiveClusters(&resident, kern, &cfg) != cudaSuccess || resident < 1) {
+      (void)cudaGetLastError();
+      return MXB_ERR_UNSUPPORTED;
+    }
+  }
   MXB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, p));
   note_launch();
   return MXB_OK;
 }
 
-int launch_topk_pivot(const mxb_topk_args* a, int cs, cudaStream_t st) {
+// MXB_ERR_UNSUPPORTED: no room for clusters of that size, nothing was launched
+static int launch_topk_clusters(const mxb_topk_args* a, int cs, cudaStream_t st) {
   TopkPivotParams p{};
   p.scores = a->scores; p.row_stride = a->row_stride; p.row_start = a->row_start; p.row_count = a->row_count;
   p.out_ids = a->out_ids; p.n = a->n; p.k = a->k;
@@ -734,7 +745,14 @@ int launch_topk_pivot(const mxb_topk_args* a, int cs, cudaStream_t st) {
     case -2: return launch_pivot<false, 512, 2>(p, a->rows, cs, st);
     case -8: return launch_pivot<false, 512, 8>(p, a->rows, cs, st);
   }
-  return fail(MXB_ERR_UNSUPPORTED, "topk: no kernel for %d samples", samples);
+  return fail(MXB_ERR_INVALID, "topk: no kernel for %d samples", samples);
+}
+
+// MXB_ERR_UNSUPPORTED: the row needs clusters of a size that the device has no room for
+int launch_topk_pivot(const mxb_topk_args* a, int cs, cudaStream_t st) {
+  int rc = launch_topk_clusters(a, cs, st);
+  if (rc == MXB_ERR_UNSUPPORTED && cs > 8 && a->n <= (int64_t)8 * kPPartMax) rc = launch_topk_clusters(a, 8, st);
+  return rc;
 }
 
 }  // namespace mxb

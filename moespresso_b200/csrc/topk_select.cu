@@ -228,8 +228,9 @@ using namespace mxb;
 
 extern "C" int64_t mxb_topk_workspace_bytes(int32_t rows, int64_t n, int32_t k) {
   if (rows <= 0 || n <= 0 || k <= 0) return 0;
-  // What the general path (topk_multi.cu) needs.  The pivot kernel uses none of it; rows above kNoScratchMax keep
-  // reporting it all the same, because callers size pools by this answer and it is part of the interface.
+  // What the general path (topk_multi.cu) needs.  The pivot kernel uses none of it, but the longest of its rows need
+  // clusters of 16 CTAs, and where there is no room for one the general path takes them.  (Callers size pools by this
+  // answer: the limit has stayed where it was when the general path took all rows above it.)
   constexpr int64_t kNoScratchMax = 360448;
   if (topk_pivot_size(rows, n) > 0 && n <= kNoScratchMax) return 0;
   return topk_multi_workspace(rows, n, k);
@@ -244,7 +245,10 @@ extern "C" int mxb_topk_select(const mxb_topk_args* a, void* stream) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   // these kernels count for themselves: only keep the promise that the counters end up clear
   if (a->digit_hist) MXB_CUDA_OK(cudaMemsetAsync(a->digit_hist, 0, (size_t)a->rows * kBigBins * sizeof(uint32_t), st));
-  if (const int cs = topk_pivot_size(a->rows, a->n)) return launch_topk_pivot(a, cs, st);
+  if (const int cs = topk_pivot_size(a->rows, a->n)) {
+    const int rc = launch_topk_pivot(a, cs, st);
+    if (rc != MXB_ERR_UNSUPPORTED) return rc;
+  }
   return launch_topk_multi(a, st);
 }
 

@@ -112,3 +112,19 @@ def test_operator_pair_and_fused_struct_layouts_match_c(tmp_path):
     subprocess.run(["gcc", str(src), "-o", str(exe)], check=True)
     got = [int(x) for x in subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()]
     assert got == [n for _, cls in pairs for n in [C.sizeof(cls)] + [getattr(cls, f[0]).offset for f in cls._fields_]]
+
+
+def test_longest_rows_go_to_the_general_selection_where_their_clusters_do_not_fit():
+    """Rows of 2^20 to 2^21 scores take clusters of 16 CTAs.  No device at all has no room for one either: the call must
+    arrive at the path that needs the workspace it reported, not end in a CUDA error."""
+    import torch
+    if torch.cuda.is_available():
+        pytest.skip("made-up addresses: for machines without a device")
+    from moespresso_b200 import _abi
+    lib = _abi.load()
+    a = _abi.TopkArgs()
+    a.scores, a.out_ids, a.rows, a.n, a.k = 4096, 4096, 1, 1 << 21, 2048
+    a.row_stride = a.n
+    assert lib.mxb_topk_workspace_bytes(a.rows, a.n, a.k) > 0
+    assert lib.mxb_topk_select(C.byref(a), None) == -3
+    assert b"workspace of" in lib.mxb_last_error()

@@ -73,6 +73,7 @@ def test_many_rows_small_clusters(n, k, rows):
 
 @pytest.mark.parametrize("n,k,rows", [(7901, 512, 2), (8191, 512, 2), (8192, 8192, 1), (8193, 2048, 3), (16384, 2048, 160),
                                       (16385, 8192, 1), (32767, 16, 33), (131072, 2048, 20), (300001, 8192, 2),
+                                      (1 << 20, 2048, 5),    # eight CTAs per row, each with the longest part there is
                                       (1 << 21, 2048, 1), ((1 << 21) + 1, 2048, 1)])
 def test_direct_and_sampled_rows(n, k, rows):
     """Either side of the direct kernel's sizes, of the cluster sizes and of the longest sampled row; random rows, and
