@@ -644,12 +644,20 @@ using namespace mxb;
 
 // How the items are dealt out.  Costs are in tiles (0.9 to 1.05 us each on a B200): a segment costs its tiles and
 // kSegCost for its Q load, first scores and drain; cutting costs kCutCost (partials out, merge launch, partials in), and
-// tiles take a tenth longer when every SM streams K and V at once.  Stretches of less than kMinShare are not worth an
-// SM of their own.  Measured (16 query / 2 KV heads, bf16, gated; tokens over past, us, one CTA per item against equal
-// stretches): 64 over 3,000 51.1 / 27.6, 64 over 30,000 404 / 74.4, 100 over 8,000 122 / 33.7, 1,200 over 4,000 132 / 105,
-// 1,500 over 7,000 221 / 183, 2,048 over 30,720 1,091 / 1,001; on the other side of the rule 700 over 1,365 39.8 / 44.2,
-// 1,000 over 1,000 40.5 / 47.5, 2,048 over 5,000 182 / 192.
-constexpr int kSegCost = 4, kCutCost = 16, kMinShare = 12;
+// the stretches must be kSaving percent shorter than the SM with the most whole items works.  That much, because tiles
+// take a tenth longer when every SM streams K and V at once, and because a cut saves time and not energy: back to back,
+// under the power cap, the SMs that idle behind whole items leave the others a higher clock.  Stretches of less than
+// kMinShare are not worth an SM of their own.  Measured (16 query / 2 KV heads, bf16, gated; tokens over past, us, one
+// CTA per item against equal stretches, alone / back to back for half a second):
+//   64 over 3,000 51.1 -> 27.6 and 64 over 30,000 404 -> 74.4 alone; 500 over 30,000 531 -> 264 / 508 -> 290;
+//   1,200 over 30,000 1,082 -> 633 / 1,011 -> 692; 1,700 over 30,000 (saving 29 %) 1,092 -> 864 / 1,073 -> 958;
+//   1,900 over 30,000 (21 %) 1,112 -> 936 / 1,106 -> 1,037;
+// below the line 2,048 over 30,720 (13 %) 1,136 -> 1,038 / 1,154 -> 1,140; 3,000 over 8,000 (11 %) 458 -> 429 / 477 -> 495;
+//   5,000 over 8,000 (10 %) 808 -> 778 / 871 -> 898; 32 heads, 2,048 over 30,720 (14 %) 2,267 -> 2,442;
+//   700 over 1,365 39.8 -> 44.2 and 1,000 over 1,000 40.5 -> 47.5 alone.
+// A cut changes the results in the last bits (P is rounded to 16 bits against each segment's own reference; the error
+// against float64 stays the same, 2.31e-3 relative in bf16 on either side).  The partials take up to 39 MB (296 slots).
+constexpr int kSegCost = 4, kCutCost = 16, kMinShare = 12, kSaving = 15;
 
 // Fills p.n_bins / p.bin_start (n_bins = 0: one CTA per item) and returns the bytes of partials the plan needs.
 static int64_t flash_plan(FlashParams& p, int sms) {
@@ -677,7 +685,7 @@ static int64_t flash_plan(FlashParams& p, int sms) {
     }
   }
   const int bins = (int)(total / kMinShare < sms ? total / kMinShare : sms);
-  if (bins < 2 || 10 * (int64_t)longest <= 11 * (total / bins) + 10 * kCutCost) return 0;
+  if (bins < 2 || 100 * (int64_t)longest <= (100 + kSaving) * (total / bins) + 100 * kCutCost) return 0;
   // Equal stretches of the items' costs.  A piece of fewer than kSegCost tiles is not worth a segment: the boundary
   // moves to the item's edge.
   uint32_t* start = p.bin_start;

@@ -128,3 +128,18 @@ def test_longest_rows_go_to_the_general_selection_where_their_clusters_do_not_fi
     assert lib.mxb_topk_workspace_bytes(a.rows, a.n, a.k) > 0
     assert lib.mxb_topk_select(C.byref(a), None) == -3
     assert b"workspace of" in lib.mxb_last_error()
+
+
+@pytest.mark.parametrize("S,past,Hq,cut", [
+    (64, 3000, 16, True), (500, 30000, 16, True), (1200, 4000, 16, True), (1900, 30000, 16, True),
+    (2048, 30720, 16, False), (2048, 30720, 32, False), (3000, 8000, 16, False), (700, 1365, 16, False), (8192, 0, 16, False),
+])
+def test_flash_items_are_cut_only_for_a_clear_saving(S, past, Hq, cut):
+    """Workspace (partials of cut items) on either side of the rule on 148 SMs: a cut that saves time but no energy is
+    slower under the power cap, and uncut items keep one order of summation."""
+    from moespresso_b200 import _abi
+    lib = _abi.load()
+    a = _abi.FlashPrefillArgs()
+    a.D, a.dtype, a.S, a.Skv, a.Hq, a.Hkv = 256, _abi.BF16, S, S + past, Hq, 2
+    a.q = a.k = a.v = a.out = 4096
+    assert (lib.mxb_flash_prefill_workspace_bytes(C.byref(a)) > 0) == cut
