@@ -163,3 +163,79 @@ def test_plan_takes_inputs_of_every_layout():
     for args in ((q.float(), iq, iw), (q.transpose(1, 2).contiguous().transpose(1, 2), iq, iw), (q.cpu(), iq, iw.cpu())):
         plan.packed.zero_()
         assert torch.equal(plan.run(*args), want)
+
+
+def _plan_over(batch, rows, k, kv):
+    from moespresso_b200.deepseek_v4.decode_step import SparseDecodePlan
+    g = torch.Generator(device="cuda").manual_seed(batch + rows)
+    mk = lambda *s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
+    n = batch * rows
+    lens = torch.full((batch,), rows, dtype=torch.int32, device="cuda")
+    cache = LatentCache(kv=mk(n, 576).mul(30).clamp(-127, 127).to(torch.int8) if kv == "int8" else mk(n, 576).to(torch.bfloat16),
+                        kv_scales=(0.01 + 0.02 * torch.rand(n, generator=g, device="cuda")).half() if kv == "int8" else None,
+                        idx_keys=mk(n, 64).to(torch.float8_e4m3fn), row_count=lens, max_rows=rows,
+                        row_start=torch.arange(batch, dtype=torch.int64, device="cuda") * rows)
+    plan = SparseDecodePlan(cache, heads=64, d_qk=576, idx_heads=16, idx_dim=64, k=k, scale=576 ** -0.5, d_v=512)
+    inputs = [(mk(batch, 64, 576).bfloat16(), mk(batch, 16, 64).bfloat16(), mk(batch, 16)) for _ in range(4)]
+    return cache, plan, inputs
+
+
+@pytest.mark.parametrize("batch,rows,k,kv", [
+    (1, 3000, 512, "int8"),        # selection of one CTA, most SMs free for the attention to set up on
+    (1, 3000, 512, "bf16"),
+    (3, 20000, 512, "bf16"),       # clusters
+    (40, 20000, 2048, "int8"),     # a partial selection wave, splits in clusters
+    (150, 3000, 512, "bf16"),      # more tokens than SMs
+])
+def test_early_start_behind_the_selection_gives_the_same_bits(batch, rows, k, kv):
+    """The attention may start while the selection finishes.  Steps with changing inputs, one after another without a
+    wait, against the selection and an attention that waits: the ids and outputs of every step."""
+    need_gpu()
+    from moespresso_b200.deepseek_v4.attention import topk_select
+    from moespresso_b200.deepseek_v4.indexed_attention_kernel import indexer_scores, sparse_attention
+    cache, plan, inputs = _plan_over(batch, rows, k, kv)
+    want = []
+    for q, iq, iw in inputs:
+        scores = indexer_scores(iq[:, :, None], iw[:, None], cache.idx_keys, n_rows=rows, row_start=cache.row_start,
+                                row_count=cache.row_count)
+        ids = topk_select(scores, k, valid=cache.row_count, row_start=cache.row_start, n=rows)
+        torch.cuda.synchronize()
+        out = sparse_attention(q[:, :, None], cache.kv, ids[:, None], None, pos0=0, window=0, ratio=0, scale=576 ** -0.5,
+                               d_v=512, kv_scales=cache.kv_scales, comp_row_start=cache.row_start,
+                               comp_row_count=cache.row_count, n_comp=rows)
+        want.append((ids, out[:, :, 0]))
+    bad = torch.zeros((), dtype=torch.int64, device="cuda")
+    for step in range(200):
+        i = (step * 7 + step // 5) % len(inputs)
+        if step % 2:
+            out, ids = plan.run(*inputs[i]), plan.ids
+        else:
+            out, ids = sparse_decode_step(*inputs[i], cache, k=k, scale=576 ** -0.5, d_v=512, return_ids=True)
+        bad += (ids != want[i][0]).sum() + (out != want[i][1]).sum()
+    assert int(bad) == 0
+
+
+def test_host_fed_steps_between_others():
+    """run(), load_inputs() and run_packed() in turn without a wait: every step's output is its own inputs'."""
+    need_gpu()
+    _, plan, inputs = _plan_over(32, 30000, 512, "bf16")
+    want = []
+    for x in inputs:
+        want.append(plan.run(*x).clone())
+        torch.cuda.synchronize()
+    host = []
+    for x in inputs:
+        buf, views = plan.host_buffer()
+        for v, t in zip(views, x):
+            v.copy_(t.cpu())
+        host.append(buf)
+    outs = []
+    for step in range(60):
+        i, j = step % 4, (step + 1 + step // 4) % 4
+        outs.append((j, plan.run(*inputs[j]).clone()) if step % 3 else (j, None))
+        if not step % 3:
+            plan.load_inputs(*inputs[j])
+        outs.append((i, plan.run_packed(host[i]).clone()))
+    torch.cuda.synchronize()
+    for i, out in outs:
+        assert out is None or torch.equal(out, want[i])

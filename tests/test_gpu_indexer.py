@@ -43,7 +43,7 @@ def test_exact_fp32_matches_oracle(B, H, T, D, R, pos0, ratio):
 @pytest.mark.parametrize("form", ["bf16", "f16", "fp8_bf16", "fp8_f16"])
 @pytest.mark.parametrize("B,H,T,D,R,pos0,ratio", [
     (1, 16, 1, 64, 4096, 0, 0),
-    (2, 16, 40, 64, 1000, 3000, 4),      # token tiles (16 tokens x 16 heads = 256 columns), ragged last tile
+    (2, 16, 40, 64, 1000, 3000, 4),      # token tiles x 16 heads: 16 tokens and a ragged last tile for FP8 keys, 8 for 16-bit ones
     (1, 64, 7, 128, 700, 2500, 4),       # D = 128 (two swizzle slabs), 64 heads
     (3, 32, 1, 64, 129, 0, 0),
     (2, 16, 1, 64, 1000, 1500, 4),       # one token WITH the causal row mask: rows >= (1500 + 1) // 4 are -inf
@@ -154,3 +154,47 @@ def test_exact_scores_of_one_token_have_the_bits_of_a_chunk(D, H, rows, qdt, kdt
     two = iak.indexer_scores(q.expand(1, H, 2, D).contiguous(), w.expand(1, 2, H).contiguous(), keys, n_rows=rows,
                              exact_fp32=True)
     assert torch.equal(one.reshape(-1), two.reshape(2, rows)[0])
+
+
+@pytest.mark.parametrize("form", ["bf16", "f16"])
+@pytest.mark.parametrize("H,T,R", [
+    (16, 9, 2049),    # 8 + 1 tokens: the second tile's drain groups 1-3 have none, group 0 has one
+    (16, 13, 700),    # a group with one token of its two between full and empty groups
+    (16, 15, 2049),   # the last group has one; 17 row tiles wrap the ring of four accumulators, the last holds one row
+    (16, 41, 4096),
+    (32, 7, 2049),    # four tokens of 32 heads per tile, the last tile ragged
+    (64, 3, 1025),    # two tokens of 64 heads
+])
+def test_partial_token_tiles_of_16bit_keys(form, H, T, R):
+    """Tiles that are not full, for the drain with the weights in registers (16 heads) and the one that reads them:
+    against the fp32 kernel on the same operands; nothing is written behind the last token or row."""
+    need_gpu()
+    dt = torch.bfloat16 if form == "bf16" else torch.float16
+    g = torch.Generator(device="cuda").manual_seed(H + T + R)
+    mk = lambda *s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
+    q, w, keys = mk(1, H, T, 64).to(dt), mk(1, T, H) / 4, mk(1, R, 64).to(dt)
+    kw = dict(pos0=2 * R, ratio=4)
+    ref = iak.indexer_scores_tiled_live(q, w, keys, exact_fp32=True, **kw)
+    store = torch.full((1, T + 3, R + 5), 12345.0, device="cuda")
+    iak.indexer_scores_tiled_live(q, w, keys, out=store[:, :T, :R], check=True, **kw)
+    got = store[:, :T, :R]
+    assert torch.equal(torch.isneginf(got), torch.isneginf(ref))
+    fin = torch.isfinite(ref)
+    np.testing.assert_allclose(got[fin].cpu().numpy(), ref[fin].cpu().numpy(), rtol=2e-4, atol=2e-3)
+    store[:, :T, :R] = 12345.0
+    assert bool((store == 12345.0).all())
+
+
+def test_more_token_tiles_than_a_grid_holds():
+    """65,535 tiles of two tokens (64 heads) and three more: the second launch continues where the first ended."""
+    need_gpu()
+    T, H, D, R = 2 * 65535 + 5, 64, 64, 33
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q = torch.randn(1, H, T, D, generator=g, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn(1, T, H, generator=g, device="cuda")
+    keys = torch.randn(1, R, D, generator=g, device="cuda").bfloat16()
+    got = iak.indexer_scores_tiled_live(q, w, keys, pos0=4 * R, ratio=4, check=True)
+    for lo in (0, 2 * 65535 - 4, 2 * 65535):     # even: the same tiles as in the whole call
+        part = iak.indexer_scores_tiled_live(q[:, :, lo:lo + 5], w[:, lo:lo + 5], keys, pos0=4 * R, ratio=4)
+        assert torch.equal(got[:, lo:lo + 5], part)
+    assert bool(torch.isfinite(got).all())

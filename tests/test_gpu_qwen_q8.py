@@ -159,3 +159,55 @@ def test_append_and_expand_of_both_tensors_at_once(dt, Hkv, L, P):
         for out, q8, tail in zip(full, (past_k, past_v), tails):
             assert torch.equal(out[:, :P], fa.dequantize_affine_q8(*(t[0].contiguous() for t in q8)))
             assert torch.equal(out[:, P:], tail)
+
+
+@pytest.mark.parametrize("width", [128, 512])
+def test_past_of_another_width_raises(width):
+    need_gpu()
+    bf, dev_ = torch.bfloat16, "cuda"
+    cache = fa.QuantizedKVCache(2, width, 40)
+    cache.update_and_fetch(*(torch.randn(1, 2, 33, width, device=dev_).to(bf) for _ in range(2)))
+    chunk = torch.randn(1, 2, 7, 256, device=dev_).to(bf)
+    with pytest.raises(ValueError):
+        fa.sdpa_fa_prefill_q8(torch.randn(1, 4, 7, 256, device=dev_).to(bf), *cache.state[0], *cache.state[1], chunk, chunk,
+                              1 / 16)
+
+
+@pytest.mark.parametrize("kind", ["compact", "rows outside heads", "longer buffers", "fp32 scales of the values"])
+def test_append_to_replaced_stores(kind):
+    """Stores that a program has put in place of the allocated ones: the same words, scales and biases in the same rows."""
+    need_gpu()
+    bf = torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(4)
+    past, new = ([torch.randn(1, 3, n, 256, generator=g, device="cuda").to(bf) for _ in range(2)] for n in (11, 5))
+    plain, other = fa.QuantizedKVCache(3, 256, 40), fa.QuantizedKVCache(3, 256, 40)
+    plain.update_and_fetch(*past)
+
+    def put(t):
+        if kind == "compact":
+            return t[:, :, :16].clone()
+        if kind == "rows outside heads":
+            return t.transpose(1, 2).contiguous().transpose(1, 2)
+        return torch.cat([t, t], 2)[:, :, :40]
+    other.keys, other.values, other.offset = tuple(map(put, plain.keys)), tuple(map(put, plain.values)), 11
+    if kind == "fp32 scales of the values":
+        other.values = (other.values[0], *(t.float() for t in other.values[1:]))
+    want, got = plain.update_and_fetch(*new), other.update_and_fetch(*new)
+    for a, b in zip(want[0], got[0]):
+        assert torch.equal(a, b)
+    if kind == "fp32 scales of the values":
+        p, s, b = fa.quantize_affine_q8(new[1].float())
+        assert torch.equal(got[1][0][:, :, 11:], p) and torch.equal(got[1][1][:, :, 11:], s) and torch.equal(got[1][2][:, :, 11:], b)
+    else:
+        for a, b in zip(want[1], got[1]):
+            assert torch.equal(a, b)
+
+
+def test_chunk_values_from_the_host():
+    need_gpu()
+    bf = torch.bfloat16
+    cache = fa.QuantizedKVCache(2, 256, 40)
+    cache.update_and_fetch(*(torch.randn(1, 2, 33, 256, device="cuda").to(bf) for _ in range(2)))
+    q, k, v = (torch.randn(1, n, 7, 256, device="cuda").to(bf) for n in (4, 2, 2))
+    past = (*cache.state[0], *cache.state[1])
+    assert torch.equal(fa.sdpa_fa_prefill_q8(q, *past, k, v, 1 / 16), fa.sdpa_fa_prefill_q8(q, *past, k, v.cpu(), 1 / 16))
