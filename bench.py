@@ -333,8 +333,8 @@ def main():
         torch.cuda.synchronize()
         return a.elapsed_time(b) / (5 * K) * 1e3
 
-    # The scan counts the selection's first radix digit (plan.digit_hist), so the selection cannot be replayed on
-    # its own (it clears the counters it starts from): it is timed as (scan + selection) - scan.
+    # With counters (plan.digit_hist; off by default) the selection clears what the scan has counted, so it is timed as
+    # (scan + selection) - scan.
     fused = plan.digit_hist is not None
     hist_a = torch.zeros_like(plan.digit_hist) if fused else None   # only ever added to: the scan's work is the same
     hist_b = torch.zeros_like(plan.digit_hist) if fused else None   # counted and cleared once per replay
@@ -451,7 +451,7 @@ def main():
         "stage_us": stage,
         "sparse_attn_us_rows_from_hbm": stage_rotating,   # the attention stage replayed over the four query sets in turn
         "stage_note": ("each entry point replayed as its own CUDA graph; topk_select = (scan + selection) - scan, because the "
-                       "scan counts the selection's first radix digit; sparse_attn replays the same ids (L2-warm rows); "
+                       "selection clears the scan's counters; sparse_attn replays the same ids (L2-warm rows); "
                        "sparse_attn_us_rows_from_hbm replays it over the four query sets in turn"
                        if fused else "each entry point replayed as its own CUDA graph; sparse_attn replays the same ids (L2-warm rows; "
                                "inside the timed steps, which rotate query sets, the rows come from HBM: sparse_attn_us_rows_from_hbm "

@@ -25,8 +25,7 @@ def topk_select(scores, k: int, *, valid=None, row_start=None, n=None, order: st
     rows, ``n`` = the longest row.  ``order="index"``: ids ascending (what the
     attention kernels walk); ``order="score"``: descending score, ties by ascending id
     (the order of the NumPy contract).  Returns int32 ``[..., k]``.  ``digit_hist``: int32 ``[rows, 2048]`` as
-    ``indexer_scores(..., digit_hist=)`` left it; the selection does not need it (it did as a radix select) and
-    leaves the counters at zero for the next step.  ``out``: contiguous int32 ``[rows, k]`` to write the ids to, in
+    ``indexer_scores(..., digit_hist=)`` left it; cleared for the next step (a launch of its own), otherwise ignored.  ``out``: contiguous int32 ``[rows, k]`` to write the ids to, in
     either order.
     """
     dev = require_cuda(scores)

@@ -66,8 +66,8 @@ def sparse_decode_step(q, idx_q, idx_w, cache: LatentCache, *, k: int, scale: fl
                        return_ids: bool = False, return_scores: bool = False, digit_hist=None):
     """q [B,H,Dqk]; idx_q [B,Hi,Di]; idx_w [B,Hi] float32.  Returns out [B,H,d_v]
     (plus ids [B,k] int32 ascending / scores flat [rows_total] on request).  ``digit_hist``: a zeroed int32
-    ``[B, 2048]`` scratch that lets the scan count the selection's first radix digit while it writes the scores
-    (used when the scan kernel takes the call, see ``scan_counts_digits``; it is zero again afterwards)."""
+    ``[B, 2048]`` scratch for the scan's counters (see ``indexer_scores``; used when the scan kernel takes the call, zero
+    again afterwards; the selection has no use for them, so a step with it is slower)."""
     B = cache.batch
     q4 = idx_q[:, :, None, :]
     if digit_hist is not None and not scan_counts_digits(q4, cache.idx_keys, n_tokens=1, ratio=0, exact_fp32=exact_fp32):
@@ -120,8 +120,8 @@ class SparseDecodePlan:
         self._dtypes = (q_dtype, q_dtype, torch.float32)
         self.packed = torch.zeros(self._offs[2] + (nw + 255) // 256 * 256, dtype=torch.uint8, device=dev)
         self.q, self.idx_q, self.idx_w = self._views(self.packed)
-        # Optional: the scan counts the scores' first radix digit (scratch, zero between steps).  The selection takes
-        # the counters and clears them, but has no use for them: off by default.
+        # Optional: the scan counts the top key bits of the scores (scratch, zero between steps).  The selection clears
+        # the counters in a launch of its own and has no use for them, so this only costs time: off by default.
         self.digit_hist = None
         if count_digits_in_scan and scan_counts_digits(self.idx_q[:, :, None, :], cache.idx_keys, n_tokens=1, ratio=0):
             self.digit_hist = torch.zeros((B, DIGIT_BINS), dtype=torch.int32, device=dev)

@@ -329,12 +329,12 @@ def indexer_scores_tiled_live(q, weights, index_comp, *, pos0: int, ratio: int =
     return scores
 
 
-DIGIT_BINS = 2048   # first radix digit of the selection: the top 11 bits of the monotone score key
+DIGIT_BINS = 2048   # the top 11 bits of the monotone score key
 
 
 def scan_counts_digits(q, keys_flat, *, n_tokens: int, ratio: int, exact_fp32: bool = False, fp8_mma: bool = False) -> bool:
-    """Does this call run on the decode scan, the kernel that can count the selection's first digit as it writes
-    the scores (``digit_hist``)?  One token, no causal mask, FP8 keys, 16-bit q, 8 / 16 / 32 / 64 heads."""
+    """Does this call run on the decode scan, the kernel that can count the top 11 key bits of the scores as it writes
+    them (``digit_hist``)?  One token, no causal mask, FP8 keys, 16-bit q, 8 / 16 / 32 / 64 heads."""
     f8 = getattr(torch, "float8_e4m3fn", None)
     return (n_tokens == 1 and ratio == 0 and keys_flat.dtype == f8 and q.dtype in (torch.float16, torch.bfloat16)
             and int(q.shape[1]) in (8, 16, 32, 64) and int(q.shape[0]) <= 4096 and not exact_fp32 and not fp8_mma)
@@ -347,8 +347,8 @@ def indexer_scores(q, weights, keys_flat, *, n_rows, pos0=0, ratio=0, row_start=
     Uniform batches (row_start None): returns [B,T,n_rows].  Ragged batches (T == 1,
     row_start / row_count int64 / int32 device vectors): returns a flat [rows_total]
     score vector laid out like the key table.  ``digit_hist``: int32 ``[B, 2048]``, zero on entry — the decode
-    scan (see ``scan_counts_digits``) adds every sequence's first-digit histogram of the scores it writes, for
-    ``topk_select(..., digit_hist=)`` to start from."""
+    scan (see ``scan_counts_digits``) adds every sequence's histogram of the top 11 bits of the keys of the scores it
+    writes.  ``topk_select`` takes the counters and clears them but makes no use of them: counting only costs time."""
     dev = require_cuda(q, weights, keys_flat)
     lib = _abi.load()
     B, H, T, D = (int(x) for x in q.shape)
