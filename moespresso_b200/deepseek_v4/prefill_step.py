@@ -9,11 +9,13 @@ than ``k`` rows every row is selected (:1393-1395).  Projections, RoPE and the Q
 are outside this operator.
 
 The [tokens x rows] fp32 score matrix is never materialised: tokens are processed in
-chunks whose scores (``token_chunk`` x rows x 4 bytes) are written to one reused buffer that mostly
-stays in the 126 MB L2 between the score kernel and the selection kernel.  The default chunk is eight
-tokens per SM (1184 on a B200: 155 MB of scores at 32768 rows; four per SM over longer pools), which fills
-whole waves of both kernels; measured per 4096-token chunk over 32768 rows: 296 -> 3343 us, 444 -> 3444,
-592 -> 3259, 888 -> 3364, 1184 -> 3201, 2072 -> 3264, 4096 (537 MB of scores) -> 3195.
+chunks whose scores (``token_chunk`` x rows x 4 bytes) are written to one reused buffer between the score
+kernel and the selection kernel.  The default chunk is eight tokens per SM (1184 on a B200): with 16 index
+heads that is one CTA of the score kernel per SM, which keeps its eight tokens and walks all rows.  The buffer
+is bounded: four tokens per SM where eight would take more than 320 MB of scores.  Scores and selection of 4096
+tokens, us at 592 / 888 / 1184 / 1480 / 4096 tokens per chunk (bf16, 16 heads of 64, k = 2048): 4096 rows 164 /
+166 / 142 / 156 / 149, 16384 rows 459 / 470 / 408 / 487 / 434, 32768 rows 699 / 770 / 657 / 773 / 672, 33000 rows
+722 / 779 / 669 / 786 / 687, 65536 rows (310 MB at 1184) 1468 / 1559 / 1350 / 1461 / 1346.
 """
 from __future__ import annotations
 
@@ -21,6 +23,8 @@ import torch
 
 from .attention import topk_select
 from .indexed_attention_kernel import indexer_scores_tiled_live, sparse_attention
+
+_SCORE_BYTES = 320_000_000
 
 
 def sparse_prefill_step(q, comp_kv, idx_q, idx_keys, idx_w, *, pos0: int, ratio: int = 4, k: int = 512,
@@ -39,7 +43,9 @@ def sparse_prefill_step(q, comp_kv, idx_q, idx_keys, idx_w, *, pos0: int, ratio:
     else:
         ids = torch.empty((T, kk), dtype=torch.int32, device=dev)
         if token_chunk is None:
-            token_chunk = (8 if R <= 32768 else 4) * torch.cuda.get_device_properties(dev).multi_processor_count
+            token_chunk = 8 * torch.cuda.get_device_properties(dev).multi_processor_count
+            if token_chunk * R * 4 > _SCORE_BYTES:
+                token_chunk //= 2
         chunk = max(1, min(int(token_chunk), T))
         buf = torch.empty((1, chunk, R), dtype=torch.float32, device=dev)
         iq = idx_q.permute(1, 0, 2)[None]            # [1,Hi,T,Di]
