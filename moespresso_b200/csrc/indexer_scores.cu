@@ -189,9 +189,26 @@ static int launch_exact_token(const IndexerParams& p, cudaStream_t st) {
   return MXB_OK;
 }
 
+// Which calls of one token per sequence go to the kernel above.  It computes 16, 32 or 64 heads whatever there are, where
+// the kernel for chunks walks the heads there are, a row per thread: the better one while that leaves SMs idle, the worse
+// one when many rows meet heads that do not fill the warps.  us, chunk kernel -> this one, 20,000 / 65,536 / 1,000,003
+// rows:  64 heads of 128, fp32 36 -> 22, 70 -> 38, 739 -> 567;  32 of 64, bf16 12 -> 8, 17 -> 14, 181 -> 146;
+// 16 of 64, fp32 8.7 -> 6.3, 13 -> 11, 136 -> 117 and FP8 keys 7.0 -> 5.9, 9.3 -> 9.9, 87 -> 96;  16 of 128, bf16
+// 12 -> 9, 22 -> 22, 218 -> 242;  48 of 64, fp32 16 -> 13, 25 -> 21, 283 -> 315;  20 of 128, bf16 14 -> 13, 25 -> 23,
+// 257 -> 324;  12 of 64, bf16 7.2 -> 6.1, 10 -> 10, 93 -> 102;  1 of 64, bf16 4.2 -> 5.8, 5.6 -> 9.7, 37 -> 98 (4,096
+// rows: 4.1 -> 4.1).
+template <int D, int KT>
+static bool exact_by_tokens(const IndexerParams& p) {
+  const int padded = p.H <= 16 ? 16 : (p.H <= 32 ? 32 : 64);
+  const int64_t rows = p.n_rows * p.B;
+  if (8 * p.H >= 7 * padded) return padded > 16 || rows <= (KT == MXB_F8E4M3 ? 32768 : (D == 128 ? 262144 : INT64_MAX));
+  if (4 * p.H >= 3 * padded && padded > 16) return rows <= 65536;
+  return rows <= (p.H >= 12 ? 24576 : (p.H >= 8 ? 16384 : 4096));
+}
+
 template <int D, int QT, int KT>
 static int launch_exact(IndexerParams& p, cudaStream_t st) {
-  if (p.T == 1) {
+  if (p.T == 1 && exact_by_tokens<D, KT>(p)) {
     // four rows per lane when that still gives every SM two CTAs
     const bool wide = ceil_div(p.n_rows, 128) * p.B >= 2 * sm_count();
     if (p.H <= 16) return wide ? launch_exact_token<D, QT, KT, 2, 4>(p, st) : launch_exact_token<D, QT, KT, 2, 1>(p, st);

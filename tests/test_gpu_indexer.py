@@ -140,11 +140,12 @@ def test_score_is_independent_of_row_partition():
 
 
 @pytest.mark.parametrize("D,H,rows", [(64, 1, 1), (64, 16, 33), (64, 17, 128 * 296 + 5), (128, 33, 31), (128, 64, 2500),
-                                      (128, 64, 128 * 296 + 1)])
+                                      (128, 64, 128 * 296 + 1), (64, 14, 128 * 296 + 7), (128, 29, 128 * 296 + 127)])
 @pytest.mark.parametrize("qdt,kdt", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16)])
 def test_exact_scores_of_one_token_have_the_bits_of_a_chunk(D, H, rows, qdt, kdt):
     """The kernel for one token splits the heads over warps; a chunk of two equal tokens takes the kernel that walks
-    them in one thread.  Edges of the row tiles (32 and 128), both row widths, heads that do not fill the warps."""
+    them in one thread.  Edges of the row tiles (32 and 128), both row widths, heads that do not fill the warps; calls
+    of few heads and many rows, which go to the kernel for chunks, among them."""
     need_gpu()
     g = torch.Generator(device="cuda").manual_seed(rows + H)
     q = torch.randn(1, H, 1, D, generator=g, device="cuda").to(qdt)
