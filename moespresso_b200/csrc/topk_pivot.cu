@@ -11,9 +11,12 @@
 //      which is expanded into the list of candidate positions in ascending order; their keys are fetched again;
 //   3. the threshold is the k-th largest key of the list: one 2,048-bin histogram over [pivot, largest key], whose
 //      threshold bin holds a handful of keys that are ranked against each other directly.
-//   The sample only steers: if fewer than k keys reach the pivot, or more than the list holds (heavy ties, rows whose
+//   Ties: if more keys than the list holds would reach the pivot and the sampled ones in its bin are one score, the pass
+//   leaves two bitmaps, larger and equal.  Either the threshold is that score and the bitmaps are emitted as they are, or
+//   it lies above and the larger ones are the candidates.
+//   The sample only steers: if fewer than k keys reach the pivot, or more than the list holds after all (rows whose
 //   large scores hide between the sampled positions), the CTAs fall back to an 11 + 11 + 10-bit radix select that
-//   streams the row.
+//   streams the row (592 rows of 32,768: 116 us; a row of 131,072: 46).
 //   A row belongs to one CTA or to a thread-block cluster, each CTA with a contiguous part of it.  The CTAs of a
 //   cluster read the same sample (same pivot, nothing exchanged); after one cluster barrier every CTA copies all
 //   lists' keys (12 KB through distributed shared memory) and finds the threshold for itself, so the second barrier
@@ -27,8 +30,14 @@
 // scores of the pass, three times as much for sample, list and threshold) and barriers.  Against the radix select over
 // whole rows before it, which spent a shared-memory atomic per score and digit: 592 rows of 32,768 scores, k = 2,048:
 // 77 -> 33 us; 32 rows of 131,072: 20.1 -> 14.6; one row of 1,048,576: 63 -> 18.3; one of 2,500, k = 512: 7.8 -> 5.6.
+// Scores rounded to integers (ties at the threshold), radix select / fallback alone / with the two bitmaps: 592 rows of
+// 32,768 79 / 116 / 43 us, 160 of 16,384 32 / 38 / 15, 32 of 131,072 21.5 / 44 / 12, one of 131,072 16 / 46 / 9.5; one row
+// of 1,048,576 equal scores 2,584 / 98 / 20.5.
+// Not better on one row of 16,384 (direct kernel): 9.9 -> 10.4 us.
 #include <cooperative_groups.h>
 #include <math.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "ptx_sm100.cuh"
@@ -72,7 +81,7 @@ __device__ __forceinline__ const float* row_scores(const TopkPivotParams& p, int
 // Shared scalars of the threshold search.
 struct TopkShared {
   uint32_t sums[2][32];   // of consecutive scans, in turn
-  uint32_t thr[4], small_n, T, need, largest;
+  uint32_t thr[4], small_n, T, need, largest, smallest;
   uint32_t small_keys[kPSmall];
 };
 
@@ -167,7 +176,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) topk_direct_kernel(TopkPivotPar
   }
   for (int i = tid; i < kBigBins; i += NT) hist_a[i] = hist_b[i] = 0;
   if (tid == 0) {
-    s.small_n = 0;
+    s.small_n = s.largest = 0;
+    s.smallest = 0xffffffffu;
     s.thr[0] = s.thr[1] = s.thr[2] = s.thr[3] = 0;
   }
   __syncthreads();
@@ -196,16 +206,38 @@ __global__ void __launch_bounds__(NT, 1024 / NT) topk_direct_kernel(TopkPivotPar
       if ((key[u] >> 10) == head && key[u]) s.small_keys[atomicAdd(&s.small_n, 1u)] = key[u];
     __syncthreads();
     rank_small(&s, cnt, want);
-  } else {
+  } else {   // ties, as a rule of a single value
+    uint32_t lo = 0xffffffffu, hi = 0;
 #pragma unroll
-    for (int u = 0; u < kDirectKeys; ++u)
-      if ((key[u] >> 10) == head && key[u]) atomicAdd(&hist_a[key[u] & 1023u], 1u);
-    for (int i = 1024 + tid; i < kBigBins; i += NT) hist_a[i] = 0;
+    for (int u = 0; u < kDirectKeys; ++u) {
+      if ((key[u] >> 10) == head && key[u]) {
+        lo = min(lo, key[u]);
+        hi = max(hi, key[u]);
+      }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0 && hi) {
+      atomicMin(&s.smallest, lo);
+      atomicMax(&s.largest, hi);
+    }
     __syncthreads();
-    threshold_bin<NT>(hist_a, want, s.sums[0], s.thr);
-    if (tid == 0) {
-      s.T = (head << 10) | s.thr[1];
-      s.need = want - s.thr[2];
+    if (s.smallest == s.largest) {
+      if (tid == 0) {
+        s.T = s.largest;
+        s.need = want;
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < kDirectKeys; ++u)
+        if ((key[u] >> 10) == head && key[u]) atomicAdd(&hist_a[key[u] & 1023u], 1u);
+      for (int i = 1024 + tid; i < kBigBins; i += NT) hist_a[i] = 0;
+      __syncthreads();
+      threshold_bin<NT>(hist_a, want, s.sums[0], s.thr);
+      if (tid == 0) {
+        s.T = (head << 10) | s.thr[1];
+        s.need = want - s.thr[2];
+      }
     }
   }
   __syncthreads();
@@ -249,7 +281,7 @@ template <bool CLUSTER, int NT, int SAMPLES>
 __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkPivotParams p) {
   extern __shared__ uint32_t dyn[];
   __shared__ TopkShared s;
-  __shared__ uint32_t s_sum[2], s_top;
+  __shared__ uint32_t s_sum[2], s_top, s_tie[2];
   __shared__ uint32_t cl_count[kPMaxCluster], cl_gt[kPMaxCluster], cl_eq[kPMaxCluster];
 
   ptx::grid_launch_dependents();   // as above
@@ -301,9 +333,12 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkP
     s.thr[0] = s.thr[1] = s.thr[2] = s.thr[3] = 0;
     s.largest = s_top = 0;
     s_sum[0] = s_sum[1] = 0;
+    s_tie[0] = 0xffffffffu;
+    s_tie[1] = 0;
   }
   __syncthreads();
   uint32_t pivot = 1;   // the smallest key of a finite score
+  bool tie = false;     // many scores equal to the pivot: the threshold may well be among them
   if (sampled) {
     const float kr = (float)p.k * (float)(4 * kTotal) / (float)n;
     const uint32_t target = (uint32_t)(kr + 5.f * sqrtf(kr) + 4.f);
@@ -333,7 +368,9 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkP
     });
     __syncthreads();
     threshold_bin<NT>(hist_a, target, s.sums[0], s.thr);
+    uint32_t width = 0, reach = s.thr[2] + s.thr[3];   // keys of the bin at the wanted rank, from the pivot on; samples reaching it
     if (s.thr[0] == target) {
+      width = 1u << 13;
       const uint32_t below = (kBigBins - s.thr[1]) << 13;   // the bin holds the keys above top - below
       pivot = top > below ? top - below + 1 : 1u;
     } else {
@@ -349,15 +386,45 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkP
         __syncthreads();
         threshold_bin<NT>(hist_b, want, s.sums[0], s.thr);
         pivot = max((bin << 21) | (s.thr[1] << 10), 1u);
+        width = 1u << 10;
+        reach = target - want + s.thr[2] + s.thr[3];
       }
+    }
+    // clearly more than wanted, so perhaps more than the list holds: is it one score that so many keys have?
+    if (width && (float)reach > (float)target + 1.5f * sqrtf((float)target)) {
+      uint32_t least = 0xffffffffu, most = 0;
+      each([&](uint32_t key) {
+        if (key - pivot < width && key) {
+          least = min(least, key);
+          most = max(most, key);
+        }
+      });
+      least = __reduce_min_sync(0xffffffffu, least);
+      most = __reduce_max_sync(0xffffffffu, most);
+      if (lane == 0 && most) {
+        atomicMin(&s_tie[0], least);
+        atomicMax(&s_tie[1], most);
+      }
+      __syncthreads();
+      tie = s_tie[0] == s_tie[1];
+      if (tie) pivot = s_tie[0];
     }
   }
 
-  // ---- the pass: a bit per score, set if it reaches the pivot
-  {
+  // ---- the pass: a bit per score, set if it reaches the pivot; with a tie, one if it is larger and one if it is equal
+  auto pass = [&](auto with_tie) {
+    constexpr bool TIE = decltype(with_tie)::value;
     const float pf = pivot <= 0x00800000u ? -kMaxScore : key_float(pivot);   // (smaller keys are no finite score's)
     for (int w0 = warp * 32; w0 < words; w0 += (NT / 32) * 32) {   // 32 words = 1,024 scores per warp
-      uint32_t mine = 0;
+      uint32_t mine = 0, equal = 0;
+      auto vote = [&](int u, float x) {
+        const uint32_t m = __ballot_sync(0xffffffffu, (TIE ? x > pf : x >= pf) && x <= kMaxScore);
+        if (lane == u) mine = m;
+        if constexpr (TIE) {
+          const uint32_t e = __ballot_sync(0xffffffffu, x == pf);
+          if (lane == u) equal = e;
+        }
+      };
       const float* at = src + lo + 32 * w0 + lane;
       if (32 * w0 + 1024 <= len) {
         constexpr int FLIGHT = NT == 512 ? 16 : 32;   // loads in flight per thread, as the registers allow
@@ -367,26 +434,89 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkP
 #pragma unroll
           for (int u = 0; u < FLIGHT; ++u) x[u] = __ldg(at + 32 * (FLIGHT * h + u));
 #pragma unroll
-          for (int u = 0; u < FLIGHT; ++u) {
-            const uint32_t m = __ballot_sync(0xffffffffu, x[u] >= pf && x[u] <= kMaxScore);
-            if (lane == FLIGHT * h + u) mine = m;
-          }
+          for (int u = 0; u < FLIGHT; ++u) vote(FLIGHT * h + u, x[u]);
         }
       } else {
         for (int u = 0; u < 32; ++u) {
           const bool in = 32 * (w0 + u) + lane < len;
-          const float x = in ? __ldg(at + 32 * u) : -INFINITY;
-          const uint32_t m = __ballot_sync(0xffffffffu, x >= pf && x <= kMaxScore);
-          if (lane == u) mine = m;
+          vote(u, in ? __ldg(at + 32 * u) : -INFINITY);
         }
       }
       bm_gt[w0 + lane] = mine;
+      if constexpr (TIE) bm_eq[w0 + lane] = equal;
     }
-  }
+  };
+  if (tie) pass(std::true_type{});
+  else pass(std::false_type{});
   __syncthreads();
-  // ---- bitmap -> ascending positions
   const int per = (words + NT - 1) / NT;
   const int w_lo = min(tid * per, words), w_hi = min(w_lo + per, words);
+  // ---- ordered emission from the two bitmaps: this CTA's ids among the row's, gt_run above and eq_run equal before them
+  auto emit_bitmaps = [&](uint32_t gt_run, uint32_t eq_run, uint32_t need) {
+    uint32_t c_gt = 0, c_eq = 0;
+    for (int w = w_lo; w < w_hi; ++w) {
+      c_gt += __popc(bm_gt[w]);
+      c_eq += __popc(bm_eq[w]);
+    }
+    uint32_t all;
+    uint32_t g_at = gt_run + scan_threads<NT>(c_gt, s.sums[0], &all);
+    uint32_t e_at = eq_run + scan_threads<NT>(c_eq, s.sums[1], &all);
+    for (int w = w_lo; w < w_hi; ++w) {
+      const uint32_t gt = bm_gt[w];
+      uint32_t m = gt | bm_eq[w];
+      while (m) {
+        const int bit = __ffs(m) - 1;
+        m &= m - 1;
+        const int32_t id = (int32_t)(lo + 32 * w + bit);
+        if ((gt >> bit) & 1u) {
+          out[g_at + min(e_at, need)] = id;
+          ++g_at;
+        } else {
+          if (e_at < need) out[g_at + e_at] = id;
+          ++e_at;
+          if (e_at >= need) m &= gt;   // (the other ties of the word are not selected)
+        }
+      }
+    }
+  };
+  if (tie) {
+    uint32_t g = 0, e = 0;
+    for (int w = w_lo; w < w_hi; ++w) {
+      g += __popc(bm_gt[w]);
+      e += __popc(bm_eq[w]);
+    }
+    g = __reduce_add_sync(0xffffffffu, g);
+    e = __reduce_add_sync(0xffffffffu, e);
+    if (lane == 0 && g) atomicAdd(&s_sum[0], g);
+    if (lane == 0 && e) atomicAdd(&s_sum[1], e);
+    __syncthreads();
+    uint32_t G = s_sum[0], E = s_sum[1], gt_run = 0, eq_run = 0;
+    if constexpr (CLUSTER) {
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // as below
+      if (tid < cs) {
+        *cluster.map_shared_rank(&cl_count[rank], tid) = G;
+        *cluster.map_shared_rank(&cl_eq[rank], tid) = E;
+      }
+      cluster.sync();
+      G = E = 0;
+      for (int q = 0; q < cs; ++q) {
+        if (q < rank) {
+          gt_run += cl_count[q];
+          eq_run += cl_eq[q];
+        }
+        G += cl_count[q];
+        E += cl_eq[q];
+      }
+    }
+    if (G < (uint32_t)p.k && (uint32_t)p.k <= G + E) {   // the threshold
+      emit_bitmaps(gt_run, eq_run, (uint32_t)p.k - G);
+      return;
+    }
+    if (G >= (uint32_t)p.k) ++pivot;   // it lies above, among the scores marked as larger
+    __syncthreads();
+    if (tid == 0) s_sum[0] = s_sum[1] = 0;
+  }
+  // ---- bitmap -> ascending positions
   uint32_t own;   // candidates of this CTA
   {
     uint32_t c = 0;
@@ -431,7 +561,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkP
   bool fits = C <= (uint32_t)p.cap;
   if constexpr (CLUSTER) {
     // every CTA of the cluster is running: its shared memory may be written
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (!tie) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (tid < cs) {
       *cluster.map_shared_rank(&cl_count[rank], tid) = C;
       *cluster.map_shared_rank(&cl_gt[rank], tid) = largest;   // (the slot is free until the fallback)
@@ -629,30 +759,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkP
     for (int i = tid + (int)k_eff; i < p.k; i += NT) out[i] = -1;
   if (k_eff == 0) return;
   __syncthreads();
-  uint32_t c_gt = 0, c_eq = 0;
-  for (int w = w_lo; w < w_hi; ++w) {
-    c_gt += __popc(bm_gt[w]);
-    c_eq += __popc(bm_eq[w]);
-  }
-  uint32_t all;
-  uint32_t g_at = gt_run + scan_threads<NT>(c_gt, s.sums[0], &all);
-  uint32_t e_at = eq_run + scan_threads<NT>(c_eq, s.sums[1], &all);
-  for (int w = w_lo; w < w_hi; ++w) {
-    const uint32_t gt = bm_gt[w];
-    uint32_t m = gt | bm_eq[w];
-    while (m) {
-      const int bit = __ffs(m) - 1;
-      m &= m - 1;
-      const int32_t id = (int32_t)(lo + 32 * w + bit);
-      if ((gt >> bit) & 1u) {
-        out[g_at + min(e_at, need)] = id;
-        ++g_at;
-      } else {
-        if (e_at < need) out[g_at + e_at] = id;
-        ++e_at;
-      }
-    }
-  }
+  emit_bitmaps(gt_run, eq_run, need);
 }
 
 // Which rows go to the direct kernel: all that 512 threads hold, and up to twice that while each row's 1,024-thread CTA

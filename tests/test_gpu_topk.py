@@ -87,8 +87,16 @@ def test_direct_and_sampled_rows(n, k, rows):
     packed[:, n // 3:n // 3 + min(k + 5, n // 2)] += 100.0
     _check(packed, k)
     _check(np.round(s), k)
+    _check(np.zeros_like(s), k)                          # the threshold is the tie
+    _check(np.maximum(s - 1.5, 0), k)                    # it is, or lies above: most scores are equal
+    _check(np.where(s > 2.5, s, np.where(s > 0, 0.0, -0.0)).astype(np.float32), k)   # few above, the tie at either zero
+    tied = np.round(s * 4)
+    tied[:, ::2] += 0.001                                # two values in the pivot's bin: no single tie
+    _check(tied, k)
+    _check((1 + rng.integers(0, 700, s.shape) * 2.0 ** -23).astype(np.float32), k)   # all within the last ten bits of a key
     s[:, n // 7:] = -np.inf
     _check(s, k)
+    _check(np.maximum(s, -2.0), k)
 
 
 def test_sampled_rows_of_a_ragged_batch():
