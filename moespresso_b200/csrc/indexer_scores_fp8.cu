@@ -53,6 +53,7 @@ struct Fp8Params {
   int32_t ratio;
   int32_t t_tile;        // tokens per CTA
   int32_t t_first;       // first token of this launch
+  int32_t t_cut;         // 16-bit keys, tiles of more than 128 columns: tokens of the first of two drain groups (0: one)
   int32_t N;             // MMA N
   int32_t acc_stride;    // TMEM columns per accumulator (N rounded up to 32)
   int32_t n_acc;         // accumulators in the TMEM ring
@@ -74,7 +75,8 @@ struct Fp8Cfg {
   // Columns of a tile = (tokens x heads).  KEYS16, where the drain sets the pace: 128 columns, so that TMEM holds four
   // accumulators and each of the four groups of drain warps has one of its own; with 256 columns and two accumulators a
   // tile's MMAs had to wait for the drain of the tile before last and the drain for them (with the packed multiply-adds of
-  // the drain: 333 tokens x 5,003 rows 27.4 -> 14.7 us, 4,096 x 32,768 in seven launches 648 -> 595 us).
+  // the drain: 333 tokens x 5,003 rows 27.4 -> 14.7 us, 4,096 x 32,768 in seven launches 648 -> 595 us).  256 columns
+  // (two groups share a tile) remain where whole waves of CTAs come out of them: see tile_shape.
   static constexpr int kCols = MODE == kKeys16 ? 128 : 256;
   static constexpr int kTileGroups = MODE == kKeys16 ? 4 : 2;   // tiles drained concurrently, four warps each
   static constexpr int kDrainWarps = 4 * kTileGroups;
@@ -154,7 +156,7 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
     }
     for (int a = 0; a < n_acc; ++a) {
       ptx::mbar_init(&acc_full[a], 1);
-      ptx::mbar_init(&acc_empty[a], pairs ? 128u * C::kTileGroups : 128u);
+      ptx::mbar_init(&acc_empty[a], pairs ? 128u * C::kTileGroups : (p.t_cut > 0 ? 256u : 128u));
     }
     *abort_flag = 0;
     ptx::mbar_fence_init();
@@ -431,7 +433,9 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
         }
       }
     }
-    for (int i = set; i < ntiles && !pairs; i += C::kTileGroups) {
+    const bool shared = K16 && p.t_cut > 0;   // groups 2 j and 2 j + 1 drain the same tiles, the tokens before and from t_cut on
+    const int t_lo = shared && (set & 1) ? min(p.t_cut, nt) : 0, t_hi = shared && !(set & 1) ? min(p.t_cut, nt) : nt;
+    for (int i = shared ? set >> 1 : set; i < ntiles && !pairs; i += shared ? C::kTileGroups / 2 : C::kTileGroups) {
       const int a = i % n_acc;
       ptx::mbar_wait(&acc_full[a], (uint32_t)((i / n_acc) & 1), abort_flag);
       ptx::tc_fence_after_sync();
@@ -439,7 +443,7 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
       const int64_t r = row0 + (int64_t)i * 128 + rloc;
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * p.acc_stride);
       const bool r_ok = r < count;
-      float* sp = p.scores + sbase + (int64_t)t0 * p.s_st + r;
+      float* sp = p.scores + sbase + (int64_t)(t0 + t_lo) * p.s_st + r;
       // two tokens per step: their TMEM loads travel together and their two head sums (each in head order) are
       // independent chains, so the loop is no longer one load latency plus one dependent chain per token
       auto load_tok = [&](int t, int c0, uint32_t* v) {
@@ -454,8 +458,8 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
           ptx::tmem_ld16(taddr + (uint32_t)(t * H + c0), v);
         }
       };
-      int t = 0;
-      for (; t + 1 < nt; t += 2, sp += 2 * p.s_st) {
+      int t = t_lo;   // even
+      for (; t + 1 < t_hi; t += 2, sp += 2 * p.s_st) {
         float2 sum = make_float2(0.f, 0.f);   // tokens t and t + 1: one packed multiply-add per head
         for (int c0 = 0; c0 < H; c0 += 16) {
           uint32_t va[16], vb[16];
@@ -477,7 +481,7 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
           sp[p.s_st] = r < (int64_t)vis_s[t + 1] ? sum.y : -INFINITY;
         }
       }
-      if (t < nt) {
+      if (t < t_hi) {
         float sum = 0.f;
         for (int c0 = 0; c0 < H; c0 += 16) {
           uint32_t v1[16];
@@ -502,6 +506,39 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
 #endif
 }
 
+// 16-bit keys, sequences of one length (all CTAs cost the same, one per SM): tokens per tile and row tiles per CTA, for the
+// cheapest waves.  A wave costs its CTAs' row tiles and about nine more for the query operand, the first keys and the last
+// scores.  In tiles of 128 columns, of 0.5 us each: a tile of 256 columns costs 2.2 (2.9 with 128 features), a narrower one
+// a little more than its share.  16 heads keep to full tiles of eight tokens, which have the weights in registers.
+// us, bf16: 256 columns / 128 columns, each in one wave where that fits and else in CTAs of 16 row tiles and more / this rule:
+//   32 heads of 64:  333 tokens x 5,003 rows 23.4 / 27.6 / 23.5;  700 x 12,000 118 / 96 / 83;  1,184 x 8,192 82 / 100 / 80
+//   32 heads of 128: 333 x 5,003 28.0 / 27.0 / 25.8;  1,184 x 8,192 101 / 95 / 75;  1,024 x 32,768 383 / 277 / 270
+//   48 heads of 64:  333 x 5,003 29.6 / 39.6 / 31.1;  700 x 12,000 112 / 140 / 118;  1,184 x 8,192 155 / 155 / 128
+//   64 heads of 64:  333 x 5,003 51.2 / 45.0 / 41.8;  1,184 x 8,192 179 / 181 / 153;  2,048 x 16,384 590 / 540 / 506
+//   64 heads of 128: 333 x 5,003 62.9 / 45.4 / 43.4;  1,184 x 8,192 212 / 159 / 138;  2,048 x 16,384 715 / 470 / 473
+static int tile_shape(const Fp8Params& p, int D, int narrow, int64_t tiles, int64_t* per) {
+  const int64_t slots = sm_count();
+  int best_t = narrow;
+  double best = 1e30;
+  for (int wide = 0; wide < (p.H == 16 ? 1 : 2); ++wide) {
+    int t = wide ? 256 / p.H : narrow;
+    if (wide && (t > p.T || t * p.H <= 128)) break;
+    const int wider = t - ((t / 2) & ~1);   // tokens of the drain group that has more of them
+    const double tile = t * p.H > 128 ? (D == 128 ? 2.9 : 2.2) * 2 * wider * p.H / 256.0 : 0.6 + 0.4 * t * p.H / 128.0;
+    for (int64_t cuts = 1; cuts <= 32; ++cuts) {
+      const int64_t n = ceil_div(tiles, cuts);
+      if (cuts > 1 && n < 8) break;
+      const double cost = (double)ceil_div(ceil_div(p.T, t) * p.B * ceil_div(tiles, n), slots) * ((double)n * tile + 9.0);
+      if (cost < best * 0.999) {
+        best = cost;
+        best_t = t;
+        *per = n;
+      }
+    }
+  }
+  return best_t;
+}
+
 template <int D, int MODE>
 static int launch_fp8_d(Fp8Params& p, const mxb_indexer_scores_args* a, cudaStream_t st) {
   using C = Fp8Cfg<D, MODE>;
@@ -510,7 +547,11 @@ static int launch_fp8_d(Fp8Params& p, const mxb_indexer_scores_args* a, cudaStre
   const int cols_per_token = (DIRECT ? 2 : 1) * p.H;
   int t_tile = C::kCols / cols_per_token;
   if (t_tile > p.T) t_tile = p.T;
+  const int64_t tiles = ceil_div(p.n_rows, 128);
+  int64_t shaped_per = 0;   // row tiles per CTA
+  if (K16 && !p.row_count) t_tile = tile_shape(p, D, t_tile, tiles, &shaped_per);
   p.t_tile = t_tile;
+  p.t_cut = K16 && t_tile * p.H > 128 ? (t_tile / 2) & ~1 : 0;
   p.N = t_tile * cols_per_token;
   p.acc_stride = (int)round_up(p.N, 32);
   int n_acc = 512 / p.acc_stride;
@@ -522,7 +563,6 @@ static int launch_fp8_d(Fp8Params& p, const mxb_indexer_scores_args* a, cudaStre
   p.tmem_cols = cols;
   p.b_bytes = (int)round_up((int64_t)p.N * D * (DIRECT ? 1 : 2), 1024);
   const int64_t t_tiles = ceil_div(p.T, t_tile);
-  const int64_t tiles = ceil_div(p.n_rows, 128);
   const int smem = C::b_off + p.b_bytes + 512 * 4 + 256 * 4 + 56 * 8 + 64 + 1024;
   const int ctas_per_sm = smem <= 113 * 1024 ? 2 : 1;
   // static chunks of rows per CTA, several per resident slot so that ragged sequences balance
@@ -538,6 +578,7 @@ static int launch_fp8_d(Fp8Params& p, const mxb_indexer_scores_args* a, cudaStre
     const int64_t one_wave = ceil_div(tiles, gx);
     if (one_wave >= 8) per = one_wave;
   }
+  if (shaped_per > 0) per = shaped_per;
   p.rows_per_cta = (int)(per * 128);
 
   CUtensorMap tmap;

@@ -165,6 +165,9 @@ def test_exact_scores_of_one_token_have_the_bits_of_a_chunk(D, H, rows, qdt, kdt
     (16, 41, 4096),
     (32, 7, 2049),    # four tokens of 32 heads per tile, the last tile ragged
     (64, 3, 1025),    # two tokens of 64 heads
+    (32, 333, 5003),  # tiles of 256 columns, shared by two drain groups: eight tokens, the last tile has five
+    (48, 333, 5003),  # five tokens of 48 heads (two and three), the last tile has three
+    (64, 331, 5003),  # four tokens, the last tile has three
 ])
 def test_partial_token_tiles_of_16bit_keys(form, H, T, R):
     """Tiles that are not full, for the drain with the weights in registers (16 heads) and the one that reads them:
@@ -187,15 +190,16 @@ def test_partial_token_tiles_of_16bit_keys(form, H, T, R):
 
 
 def test_more_token_tiles_than_a_grid_holds():
-    """65,535 tiles of two tokens (64 heads) and three more: the second launch continues where the first ended."""
+    """65,535 tiles of eight tokens (16 heads) and two more: the second launch continues where the first ended."""
     need_gpu()
-    T, H, D, R = 2 * 65535 + 5, 64, 64, 33
+    first = 8 * 65535
+    T, H, D, R = first + 13, 16, 64, 33
     g = torch.Generator(device="cuda").manual_seed(1)
     q = torch.randn(1, H, T, D, generator=g, device="cuda", dtype=torch.bfloat16)
     w = torch.randn(1, T, H, generator=g, device="cuda")
     keys = torch.randn(1, R, D, generator=g, device="cuda").bfloat16()
     got = iak.indexer_scores_tiled_live(q, w, keys, pos0=4 * R, ratio=4, check=True)
-    for lo in (0, 2 * 65535 - 4, 2 * 65535):     # even: the same tiles as in the whole call
-        part = iak.indexer_scores_tiled_live(q[:, :, lo:lo + 5], w[:, lo:lo + 5], keys, pos0=4 * R, ratio=4)
-        assert torch.equal(got[:, lo:lo + 5], part)
+    for lo in (0, first - 8, first):
+        part = iak.indexer_scores_tiled_live(q[:, :, lo:lo + 13], w[:, lo:lo + 13], keys, pos0=4 * R, ratio=4)
+        assert torch.equal(got[:, lo:lo + 13], part)
     assert bool(torch.isfinite(got).all())
