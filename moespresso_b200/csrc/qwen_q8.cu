@@ -74,19 +74,27 @@ __device__ __forceinline__ void store8(void* p, int64_t i, const float (&v)[8]) 
   }
 }
 
-// One warp per row; grid.y = tensor * heads + head.
-template <int XT, bool VEC>
+// One warp per row; PAIR: grid.y = head, grid.z = tensor (without: one tensor of consecutive packed rows).
+template <int XT, bool VEC, bool PAIR>
 __global__ void __launch_bounds__(128) affine_q8_quantize_kernel(const __grid_constant__ Q8Rows p) {
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (row >= p.n_rows) return;
-  const int which = (int)blockIdx.y / p.heads, head = (int)blockIdx.y % p.heads;
-  const int64_t xo = head * p.x_head_stride + row * p.x_row_stride, po = head * p.head_rows + p.row0 + row;
+  const bool second = PAIR && blockIdx.z != 0;   // (selected, not indexed: an indexed parameter is a dependent load)
+  const void* x = second ? p.x[1] : p.x[0];
+  uint32_t* packed = second ? p.packed[1] : p.packed[0];
+  void* scales = second ? p.scales[1] : p.scales[0];
+  void* biases = second ? p.biases[1] : p.biases[0];
+  int64_t xo = row * p.x_row_stride, po = row;
+  if constexpr (PAIR) {
+    xo += blockIdx.y * p.x_head_stride;
+    po += blockIdx.y * p.head_rows + p.row0;
+  }
   // 8 lanes share a group of 64 features: lane l of a 256-feature span holds features 8 l .. 8 l + 7
   for (int f0 = 0; f0 < p.width; f0 += 256) {
     const int f = f0 + lane * 8;
     float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (f < p.width) load8<XT, VEC>(p.x[which], xo + f, v);
+    if (f < p.width) load8<XT, VEC>(x, xo + f, v);
     float lo = v[0], hi = v[0];
 #pragma unroll
     for (int e = 1; e < 8; ++e) {
@@ -117,43 +125,48 @@ __global__ void __launch_bounds__(128) affine_q8_quantize_kernel(const __grid_co
       const float q = fminf(fmaxf(floorf(__fadd_rn(__fmul_rn(__fsub_rn(v[e], bias), inv), 0.5f)), 0.f), 255.f);
       w[e >> 2] |= (uint32_t)q << (8 * (e & 3));
     }
-    *reinterpret_cast<uint2*>(p.packed[which] + po * (p.width / 4) + f / 4) = make_uint2(w[0], w[1]);
+    *reinterpret_cast<uint2*>(packed + po * (p.width / 4) + f / 4) = make_uint2(w[0], w[1]);
     if ((lane & 7) == 0) {
       const int64_t g = po * (p.width / Q8_GROUP) + f / Q8_GROUP;
-      store_elem<XT>(p.scales[which], g, scale);
-      store_elem<XT>(p.biases[which], g, bias);
+      store_elem<XT>(scales, g, scale);
+      store_elem<XT>(biases, g, bias);
     }
   }
 }
 
-// One warp per four rows, all of whose loads are issued before the first is used; grid.y = tensor * heads + head.
+// One warp per ROWS rows, all of whose loads are issued before the first is used; grid.y = head, grid.z = tensor.
 // Rows behind the packed ones (n_tail) are copied: a past and the chunk behind it become one operand in one launch.
 // HBM-bound.  Keys and values of 2 heads, 30,720 rows and 2,048 behind them: 29 us (3.4 TB/s); one launch per head
-// and tensor with two-byte stores, and copies for the rows behind, took 108 us.
+// and tensor with two-byte stores, and copies for the rows behind, took 108 us.  Calls whose rows are all resident with
+// a warp each take ROWS = 1: what they cost is the chain of one row (7 rows of 256, 2.3 -> 1.5 us; 5,000 of 64, 2.8 -> 2.2).
 constexpr int kDqRows = 4;
-template <int ST, int OT, bool VEC>
+template <int ST, int OT, bool VEC, int ROWS>
 __global__ void __launch_bounds__(128) affine_q8_dequantize_kernel(const __grid_constant__ Q8Rows p) {
   const int lane = threadIdx.x & 31;
-  const int64_t row_lo = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * kDqRows;
-  const int which = (int)blockIdx.y / p.heads, head = (int)blockIdx.y % p.heads;
-  void* out = const_cast<void*>(p.x[which]);
+  const int64_t row_lo = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * ROWS;
+  const bool second = blockIdx.z != 0;
+  const uint32_t* packed = second ? p.packed[1] : p.packed[0];
+  const void* scales = second ? p.scales[1] : p.scales[0];
+  const void* biases = second ? p.biases[1] : p.biases[0];
+  const int head = (int)blockIdx.y;
+  void* out = const_cast<void*>(second ? p.x[1] : p.x[0]);
   const int64_t oo = head * p.x_head_stride, n_all = p.n_rows + p.n_tail;
   for (int f = lane * 8; f < p.width; f += 256) {
-    uint2 w[kDqRows];
-    float scale[kDqRows], bias[kDqRows];
+    uint2 w[ROWS];
+    float scale[ROWS], bias[ROWS];
 #pragma unroll
-    for (int u = 0; u < kDqRows; ++u) {
+    for (int u = 0; u < ROWS; ++u) {
       const int64_t row = row_lo + u;
       if (row < p.n_rows) {
         const int64_t po = head * p.head_rows + p.row0 + row;
-        w[u] = __ldg(reinterpret_cast<const uint2*>(p.packed[which] + po * (p.width / 4) + f / 4));
+        w[u] = __ldg(reinterpret_cast<const uint2*>(packed + po * (p.width / 4) + f / 4));
         const int64_t g = po * (p.width / Q8_GROUP) + f / Q8_GROUP;
-        scale[u] = load_elem<ST>(p.scales[which], g);
-        bias[u] = load_elem<ST>(p.biases[which], g);
+        scale[u] = load_elem<ST>(scales, g);
+        bias[u] = load_elem<ST>(biases, g);
       }
     }
 #pragma unroll
-    for (int u = 0; u < kDqRows; ++u) {
+    for (int u = 0; u < ROWS; ++u) {
       const int64_t row = row_lo + u;
       float v[8];
       if (row < p.n_rows) {
@@ -161,7 +174,7 @@ __global__ void __launch_bounds__(128) affine_q8_dequantize_kernel(const __grid_
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = fmaf((float)((ww[e >> 2] >> (8 * (e & 3))) & 0xffu), scale[u], bias[u]);
       } else if (row < n_all) {
-        load8<OT, VEC>(p.tail[which], head * p.tail_head_stride + (row - p.n_rows) * p.tail_row_stride + f, v);
+        load8<OT, VEC>(second ? p.tail[1] : p.tail[0], head * p.tail_head_stride + (row - p.n_rows) * p.tail_row_stride + f, v);
       }
       if (row < n_all) store8<OT, VEC>(out, oo + row * p.x_row_stride + f, v);
     }
@@ -541,11 +554,13 @@ static bool vec16(const void* p, int dt, int64_t stride_a, int64_t stride_b) {
 static int launch_quantize(const Q8Rows& p, int tensors, int x_dtype, cudaStream_t st) {
   bool vec = true;
   for (int i = 0; i < tensors; ++i) vec = vec && vec16(p.x[i], x_dtype, p.x_head_stride, p.x_row_stride);
-  const dim3 grid((unsigned)ceil_div(p.n_rows, 4), (unsigned)(tensors * p.heads));
-#define MXB_Q(XT)                                                    \
-  if (x_dtype == XT) {                                               \
-    if (vec) affine_q8_quantize_kernel<XT, true><<<grid, 128, 0, st>>>(p);  \
-    else affine_q8_quantize_kernel<XT, false><<<grid, 128, 0, st>>>(p);     \
+  const dim3 grid((unsigned)ceil_div(p.n_rows, 4), (unsigned)p.heads, (unsigned)tensors);
+#define MXB_Q(XT)                                                                                  \
+  if (x_dtype == XT) {                                                                             \
+    if (tensors == 1 && vec) affine_q8_quantize_kernel<XT, true, false><<<grid, 128, 0, st>>>(p);  \
+    else if (tensors == 1) affine_q8_quantize_kernel<XT, false, false><<<grid, 128, 0, st>>>(p);   \
+    else if (vec) affine_q8_quantize_kernel<XT, true, true><<<grid, 128, 0, st>>>(p);              \
+    else affine_q8_quantize_kernel<XT, false, true><<<grid, 128, 0, st>>>(p);                      \
   }
   MXB_Q(MXB_F32) else MXB_Q(MXB_F16) else MXB_Q(MXB_BF16)
 #undef MXB_Q
@@ -559,11 +574,14 @@ static int launch_dequantize(const Q8Rows& p, int tensors, int sb_dtype, int x_d
   for (int i = 0; i < tensors; ++i)
     vec = vec && vec16(p.x[i], x_dtype, p.x_head_stride, p.x_row_stride) &&
           (p.n_tail == 0 || vec16(p.tail[i], x_dtype, p.tail_head_stride, p.tail_row_stride));
-  const dim3 grid((unsigned)ceil_div(p.n_rows + p.n_tail, 4 * kDqRows), (unsigned)(tensors * p.heads));
-#define MXB_DQ(ST, OT)                                                              \
-  if (sb_dtype == ST && x_dtype == OT) {                                            \
-    if (vec) affine_q8_dequantize_kernel<ST, OT, true><<<grid, 128, 0, st>>>(p);    \
-    else affine_q8_dequantize_kernel<ST, OT, false><<<grid, 128, 0, st>>>(p);       \
+  const int64_t rows = p.n_rows + p.n_tail;
+  const bool few = vec && rows * p.heads * tensors <= 48 * (int64_t)sm_count();
+  const dim3 grid((unsigned)ceil_div(rows, few ? 4 : 4 * kDqRows), (unsigned)p.heads, (unsigned)tensors);
+#define MXB_DQ(ST, OT)                                                                         \
+  if (sb_dtype == ST && x_dtype == OT) {                                                       \
+    if (few) affine_q8_dequantize_kernel<ST, OT, true, 1><<<grid, 128, 0, st>>>(p);            \
+    else if (vec) affine_q8_dequantize_kernel<ST, OT, true, kDqRows><<<grid, 128, 0, st>>>(p); \
+    else affine_q8_dequantize_kernel<ST, OT, false, kDqRows><<<grid, 128, 0, st>>>(p);         \
   } else
   MXB_DQ(MXB_F32, MXB_F32) MXB_DQ(MXB_F32, MXB_F16) MXB_DQ(MXB_F32, MXB_BF16)
   MXB_DQ(MXB_F16, MXB_F32) MXB_DQ(MXB_F16, MXB_F16) MXB_DQ(MXB_F16, MXB_BF16)
