@@ -137,8 +137,8 @@ def _q8_call(name, rows, row_stride, packed, scales, biases, n, D):
 
 def _q8_head_rows(tensors) -> int:
     """Rows between consecutive heads of (packed, scales, biases) x (keys, values), all row-contiguous views
-    ``[1, Hkv, P, w]`` of one capacity and one row width, with scales of one type; 0 when they are not (the paired
-    kernels take the widths and the rows of a head on trust)."""
+    ``[1, Hkv, P, w]`` of one capacity and one row width on one device, with scales of one type; 0 when they are not
+    (the paired kernels take the widths and the rows of a head on trust)."""
     kp, ks, kb, vp, vs, vb = tensors
     _, heads, n, words = shape = kp.shape
     strides, groups = kp.stride(), words * 4 // Q8_GROUP
@@ -147,7 +147,8 @@ def _q8_head_rows(tensors) -> int:
             not (kb.shape == vs.shape == vb.shape == s_shape) or
             strides[2:] != (words, 1) or vp.stride() != strides or
             s_strides[2:] != (groups, 1) or not (kb.stride() == vs.stride() == vb.stride() == s_strides) or
-            not (kb.dtype == vs.dtype == vb.dtype == dt) or kp.element_size() != 4 or vp.element_size() != 4):
+            not (kb.dtype == vs.dtype == vb.dtype == dt) or kp.element_size() != 4 or vp.element_size() != 4 or
+            not (kp.get_device() == ks.get_device() == kb.get_device() == vp.get_device() == vs.get_device() == vb.get_device())):
         return 0
     if heads == 1:
         return n
@@ -198,10 +199,11 @@ class QuantizedKVCache:
         if self.offset + L > self.capacity:
             raise ValueError("QuantizedKVCache capacity exceeded")
         stores, words = (*self.keys, *self.values), self.keys[0]
-        dev, shape = words.device, (1, int(words.shape[1]), L, 4 * int(words.shape[3]))
+        one, heads, rows, width = words.shape
+        shape = (1, heads, L, 4 * width)
         # the paired kernel writes whole rows of both tensors by address; the stores are public and may have been replaced
-        paired = (L and 0 <= self.offset <= words.shape[2] - L and words.shape[0] == 1 and
-                  keys.shape == shape and values.shape == shape and all(t.device == dev for t in (keys, values, *stores)))
+        paired = (L and one == 1 and 0 <= self.offset <= rows - L and keys.shape == shape and values.shape == shape and
+                  keys.get_device() == values.get_device() == words.get_device())
         head_rows = _q8_head_rows(stores) if paired else 0
         if head_rows:
             dt = stores[1].dtype
@@ -257,7 +259,7 @@ def sdpa_fa_prefill_q8(queries, k_packed, k_scales, k_biases, v_packed, v_scales
     self_k, self_v = self_k[0], self_v[0]
     past = (k_packed, k_scales, k_biases, v_packed, v_scales, v_biases)
     paired = (P and 4 * int(k_packed.shape[3]) == D and tuple(self_k.shape) == tuple(self_v.shape) == (Hkv, L, D) and
-              all(t.device == dev for t in (self_k, self_v, *past)))
+              self_k.get_device() == self_v.get_device() == k_packed.get_device())
     head_rows = _q8_head_rows(past) if paired else 0
     if head_rows:
         self_k, self_v = self_k.to(op), self_v.to(op)
@@ -295,9 +297,12 @@ def sdpa_decode_q8(queries, k_packed, k_scales, k_biases, v_packed, v_scales, v_
     if B != 1 or T != 1 or D != FLASH_HEAD_DIM:
         raise ValueError("q8 decode requires one token of batch 1 and head_dim=256")
     tensors = (k_packed, k_scales, k_biases, v_packed, v_scales, v_biases)
-    strides = {int(t.stride(1)) // int(t.shape[3]) for t in tensors}
-    if len(strides) != 1 or any(t.stride(3) != 1 or t.stride(2) != t.shape[3] for t in tensors):
-        raise ValueError("q8 decode: cache tensors must be row-contiguous views with one capacity")
+    head_rows = _q8_head_rows(tensors)
+    if not head_rows:            # keys and values that differ in what does not matter here
+        strides = {int(t.stride(1)) // int(t.shape[3]) for t in tensors}
+        if len(strides) != 1 or any(t.stride(3) != 1 or t.stride(2) != t.shape[3] for t in tensors):
+            raise ValueError("q8 decode: cache tensors must be row-contiguous views with one capacity")
+        head_rows = strides.pop()
     splits = max(1, min(int(splits), P))
     q = queries.reshape(Hq, D).contiguous()
     o_parts = torch.empty((splits, 1, 1, Hq, D), dtype=torch.float32, device=dev)
@@ -306,7 +311,7 @@ def sdpa_decode_q8(queries, k_packed, k_scales, k_biases, v_packed, v_scales, v_
     a.q, a.q_dtype = ptr(q), dtype_code(q)
     a.k_packed, a.k_scales, a.k_biases = ptr(k_packed), ptr(k_scales), ptr(k_biases)
     a.v_packed, a.v_scales, a.v_biases = ptr(v_packed), ptr(v_scales), ptr(v_biases)
-    a.sb_dtype, a.head_stride_rows = dtype_code(k_scales), strides.pop()
+    a.sb_dtype, a.head_stride_rows = dtype_code(k_scales), head_rows
     a.P, a.Hq, a.Hkv, a.D, a.scale, a.n_splits = P, Hq, Hkv, D, float(scale), splits
     a.o_parts, a.ml_parts = ptr(o_parts), ptr(ml_parts)
     _abi.check(_t.launch("sdpa_decode_q8", _abi.load().mxb_sdpa_decode_q8, a))
