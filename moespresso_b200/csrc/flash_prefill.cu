@@ -653,8 +653,9 @@ using namespace mxb;
 //   1,200 over 30,000 1,082 -> 633 / 1,011 -> 692; 1,700 over 30,000 (saving 29 %) 1,092 -> 864 / 1,073 -> 958;
 //   1,900 over 30,000 (21 %) 1,112 -> 936 / 1,106 -> 1,037;
 // below the line 2,048 over 30,720 (13 %) 1,136 -> 1,038 / 1,154 -> 1,140; 3,000 over 8,000 (11 %) 458 -> 429 / 477 -> 495;
-//   5,000 over 8,000 (10 %) 808 -> 778 / 871 -> 898; 32 heads, 2,048 over 30,720 (14 %) 2,267 -> 2,442;
-//   700 over 1,365 39.8 -> 44.2 and 1,000 over 1,000 40.5 -> 47.5 alone.
+//   5,000 over 8,000 (10 %) 808 -> 778 / 871 -> 898; 704 over 2,000 (12 %) 63 -> 66 / 48 -> 53; 1,728 over 4,000 (13 %)
+//   185 -> 168 / 161 -> 165; 1,024 over 12,000 (10 %) 240 -> 219 / 214 -> 227; 2,048 over 24,000 (13 %) 913 -> 762 / 893 -> 847;
+//   32 heads, 2,048 over 30,720 (14 %) 2,267 -> 2,442; 700 over 1,365 39.8 -> 44.2 and 1,000 over 1,000 40.5 -> 47.5 alone.
 // A cut changes the results in the last bits (P is rounded to 16 bits against each segment's own reference; the error
 // against float64 stays the same, 2.31e-3 relative in bf16 on either side).  The partials take up to 39 MB (296 slots).
 constexpr int kSegCost = 4, kCutCost = 16, kMinShare = 12, kSaving = 15;

@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkP
   uint32_t* keys = CLUSTER ? lkey + p.cap : lkey;   // [cap] the keys of all candidates of the row
   const int max_words = p.part / 32;
   uint32_t* bm_gt = (CLUSTER ? keys : lkey) + p.cap;   // [max_words]; the pass's bitmap
-  uint32_t* bm_eq = bm_gt + max_words;                  // [max_words]; fallback only
+  uint32_t* bm_eq = bm_gt + max_words;                  // [max_words]; with a tie, and in the fallback
   uint32_t* w_gt = hist_a;                       // [cap / 32] each, once the threshold is known
   uint32_t* w_eq = hist_a + 512;
   uint32_t* w_at = hist_b;
