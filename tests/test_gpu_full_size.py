@@ -21,7 +21,7 @@ def test_batched_decode_step_at_full_size():
     cache = LatentCache(kv=dev(c["kv"]), kv_scales=dev(c["kv_scales"]), idx_keys=fp8_from_bits(c["idx_key_bits"]),
                         row_start=dev(c["row_start"]), row_count=dev(c["lens"].astype(np.int32)),
                         max_rows=int(c["lens"].max()))
-    hist = torch.zeros((B, 2048), dtype=torch.int32, device="cuda")   # the scan counts the selection's first digit
+    hist = torch.zeros((B, 2048), dtype=torch.int32, device="cuda")   # counters that the scan fills and the selection clears
     out, ids, scores = sparse_decode_step(dev(c["q"], torch.bfloat16), dev(c["idx_q"], torch.bfloat16),
                                           dev(c["idx_w"]), cache, k=k, scale=c["scale"], d_v=c["d_v"],
                                           return_ids=True, return_scores=True, digit_hist=hist)

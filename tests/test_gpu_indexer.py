@@ -158,6 +158,7 @@ def test_exact_scores_of_one_token_have_the_bits_of_a_chunk(D, H, rows, qdt, kdt
 
 
 @pytest.mark.parametrize("form", ["bf16", "f16"])
+@pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("H,T,R", [
     (16, 9, 2049),    # 8 + 1 tokens: the second tile's drain groups 1-3 have none, group 0 has one
     (16, 13, 700),    # a group with one token of its two between full and empty groups
@@ -169,14 +170,14 @@ def test_exact_scores_of_one_token_have_the_bits_of_a_chunk(D, H, rows, qdt, kdt
     (48, 333, 5003),  # five tokens of 48 heads (two and three), the last tile has three
     (64, 331, 5003),  # four tokens, the last tile has three
 ])
-def test_partial_token_tiles_of_16bit_keys(form, H, T, R):
+def test_partial_token_tiles_of_16bit_keys(form, H, T, R, D):
     """Tiles that are not full, for the drain with the weights in registers (16 heads) and the one that reads them:
     against the fp32 kernel on the same operands; nothing is written behind the last token or row."""
     need_gpu()
     dt = torch.bfloat16 if form == "bf16" else torch.float16
     g = torch.Generator(device="cuda").manual_seed(H + T + R)
     mk = lambda *s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
-    q, w, keys = mk(1, H, T, 64).to(dt), mk(1, T, H) / 4, mk(1, R, 64).to(dt)
+    q, w, keys = mk(1, H, T, D).to(dt), mk(1, T, H) / 4, mk(1, R, D).to(dt)
     kw = dict(pos0=2 * R, ratio=4)
     ref = iak.indexer_scores_tiled_live(q, w, keys, exact_fp32=True, **kw)
     store = torch.full((1, T + 3, R + 5), 12345.0, device="cuda")
