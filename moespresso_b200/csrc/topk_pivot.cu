@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkP
       }
     }
     // clearly more than wanted, so perhaps more than the list holds: is it one score that so many keys have?
-    if (width && (float)reach > (float)target + 1.5f * sqrtf((float)target)) {
+    if (__builtin_expect(width && (float)reach > (float)target + 1.5f * sqrtf((float)target), 0)) {
       uint32_t least = 0xffffffffu, most = 0;
       each([&](uint32_t key) {
         if (key - pivot < width && key) {
@@ -446,8 +446,8 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkP
       if constexpr (TIE) bm_eq[w0 + lane] = equal;
     }
   };
-  if (tie) pass(std::true_type{});
-  else pass(std::false_type{});
+  if (__builtin_expect(!tie, 1)) pass(std::false_type{});
+  else pass(std::true_type{});
   __syncthreads();
   const int per = (words + NT - 1) / NT;
   const int w_lo = min(tid * per, words), w_hi = min(w_lo + per, words);
@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkP
       }
     }
   };
-  if (tie) {
+  if (__builtin_expect(tie, 0)) {
     uint32_t g = 0, e = 0;
     for (int w = w_lo; w < w_hi; ++w) {
       g += __popc(bm_gt[w]);
