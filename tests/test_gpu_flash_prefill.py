@@ -63,6 +63,27 @@ def test_items_cut_at_equal_stretches(S, past, Hq, Hkv, dt, gate):
     assert max_abs(out, ref) <= 2 * 2.0 ** -9 * float(np.abs(v).max())
 
 
+@pytest.mark.parametrize("S,past,Hq,Hkv", [
+    (1, 0, 1, 1),         # one row; the pair's second query tile lies past the end
+    (128, 1, 3, 1),       # a full first tile, an empty second one
+    (129, 127, 2, 2),     # the second tile holds one row; 256 keys, two tiles exactly
+    (300, 200, 3, 1),     # an odd number of query tiles
+    (65, 3000, 3, 3),     # items cut between pairs that take 256 rows
+    (257, 129, 6, 3),     # two heads of one KV head: three query tiles, a last key tile of two keys
+])
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+def test_pairs_of_query_tiles(S, past, Hq, Hkv, dt):
+    """A pair of CTAs takes two heads of one KV head, or 256 rows of one head where the heads per KV head are odd."""
+    need_gpu()
+    rng = np.random.default_rng(S + past)
+    tdt = torch.bfloat16 if dt == "bf16" else torch.float16
+    q, k, v, g = _inputs(rng, S, past, Hq, Hkv, bf16_round if dt == "bf16" else f16_round)
+    out = fa.sdpa_fa_prefill(dev(q, tdt), dev(k, tdt), dev(v, tdt), 1.0 / 16.0, gate=dev(g, tdt), layout="lhd", check=True)
+    ref = qwen.causal_gqa_prefill(q, k, v, g, scale=1.0 / 16.0, past_len=past)
+    # half a unit of bf16 (2^-9) for P and for the result, relative to the largest |v| a row can average
+    assert max_abs(out, ref) <= 2 * 2.0 ** -9 * float(np.abs(v).max())
+
+
 def test_gate_layout_without_tensor_map():
     """A gate whose row stride is not a multiple of its head stride cannot be described by a tensor map: the drain
     then reads the gate and writes the output with per-thread accesses.  Same result as the tiled drain."""
