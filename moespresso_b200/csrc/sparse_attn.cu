@@ -608,6 +608,8 @@ extern "C" int mxb_sparse_attn(const mxb_sparse_attn_args* a, void* stream) {
 
   const int kt = a->kv_dtype, qt = a->q_dtype;
   if (use_tc(a)) {
+    rc = launch_sparse_few(p, kt, qt, a->out_dtype, st);
+    if (rc != MXB_ERR_UNSUPPORTED) return rc;
     rc = launch_sparse_tc(p, kt, qt, a->out_dtype, st);
   } else
 #define MXB_PAIR(QT, KT) \

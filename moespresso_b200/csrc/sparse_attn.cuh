@@ -44,6 +44,8 @@ struct SparseParams {
 // tcgen05 path (16-bit / int8 KV).  Returns MXB_ERR_UNSUPPORTED when the shape is outside its range.
 bool sparse_tc_eligible(int kv_dtype, int q_dtype, int H, int Dqk, int Dv);
 int sparse_tc_splits(int B, int T, int H, int k, int raw_cap, int requested);
+// A few tokens (sparse_attn_few.cu).  MXB_ERR_UNSUPPORTED: nothing was launched.
+int launch_sparse_few(const SparseParams& p, int kv_dtype, int q_dtype, int out_dtype, cudaStream_t st);
 int launch_sparse_tc(SparseParams& p, int kv_dtype, int q_dtype, int out_dtype, cudaStream_t st);
 
 }  // namespace mxb
