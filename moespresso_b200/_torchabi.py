@@ -70,6 +70,30 @@ def last_dim_contiguous(t: torch.Tensor) -> torch.Tensor:
 TIMER = None
 
 
+_NATIVE_CALLS = ("mxb_indexer_scores", "mxb_topk_workspace_bytes", "mxb_topk_select", "mxb_sparse_attn_workspace_bytes",
+                 "mxb_sparse_attn", "mxb_fused_decode_prep_workspace_bytes", "mxb_fused_decode_prep",
+                 "mxb_fused_decode_sdpa_workspace_bytes", "mxb_fused_decode_sdpa", "mxb_affine_q8_append",
+                 "mxb_sdpa_decode_q8", "mxb_merge_partials")
+_native = None
+
+
+def native(name: str, *args):
+    """One of the native host calls (``csrc/host_calls.cpp``), which take an operator's plain case in one go.  None: not
+    such a case, nothing has been done, the caller goes on in Python."""
+    global _native
+    if _native is None:
+        lib = _abi.load()
+        from . import _native as mod
+        mod.bind(*(C.cast(getattr(lib, n), C.c_void_p).value for n in _NATIVE_CALLS))
+        _native = mod
+    if TIMER is not None:
+        return None
+    r = getattr(_native, name)(*args)
+    if type(r) is int:
+        _abi.check(r)
+    return r
+
+
 def launch(name: str, fn, args) -> int:
     if TIMER is None:
         return fn(C.byref(args), stream_ptr())

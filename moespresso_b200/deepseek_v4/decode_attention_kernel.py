@@ -18,7 +18,7 @@ import torch
 
 from .. import _abi
 from .. import _torchabi as _t
-from .._torchabi import ptr, require_cuda
+from .._torchabi import native, ptr, require_cuda
 
 _HEAD_DIM = 512
 
@@ -69,6 +69,9 @@ def fused_decode_prep(q_idx, pooled_qat, weights, kv_row, inv_freq, params, *, s
     top-k with ties to the lower row; ids ASCENDING here, where the reference emits the strictly-above rows first
     and the boundary ties after them — the same set), the roped and FP8-rounded KV row, and the scores.
     Three launches: everything that precedes the scan, the exact fp32 scores, the top-k."""
+    r = native("fused_decode_prep", q_idx, pooled_qat, weights, kv_row, inv_freq, params, scale, topk)
+    if r is not None:
+        return r
     if q_idx.ndim != 2 or int(q_idx.shape[1]) != _INDEX_HEAD_DIM:
         raise ValueError("q_idx must have shape [n_heads, 128]")
     n_heads = int(q_idx.shape[0])
@@ -114,6 +117,9 @@ def fused_decode_sdpa(q, window, row, pooled, sel, sinks, inv_freq, params, *, s
     ``[position, write_idx]``.  Every window row and every selected row is a key and a value; the sink joins the
     maximum and the denominator once.  Returns float16 ``[n_heads, 512]`` after the inverse rope.
     Launches: the operands (rope, window, sinks), the attention (and its merge), the inverse rope."""
+    r = native("fused_decode_sdpa", q, window, row, pooled, sel, sinks, inv_freq, params, scale)
+    if r is not None:
+        return r
     if q.ndim != 2 or int(q.shape[1]) != _HEAD_DIM or q.dtype != torch.float16:
         raise ValueError("q must be float16 [n_heads, 512]")
     n_heads = int(q.shape[0])

@@ -15,6 +15,7 @@ from dataclasses import dataclass
 
 import torch
 
+from .._torchabi import native
 from .attention import topk_select
 from .indexed_attention_kernel import DIGIT_BINS, indexer_scores, scan_counts_digits, sparse_attention
 
@@ -68,6 +69,13 @@ def sparse_decode_step(q, idx_q, idx_w, cache: LatentCache, *, k: int, scale: fl
     (plus ids [B,k] int32 ascending / scores flat [rows_total] on request).  ``digit_hist``: a zeroed int32
     ``[B, 2048]`` scratch for the scan's counters (see ``indexer_scores``; used when the scan kernel takes the call, zero
     again afterwards; the selection has no use for them, so a step with it is slower)."""
+    if digit_hist is None and not partial:
+        r = native("decode_step", q, idx_q, idx_w, cache.kv, cache.kv_scales, cache.idx_keys, cache.row_start, cache.row_count,
+                   cache.max_rows, k, scale, d_v, sinks, out_dtype, exact_fp32)
+        if r is not None:
+            out, ids, scores = r
+            extra = (ids,) * bool(return_ids) + (scores,) * bool(return_scores)
+            return (out, *extra) if extra else out
     B = cache.batch
     q4 = idx_q[:, :, None, :]
     if digit_hist is not None and not scan_counts_digits(q4, cache.idx_keys, n_tokens=1, ratio=0, exact_fp32=exact_fp32):

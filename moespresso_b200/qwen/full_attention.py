@@ -17,7 +17,7 @@ import torch
 
 from .. import _abi
 from .. import _torchabi as _t
-from .._torchabi import dtype_code, last_dim_contiguous, ptr, require_cuda, status_word, stream_ptr, workspace
+from .._torchabi import dtype_code, last_dim_contiguous, native, ptr, require_cuda, status_word, stream_ptr, workspace
 
 FLASH_HEAD_DIM = 256
 
@@ -195,6 +195,10 @@ class QuantizedKVCache:
     def update_and_fetch(self, keys, values):
         """keys / values ``[1, Hkv, L, D]``: quantised into rows ``offset .. offset + L``; returns the quantised
         prefix including them."""
+        r = native("q8_append", self.keys, self.values, self.offset, self.capacity, keys, values)
+        if r is not None:
+            self.offset += int(keys.shape[2])
+            return r
         L = int(keys.shape[2])
         if self.offset + L > self.capacity:
             raise ValueError("QuantizedKVCache capacity exceeded")
@@ -291,6 +295,9 @@ def sdpa_decode_q8(queries, k_packed, k_scales, k_biases, v_packed, v_scales, v_
     from ..deepseek_v4.indexed_attention_kernel import merge_partials
     if group_size != Q8_GROUP or bits != Q8_BITS:
         raise ValueError("q8 decode requires group_size=64 and bits=8")
+    r = native("q8_decode", queries, k_packed, k_scales, k_biases, v_packed, v_scales, v_biases, scale, splits)
+    if r is not None:
+        return r
     dev = require_cuda(queries, k_packed, v_packed)
     B, Hq, T, D = (int(x) for x in queries.shape)
     Hkv, P = int(k_packed.shape[1]), int(k_packed.shape[2])

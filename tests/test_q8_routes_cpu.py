@@ -112,3 +112,12 @@ def test_state_of_an_offset_past_the_stores_clips():
     cache.keys, cache.values = (tuple(t[:, :, :9] for t in six) for six in (cache.keys, cache.values))
     cache.offset = 12
     assert all(t.shape[2] == 9 for six in cache.state for t in six)
+
+
+def test_native_calls_leave_cpu_tensors_to_python():
+    """Without a device the native calls take nothing: the Python operators raise their own error."""
+    import torch
+    from moespresso_b200 import _torchabi
+    x = torch.zeros(1, 2, 1, 256)
+    assert _torchabi.native("q8_decode", x, x, x, x, x, x, x, 0.1, 4) is None
+    assert _torchabi.native("decode_step") is None
