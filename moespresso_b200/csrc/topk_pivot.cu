@@ -1,8 +1,11 @@
 // Exact top-k of fp32 score rows of up to 2^21 scores: rows of up to 16,384 scores in registers, longer ones through a
 // sampled pivot that lets one pass over the row throw nearly all of it away.
 //
-// topk_direct_kernel (rows of at most kDirectMax scores): one CTA, up to 16 keys per thread in registers.  Two
-// histogram levels (11 + 11 key bits) and a direct ranking of what is left in the threshold bin.
+// topk_direct_kernel (rows of at most kDirectMax scores): one CTA, up to 16 keys per thread in registers.  One histogram
+// of 2,048 equal bins over the row's range without outliers and a direct ranking of what is left in the threshold bin;
+// rows that this does not resolve go by the key's bits (11 + 11 + 10).  Bins of values and not of key bits, because
+// ordinary scores have some twenty values of the top 11 bits: the atomics of a warp then meet in a few words, and the
+// threshold bin always needs a second level.
 //
 // topk_pivot_kernel (longer rows):
 //   1. a strided sample of the row (4,096 to 32,768 scores, a histogram of the keys below its largest) gives a
@@ -29,11 +32,11 @@
 // Bound: few rows, the chain of barriers and L2 round trips; many rows, instruction issue (6 warp instructions per 32
 // scores of the pass, three times as much for sample, list and threshold) and barriers.  Against the radix select over
 // whole rows before it, which spent a shared-memory atomic per score and digit: 592 rows of 32,768 scores, k = 2,048:
-// 77 -> 33 us; 32 rows of 131,072: 20.1 -> 14.6; one row of 1,048,576: 63 -> 18.3; one of 2,500, k = 512: 7.8 -> 5.6.
+// 77 -> 33 us; 32 rows of 131,072: 20.1 -> 14.6; one row of 1,048,576: 63 -> 18.3; one of 2,500, k = 512: 7.8 -> 5.6
+// (key bits) -> 4.2 (bins of values, 1,024 threads); 4,096: 6.0 -> 4.4; 333 of 5,003: 13.7 -> 11.9; 1,184 of 8,192: 37.5 -> 34.1.
 // Scores rounded to integers (ties at the threshold), radix select / fallback alone / with the two bitmaps: 592 rows of
 // 32,768 79 / 116 / 43 us, 160 of 16,384 32 / 38 / 15, 32 of 131,072 21.5 / 44 / 12, one of 131,072 16 / 46 / 9.5; one row
 // of 1,048,576 equal scores 2,584 / 98 / 20.5.
-// Not better on one row of 16,384 (direct kernel): 9.9 -> 10.4 us.
 #include <cooperative_groups.h>
 #include <math.h>
 
@@ -155,11 +158,14 @@ __device__ __forceinline__ void rank_small(TopkShared* s, uint32_t cnt, uint32_t
 // --------------------------------------------------------------------------
 // rows of at most 16 keys per thread
 // --------------------------------------------------------------------------
-template <int NT>
-__global__ void __launch_bounds__(NT, 1024 / NT) topk_direct_kernel(TopkPivotParams p) {
-  constexpr int kWords = NT / 32 * kDirectKeys;
+template <int NT, int KEYS, int CTAS>
+__global__ void __launch_bounds__(NT, CTAS) topk_direct_kernel(TopkPivotParams p) {
+  constexpr int kWords = NT / 32 * KEYS;
+  // rows of more than 8,192 scores go by the key's bits: 2,048 bins of values hold too many of their keys to pay
+  constexpr bool kValueBins = NT * KEYS <= 8192;
   __shared__ uint32_t hist_a[kBigBins], hist_b[kBigBins];
   __shared__ uint32_t w_gt[kWords], w_eq[kWords], w_at[kWords];
+  __shared__ uint32_t w_max[32], w_min[32];
   __shared__ TopkShared s;
   ptx::grid_launch_dependents();   // the attention may set up on idle SMs; it waits for this grid before it reads ids
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -168,68 +174,139 @@ __global__ void __launch_bounds__(NT, 1024 / NT) topk_direct_kernel(TopkPivotPar
   const int n = (int)n64;
   int32_t* out = p.out_ids + (int64_t)row * p.k;
 
-  uint32_t key[kDirectKeys];
+  uint32_t key[KEYS];
 #pragma unroll
-  for (int u = 0; u < kDirectKeys; ++u) {
+  for (int u = 0; u < KEYS; ++u) {
     key[u] = 0xFF800000u;   // -inf
     if (u * NT + tid < n) key[u] = __float_as_uint(__ldg(src + u * NT + tid));
   }
-  for (int i = tid; i < kBigBins; i += NT) hist_a[i] = hist_b[i] = 0;
+  if constexpr (kValueBins)
+    for (int i = tid; i < kBigBins; i += NT) hist_a[i] = 0;
   if (tid == 0) {
     s.small_n = s.largest = 0;
     s.smallest = 0xffffffffu;
     s.thr[0] = s.thr[1] = s.thr[2] = s.thr[3] = 0;
   }
-  __syncthreads();
+  uint32_t top = 0, low = 0xffffffffu;
 #pragma unroll
-  for (int u = 0; u < kDirectKeys; ++u) {
+  for (int u = 0; u < KEYS; ++u) {
     key[u] = score_key_full(__uint_as_float(key[u]));
-    if (key[u]) atomicAdd(&hist_a[key[u] >> 21], 1u);
+    top = max(top, key[u]);
+    if (key[u]) low = min(low, key[u]);
   }
-  __syncthreads();
-  threshold_bin<NT>(hist_a, (uint32_t)p.k, s.sums[0], s.thr);
-  const uint32_t k_eff = s.thr[0], bin = s.thr[1];
-  uint32_t want = k_eff - s.thr[2];
-  for (int i = tid + (int)k_eff; i < p.k; i += NT) out[i] = -1;
-  if (k_eff == 0) return;
-#pragma unroll
-  for (int u = 0; u < kDirectKeys; ++u)
-    if ((key[u] >> 21) == bin && key[u]) atomicAdd(&hist_b[(key[u] >> 10) & 2047u], 1u);
-  __syncthreads();
-  for (int i = tid; i < 1024; i += NT) hist_a[i] = 0;   // read for the last time before the barrier
-  threshold_bin<NT>(hist_b, want, s.sums[1], s.thr);
-  const uint32_t head = (bin << 11) | s.thr[1], cnt = s.thr[3];   // the top 22 bits of the threshold
-  want -= s.thr[2];
-  if (cnt <= (uint32_t)kPSmall) {
-#pragma unroll
-    for (int u = 0; u < kDirectKeys; ++u)
-      if ((key[u] >> 10) == head && key[u]) s.small_keys[atomicAdd(&s.small_n, 1u)] = key[u];
-    __syncthreads();
-    rank_small(&s, cnt, want);
-  } else {   // ties, as a rule of a single value
-    uint32_t lo = 0xffffffffu, hi = 0;
-#pragma unroll
-    for (int u = 0; u < kDirectKeys; ++u) {
-      if ((key[u] >> 10) == head && key[u]) {
-        lo = min(lo, key[u]);
-        hi = max(hi, key[u]);
-      }
-    }
-    lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    if (lane == 0 && hi) {
-      atomicMin(&s.smallest, lo);
-      atomicMax(&s.largest, hi);
+  if constexpr (kValueBins) {
+    top = __reduce_max_sync(0xffffffffu, top);
+    low = __reduce_min_sync(0xffffffffu, low);
+    if (lane == 0) {
+      w_max[warp] = top;
+      w_min[warp] = low;
     }
     __syncthreads();
-    if (s.smallest == s.largest) {
-      if (tid == 0) {
-        s.T = s.largest;
-        s.need = want;
+  }
+  // ---- 2,048 equal bins over the range of the row without its outliers: from the second smallest of the warps' smallest
+  // scores to the second largest of their largest, what lies beyond goes to the outer bins (subtraction, product and
+  // clamps are monotone, so bins are in the order of the keys).  The threshold bin holds a few keys of an ordinary row.
+  uint32_t hi = 0, lo = 0;
+  if constexpr (kValueBins) {
+    top = lane < NT / 32 ? w_max[lane] : 0u;
+    low = lane < NT / 32 ? w_min[lane] : 0xffffffffu;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t h = __reduce_max_sync(0xffffffffu, top), l = __reduce_min_sync(0xffffffffu, low);
+      if (h) hi = h;
+      if (l != 0xffffffffu) lo = l;
+      if (top == h) top = 0;
+      if (low == l) low = 0xffffffffu;
+    }
+  }
+  const float x_lo = key_float(lo), scale = 2048.f / (key_float(hi) - x_lo);
+  const bool spread = kValueBins && hi > lo && lo != 0 && scale > 0.f && scale <= kMaxScore;   // not without a range that float can hold
+  auto bin_of = [&](uint32_t k) { return (int)fminf(fmaxf((key_float(k) - x_lo) * scale, 0.f), (float)(kBigBins - 1)); };
+  // Do all keys that `in` picks have one value (ties)?  Then that is the threshold.
+  auto one_value = [&](auto in, uint32_t need_of) -> bool {
+    uint32_t least = 0xffffffffu, most = 0;
+#pragma unroll
+    for (int u = 0; u < KEYS; ++u) {
+      if (in(key[u])) {
+        least = min(least, key[u]);
+        most = max(most, key[u]);
       }
+    }
+    least = __reduce_min_sync(0xffffffffu, least);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0 && most) {
+      atomicMin(&s.smallest, least);
+      atomicMax(&s.largest, most);
+    }
+    __syncthreads();
+    const bool one = s.smallest == s.largest;
+    if (one && tid == 0) {
+      s.T = s.largest;
+      s.need = need_of;
+    }
+    return one;
+  };
+  uint32_t k_eff, want;
+  bool found = false;
+  if (spread) {
+#pragma unroll
+    for (int u = 0; u < KEYS; ++u)
+      if (key[u]) atomicAdd(&hist_a[bin_of(key[u])], 1u);
+    __syncthreads();
+    threshold_bin<NT>(hist_a, (uint32_t)p.k, s.sums[0], s.thr);
+    const int bin = (int)s.thr[1];
+    const uint32_t cnt = s.thr[3];
+    k_eff = s.thr[0];
+    want = k_eff - s.thr[2];
+    if (cnt <= (uint32_t)kPSmall) {
+#pragma unroll
+      for (int u = 0; u < KEYS; ++u)
+        if (key[u] && bin_of(key[u]) == bin) s.small_keys[atomicAdd(&s.small_n, 1u)] = key[u];
+      __syncthreads();
+      rank_small(&s, cnt, want);
+      found = true;
     } else {
+      found = one_value([&](uint32_t k) { return k && bin_of(k) == bin; }, want);
+    }
+  }
+  if (!found) {
+    // ---- rows whose scores crowd into one bin, long ones, one value only: 11 + 11 + 10 key bits
+    if constexpr (kValueBins) __syncthreads();   // (the counters below have been read)
+    for (int i = tid; i < kBigBins; i += NT) hist_a[i] = hist_b[i] = 0;
+    if (tid == 0) {
+      s.small_n = s.largest = s.thr[0] = s.thr[1] = s.thr[2] = s.thr[3] = 0;
+      s.smallest = 0xffffffffu;
+    }
+    __syncthreads();
 #pragma unroll
-      for (int u = 0; u < kDirectKeys; ++u)
+    for (int u = 0; u < KEYS; ++u)
+      if (key[u]) atomicAdd(&hist_a[key[u] >> 21], 1u);
+    __syncthreads();
+    threshold_bin<NT>(hist_a, (uint32_t)p.k, s.sums[0], s.thr);
+    const uint32_t bin = s.thr[1];
+    k_eff = s.thr[0];
+    want = k_eff - s.thr[2];
+    if (k_eff == 0) {   // no finite score
+      for (int i = tid; i < p.k; i += NT) out[i] = -1;
+      return;
+    }
+#pragma unroll
+    for (int u = 0; u < KEYS; ++u)
+      if ((key[u] >> 21) == bin && key[u]) atomicAdd(&hist_b[(key[u] >> 10) & 2047u], 1u);
+    __syncthreads();
+    for (int i = tid; i < 1024; i += NT) hist_a[i] = 0;   // read for the last time before the barrier
+    threshold_bin<NT>(hist_b, want, s.sums[1], s.thr);
+    const uint32_t head = (bin << 11) | s.thr[1], cnt = s.thr[3];   // the top 22 bits of the threshold
+    want -= s.thr[2];
+    if (cnt <= (uint32_t)kPSmall) {
+#pragma unroll
+      for (int u = 0; u < KEYS; ++u)
+        if ((key[u] >> 10) == head && key[u]) s.small_keys[atomicAdd(&s.small_n, 1u)] = key[u];
+      __syncthreads();
+      rank_small(&s, cnt, want);
+    } else if (!one_value([&](uint32_t k) { return k && (k >> 10) == head; }, want)) {
+#pragma unroll
+      for (int u = 0; u < KEYS; ++u)
         if ((key[u] >> 10) == head && key[u]) atomicAdd(&hist_a[key[u] & 1023u], 1u);
       for (int i = 1024 + tid; i < kBigBins; i += NT) hist_a[i] = 0;
       __syncthreads();
@@ -240,12 +317,13 @@ __global__ void __launch_bounds__(NT, 1024 / NT) topk_direct_kernel(TopkPivotPar
       }
     }
   }
+  for (int i = tid + (int)k_eff; i < p.k; i += NT) out[i] = -1;
   __syncthreads();
   const uint32_t thr = s.T, need = s.need;
 
   // ---- ordered emission: word u * (NT / 32) + warp votes on positions u * NT + 32 * warp + (0 .. 31)
 #pragma unroll
-  for (int u = 0; u < kDirectKeys; ++u) {
+  for (int u = 0; u < KEYS; ++u) {
     const uint32_t gt = __ballot_sync(0xffffffffu, key[u] > thr), eq = __ballot_sync(0xffffffffu, key[u] == thr);
     if (lane == 0) {
       w_gt[u * (NT / 32) + warp] = gt;
@@ -263,7 +341,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) topk_direct_kernel(TopkPivotPar
   __syncthreads();
   const uint32_t below = (1u << lane) - 1u;
 #pragma unroll
-  for (int u = 0; u < kDirectKeys; ++u) {
+  for (int u = 0; u < KEYS; ++u) {
     if (key[u] >= thr) {   // thr > 0
       const int w = u * (NT / 32) + warp;
       const uint32_t g = (w_at[w] & 0xffffu) + __popc(w_gt[w] & below), q = (w_at[w] >> 16) + __popc(w_eq[w] & below);
@@ -821,9 +899,18 @@ static int launch_topk_clusters(const mxb_topk_args* a, int cs, cudaStream_t st)
   p.scores = a->scores; p.row_stride = a->row_stride; p.row_start = a->row_start; p.row_count = a->row_count;
   p.out_ids = a->out_ids; p.n = a->n; p.k = a->k;
   if (topk_direct(a->rows, a->n)) {
-    if (a->n <= 256 * kDirectKeys) topk_direct_kernel<256><<<(unsigned)a->rows, 256, 0, st>>>(p);
-    else if (a->n <= 512 * kDirectKeys) topk_direct_kernel<512><<<(unsigned)a->rows, 512, 0, st>>>(p);
-    else topk_direct_kernel<1024><<<(unsigned)a->rows, 1024, 0, st>>>(p);
+    const unsigned rows = (unsigned)a->rows;
+    // Every row has an SM to itself: all the threads there are, few keys each (148 rows of 4,096: 6.6 -> 5.0 us).  More
+    // rows: as many CTAs per SM as the registers of 16 keys allow (333 rows of 5,003 need one wave, not two).
+    if (a->rows <= sm_count()) {
+      if (a->n <= 1024 * 4) topk_direct_kernel<1024, 4, 1><<<rows, 1024, 0, st>>>(p);
+      else if (a->n <= 1024 * 8) topk_direct_kernel<1024, 8, 1><<<rows, 1024, 0, st>>>(p);
+      else topk_direct_kernel<1024, kDirectKeys, 1><<<rows, 1024, 0, st>>>(p);
+    } else if (a->n <= 256 * kDirectKeys) {
+      topk_direct_kernel<256, kDirectKeys, 6><<<rows, 256, 0, st>>>(p);
+    } else {
+      topk_direct_kernel<512, kDirectKeys, 3><<<rows, 512, 0, st>>>(p);
+    }
     note_launch();
     MXB_CUDA_OK(cudaGetLastError());
     return MXB_OK;

@@ -186,3 +186,28 @@ def test_causal_indexer_topk_known_answers(golden):
         got = causal_indexer_topk(dev(raw), dev(w), qp, np.arange(raw.shape[2]), ratio, topk=k,
                                   index_head_dim=D, n_heads=H).cpu().numpy()
         np.testing.assert_array_equal(got, golden[f"idx{i}_topk"])
+
+
+@pytest.mark.parametrize("rows,n,k", [(1, 33, 7), (1, 1025, 64), (2, 4096, 512), (3, 4097, 512), (2, 8192, 700), (2, 8193, 64),
+                                      (150, 300, 64), (150, 4097, 512)])
+def test_bins_of_values(rows, n, k):
+    """Rows in registers: the bins between a row's extremes with outliers that they leave out, with more keys in the
+    threshold bin than are ranked directly, and with ranges that give no bins at all."""
+    need_gpu()
+    rng = np.random.default_rng(n + rows)
+    base = rng.standard_normal((rows, n)).astype(np.float32)
+    few = base.copy()
+    few[:, 0], few[:, n // 2], few[:, -1] = 1e30, -1e30, 3e38
+    many = base.copy()
+    many[:, ::20] = 1e20 * (1 + np.abs(base[:, ::20]))       # every warp holds one
+    crowd = (100 + 1e-4 * base).astype(np.float32)
+    crowd[:, ::3] = base[:, ::3]                             # two thirds of the row in one bin
+    wide = base.copy()
+    wide[:, : n // 2] = 3.3e38 * np.sign(base[:, : n // 2])  # a range beyond float32
+    tiny = (base * 1e-41).astype(np.float32)                 # subnormal scores
+    flat = np.full((rows, n), -2.5, np.float32)
+    flat[:, n // 3] = 7.0
+    holes = base.copy()
+    holes[:, : n - n // 4] = -np.inf                         # warps without a score
+    for s in (base, few, many, crowd, wide, tiny, flat, holes, np.round(base), np.where(base > 0, 0.0, -0.0).astype(np.float32)):
+        _check(s, min(k, n))
