@@ -7,6 +7,7 @@
 // the scan, the selection and the attention are the package's kernels.  At 2,500 rows a token takes 57 us (44 us of it
 // in eight kernels); as some twenty single operators it took 378 us, 104 of them in kernels.
 #include "decode_rows.cuh"
+#include "ptx_sm100.cuh"
 
 namespace mxb {
 
@@ -48,6 +49,7 @@ struct DecodePrepParams {
 template <int QT>
 __global__ void __launch_bounds__(128) decode_prep_kernel(DecodePrepParams p) {
   const int lane = threadIdx.x & 31, w = (int)blockIdx.x * 4 + (threadIdx.x >> 5);
+  ptx::grid_chain();
   if (w < p.H) {
     float v[4], o[4];
 #pragma unroll
@@ -101,6 +103,7 @@ __global__ void __launch_bounds__(128) decode_sdpa_prep_kernel(SdpaPrepParams p)
   const int lane = threadIdx.x & 31, w = (int)blockIdx.x * 4 + (threadIdx.x >> 5);
   const bool vec = ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.window) |
                      reinterpret_cast<uintptr_t>(p.row)) & 15) == 0;
+  ptx::grid_chain();
   if (w < p.H) {
     const __half* src = p.q + (int64_t)w * kRowDim;
     __half* dst = p.q_roped + (int64_t)w * kRowDim;
@@ -121,6 +124,7 @@ __global__ void __launch_bounds__(128) decode_sdpa_prep_kernel(SdpaPrepParams p)
 
 __global__ void __launch_bounds__(128) decode_unrope_kernel(__half* out, const float* inv_freq, TokenParams token, int H) {
   const int lane = threadIdx.x & 31, w = (int)blockIdx.x * 4 + (threadIdx.x >> 5);
+  ptx::grid_chain();
   if (w < H) rope_row(out + (int64_t)w * kRowDim, out + (int64_t)w * kRowDim, token.at(0), inv_freq, true, lane);
 }
 
@@ -176,11 +180,11 @@ extern "C" int mxb_fused_decode_prep(const mxb_fused_decode_prep_args* a, void* 
   const int64_t topk_bytes = mxb_topk_workspace_bytes(1, a->n_rows, a->topk);
   void* topk_ws = ws.take(topk_bytes);
   const unsigned grid = (unsigned)ceil_div(a->n_heads + 3, 4);
-  if (a->q_dtype == MXB_F32) decode_prep_kernel<MXB_F32><<<grid, 128, 0, st>>>(p);
-  else if (a->q_dtype == MXB_F16) decode_prep_kernel<MXB_F16><<<grid, 128, 0, st>>>(p);
-  else decode_prep_kernel<MXB_BF16><<<grid, 128, 0, st>>>(p);
+  auto* prep = a->q_dtype == MXB_F32   ? decode_prep_kernel<MXB_F32>
+               : a->q_dtype == MXB_F16 ? decode_prep_kernel<MXB_F16>
+                                       : decode_prep_kernel<MXB_BF16>;
+  MXB_CUDA_OK(launch_early(prep, dim3(grid), 128, 0, st, p));
   note_launch();
-  MXB_CUDA_OK(cudaGetLastError());
 
   mxb_indexer_scores_args s{};
   s.q = p.q_qat; s.q_dtype = MXB_F32;
@@ -247,18 +251,17 @@ extern "C" int mxb_fused_decode_sdpa(const mxb_fused_decode_sdpa_args* a, void* 
   const int64_t attn_bytes = mxb_sparse_attn_workspace_bytes(&s);
   s.workspace = ws.take(attn_bytes);
   s.workspace_bytes = attn_bytes;
-  decode_sdpa_prep_kernel<<<(unsigned)ceil_div((int64_t)a->n_heads + a->window_rows + 1, 4), 128, 0, st>>>(p);
+  MXB_CUDA_OK(launch_early(decode_sdpa_prep_kernel, dim3((unsigned)ceil_div((int64_t)a->n_heads + a->window_rows + 1, 4)), 128, 0,
+                           st, p));
   note_launch();
-  MXB_CUDA_OK(cudaGetLastError());
   s.q = p.q_roped;
   s.raw_kv = a->window_rows > 0 ? p.keys : nullptr;
   s.sinks = p.sinks_f;
   s.pos0_dev = p.pos0;
   int rc = mxb_sparse_attn(&s, stream);
   if (rc != MXB_OK) return rc;
-  decode_unrope_kernel<<<(unsigned)ceil_div(a->n_heads, 4), 128, 0, st>>>(reinterpret_cast<__half*>(a->out), a->inv_freq,
-                                                                          p.token, a->n_heads);
+  MXB_CUDA_OK(launch_early(decode_unrope_kernel, dim3((unsigned)ceil_div(a->n_heads, 4)), 128, 0, st,
+                           reinterpret_cast<__half*>(a->out), a->inv_freq, p.token, a->n_heads));
   note_launch();
-  MXB_CUDA_OK(cudaGetLastError());
   return MXB_OK;
 }

@@ -24,6 +24,7 @@
 // tensor work is tiny (32 flop per byte); this kernel is bound by HBM, which is why it uses
 // warp-level MMA rather than the tcgen05 pipeline the prefill form needs.
 #include "common.cuh"
+#include "ptx_sm100.cuh"
 #include "topk_common.cuh"
 
 namespace mxb {
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, (D == 64 && NT <= 2) ? 3 : 1) 
   constexpr int VPL = EPL / 16; // 16-byte loads per lane per row
   extern __shared__ int64_t pre_s[];   // [B + 1] exclusive prefix sums of the row counts
   __shared__ uint32_t hist_s[HIST ? kBigBins : 1];
+  ptx::grid_launch_dependents();   // the selection may be launched meanwhile; it waits for this grid
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   if constexpr (HIST)

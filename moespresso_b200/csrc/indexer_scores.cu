@@ -43,6 +43,8 @@ template <int D, int QT, int KT>
 __global__ void __launch_bounds__(128) indexer_exact_kernel(IndexerParams p) {
   extern __shared__ float q_s[];  // [t_tile][H][D]
   float* w_s = q_s + (size_t)p.t_tile * p.H * D;
+  ptx::grid_chain();
+  p.keys = ptx::behind_wait(p.keys);
   const int b = blockIdx.z;
   const int t0 = blockIdx.y * p.t_tile;
   const int64_t count = p.row_count ? (int64_t)p.row_count[b] : p.n_rows;
@@ -108,6 +110,8 @@ __global__ void __launch_bounds__(256) indexer_exact_token_kernel(IndexerParams 
   float4* q_s = k_s + ROWS * LD;                   // [8 HPW][D / 4], heads beyond H are zeros
   float* w_s = reinterpret_cast<float*>(q_s + 8 * HPW * (D / 4));   // [8 HPW]
   float* d_s = reinterpret_cast<float*>(k_s);      // afterwards: rectified dots [8 HPW][ROWS]
+  ptx::grid_chain();
+  p.keys = ptx::behind_wait(p.keys);
   const int b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t count = p.row_count ? (int64_t)p.row_count[b] : p.n_rows;
   const int64_t rbase = p.row_start ? p.row_start[b] : (int64_t)b * p.n_rows;
@@ -183,9 +187,8 @@ static int launch_exact_token(const IndexerParams& p, cudaStream_t st) {
   static_assert(8 * HPW <= D, "the dots take the keys' place");
   auto kern = indexer_exact_token_kernel<D, QT, KT, HPW, RPL>;
   if (smem > 48 * 1024) MXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<dim3((unsigned)ceil_div(p.n_rows, 32 * RPL), 1, (unsigned)p.B), 256, smem, st>>>(p);
+  MXB_CUDA_OK(launch_early(kern, dim3((unsigned)ceil_div(p.n_rows, 32 * RPL), 1, (unsigned)p.B), 256, smem, st, p));
   note_launch();
-  MXB_CUDA_OK(cudaGetLastError());
   return MXB_OK;
 }
 
@@ -223,9 +226,8 @@ static int launch_exact(IndexerParams& p, cudaStream_t st) {
   auto kern = indexer_exact_kernel<D, QT, KT>;
   if (smem > 48 * 1024) MXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((unsigned)ceil_div(p.n_rows, 128), (unsigned)ceil_div(p.T, t_tile), (unsigned)p.B);
-  kern<<<grid, 128, smem, st>>>(p);
+  MXB_CUDA_OK(launch_early(kern, grid, 128, smem, st, p));
   note_launch();
-  MXB_CUDA_OK(cudaGetLastError());
   return MXB_OK;
 }
 

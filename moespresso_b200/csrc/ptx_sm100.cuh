@@ -30,6 +30,18 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 // if that was launched with the attribute for it; the next one waits for its completion before it reads its results.
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The first lines of a kernel launched with launch_early: wait for the kernel before, then let the next one start.  In
+// this order, so that a kernel which starts while the one before it runs finds everything further back complete.
+__device__ __forceinline__ void grid_chain() {
+  grid_dependency_wait();
+  grid_launch_dependents();
+}
+// A pointer whose loads cannot move above the wait (read-only loads are free to move across a memory barrier).
+template <class T>
+__device__ __forceinline__ T* behind_wait(T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");

@@ -16,6 +16,7 @@
 //    rows (see the comment at the kernel); every split writes (o, m, l) partials for the log-sum-exp merge kernel
 //    (mxb_merge_partials).  HBM-bound: 2 x (256 + 16) bytes per key and KV head are read once.
 #include "common.cuh"
+#include "ptx_sm100.cuh"
 
 namespace mxb {
 
@@ -79,9 +80,10 @@ template <int XT, bool VEC, bool PAIR>
 __global__ void __launch_bounds__(128) affine_q8_quantize_kernel(const __grid_constant__ Q8Rows p) {
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  ptx::grid_chain();
   if (row >= p.n_rows) return;
   const bool second = PAIR && blockIdx.z != 0;   // (selected, not indexed: an indexed parameter is a dependent load)
-  const void* x = second ? p.x[1] : p.x[0];
+  const void* x = ptx::behind_wait(second ? p.x[1] : p.x[0]);
   uint32_t* packed = second ? p.packed[1] : p.packed[0];
   void* scales = second ? p.scales[1] : p.scales[0];
   void* biases = second ? p.biases[1] : p.biases[0];
@@ -287,6 +289,7 @@ __global__ void __launch_bounds__(QD_WARPS * 32, 3) q8_decode_kernel(Q8DecodePar
   const int g = lane >> 2, t = lane & 3;
   const int G = p.Hq / p.Hkv;
   uint8_t* my_stage = q8_smem + (size_t)warp * QD_STAGES * STAGE_BYTES;
+  ptx::grid_chain();
 
   // q as B fragments of k-step i = 4 grp + w: head g, features 64 grp + 16 t + 4 w + {0, 1} and + {2, 3}, times
   // scale * log2(e), fp16.  The sixteen features of a k-step lie in ONE quantisation group.
@@ -557,15 +560,15 @@ static int launch_quantize(const Q8Rows& p, int tensors, int x_dtype, cudaStream
   const dim3 grid((unsigned)ceil_div(p.n_rows, 4), (unsigned)p.heads, (unsigned)tensors);
 #define MXB_Q(XT)                                                                                  \
   if (x_dtype == XT) {                                                                             \
-    if (tensors == 1 && vec) affine_q8_quantize_kernel<XT, true, false><<<grid, 128, 0, st>>>(p);  \
-    else if (tensors == 1) affine_q8_quantize_kernel<XT, false, false><<<grid, 128, 0, st>>>(p);   \
-    else if (vec) affine_q8_quantize_kernel<XT, true, true><<<grid, 128, 0, st>>>(p);              \
-    else affine_q8_quantize_kernel<XT, false, true><<<grid, 128, 0, st>>>(p);                      \
+    MXB_CUDA_OK(launch_early(tensors == 1 && vec ? affine_q8_quantize_kernel<XT, true, false>      \
+                             : tensors == 1      ? affine_q8_quantize_kernel<XT, false, false>     \
+                             : vec               ? affine_q8_quantize_kernel<XT, true, true>       \
+                                                 : affine_q8_quantize_kernel<XT, false, true>,     \
+                             grid, 128, 0, st, p));                                                \
   }
   MXB_Q(MXB_F32) else MXB_Q(MXB_F16) else MXB_Q(MXB_BF16)
 #undef MXB_Q
   note_launch();
-  MXB_CUDA_OK(cudaGetLastError());
   return MXB_OK;
 }
 
@@ -702,7 +705,7 @@ extern "C" int mxb_sdpa_decode_q8(const mxb_sdpa_decode_q8_args* a, void* stream
     const int out_bytes = QD_WARPS * QD_MAXG * QD_D * 4;                                                         \
     const int smem = stage_bytes > out_bytes ? stage_bytes : out_bytes;                                          \
     MXB_CUDA_OK(cudaFuncSetAttribute(q8_decode_kernel<ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
-    q8_decode_kernel<ST><<<grid, QD_WARPS * 32, smem, st>>>(p);                                                 \
+    MXB_CUDA_OK(launch_early(q8_decode_kernel<ST>, grid, QD_WARPS * 32, smem, st, p));                          \
   }
   if (a->sb_dtype == MXB_F32) MXB_QD(MXB_F32)
   else if (a->sb_dtype == MXB_F16) MXB_QD(MXB_F16)
@@ -710,6 +713,5 @@ extern "C" int mxb_sdpa_decode_q8(const mxb_sdpa_decode_q8_args* a, void* stream
   else return fail(MXB_ERR_INVALID, "q8 decode: scales and biases must be float32, float16 or bfloat16");
 #undef MXB_QD
   note_launch();
-  MXB_CUDA_OK(cudaGetLastError());
   return MXB_OK;
 }

@@ -10,6 +10,7 @@
 // the row list write (o, m, l) partials that merge_kernel combines by log-sum-exp; the
 // sink joins once, in the merge (or in the single-split epilogue).
 #include "common.cuh"
+#include "ptx_sm100.cuh"
 #include "sparse_attn.cuh"
 
 namespace mxb {
@@ -62,6 +63,9 @@ __global__ void __launch_bounds__(256) sparse_attn_kernel(SparseParams p) {
   int* valid_s = reinterpret_cast<int*>(p_s + kHeadsPerCta * kTileRows);  // [32]
   __shared__ int s_keff;
 
+  ptx::grid_chain();
+  p.comp_kv = ptx::behind_wait(p.comp_kv);
+  p.raw_kv = ptx::behind_wait(p.raw_kv);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int split = blockIdx.x;
   const int h = blockIdx.y * kHeadsPerCta + warp;
@@ -278,6 +282,9 @@ struct MergeParams {
 template <int OT, int VEC>
 __global__ void __launch_bounds__(256) merge_kernel(MergeParams p) {
   // one thread = one (row, VEC consecutive features); partial loads are independent, so many are in flight
+  ptx::grid_chain();
+  p.ml_parts = ptx::behind_wait(p.ml_parts);
+  p.o_parts = ptx::behind_wait(p.o_parts);
   const int64_t N = (int64_t)p.B * p.T * p.H;
   const int per_row = p.Dv / VEC;
   const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -395,6 +402,9 @@ __global__ void __launch_bounds__(256) merge_rows_kernel(MergeParams p) {
   __shared__ float w_s[kMergeRowsMaxP];
   __shared__ float red[256];
   __shared__ float4 part[256];
+  ptx::grid_chain();
+  p.ml_parts = ptx::behind_wait(p.ml_parts);
+  p.o_parts = ptx::behind_wait(p.o_parts);
   const int64_t N = (int64_t)p.B * p.T * p.H;
   const int64_t n = blockIdx.x;
   const int tid = threadIdx.x;
@@ -483,23 +493,21 @@ static int launch_merge(const MergeParams& mp, int out_dtype, cudaStream_t st) {
   // few rows, many splits: spread the splits over a CTA per row instead of one thread walking them all
   if (vec && mp.P > 16 && mp.P <= kMergeRowsMaxP && mp.Dv / 4 <= 256 && 256 % (mp.Dv / 4) == 0 && items < 148 * 2 * 256) {
     const dim3 rows((unsigned)N, mp.Dv >= 64 && 4 * N <= sm_count() ? 4u : 1u);
-    if (out_dtype == MXB_F32) merge_rows_kernel<MXB_F32><<<rows, 256, 0, st>>>(mp);
-    else if (out_dtype == MXB_BF16) merge_rows_kernel<MXB_BF16><<<rows, 256, 0, st>>>(mp);
-    else merge_rows_kernel<MXB_F16><<<rows, 256, 0, st>>>(mp);
+    MXB_CUDA_OK(launch_early(out_dtype == MXB_F32    ? merge_rows_kernel<MXB_F32>
+                             : out_dtype == MXB_BF16 ? merge_rows_kernel<MXB_BF16>
+                                                     : merge_rows_kernel<MXB_F16>,
+                             rows, 256, 0, st, mp));
     note_launch();
-    MXB_CUDA_OK(cudaGetLastError());
     return MXB_OK;
   }
   dim3 grid((unsigned)ceil_div(items, 256));
 #define MXB_MG(OT)                                             \
-  if (vec) merge_kernel<OT, 4><<<grid, 256, 0, st>>>(mp);      \
-  else merge_kernel<OT, 1><<<grid, 256, 0, st>>>(mp);
+  MXB_CUDA_OK(launch_early(vec ? merge_kernel<OT, 4> : merge_kernel<OT, 1>, grid, 256, 0, st, mp));
   if (out_dtype == MXB_F32) { MXB_MG(MXB_F32) }
   else if (out_dtype == MXB_BF16) { MXB_MG(MXB_BF16) }
   else { MXB_MG(MXB_F16) }
 #undef MXB_MG
   note_launch();
-  MXB_CUDA_OK(cudaGetLastError());
   return MXB_OK;
 }
 
@@ -527,7 +535,7 @@ static int launch_sparse(SparseParams& p, int out_dtype, size_t smem, dim3 grid,
   {                                                                                                        \
     auto kern = sparse_attn_kernel<KVT, QT, OT>;                                                           \
     MXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));       \
-    kern<<<grid, 256, smem, st>>>(p);                                                                      \
+    MXB_CUDA_OK(launch_early(kern, grid, 256, smem, st, p));                                               \
   }
   if (out_dtype == MXB_F32 || p.nsplit > 1 || p.partial_ml) MXB_SP(MXB_F32)
   else if (out_dtype == MXB_BF16) MXB_SP(MXB_BF16)

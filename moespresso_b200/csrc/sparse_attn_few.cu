@@ -149,6 +149,8 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
   const int unit = (int)(blockIdx.x / (unsigned)C);
   const int bt = unit / fp.groups, h0 = (unit - bt * fp.groups) * kFewHeads;
   const int b = bt / p.T, t = bt - b * p.T;
+  if (!p.after_select) ptx::grid_dependency_wait();   // behind a selection q and all else but the list are complete
+  const void* q_in = ptx::behind_wait(p.q);
   ptx::cluster_arrive();   // (0) every CTA of the cluster has started: waited for before the first remote store
   if (tid == 0) *keff_s = p.k;
 
@@ -156,7 +158,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
   uint32_t qf[NB][4][4];        // [block][step][A registers]
   float q_mul[2] = {1.f, 1.f};  // int8 rows: what undoes the power of two that q was scaled by
   {
-    const bool vec = fp.q_dtype != MXB_F32 && ((reinterpret_cast<uintptr_t>(p.q) & 15) == 0) && p.q_sb % 8 == 0 &&
+    const bool vec = fp.q_dtype != MXB_F32 && ((reinterpret_cast<uintptr_t>(q_in) & 15) == 0) && p.q_sb % 8 == 0 &&
                      p.q_sh % 8 == 0 && p.q_st % 8 == 0;
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh) {
@@ -166,7 +168,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
       if (h < p.H && vec) {
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
-          const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.q) + base + i * 64);
+          const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(q_in) + base + i * 64);
           const uint4 x = __ldg(src), y = __ldg(src + 1);
           w[i][0] = x.x; w[i][1] = x.y; w[i][2] = x.z; w[i][3] = x.w;
           w[i][4] = y.x; w[i][5] = y.y; w[i][6] = y.z; w[i][7] = y.w;
@@ -180,9 +182,9 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
             if (h < p.H) {
               const int64_t at = base + i * 64 + 2 * e;
               if (fp.q_dtype == MXB_F32) {
-                w[i][e] = pack16<BF16>(reinterpret_cast<const float*>(p.q)[at], reinterpret_cast<const float*>(p.q)[at + 1]);
+                w[i][e] = pack16<BF16>(reinterpret_cast<const float*>(q_in)[at], reinterpret_cast<const float*>(q_in)[at + 1]);
               } else {
-                const uint16_t* src = reinterpret_cast<const uint16_t*>(p.q) + at;
+                const uint16_t* src = reinterpret_cast<const uint16_t*>(q_in) + at;
                 w[i][e] = (uint32_t)src[0] | ((uint32_t)src[1] << 16);
               }
             }
@@ -249,6 +251,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
   __syncthreads();   // the list's end is initialised
   // The list is all that the selection right before this launch writes: it may still have been running so far.
   if (p.after_select) ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   const int32_t* ids = p.topk + (int64_t)bt * p.k;
   {
     // this CTA's rows; whether the list ends before them is known only after the scan, but a row inside the visible range
@@ -537,7 +540,7 @@ static int launch_few_typed(const FewParams& fp, int smem, int clusters, cudaStr
   at[0].val.clusterDim.x = (unsigned)C;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // behind a selection: see launch_tc_typed
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // (the kernel waits, see grid_chain)
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
@@ -555,7 +558,7 @@ static int launch_few_typed(const FewParams& fp, int smem, int clusters, cudaStr
     if (cached) *cached = resident;
   }
   if (resident < clusters) return MXB_ERR_UNSUPPORTED;
-  cfg.numAttrs = fp.s.after_select ? 2 : 1;
+  cfg.numAttrs = 2;
   MXB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, fp));
   note_launch();
   return MXB_OK;

@@ -167,10 +167,10 @@ __global__ void __launch_bounds__(NT, CTAS) topk_direct_kernel(TopkPivotParams p
   __shared__ uint32_t w_gt[kWords], w_eq[kWords], w_at[kWords];
   __shared__ uint32_t w_max[32], w_min[32];
   __shared__ TopkShared s;
-  ptx::grid_launch_dependents();   // the attention may set up on idle SMs; it waits for this grid before it reads ids
+  ptx::grid_chain();   // (the attention may set up on idle SMs; it waits for this grid before it reads ids)
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int64_t n64;
-  const float* src = row_scores(p, row, &n64);
+  const float* src = ptx::behind_wait(row_scores(p, row, &n64));
   const int n = (int)n64;
   int32_t* out = p.out_ids + (int64_t)row * p.k;
 
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkP
   __shared__ uint32_t s_sum[2], s_top, s_tie[2];
   __shared__ uint32_t cl_count[kPMaxCluster], cl_gt[kPMaxCluster], cl_eq[kPMaxCluster];
 
-  ptx::grid_launch_dependents();   // as above
+  ptx::grid_chain();   // as above
   cg::cluster_group cluster = cg::this_cluster();
   const int cs = CLUSTER ? (int)cluster.num_blocks() : 1;
   const int rank = CLUSTER ? (int)cluster.block_rank() : 0;
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 3 : 1) topk_pivot_kernel(TopkP
   uint32_t* w_at = hist_b;
 
   int64_t n;
-  const float* src = row_scores(p, row, &n);
+  const float* src = ptx::behind_wait(row_scores(p, row, &n));
   // this CTA's scores: equal parts of the row's own length, which may be far below the longest of a ragged batch
   const int64_t share = cs > 1 ? round_up(ceil_div(n, (int64_t)cs), (int64_t)1024) : (int64_t)p.part;
   const int64_t lo = min((int64_t)rank * share, n);
@@ -874,13 +874,15 @@ static int launch_pivot(const TopkPivotParams& p, int rows, int cs, cudaStream_t
   cfg.blockDim = dim3(NT);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)cs;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)cs;
+  at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = CLUSTER ? 1 : 0;
+  cfg.numAttrs = CLUSTER ? 2 : 1;
   if (cs > 8) {   // sixteen SMs of one GPC are not there on every device or SM set
     int resident = 0;
     if (cudaOccupancyMaxActiveClusters(&resident, kern, &cfg) != cudaSuccess || resident < 1) {
@@ -903,16 +905,16 @@ static int launch_topk_clusters(const mxb_topk_args* a, int cs, cudaStream_t st)
     // Every row has an SM to itself: all the threads there are, few keys each (148 rows of 4,096: 6.6 -> 5.0 us).  More
     // rows: as many CTAs per SM as the registers of 16 keys allow (333 rows of 5,003 need one wave, not two).
     if (a->rows <= sm_count()) {
-      if (a->n <= 1024 * 4) topk_direct_kernel<1024, 4, 1><<<rows, 1024, 0, st>>>(p);
-      else if (a->n <= 1024 * 8) topk_direct_kernel<1024, 8, 1><<<rows, 1024, 0, st>>>(p);
-      else topk_direct_kernel<1024, kDirectKeys, 1><<<rows, 1024, 0, st>>>(p);
+      MXB_CUDA_OK(launch_early(a->n <= 1024 * 4   ? topk_direct_kernel<1024, 4, 1>
+                               : a->n <= 1024 * 8 ? topk_direct_kernel<1024, 8, 1>
+                                                  : topk_direct_kernel<1024, kDirectKeys, 1>,
+                               dim3(rows), 1024, 0, st, p));
     } else if (a->n <= 256 * kDirectKeys) {
-      topk_direct_kernel<256, kDirectKeys, 6><<<rows, 256, 0, st>>>(p);
+      MXB_CUDA_OK(launch_early(topk_direct_kernel<256, kDirectKeys, 6>, dim3(rows), 256, 0, st, p));
     } else {
-      topk_direct_kernel<512, kDirectKeys, 3><<<rows, 512, 0, st>>>(p);
+      MXB_CUDA_OK(launch_early(topk_direct_kernel<512, kDirectKeys, 3>, dim3(rows), 512, 0, st, p));
     }
     note_launch();
-    MXB_CUDA_OK(cudaGetLastError());
     return MXB_OK;
   }
   p.part = (int32_t)round_up(ceil_div(a->n, (int64_t)cs), (int64_t)1024);
