@@ -7,7 +7,8 @@
 // rows), the row splits of a head group form one thread-block cluster (up to 16 CTAs), and nothing is pipelined because
 // nothing repeats:
 //
-//   q fragments into registers, before the selection is waited for
+//   q once into shared memory (int8 rows: scaled, two heads per warp) and from there into every warp's registers, before
+//   the selection is waited for (eight warps loading the fragments from global memory took 4,000 cycles, int8 7,700)
 //   list ids -> rows; every warp fetches its own eight rows of every 64 (16-byte asynchronous copies) and multiplies them
 //   as soon as they are there:  S[16 heads x 8 rows] = Q . K^T
 //   softmax over the CTA's rows with their exact maximum
@@ -30,7 +31,7 @@
 // logit + log2(scale), the denominator takes the rounded weights divided by the scale.
 //
 // What bounds it: latency, front to back (launch, list, rows, two contractions of one pass, cluster barrier, output); a
-// further 64 rows per CTA cost 2.1 (bf16) to 2.3 us (int8).  Both sides measured: at the rule in launch_sparse_few.
+// further 64 rows per CTA cost 2 us.  Both sides measured: at the rule in launch_sparse_few.
 #include "common.cuh"
 #include "ptx_sm100.cuh"
 #include "sparse_attn.cuh"
@@ -50,20 +51,22 @@ __host__ __device__ constexpr int few_max_rows(int eb) { return eb == 1 ? 256 : 
 struct FewLayout {
   int row_pitch;    // bytes of a staged row: an odd multiple of 16, so that eight rows cover all banks
   int s_pitch;      // floats of a head's logits; its 16-bit weights are written over them
-  int s_off, ref_off, scale_off, recv_off, ml_off, fac_off, misc_off, total;
+  int q_off;        // the 16 heads as operands: where partials arrive later
+  int s_off, row_off, scale_off, recv_off, ml_off, fac_off, misc_off, total;
 };
 __host__ __device__ inline FewLayout few_layout(int Dqk, int eb, int rows, int splits) {
   FewLayout L;
   L.row_pitch = Dqk * eb + 16;
   L.s_pitch = rows + 4;
   L.s_off = rows * L.row_pitch;
-  L.ref_off = L.s_off + kFewHeads * L.s_pitch * 4;
-  L.scale_off = L.ref_off + rows * 4;
-  L.recv_off = L.scale_off + rows * 4;
+  L.row_off = L.s_off + kFewHeads * L.s_pitch * 4;
+  L.scale_off = L.row_off + rows * 8;
+  L.recv_off = L.scale_off + (eb == 1 ? rows * 12 : 0);
+  L.q_off = L.recv_off;
   L.ml_off = L.recv_off + (kFewDv / kFewBlk + splits - 1) / splits * splits * kFewBlkBytes;
   L.fac_off = L.ml_off + splits * kFewHeads * 8;
   L.misc_off = L.fac_off + splits * kFewHeads * 4;
-  L.total = L.misc_off + 16;
+  L.total = L.misc_off + 80;
   return L;
 }
 
@@ -136,12 +139,15 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
   const int C = p.nsplit, R = fp.rows;
   const FewLayout L = few_layout(NB * 64, EB, R, C);
   float* s_s = reinterpret_cast<float*>(smem + L.s_off);
-  uint32_t* ref_s = reinterpret_cast<uint32_t*>(smem + L.ref_off);
-  float* scale_s = reinterpret_cast<float*>(smem + L.scale_off);
+  const uint8_t** row_s = reinterpret_cast<const uint8_t**>(smem + L.row_off);   // [R] address of the row, or null
+  float* scale_s = reinterpret_cast<float*>(smem + L.scale_off);                 // int8 rows, [R] each: scale,
+  float* lscale_s = scale_s + R;                                                 //   its log2,
+  float* iscale_s = lscale_s + R;                                                //   and its inverse
   const float* recv = reinterpret_cast<const float*>(smem + L.recv_off);
   float2* ml_s = reinterpret_cast<float2*>(smem + L.ml_off);
   float* fac_s = reinterpret_cast<float*>(smem + L.fac_off);
   int* keff_s = reinterpret_cast<int*>(smem + L.misc_off);
+  float* qmul_s = reinterpret_cast<float*>(smem + L.misc_off + 16);   // [16] int8 rows: undoes the power of two that q was scaled by
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t4 = lane & 3;
@@ -151,81 +157,100 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
   const int b = bt / p.T, t = bt - b * p.T;
   if (!p.after_select) ptx::grid_dependency_wait();   // behind a selection q and all else but the list are complete
   const void* q_in = ptx::behind_wait(p.q);
-  ptx::cluster_arrive();   // (0) every CTA of the cluster has started: waited for before the first remote store
   if (tid == 0) *keff_s = p.k;
 
-  // ---- q: fragments of the 16 heads, every warp the same
-  uint32_t qf[NB][4][4];        // [block][step][A registers]
-  float q_mul[2] = {1.f, 1.f};  // int8 rows: what undoes the power of two that q was scaled by
+  // ---- q: every warp turns two heads into operands in shared memory, then all warps read the fragments of all 16
   {
+    constexpr int kQPitch = NB * 128 + 16;   // an odd multiple of 16 bytes
+    uint8_t* q_s = smem + L.q_off;
     const bool vec = fp.q_dtype != MXB_F32 && ((reinterpret_cast<uintptr_t>(q_in) & 15) == 0) && p.q_sb % 8 == 0 &&
                      p.q_sh % 8 == 0 && p.q_st % 8 == 0;
+    auto two = [&](uint32_t x) -> float2 {
+      if (fp.q_dtype == MXB_BF16) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x));
+      return __half22float2(*reinterpret_cast<const __half2*>(&x));
+    };
+    uint32_t w[2][3][4];   // [head][piece of eight features][pair]
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh) {
-      const int h = h0 + g + 8 * hh;
-      const int64_t base = (int64_t)b * p.q_sb + (int64_t)h * p.q_sh + (int64_t)t * p.q_st + 16 * t4;
-      uint32_t w[NB][8];
-      if (h < p.H && vec) {
+      const int h = h0 + 2 * warp + hh;
+      const int64_t base = (int64_t)b * p.q_sb + (int64_t)h * p.q_sh + (int64_t)t * p.q_st;
 #pragma unroll
-        for (int i = 0; i < NB; ++i) {
-          const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(q_in) + base + i * 64);
-          const uint4 x = __ldg(src), y = __ldg(src + 1);
-          w[i][0] = x.x; w[i][1] = x.y; w[i][2] = x.z; w[i][3] = x.w;
-          w[i][4] = y.x; w[i][5] = y.y; w[i][6] = y.z; w[i][7] = y.w;
-        }
-      } else {
+      for (int c = 0; c < 3; ++c) {
+        const int ck = c * 32 + lane;
+        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+        if (h < p.H && ck < NB * 8) {
+          if (vec) {
+            x = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(q_in) + base) + ck);
+          } else {
+            uint32_t e4[4];
 #pragma unroll
-        for (int i = 0; i < NB; ++i)
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            w[i][e] = 0u;
-            if (h < p.H) {
-              const int64_t at = base + i * 64 + 2 * e;
+            for (int e = 0; e < 4; ++e) {
+              const int64_t at = base + 8 * ck + 2 * e;
               if (fp.q_dtype == MXB_F32) {
-                w[i][e] = pack16<BF16>(reinterpret_cast<const float*>(q_in)[at], reinterpret_cast<const float*>(q_in)[at + 1]);
+                e4[e] = pack16<BF16>(reinterpret_cast<const float*>(q_in)[at], reinterpret_cast<const float*>(q_in)[at + 1]);
               } else {
                 const uint16_t* src = reinterpret_cast<const uint16_t*>(q_in) + at;
-                w[i][e] = (uint32_t)src[0] | ((uint32_t)src[1] << 16);
+                e4[e] = (uint32_t)src[0] | ((uint32_t)src[1] << 16);
               }
             }
+            x = make_uint4(e4[0], e4[1], e4[2], e4[3]);
           }
+        }
+        w[hh][c][0] = x.x; w[hh][c][1] = x.y; w[hh][c][2] = x.z; w[hh][c][3] = x.w;
       }
+    }
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
       if constexpr (I8) {
-        auto two = [&](uint32_t x) -> float2 {
-          if (fp.q_dtype == MXB_BF16) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x));
-          return __half22float2(*reinterpret_cast<const __half2*>(&x));
-        };
         float amax = 0.f;
 #pragma unroll
-        for (int i = 0; i < NB; ++i)
+        for (int c = 0; c < 3; ++c)
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float2 v = two(w[i][e]);
+          for (int e = 0; e < 4; ++e) {
+            const float2 v = two(w[hh][c][e]);
             amax = fmaxf(amax, fmaxf(fabsf(v.x), fabsf(v.y)));
           }
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+        amax = warp_max(amax);
         const int ex = (int)(__float_as_uint(amax) >> 23) - 127;   // floor(log2(max)); zeros and denormals: any power does
         const int sh = min(max(14 - ex, -100), 100);
         const float up = __uint_as_float((uint32_t)(127 + sh) << 23);
-        q_mul[hh] = __uint_as_float((uint32_t)(127 - sh) << 23);
+        if (lane == 0) qmul_s[2 * warp + hh] = __uint_as_float((uint32_t)(127 - sh) << 23);
 #pragma unroll
-        for (int i = 0; i < NB; ++i)
+        for (int c = 0; c < 3; ++c)
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float2 v = two(w[i][e]);
-            w[i][e] = pack16<false>(v.x * up, v.y * up);
+          for (int e = 0; e < 4; ++e) {
+            const float2 v = two(w[hh][c][e]);
+            w[hh][c][e] = pack16<false>(v.x * up, v.y * up);
           }
       }
 #pragma unroll
-      for (int i = 0; i < NB; ++i)
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-          qf[i][s][hh] = w[i][2 * s];
-          qf[i][s][2 + hh] = w[i][2 * s + 1];
-        }
+      for (int c = 0; c < 3; ++c) {
+        const int ck = c * 32 + lane;
+        if (ck < NB * 8)
+          *reinterpret_cast<uint4*>(q_s + (2 * warp + hh) * kQPitch + ck * 16) =
+              make_uint4(w[hh][c][0], w[hh][c][1], w[hh][c][2], w[hh][c][3]);
+      }
     }
   }
+  __syncthreads();   // (the list's end is initialised, too)
+  uint32_t qf[NB][4][4];        // fragments: [block][step][A registers]
+  float q_mul[2] = {1.f, 1.f};
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {
+    const uint8_t* qrow = smem + L.q_off + (g + 8 * hh) * (NB * 128 + 16) + 32 * t4;
+    if constexpr (I8) q_mul[hh] = qmul_s[g + 8 * hh];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const uint4 x = *reinterpret_cast<const uint4*>(qrow + i * 128), y = *reinterpret_cast<const uint4*>(qrow + i * 128 + 16);
+      qf[i][0][hh] = x.x; qf[i][0][2 + hh] = x.y;
+      qf[i][1][hh] = x.z; qf[i][1][2 + hh] = x.w;
+      qf[i][2][hh] = y.x; qf[i][2][2 + hh] = y.y;
+      qf[i][3][hh] = y.z; qf[i][3][2 + hh] = y.w;
+    }
+  }
+  // (0) Every CTA of the cluster has started and has read its q out of the place where partials arrive: waited for before
+  // the first remote store.
+  ptx::cluster_arrive();
 
   // ---- what token (b, t) sees, and this CTA's entries of its list: raw window rows, then the selected rows
   const int64_t pos_b = p.pos0_dev ? p.pos0_dev[b] : p.pos0;
@@ -248,7 +273,6 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
     n_raw = last >= first ? (int)(last - first + 1) : 0;
   }
   const int e_lo = split * R;
-  __syncthreads();   // the list's end is initialised
   // The list is all that the selection right before this launch writes: it may still have been running so far.
   if (p.after_select) ptx::grid_dependency_wait();
   ptx::grid_launch_dependents();
@@ -256,16 +280,23 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
   {
     // this CTA's rows; whether the list ends before them is known only after the scan, but a row inside the visible range
     // may be looked at either way
-    uint32_t ref = 0xFFFFFFFFu;
+    const uint8_t* row = nullptr;
     float rs = 1.f;
     if (tid < R) {
       const int e = e_lo + tid;
+      int64_t r = -1;
+      bool raw = false;
       if (e < n_raw) {
-        const int64_t phys = ((int64_t)p.raw_start + (first + e - first_raw_pos)) % p.raw_cap;
-        ref = (uint32_t)((int64_t)b * p.raw_cap + phys) | 0x80000000u;
+        r = (int64_t)b * p.raw_cap + ((int64_t)p.raw_start + (first + e - first_raw_pos)) % p.raw_cap;
+        raw = true;
       } else if (e - n_raw < p.k) {
         const int32_t id = ids[e - n_raw];
-        if (id >= 0 && (int64_t)id < visible) ref = (uint32_t)(cbase + id);
+        if (id >= 0 && (int64_t)id < visible) r = cbase + id;
+      }
+      if (r >= 0) {
+        row = reinterpret_cast<const uint8_t*>(raw ? p.raw_kv : p.comp_kv) + r * (NB * 64 * EB);
+        // (a zero scale, i.e. an all-zero row, still counts in the denominator: it is taken as fp16's smallest number)
+        if (I8) rs = fmaxf(__half2float(raw ? p.raw_scales[r] : p.comp_scales[r]), 5.9604645e-8f);
       }
     }
     int mine = p.k;   // first list entry that ends the walk
@@ -278,14 +309,13 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
         if ((int64_t)v[u] >= visible && j0 + u * kFewThreads < mine) mine = j0 + u * kFewThreads;
     }
     if (mine < p.k) atomicMin(keff_s, mine);
-    if (I8 && ref != 0xFFFFFFFFu) {
-      // (a zero scale, i.e. an all-zero row, still counts in the denominator: it is taken as fp16's smallest number)
-      const __half* sc = (ref >> 31) ? p.raw_scales : p.comp_scales;
-      rs = fmaxf(__half2float(sc[ref & 0x7FFFFFFFu]), 5.9604645e-8f);
-    }
     if (tid < R) {
-      ref_s[tid] = ref;
-      scale_s[tid] = rs;
+      row_s[tid] = row;
+      if constexpr (I8) {
+        scale_s[tid] = rs;
+        lscale_s[tid] = log2f(rs);
+        iscale_s[tid] = __frcp_rn(rs);
+      }
     }
   }
   __syncthreads();
@@ -294,17 +324,23 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
   // ---- every warp fetches its own rows: row tile i holds rows 64 i + 8 warp .. + 7
   const int tiles = R >> 6;
   const uint32_t row0 = ptx::smem_u32(smem);
-  auto row_ok = [&](int r) { return ref_s[r] != 0xFFFFFFFFu && e_lo + r < e_end; };
+  const int live = e_end - e_lo;   // entries before the list's end
+  auto row_ok = [&](int r) { return row_s[r] != nullptr && r < live; };
   for (int i = 0; i < tiles; ++i) {
+    int rr = lane / kChunks, ck = lane % kChunks;   // (a row is 32 to 72 pieces)
 #pragma unroll
     for (int c0 = 0; c0 < 8 * kChunks; c0 += 32) {
-      const int c = c0 + lane, rr = c / kChunks, ck = c - rr * kChunks;
       const int r = i * 64 + warp * 8 + rr;
       const uint32_t dst = row0 + (uint32_t)(r * L.row_pitch + ck * 16);
-      if (row_ok(r)) {
-        const uint32_t ref = ref_s[r];
-        const uint8_t* table = reinterpret_cast<const uint8_t*>((ref >> 31) ? p.raw_kv : p.comp_kv);
-        cp_async16(dst, table + (int64_t)(ref & 0x7FFFFFFFu) * (NB * 64 * EB) + ck * 16);
+      const uint8_t* row = r < live ? row_s[r] : nullptr;
+      const int at = ck * 16;
+      ck += 32;
+      if (ck >= kChunks) {
+        ck -= kChunks;
+        ++rr;
+      }
+      if (row) {
+        cp_async16(dst, row + at);
       } else {
         asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0u) : "memory");   // zeros: 0 weight x 0
       }
@@ -352,8 +388,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
       const int r = rt + 2 * t4 + (e & 1), h = g + 8 * (e >> 1);
       float x = (acc[0][e] + acc[1][e]) + (acc[2][e] + acc[3][e]);
       if constexpr (I8) {
-        const float rs = scale_s[r];
-        x = fmaf(x, scale_log2 * q_mul[e >> 1] * rs, log2f(rs));
+        x = fmaf(x, scale_log2 * q_mul[e >> 1] * scale_s[r], lscale_s[r]);
       } else {
         x *= scale_log2;
       }
@@ -391,8 +426,9 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
       if constexpr (BF16) back = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
       else back = __half22float2(*reinterpret_cast<const __half2*>(&w));
       if constexpr (I8) {
-        l = fmaf(back.x, __frcp_rn(scale_s[i * 64 + 2 * lane]), l);
-        l = fmaf(back.y, __frcp_rn(scale_s[i * 64 + 2 * lane + 1]), l);
+        const float2 inv = *reinterpret_cast<const float2*>(iscale_s + i * 64 + 2 * lane);
+        l = fmaf(back.x, inv.x, l);
+        l = fmaf(back.y, inv.y, l);
       } else {
         l += back.x + back.y;
       }
@@ -466,26 +502,24 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
   ptx::cluster_wait();
 
   // ---- weights: exp2(m - m*) over the denominator of the whole token, the sink joining once
-  if (tid < kFewHeads) {
-    const int h = h0 + tid;
+  {   // half a warp per head, a lane per split; the sums over the splits are shuffles, in the same order on every run
+    const int hl = 2 * warp + (lane >> 4), r = lane & 15, h = h0 + hl;
     const bool partial = p.partial_ml != nullptr;   // un-normalised output and (m, l): the sink joins in the caller's merge
     const float sink2 = (p.sinks && h < p.H && !partial) ? p.sinks[h] * 1.4426950408889634f : -INFINITY;
-    float m2 = sink2;
-    for (int r = 0; r < C; ++r) m2 = fmaxf(m2, ml_s[r * kFewHeads + tid].x);
-    float den = 0.f;
-    if (m2 > -INFINITY) {
-      for (int r = 0; r < C; ++r) {
-        const float2 v = ml_s[r * kFewHeads + tid];
-        const float w = v.x == -INFINITY ? 0.f : exp2f(v.x - m2);
-        den = fmaf(v.y, w, den);
-        fac_s[r * kFewHeads + tid] = w;
-      }
-      den += sink2 == -INFINITY ? 0.f : exp2f(sink2 - m2);
-    }
-    if (partial && split == 0 && h < p.H)
+    const float2 v = r < C ? ml_s[r * kFewHeads + hl] : make_float2(-INFINITY, 0.f);
+    float m2 = v.x;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) m2 = fmaxf(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+    m2 = fmaxf(m2, sink2);
+    const float w = v.x == -INFINITY ? 0.f : exp2f(v.x - m2);
+    float den = v.y * w;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+    den += sink2 == -INFINITY ? 0.f : exp2f(sink2 - m2);
+    if (partial && split == 0 && r == 0 && h < p.H)
       *reinterpret_cast<float2*>(p.partial_ml + ((int64_t)bt * p.H + h) * 2) = make_float2(m2 * 0.6931471805599453f, den);
     const float inv = partial ? 1.f : den > 0.f ? 1.f / den : 0.f;
-    for (int r = 0; r < C; ++r) fac_s[r * kFewHeads + tid] = m2 > -INFINITY ? fac_s[r * kFewHeads + tid] * inv : 0.f;
+    if (r < C) fac_s[r * kFewHeads + hl] = w * inv;
   }
   __syncthreads();
   const int64_t ob = (int64_t)b * p.o_sb + (int64_t)t * p.o_st;
@@ -591,10 +625,10 @@ int launch_sparse_few(const SparseParams& p, int kv_dtype, int q_dtype, int out_
   const int64_t clusters = (int64_t)p.B * p.T * fp.groups;
   // The fewest rows per CTA whose clusters are all resident at once; a second wave of them would take as long as the kernel
   // for many tokens.  us per launch, 64 heads of 576 features, that kernel -> this one (rows per CTA):
-  //   bf16  k = 512: 1 token 18.4 -> 9.8 (64), 4 18.6 -> 11.9 (128), 8 18.6 -> 12.2, from 9 on the other's;
-  //         k = 2,048: 1 token 21.6 -> 12.9 (128), from 2 on the other's
-  //   int8  k = 512: 1 token 23.2 -> 12.5 (64), 8 24.1 -> 15.1 (128), 12 24.1 -> 19.8 (256);
-  //         k = 2,048: 1 token 27.2 -> 15.7 (128), 3 27.3 -> 19.5 (256), from 4 on the other's
+  //   bf16  k = 512: 1 token 18.4 -> 8.5 (64), 8 18.6 -> 10.5 (128), from 9 on the other's;
+  //         k = 2,048: 1 token 21.6 -> 10.8 (128), from 2 on the other's
+  //   int8  k = 512: 1 token 23.2 -> 9.4 (64), 8 24.1 -> 11.4 (128), 12 24.1 -> 15.5 (256);
+  //         k = 2,048: 1 token 27.2 -> 11.6 (128), 3 27.3 -> 14.8 (256), from 4 on the other's
   for (int rows = 64; rows <= few_max_rows(eb); rows *= 2) {
     const int64_t splits = ceil_div(entries, rows);
     if (splits < 1 || splits > kFewMaxSplits || clusters * splits > sm_count()) continue;
