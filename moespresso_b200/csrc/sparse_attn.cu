@@ -615,9 +615,11 @@ extern "C" int mxb_sparse_attn(const mxb_sparse_attn_args* a, void* stream) {
   dim3 grid((unsigned)p.nsplit, (unsigned)ceil_div(a->H, kHeadsPerCta), (unsigned)(a->B * a->T));
 
   const int kt = a->kv_dtype, qt = a->q_dtype;
-  if (use_tc(a)) {
+  if (use_tc(a) || kt == MXB_F32) {   // a few tokens
     rc = launch_sparse_few(p, kt, qt, a->out_dtype, st);
     if (rc != MXB_ERR_UNSUPPORTED) return rc;
+  }
+  if (use_tc(a)) {
     rc = launch_sparse_tc(p, kt, qt, a->out_dtype, st);
   } else
 #define MXB_PAIR(QT, KT) \

@@ -127,6 +127,87 @@ __device__ __forceinline__ float few_exp2(float x) {
   return y;
 }
 
+// What token (b, t) sees, and entry e_lo + threadIdx.x of its list (raw window rows, then the selected rows) for the threads
+// below R: the address of the row or null, int8 rows also the scale.  *keff becomes the number of selected entries before
+// the walk ends (p.k on entry); returns the number of raw rows.  The list is all that the selection right before the launch
+// writes: it is waited for here.
+template <int ROW_BYTES, bool I8>
+__device__ __forceinline__ int few_list(const SparseParams& p, int b, int t, const int32_t* ids, int e_lo, int R, int* keff,
+                                        const uint8_t*& row, float& rs) {
+  const int tid = threadIdx.x;
+  const int64_t pos_b = p.pos0_dev ? p.pos0_dev[b] : p.pos0;
+  const int64_t qpos = pos_b + t, last_pos = pos_b + p.T - 1;
+  const int64_t count = p.comp_row_count ? (int64_t)p.comp_row_count[b] : p.n_comp;
+  const int64_t cbase = p.comp_row_start ? p.comp_row_start[b] : (int64_t)b * p.n_comp;
+  int64_t visible = count;
+  if (p.ratio > 0) {
+    visible = (qpos + 1) / p.ratio;
+    if (visible > count) visible = count;
+  }
+  int64_t first_raw_pos = 0, first = 0;
+  int n_raw = 0;
+  if (p.raw_cap > 0) {
+    first_raw_pos = last_pos + 1 - p.raw_cap;
+    const int64_t window_first = (p.window != 0 && qpos + 1 > p.window) ? qpos + 1 - p.window : 0;
+    first = first_raw_pos > window_first ? first_raw_pos : window_first;
+    if (first < 0) first = 0;
+    const int64_t last = qpos < last_pos ? qpos : last_pos;
+    n_raw = last >= first ? (int)(last - first + 1) : 0;
+  }
+  if (p.after_select) ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
+  // whether the list ends before this CTA's rows is known only after the scan, but a row inside the visible range may be
+  // looked at either way
+  row = nullptr;
+  rs = 1.f;
+  if (tid < R) {
+    const int e = e_lo + tid;
+    int64_t r = -1;
+    bool raw = false;
+    if (e < n_raw) {
+      r = (int64_t)b * p.raw_cap + ((int64_t)p.raw_start + (first + e - first_raw_pos)) % p.raw_cap;
+      raw = true;
+    } else if (e - n_raw < p.k) {
+      const int32_t id = ids[e - n_raw];
+      if (id >= 0 && (int64_t)id < visible) r = cbase + id;
+    }
+    if (r >= 0) {
+      row = reinterpret_cast<const uint8_t*>(raw ? p.raw_kv : p.comp_kv) + r * ROW_BYTES;
+      // (a zero scale, i.e. an all-zero row, still counts in the denominator: it is taken as fp16's smallest number)
+      if (I8) rs = fmaxf(__half2float(raw ? p.raw_scales[r] : p.comp_scales[r]), 5.9604645e-8f);
+    }
+  }
+  int mine = p.k;   // first list entry that ends the walk
+  for (int j0 = tid; j0 < p.k; j0 += 8 * kFewThreads) {   // eight ids in flight
+    int32_t v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = j0 + u * kFewThreads < p.k ? ids[j0 + u * kFewThreads] : -1;
+#pragma unroll
+    for (int u = 7; u >= 0; --u)
+      if ((int64_t)v[u] >= visible && j0 + u * kFewThreads < mine) mine = j0 + u * kFewThreads;
+  }
+  if (mine < p.k) atomicMin(keff, mine);
+  return n_raw;
+}
+
+// One split's share of its head, lane r of a half warp = split r: exp(m - m*) over the denominator of the whole token, the
+// sink joining once, and m*, the denominator themselves (partial output: no sink, not divided).  LOG2: m and sink in log2
+// units; otherwise in natural ones, which float32 tables keep (a product with log2(e) would round a large m).
+template <bool LOG2>
+__device__ __forceinline__ float few_weight(float2 ml, float sink2, bool partial, float& m2, float& den) {
+  m2 = ml.x;
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) m2 = fmaxf(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+  m2 = fmaxf(m2, sink2);
+  auto e = [](float x) { return LOG2 ? exp2f(x) : expf(x); };
+  const float w = ml.x == -INFINITY ? 0.f : e(ml.x - m2);
+  den = ml.y * w;
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);   // the same order on every run
+  den += sink2 == -INFINITY ? 0.f : e(sink2 - m2);
+  return w * (partial ? 1.f : den > 0.f ? 1.f / den : 0.f);
+}
+
 // NB: 64-feature blocks of a row (Dqk / 64).
 template <int KVT, int NB>
 __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const __grid_constant__ FewParams fp) {
@@ -252,63 +333,13 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
   // the first remote store.
   ptx::cluster_arrive();
 
-  // ---- what token (b, t) sees, and this CTA's entries of its list: raw window rows, then the selected rows
-  const int64_t pos_b = p.pos0_dev ? p.pos0_dev[b] : p.pos0;
-  const int64_t qpos = pos_b + t, last_pos = pos_b + p.T - 1;
-  const int64_t count = p.comp_row_count ? (int64_t)p.comp_row_count[b] : p.n_comp;
-  const int64_t cbase = p.comp_row_start ? p.comp_row_start[b] : (int64_t)b * p.n_comp;
-  int64_t visible = count;
-  if (p.ratio > 0) {
-    visible = (qpos + 1) / p.ratio;
-    if (visible > count) visible = count;
-  }
-  int64_t first_raw_pos = 0, first = 0;
-  int n_raw = 0;
-  if (p.raw_cap > 0) {
-    first_raw_pos = last_pos + 1 - p.raw_cap;
-    const int64_t window_first = (p.window != 0 && qpos + 1 > p.window) ? qpos + 1 - p.window : 0;
-    first = first_raw_pos > window_first ? first_raw_pos : window_first;
-    if (first < 0) first = 0;
-    const int64_t last = qpos < last_pos ? qpos : last_pos;
-    n_raw = last >= first ? (int)(last - first + 1) : 0;
-  }
   const int e_lo = split * R;
-  // The list is all that the selection right before this launch writes: it may still have been running so far.
-  if (p.after_select) ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();
   const int32_t* ids = p.topk + (int64_t)bt * p.k;
+  int n_raw;
   {
-    // this CTA's rows; whether the list ends before them is known only after the scan, but a row inside the visible range
-    // may be looked at either way
-    const uint8_t* row = nullptr;
-    float rs = 1.f;
-    if (tid < R) {
-      const int e = e_lo + tid;
-      int64_t r = -1;
-      bool raw = false;
-      if (e < n_raw) {
-        r = (int64_t)b * p.raw_cap + ((int64_t)p.raw_start + (first + e - first_raw_pos)) % p.raw_cap;
-        raw = true;
-      } else if (e - n_raw < p.k) {
-        const int32_t id = ids[e - n_raw];
-        if (id >= 0 && (int64_t)id < visible) r = cbase + id;
-      }
-      if (r >= 0) {
-        row = reinterpret_cast<const uint8_t*>(raw ? p.raw_kv : p.comp_kv) + r * (NB * 64 * EB);
-        // (a zero scale, i.e. an all-zero row, still counts in the denominator: it is taken as fp16's smallest number)
-        if (I8) rs = fmaxf(__half2float(raw ? p.raw_scales[r] : p.comp_scales[r]), 5.9604645e-8f);
-      }
-    }
-    int mine = p.k;   // first list entry that ends the walk
-    for (int j0 = tid; j0 < p.k; j0 += 8 * kFewThreads) {   // eight ids in flight
-      int32_t v[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = j0 + u * kFewThreads < p.k ? ids[j0 + u * kFewThreads] : -1;
-#pragma unroll
-      for (int u = 7; u >= 0; --u)
-        if ((int64_t)v[u] >= visible && j0 + u * kFewThreads < mine) mine = j0 + u * kFewThreads;
-    }
-    if (mine < p.k) atomicMin(keff_s, mine);
+    const uint8_t* row;
+    float rs;
+    n_raw = few_list<NB * 64 * EB, I8>(p, b, t, ids, e_lo, R, keff_s, row, rs);
     if (tid < R) {
       row_s[tid] = row;
       if constexpr (I8) {
@@ -502,24 +533,16 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
   ptx::cluster_wait();
 
   // ---- weights: exp2(m - m*) over the denominator of the whole token, the sink joining once
-  {   // half a warp per head, a lane per split; the sums over the splits are shuffles, in the same order on every run
+  {   // half a warp per head, a lane per split
     const int hl = 2 * warp + (lane >> 4), r = lane & 15, h = h0 + hl;
     const bool partial = p.partial_ml != nullptr;   // un-normalised output and (m, l): the sink joins in the caller's merge
     const float sink2 = (p.sinks && h < p.H && !partial) ? p.sinks[h] * 1.4426950408889634f : -INFINITY;
     const float2 v = r < C ? ml_s[r * kFewHeads + hl] : make_float2(-INFINITY, 0.f);
-    float m2 = v.x;
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) m2 = fmaxf(m2, __shfl_xor_sync(0xffffffffu, m2, o));
-    m2 = fmaxf(m2, sink2);
-    const float w = v.x == -INFINITY ? 0.f : exp2f(v.x - m2);
-    float den = v.y * w;
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
-    den += sink2 == -INFINITY ? 0.f : exp2f(sink2 - m2);
+    float m2, den;
+    const float f = few_weight<true>(v, sink2, partial, m2, den);
     if (partial && split == 0 && r == 0 && h < p.H)
       *reinterpret_cast<float2*>(p.partial_ml + ((int64_t)bt * p.H + h) * 2) = make_float2(m2 * 0.6931471805599453f, den);
-    const float inv = partial ? 1.f : den > 0.f ? 1.f / den : 0.f;
-    if (r < C) fac_s[r * kFewHeads + hl] = w * inv;
+    if (r < C) fac_s[r * kFewHeads + hl] = f;
   }
   __syncthreads();
   const int64_t ob = (int64_t)b * p.o_sb + (int64_t)t * p.o_st;
@@ -551,16 +574,220 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
   }
 }
 
+// float32 tables and queries: the same cut with HG heads and up to 64 rows per CTA, on the FMA pipe.  Bound by latency and by
+// shared-memory reads (a row once for HG heads).  The kernel of sparse_attn.cu walks 32-row tiles with eight heads a CTA, a
+// chain of staging, dots, softmax and values per tile, and leaves partials to a merge kernel: k = 512, 64 heads of 576, 20.6
+// and 5 us, a float32 decode step over 4,096 rows 33.1 us; with this kernel 19.6.
+template <int HG>
+struct FewF32Layout {
+  static constexpr int kRows = 64, kHP = (HG + 3) / 4 * 4;
+  int pitch;        // floats of a staged row: + 16 bytes, so that eight rows cover all banks
+  int q_off, part_off, p_off, row_off, recv_off, ml_off, fac_off, misc_off, total;
+  __host__ __device__ FewF32Layout(int Dqk, int splits) {
+    pitch = Dqk + 4;
+    q_off = kRows * pitch * 4;
+    part_off = q_off + HG * Dqk * 4;
+    p_off = part_off + 4 * HG * kRows * 4;
+    row_off = p_off + kRows * kHP * 4;
+    recv_off = row_off + kRows * 8;
+    ml_off = recv_off + (kFewDv / kFewBlk + splits - 1) / splits * splits * HG * kFewBlk * 4;
+    fac_off = ml_off + splits * HG * 8;
+    misc_off = (fac_off + splits * HG * 4 + 15) / 16 * 16;
+    total = misc_off + 16;
+  }
+};
+
+template <int NB, int HG>
+__global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_f32_kernel(const __grid_constant__ FewParams fp) {
+  using Lay = FewF32Layout<HG>;
+  constexpr int R = Lay::kRows, HP = Lay::kHP, D = NB * 64;
+  constexpr int kChunks = D / 4;   // 16-byte pieces of a row
+  const SparseParams& p = fp.s;
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int C = p.nsplit;
+  const Lay L(D, C);
+  const float* rows_s = reinterpret_cast<const float*>(smem);
+  float* q_s = reinterpret_cast<float*>(smem + L.q_off);         // [HG][D]
+  float* part_s = reinterpret_cast<float*>(smem + L.part_off);   // [4 feature quarters][HG][R]
+  float* p_s = reinterpret_cast<float*>(smem + L.p_off);         // [R][HP]
+  const uint8_t** row_s = reinterpret_cast<const uint8_t**>(smem + L.row_off);
+  const float* recv = reinterpret_cast<const float*>(smem + L.recv_off);   // [slot][split][HG][32]
+  float2* ml_s = reinterpret_cast<float2*>(smem + L.ml_off);     // [split][HG]
+  float* fac_s = reinterpret_cast<float*>(smem + L.fac_off);     // [split][HG]
+  int* keff_s = reinterpret_cast<int*>(smem + L.misc_off);
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int split = (int)(blockIdx.x % (unsigned)C);
+  const int unit = (int)(blockIdx.x / (unsigned)C);
+  const int bt = unit / fp.groups, h0 = (unit - bt * fp.groups) * HG;
+  const int b = bt / p.T, t = bt - b * p.T;
+  if (!p.after_select) ptx::grid_dependency_wait();   // behind a selection q and all else but the list are complete
+  const float* q_in = reinterpret_cast<const float*>(ptx::behind_wait(p.q));
+  ptx::cluster_arrive();   // (0) every CTA of the cluster has started: waited for before the first remote store
+  if (tid == 0) *keff_s = p.k;
+  {
+    const int64_t qbase = (int64_t)b * p.q_sb + (int64_t)t * p.q_st;
+#pragma unroll 4
+    for (int i = tid; i < HG * D; i += kFewThreads) {
+      const int hl = i / D, h = h0 + hl;
+      q_s[i] = h < p.H ? q_in[qbase + (int64_t)h * p.q_sh + (i - hl * D)] : 0.f;
+    }
+  }
+  __syncthreads();   // the list's end is initialised
+  const int e_lo = split * R;
+  const uint8_t* my_row;
+  float unused;
+  const int n_raw = few_list<D * 4, false>(p, b, t, p.topk + (int64_t)bt * p.k, e_lo, R, keff_s, my_row, unused);
+  if (tid < R) row_s[tid] = my_row;
+  __syncthreads();
+  const int live = n_raw + *keff_s - e_lo;   // entries before the list's end
+
+  // ---- a warp fetches eight rows
+  {
+    const uint32_t row0 = ptx::smem_u32(smem);
+    int rr = 0, ck = lane;
+#pragma unroll 12
+    for (int c0 = 0; c0 < 8 * kChunks; c0 += 32) {
+      const int r = warp * 8 + rr;
+      const uint32_t dst = row0 + (uint32_t)(r * L.pitch * 4 + ck * 16);
+      const uint8_t* row = r < live ? row_s[r] : nullptr;
+      const int at = ck * 16;
+      ck += 32;
+      if (ck >= kChunks) {
+        ck -= kChunks;
+        ++rr;
+      }
+      if (row) cp_async16(dst, row + at);
+      else asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0u) : "memory");
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+  }
+  __syncthreads();
+
+  // ---- S: thread = (row, quarter of the features), all heads
+  {
+    const int r = (warp & 1) * 32 + lane, quarter = warp >> 1;
+    constexpr int N4 = D / 16;   // float4 of a quarter
+    const float4* kr = reinterpret_cast<const float4*>(rows_s + r * L.pitch) + quarter * N4;
+    const float4* qr = reinterpret_cast<const float4*>(q_s) + quarter * N4;
+    float acc[HG];
+#pragma unroll
+    for (int h = 0; h < HG; ++h) acc[h] = 0.f;
+#pragma unroll 4
+    for (int c = 0; c < N4; ++c) {
+      const float4 k4 = kr[c];
+#pragma unroll
+      for (int h = 0; h < HG; ++h) {
+        const float4 x = qr[h * (D / 4) + c];
+        acc[h] = fmaf(x.x, k4.x, acc[h]);
+        acc[h] = fmaf(x.y, k4.y, acc[h]);
+        acc[h] = fmaf(x.z, k4.z, acc[h]);
+        acc[h] = fmaf(x.w, k4.w, acc[h]);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < HG; ++h) part_s[(quarter * HG + h) * R + r] = acc[h];
+  }
+  __syncthreads();
+
+  // ---- softmax: a warp takes heads warp, warp + 8; (m, l) go to every CTA of the cluster
+  ptx::cluster_wait();   // (0)
+  for (int h = warp; h < HG; h += 8) {
+    float x[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = i * 32 + lane;
+      const float dot = (part_s[h * R + r] + part_s[(HG + h) * R + r]) + (part_s[(2 * HG + h) * R + r] + part_s[(3 * HG + h) * R + r]);
+      x[i] = row_s[r] != nullptr && r < live ? dot * p.scale : -INFINITY;
+    }
+    const float m = warp_max(fmaxf(x[0], x[1]));
+    float l = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float w = x[i] == -INFINITY ? 0.f : expf(x[i] - m);
+      p_s[(i * 32 + lane) * HP + h] = w;
+      l += w;
+    }
+    l = warp_sum(l);
+    if (lane < C) {
+      const uint32_t dst = ptx::cluster_map(ptx::smem_u32(ml_s + split * HG + h), (uint32_t)lane);
+      ptx::st_cluster_f32(dst, m);
+      ptx::st_cluster_f32(dst + 4, l);
+    }
+  }
+  __syncthreads();
+
+  // ---- O: thread = two features, all heads
+  float2 o[HG];
+#pragma unroll
+  for (int h = 0; h < HG; ++h) o[h] = make_float2(0.f, 0.f);
+  const int n_rows = min(R, max(live, 0));   // (the rows behind them weigh nothing)
+#pragma unroll 4
+  for (int r = 0; r < n_rows; ++r) {
+    const float2 v = *reinterpret_cast<const float2*>(rows_s + r * L.pitch + 2 * tid);
+    float w[HP];
+#pragma unroll
+    for (int i = 0; i < HP; i += 4) *reinterpret_cast<float4*>(&w[i]) = *reinterpret_cast<const float4*>(p_s + r * HP + i);
+#pragma unroll
+    for (int h = 0; h < HG; ++h) {
+      o[h].x = fmaf(w[h], v.x, o[h].x);
+      o[h].y = fmaf(w[h], v.y, o[h].y);
+    }
+  }
+  {
+    const int blk = tid >> 4;   // block of 32 features, of CTA blk % C
+    const uint32_t dst = ptx::cluster_map(
+        ptx::smem_u32(recv + (size_t)((blk / C) * C + split) * HG * kFewBlk + ((2 * tid) & (kFewBlk - 1))), (uint32_t)(blk % C));
+#pragma unroll
+    for (int h = 0; h < HG; ++h)
+      asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dst + (uint32_t)(h * kFewBlk * 4)), "f"(o[h].x), "f"(o[h].y)
+                   : "memory");
+  }
+  __syncwarp();
+  ptx::cluster_arrive();   // (1) everything has arrived; nothing remote is touched after this
+  ptx::cluster_wait();
+  for (int h1 = 2 * warp; h1 < HG; h1 += 16) {   // (the same trips for both halves of a warp)
+    const int hl = h1 + (lane >> 4), r = lane & 15, h = h0 + hl;
+    const bool partial = p.partial_ml != nullptr, on = hl < HG;
+    const float sink = (p.sinks && on && h < p.H && !partial) ? p.sinks[h] : -INFINITY;
+    const float2 v = on && r < C ? ml_s[r * HG + hl] : make_float2(-INFINITY, 0.f);
+    float m2, den;
+    const float f = few_weight<false>(v, sink, partial, m2, den);
+    if (partial && on && split == 0 && r == 0 && h < p.H)
+      *reinterpret_cast<float2*>(p.partial_ml + ((int64_t)bt * p.H + h) * 2) = make_float2(m2, den);
+    if (on && r < C) fac_s[r * HG + hl] = f;
+  }
+  __syncthreads();
+  const int64_t ob = (int64_t)b * p.o_sb + (int64_t)t * p.o_st;
+  for (int x = tid;; x += kFewThreads) {   // item: (slot, head, feature of the block)
+    const int slot = x / (HG * kFewBlk), i = x - slot * (HG * kFewBlk), blk = slot * C + split;
+    if (blk >= kFewDv / kFewBlk) break;
+    const int hl = i / kFewBlk, h = h0 + hl;
+    const float* src = recv + (size_t)slot * C * HG * kFewBlk + i;
+    float acc = 0.f;
+#pragma unroll 4
+    for (int r = 0; r < C; ++r) acc = fmaf(src[(size_t)r * HG * kFewBlk], fac_s[r * HG + hl], acc);
+    if (h < p.H) {
+      const int64_t at = ob + (int64_t)h * p.o_sh + blk * kFewBlk + (i & (kFewBlk - 1));
+      if (fp.out_dtype == MXB_F32) store_elem<MXB_F32>(p.out, at, acc);
+      else if (fp.out_dtype == MXB_F16) store_elem<MXB_F16>(p.out, at, acc);
+      else store_elem<MXB_BF16>(p.out, at, acc);
+    }
+  }
+}
+
 // Which calls come here: splits left to the library, 512 values of 512 or 576 features.  int8 rows need a
 // 16-bit q (a float32 one would be rounded to 11 bits; the other kernel keeps 15).
 static bool sparse_few_eligible(const SparseParams& p, int kv_dtype, int q_dtype) {
+  if (p.H < 1) return false;
   return p.may_split && p.Dv == kFewDv && (p.Dqk == 512 || p.Dqk == 576) && p.H <= 64 &&
          !(kv_dtype == MXB_I8 && q_dtype == MXB_F32);
 }
 
-template <int KVT, int NB>
-static int launch_few_typed(const FewParams& fp, int smem, int clusters, cudaStream_t st) {
-  auto* kern = sparse_attn_few_kernel<KVT, NB>;
+// MXB_ERR_UNSUPPORTED: the clusters are not all resident at once, nothing was launched.  `cached`: how many are, 0 = not asked
+// yet (one per kernel, device, shared memory and cluster size).
+static int launch_few_kernel(void (*kern)(FewParams), const FewParams& fp, int smem, int clusters, int* cached, cudaStream_t st) {
   const int C = fp.s.nsplit;
   MXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
   if (C > 8) MXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -578,10 +805,6 @@ static int launch_few_typed(const FewParams& fp, int smem, int clusters, cudaStr
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  static int resident_cache[16][3][kFewMaxSplits + 1];   // per device, rows (64, 128, 256) and cluster size; 0 = not asked yet
-  int dev = 0;
-  MXB_CUDA_OK(cudaGetDevice(&dev));
-  int* cached = dev >= 0 && dev < 16 ? &resident_cache[dev][fp.rows >> 7][C] : nullptr;
   int resident = cached ? *cached : 0;
   if (resident == 0) {
     if (cudaOccupancyMaxActiveClusters(&resident, kern, &cfg) != cudaSuccess) {
@@ -596,6 +819,28 @@ static int launch_few_typed(const FewParams& fp, int smem, int clusters, cudaStr
   MXB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, fp));
   note_launch();
   return MXB_OK;
+}
+
+template <int KVT, int NB>
+static int launch_few_typed(const FewParams& fp, int smem, int clusters, cudaStream_t st) {
+  static int resident[16][3][kFewMaxSplits + 1];   // rows 64, 128, 256
+  int dev = 0;
+  MXB_CUDA_OK(cudaGetDevice(&dev));
+  int* cached = dev >= 0 && dev < 16 ? &resident[dev][fp.rows >> 7][fp.s.nsplit] : nullptr;
+  return launch_few_kernel(sparse_attn_few_kernel<KVT, NB>, fp, smem, clusters, cached, st);
+}
+
+template <int NB, int HG>
+static int launch_few_f32(FewParams fp, cudaStream_t st) {
+  static int resident[16][kFewMaxSplits + 1];
+  int dev = 0;
+  MXB_CUDA_OK(cudaGetDevice(&dev));
+  int* cached = dev >= 0 && dev < 16 ? &resident[dev][fp.s.nsplit] : nullptr;
+  fp.groups = (fp.s.H + HG - 1) / HG;
+  const int64_t clusters = (int64_t)fp.s.B * fp.s.T * fp.groups;
+  const int smem = FewF32Layout<HG>(NB * 64, fp.s.nsplit).total;
+  if (clusters * fp.s.nsplit > sm_count() || smem > 227 * 1024) return MXB_ERR_UNSUPPORTED;
+  return launch_few_kernel(sparse_attn_few_f32_kernel<NB, HG>, fp, smem, (int)clusters, cached, st);
 }
 
 static int launch_few(const FewParams& fp, int kv_dtype, int smem, int clusters, cudaStream_t st) {
@@ -622,6 +867,18 @@ int launch_sparse_few(const SparseParams& p, int kv_dtype, int q_dtype, int out_
   fp.groups = (p.H + kFewHeads - 1) / kFewHeads;
   fp.out_dtype = out_dtype;
   fp.q_dtype = q_dtype;
+  if (kv_dtype == MXB_F32) {
+    // The fewest heads per CTA whose clusters are all resident at once (16 of eight CTAs are not, 13 are; 7 of sixteen).
+    if (q_dtype != MXB_F32 || entries < 1 || entries > 64 * kFewMaxSplits) return MXB_ERR_UNSUPPORTED;
+    fp.rows = 64;
+    fp.s.nsplit = (int)ceil_div(entries, (int64_t)64);
+    int rc = MXB_ERR_UNSUPPORTED;
+#define MXB_FEW32(HG) \
+  if (rc == MXB_ERR_UNSUPPORTED) rc = p.Dqk == 576 ? launch_few_f32<9, HG>(fp, st) : launch_few_f32<8, HG>(fp, st);
+    MXB_FEW32(4) MXB_FEW32(5) MXB_FEW32(10)
+#undef MXB_FEW32
+    return rc;
+  }
   const int64_t clusters = (int64_t)p.B * p.T * fp.groups;
   // The fewest rows per CTA whose clusters are all resident at once; a second wave of them would take as long as the kernel
   // for many tokens.  us per launch, 64 heads of 576 features, that kernel -> this one (rows per CTA):

@@ -18,7 +18,8 @@ def _tables(rng, kind, R, raw_cap, D):
         (comp, cs), (raw, rs) = mk(R), mk(max(raw_cap, 1))
         return dict(comp=comp, raw=raw, cs=cs, rs=rs, ct=dev(comp), rt=dev(raw), cst=dev(cs), rst=dev(rs),
                     okw=dict(kv_scales=cs, raw_scales=rs))
-    rnd, kt = (f16_round, torch.float16) if kind == "f16" else (bf16_round, torch.bfloat16)
+    rnd, kt = {"f16": (f16_round, torch.float16), "bf16": (bf16_round, torch.bfloat16),
+               "f32": (lambda x: x.astype(np.float32), torch.float32)}[kind]
     comp, raw = rnd(rng.standard_normal((R, D))), rnd(rng.standard_normal((max(raw_cap, 1), D)))
     return dict(comp=comp, raw=raw, ct=dev(comp, kt), rt=dev(raw, kt), cst=None, rst=None, okw={})
 
@@ -147,3 +148,39 @@ def test_partials_of_list_halves_merge_to_the_whole(kind, k):
         out = sum(x[0] * y[:, None] for x, y in zip(parts, w)) / sum(x[2] * y for x, y in zip(parts, w))[:, None]
         # the weights of either side are rounded to 16 bits (2^-9, fp16 2^-12) relative to another maximum
         assert float((out - whole).abs().max()) <= (2 ** -8 if kind == "bf16" else 2 ** -11) * float(np.abs(whole.cpu().numpy()).max() * 4)
+
+
+@pytest.mark.parametrize("D,H,k,window,raw_cap,B", [
+    (576, 64, 1, 0, 0, 1),
+    (512, 3, 65, 0, 0, 1),        # three of a group's four heads, a second split of one row
+    (576, 64, 512, 0, 0, 1),      # eight splits: more than four heads per CTA, the last group not full
+    (576, 40, 1024, 0, 0, 1),     # sixteen splits
+    (512, 64, 400, 101, 128, 1),  # a ragged window before the list
+    (576, 16, 256, 0, 0, 7),      # a batch
+])
+def test_float32_tables(D, H, k, window, raw_cap, B):
+    """1e-4 as for the other float32 kernel, which exact_fp32 with a fixed number of splits still takes."""
+    need_gpu()
+    rng = np.random.default_rng(k * 7 + D + H)
+    R = max(2 * k, 40)
+    t = _tables(rng, "f32", R, raw_cap, D)
+    q = rng.standard_normal((B, H, 1, D)).astype(np.float32)
+    sinks = rng.standard_normal(H).astype(np.float32)
+    ids = np.stack([np.sort(rng.choice(R, size=k, replace=False)) for _ in range(B)]).astype(np.int32)[:, None]
+    if k > 60:
+        ids[:, 0, [0, 5, 59]] = -1
+        ids[:, 0, -2] = R + 7
+    pos0 = 128 + R * 4 - 1
+    kw = dict(pos0=pos0, window=window, ratio=4, raw_kv=t["rt"][None] if raw_cap else None, raw_start=11 if raw_cap else 0,
+              scale=D ** -0.5, d_v=512, comp_row_start=torch.zeros(B, dtype=torch.int64, device="cuda"), n_comp=R, check=True)
+    out = iak.sparse_attention(dev(q), t["ct"], dev(ids), dev(sinks), **kw)
+    other = iak.sparse_attention(dev(q), t["ct"], dev(ids), dev(sinks), n_splits=2, **kw)
+    for b in range(B):
+        ref = ds4.indexed_mixed_attention_decode(q[b, :, 0], t["raw"] if raw_cap else None, t["comp"], ids[b, 0], sinks, pos0=pos0,
+                                                 window=window, ratio=4, raw_start=11 if raw_cap else 0, scale=D ** -0.5, d_v=512)
+        assert max_abs(out[b, :, 0], ref) <= 1e-4 and max_abs(other[b, :, 0], ref) <= 1e-4
+    half = iak.sparse_attention(dev(q), t["ct"], dev(ids), dev(sinks), out_dtype=torch.bfloat16, **kw)
+    assert torch.equal(half, out.to(torch.bfloat16))
+    o, ml = iak.sparse_attention(dev(q), t["ct"], dev(ids), None, partial=True, **kw)
+    plain = iak.sparse_attention(dev(q), t["ct"], dev(ids), None, **kw)
+    assert max_abs(o / ml[:, 0, :, 1][:, :, None, None], plain) <= 1e-5
