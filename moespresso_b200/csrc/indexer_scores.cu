@@ -98,8 +98,8 @@ __global__ void __launch_bounds__(128) indexer_exact_kernel(IndexerParams p) {
 // owns RPL rows, all staged in shared memory.  Every dot product and the head sum (over the rectified dots, parked in
 // shared memory) are formed in the same order as above, so the two kernels give the same bits.  What the kernel above
 // is short of on a decode call is parallelism: a thread walks all heads of its row, 64 x 128 dependent steps.
-// fp32, us before -> after: 64 heads of 128: 2,500 rows 28.0 -> 8.2, 16,384 rows 28.5 -> 17.2, 131,072 rows 110 -> 68;
-// 16 heads of 64: 4,096 rows 6.8 -> 3.9, 131,072 rows 23.1 -> 16.7.
+// fp32, us before -> after: 64 heads of 128: 2,500 rows 28.0 -> 5.3, 16,384 rows 28.5 -> 15.2, 131,072 rows 110 -> 57;
+// 16 heads of 64: 4,096 rows 6.8 -> 2.3, 131,072 rows 23.1 -> 14.3.
 // Shared-memory reads set its pace (per four features RPL row reads, 4 cycles each, and HPW broadcasts for
 // 4 x RPL x HPW multiply-adds a lane), hence four rows per lane once the rows fill the SMs anyway.
 template <int D, int QT, int KT, int HPW, int RPL>
@@ -112,13 +112,41 @@ __global__ void __launch_bounds__(256) indexer_exact_token_kernel(IndexerParams 
   float* d_s = reinterpret_cast<float*>(k_s);      // afterwards: rectified dots [8 HPW][ROWS]
   ptx::grid_chain();
   p.keys = ptx::behind_wait(p.keys);
+  p.q = ptx::behind_wait(p.q);
   const int b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t count = p.row_count ? (int64_t)p.row_count[b] : p.n_rows;
   const int64_t rbase = p.row_start ? p.row_start[b] : (int64_t)b * p.n_rows;
   const int64_t r0 = (int64_t)blockIdx.x * ROWS;
   if (r0 >= count) return;
 
+  // q first, sixteen bytes a load where its layout allows: all of it in flight while the keys are fetched (64 heads of 128
+  // in float32 by single elements were 32 loads a thread, eight at a time: 2,500 rows 7.7 -> 5.3 us,
+  // 131,072 67.7 -> 56.6)
+  constexpr int EPQ = 16 / ElemBytes<QT>::v;
+  if ((reinterpret_cast<uintptr_t>(p.q) & 15) == 0 && p.q_sb % EPQ == 0 && p.q_sh % EPQ == 0) {
+#pragma unroll
+    for (int i = tid; i < 8 * HPW * (D / EPQ); i += 256) {
+      const int h = i / (D / EPQ), c = i % (D / EPQ);
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (h < p.H) {
+        const int64_t at = (int64_t)b * p.q_sb + (int64_t)h * p.q_sh + c * EPQ;
+        v = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(p.q) + at * ElemBytes<QT>::v));
+      }
+      float f[EPQ];
+      unpack16<QT>(v, f);
+#pragma unroll
+      for (int e = 0; e < EPQ / 4; ++e)
+        q_s[h * (D / 4) + c * (EPQ / 4) + e] = make_float4(f[4 * e], f[4 * e + 1], f[4 * e + 2], f[4 * e + 3]);
+    }
+  } else {
+#pragma unroll 8
+    for (int i = tid; i < 8 * HPW * D; i += 256) {
+      const int h = i / D, d = i % D;
+      reinterpret_cast<float*>(q_s)[i] = h < p.H ? load_elem<QT>(p.q, (int64_t)b * p.q_sb + (int64_t)h * p.q_sh + d) : 0.f;
+    }
+  }
   constexpr int EPV = 16 / ElemBytes<KT>::v;
+#pragma unroll
   for (int i = tid; i < ROWS * (D / EPV); i += 256) {
     const int row = i / (D / EPV), c = i % (D / EPV);
     float f[EPV];
@@ -129,11 +157,6 @@ __global__ void __launch_bounds__(256) indexer_exact_token_kernel(IndexerParams 
 #pragma unroll
     for (int e = 0; e < EPV / 4; ++e)
       k_s[row * LD + c * (EPV / 4) + e] = make_float4(f[4 * e], f[4 * e + 1], f[4 * e + 2], f[4 * e + 3]);
-  }
-#pragma unroll 8
-  for (int i = tid; i < 8 * HPW * D; i += 256) {
-    const int h = i / D, d = i % D;
-    reinterpret_cast<float*>(q_s)[i] = h < p.H ? load_elem<QT>(p.q, (int64_t)b * p.q_sb + (int64_t)h * p.q_sh + d) : 0.f;
   }
   if (tid < p.H) w_s[tid] = p.weights[(int64_t)b * p.H + tid];
   __syncthreads();
