@@ -388,7 +388,8 @@ PyObject* q8_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
               (type == at::kFloat || type == at::kHalf || type == at::kBFloat16) && dtype_code(t[1]->scalar_type()) >= 0);
     PLAIN(c);
     const int64_t Hq = q.size(1), P = t[0]->size(2);
-    c.require(q.size(0) == 1 && q.size(2) == 1 && q.size(3) == 256 && Hq > 0 && P > 0);
+    c.require(q.size(0) == 1 && q.size(2) == 1 && q.size(3) == 256 && Hq > 0 && P > 0 &&
+              t[0]->size(3) == 64);   // rows of 256 features: the library is not told the cache's width
     PLAIN(c);
     splits = std::max<int64_t>(1, std::min(splits, P));
     const at::Tensor parts = c.empty({splits * Hq * 258}, at::kFloat), out = c.empty({1, Hq, 1, 256}, type);

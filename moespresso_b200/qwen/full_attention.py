@@ -298,16 +298,25 @@ def sdpa_decode_q8(queries, k_packed, k_scales, k_biases, v_packed, v_scales, v_
     r = native("q8_decode", queries, k_packed, k_scales, k_biases, v_packed, v_scales, v_biases, scale, splits)
     if r is not None:
         return r
-    dev = require_cuda(queries, k_packed, v_packed)
+    tensors = (k_packed, k_scales, k_biases, v_packed, v_scales, v_biases)
+    dev = require_cuda(queries, *tensors)
     B, Hq, T, D = (int(x) for x in queries.shape)
     Hkv, P = int(k_packed.shape[1]), int(k_packed.shape[2])
     if B != 1 or T != 1 or D != FLASH_HEAD_DIM:
         raise ValueError("q8 decode requires one token of batch 1 and head_dim=256")
-    tensors = (k_packed, k_scales, k_biases, v_packed, v_scales, v_biases)
+    # (the kernel takes the width, rows and types on trust: rows of another width would be read past their end)
+    for i, t in enumerate(tensors):
+        if (t.ndim != 4 or t.shape[0] < 1 or t.shape[1] != Hkv or t.shape[2] < P or
+                t.shape[3] != (D // Q8_GROUP if i % 3 else D // 4)):
+            raise ValueError("q8 decode: every head of the cache needs packed rows of 256 features and four scales and biases "
+                             "to each, of keys and values alike")
+        if t.dtype != k_scales.dtype if i % 3 else t.element_size() != 4:
+            raise ValueError("q8 decode: packed words must be 32-bit, scales and biases of one type")
     head_rows = _q8_head_rows(tensors)
     if not head_rows:            # keys and values that differ in what does not matter here
         strides = {int(t.stride(1)) // int(t.shape[3]) for t in tensors}
-        if len(strides) != 1 or any(t.stride(3) != 1 or t.stride(2) != t.shape[3] for t in tensors):
+        if len(strides) != 1 or any(t.stride(3) != 1 or t.stride(2) != t.shape[3] or (Hkv > 1 and t.stride(1) % t.shape[3])
+                                    for t in tensors):
             raise ValueError("q8 decode: cache tensors must be row-contiguous views with one capacity")
         head_rows = strides.pop()
     splits = max(1, min(int(splits), P))

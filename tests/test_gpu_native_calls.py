@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 import torch
 
+from moespresso_b200 import _abi
 from moespresso_b200 import _torchabi as _t
 from moespresso_b200.deepseek_v4.attention import rope_inverse_frequencies
 from moespresso_b200.deepseek_v4.decode_attention_kernel import fused_decode_prep, fused_decode_sdpa
@@ -157,3 +158,11 @@ def test_q8_token(taken):
     with pytest.raises(ValueError):
         c.update_and_fetch(k, v)                                                             # capacity
     assert c.offset == 508
+    # rows of another width than the kernel's 256 features: not the native call's, and refused before any launch
+    del taken[:]
+    narrow = QuantizedKVCache(2, 128, 600)
+    narrow.offset = 500
+    before = _abi.load().mxb_kernel_launches()
+    with pytest.raises(ValueError):
+        sdpa_decode_q8(q, *narrow.state[0], *narrow.state[1], 0.0625)
+    assert taken == [] and _abi.load().mxb_kernel_launches() == before

@@ -121,3 +121,40 @@ def test_native_calls_leave_cpu_tensors_to_python():
     x = torch.zeros(1, 2, 1, 256)
     assert _torchabi.native("q8_decode", x, x, x, x, x, x, x, 0.1, 4) is None
     assert _torchabi.native("decode_step") is None
+
+
+def _narrow(i, n):       # tensor i of the six with rows of n values
+    return lambda six: [t[..., :n].contiguous() if j == i else t for j, t in enumerate(six)]
+
+
+@pytest.mark.parametrize("cache", [
+    lambda six: _past(2, 5, 32, 2), lambda six: _past(2, 5, 128, 8), lambda six: _past(2, 5, 64, 2), lambda six: _past(2, 5, 16, 1),
+    _narrow(0, 32), _narrow(3, 16), _narrow(1, 2), _narrow(2, 1), _narrow(5, 3),
+    lambda six: [*six[:3], *(t[:, :, :4] for t in six[3:])],                         # fewer values than keys
+    lambda six: [*six[:3], *(t[:, :1] for t in six[3:])],                            # values of fewer heads
+    lambda six: [*six[:4], six[4].float(), six[5]],                                  # scales of two types
+    lambda six: [six[0].to(torch.int16), *six[1:]],
+    lambda six: [torch.zeros(1, 2, 5 * 64 + 32, dtype=torch.int32).as_strided((1, 2, 5, 64), (0, 5 * 64 + 32, 64, 1)), *six[1:]],
+    lambda six: [t[:0] for t in six],
+])
+def test_decode_refuses_rows_that_the_kernel_would_misread(monkeypatch, cache):
+    """The decode kernel is told head_dim 256, the rows of a head and one type of scales, and reads by them."""
+    monkeypatch.setattr(fa, "require_cuda", lambda *tensors: torch.device("cpu"))
+    monkeypatch.setattr(fa._t, "launch", lambda *a: pytest.fail("a kernel would have been launched"))
+    with pytest.raises(ValueError):
+        fa.sdpa_decode_q8(torch.zeros(1, 4, 1, 256, dtype=BF), *cache(_past(2, 5, 64, 4)), 1 / 16)
+
+
+@pytest.mark.parametrize("layout,head_rows", [
+    (lambda six: six, 5), (_wide, 50),
+    (lambda six: [*(t[:, :, :3] for t in six[:3]), *six[3:]], 5),                    # values of keys to come
+    (lambda six: [torch.cat([t, t]) for t in six], 5),                               # the first entry of a batch
+])
+def test_decode_takes_the_caches_that_it_can_address(monkeypatch, layout, head_rows):
+    seen = []
+    monkeypatch.setattr(fa, "require_cuda", lambda *tensors: torch.device("cpu"))
+    monkeypatch.setattr(fa._t, "launch", lambda name, fn, a: seen.append(a) or 0)
+    monkeypatch.setattr("moespresso_b200.deepseek_v4.indexed_attention_kernel.require_cuda", lambda *t: torch.device("cpu"))
+    six = layout(_past(2, 5, 64, 4))
+    fa.sdpa_decode_q8(torch.zeros(1, 4, 1, 256, dtype=BF), *six, 1 / 16)
+    assert (seen[0].P, seen[0].head_stride_rows) == (six[0].shape[2], head_rows)
