@@ -192,8 +192,8 @@ def load():
     global _lib
     if _lib is not None:
         return _lib
-    if not os.path.exists(_build.LIB) or (not _build.is_current() and _can_build()):
-        _build.build()
+    if not os.path.exists(_build.LIB) or (not _build.library_is_current() and _can_build()):
+        _build.build_library()
     lib = C.CDLL(_build.LIB)
     for name, (res, args) in EXPORTS.items():
         fn = getattr(lib, name)

@@ -3,6 +3,7 @@ argument structures.  Torch is used for device memory and streams only."""
 from __future__ import annotations
 
 import ctypes as C
+import warnings
 
 import torch
 
@@ -74,19 +75,33 @@ _NATIVE_CALLS = ("mxb_indexer_scores", "mxb_topk_workspace_bytes", "mxb_topk_sel
                  "mxb_sparse_attn", "mxb_fused_decode_prep_workspace_bytes", "mxb_fused_decode_prep",
                  "mxb_fused_decode_sdpa_workspace_bytes", "mxb_fused_decode_sdpa", "mxb_affine_q8_append",
                  "mxb_sdpa_decode_q8", "mxb_merge_partials")
-_native = None
+_native = None     # the extension; False: there is none, every call is the Python operators'
+
+
+def _load_native():
+    """The CPython extension, built first where it is missing or belongs to another torch or interpreter (loaded all the
+    same it would misread their objects).  Where that cannot be done the Python operators take every call, at their own pace."""
+    from . import _build
+    lib = _abi.load()
+    try:
+        if not _build.native_is_current():
+            _build.build_native()
+        from . import _native as mod
+        mod.bind(*(C.cast(getattr(lib, n), C.c_void_p).value for n in _NATIVE_CALLS))
+        return mod
+    except (ImportError, OSError, RuntimeError) as e:
+        warnings.warn(f"moespresso_b200: no native host calls, short steps run from Python and take longer ({e})", RuntimeWarning,
+                      stacklevel=4)
+        return False
 
 
 def native(name: str, *args):
     """One of the native host calls (``csrc/host_calls.cpp``), which take an operator's plain case in one go.  None: not
-    such a case, nothing has been done, the caller goes on in Python."""
+    such a case, the caller goes on in Python."""
     global _native
     if _native is None:
-        lib = _abi.load()
-        from . import _native as mod
-        mod.bind(*(C.cast(getattr(lib, n), C.c_void_p).value for n in _NATIVE_CALLS))
-        _native = mod
-    if TIMER is not None:
+        _native = _load_native()
+    if TIMER is not None or _native is False:
         return None
     r = getattr(_native, name)(*args)
     if type(r) is int:

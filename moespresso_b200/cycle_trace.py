@@ -56,7 +56,7 @@ def trace(case: str):
     import torch
     lib = TRACE_LIB if os.path.exists(TRACE_LIB) else build_trace_library()
     _build.LIB = lib                       # this process talks to the traced library only
-    _build.is_current = lambda: True
+    _build.library_is_current = lambda: True
     from . import synth
     from .deepseek_v4 import indexed_attention_kernel as iak
     dev = torch.device("cuda")
