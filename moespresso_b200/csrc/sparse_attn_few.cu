@@ -292,8 +292,8 @@ __global__ void __launch_bounds__(kFewThreads, 1) sparse_attn_few_kernel(const _
             amax = fmaxf(amax, fmaxf(fabsf(v.x), fabsf(v.y)));
           }
         amax = warp_max(amax);
-        const int ex = (int)(__float_as_uint(amax) >> 23) - 127;   // floor(log2(max)); zeros and denormals: any power does
-        const int sh = min(max(14 - ex, -100), 100);
+        const int ex = (int)(__float_as_uint(amax) >> 23) - 127;   // floor(log2(max)); zeros and denormals: -127
+        const int sh = min(14 - ex, 126);   // at least -114; 2^126 brings any 16-bit q to where fp16 holds all its bits
         const float up = __uint_as_float((uint32_t)(127 + sh) << 23);
         if (lane == 0) qmul_s[2 * warp + hh] = __uint_as_float((uint32_t)(127 - sh) << 23);
 #pragma unroll

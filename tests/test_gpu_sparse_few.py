@@ -123,6 +123,27 @@ def test_q_of_any_magnitude_over_int8_rows():
     assert max_abs(base[0, 3, 0], mean) <= 2e-2
 
 
+@pytest.mark.parametrize("e", [-126, -112, 99, 116, 125])
+def test_int8_tables_take_any_finite_q(e):
+    """q is scaled by a power of two into fp16's range: over all of bfloat16's range the same bits as for q of 1."""
+    need_gpu()
+    rng = np.random.default_rng(5)
+    D, H, k, R = 576, 20, 300, 900
+    t = _tables(rng, "int8", R, 0, D)
+    q = np.round(8 * rng.standard_normal((H, D)).clip(-3.9, 3.9)) / 8       # times 2^e exactly a bfloat16
+    ids = np.sort(rng.choice(R, size=k, replace=False)).astype(np.int32)
+
+    def f(e):
+        x = dev((q * 2.0 ** e).astype(np.float32), torch.bfloat16)[None, :, None, :]
+        return iak.sparse_attention(x, t["ct"], dev(ids)[None, None], None, pos0=0, window=0, ratio=0, scale=0.7 * 2.0 ** -e, d_v=512,
+                                    kv_scales=t["cst"], n_comp=R)
+    base = f(0)
+    assert bool(base.isfinite().all()) and torch.equal(f(e), base)
+    ref = ds4.indexed_mixed_attention_decode(q.astype(np.float32), None, t["comp"], ids, None, pos0=0, window=0, ratio=0, scale=0.7,
+                                             d_v=512, kv_scales=t["cs"])
+    assert max_abs(base[0, :, 0], ref) <= 2e-2
+
+
 @pytest.mark.parametrize("kind", ["bf16", "int8"])
 @pytest.mark.parametrize("k", [64, 700, 2048])
 def test_partials_of_list_halves_merge_to_the_whole(kind, k):
