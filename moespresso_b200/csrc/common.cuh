@@ -36,9 +36,10 @@ void note_launch(int n = 1);   // counts kernels enqueued by this library (mxb_k
 
 // Launches a kernel that may start while the one before it on the stream runs, if that lets it (grid_launch_dependents);
 // the kernel calls grid_chain() before it touches global memory.  What it saves is the launch itself, 1 to 1.5 us between
-// two short kernels.
+// two short kernels.  early = false: a plain launch of such a kernel.
 template <class... P, class... A>
-inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+inline cudaError_t launch_early_if(bool early, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st,
+                                   A... args) {
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
@@ -48,9 +49,19 @@ inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned block,
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
+template <class... P, class... A>
+inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+  return launch_early_if(true, kernel, grid, block, smem, st, args...);
+}
+// For kernels that compute for longer than a launch takes: CTAs that are dealt out while another kernel's still sit on some
+// SMs pile up on the others, and a grid of two to six CTAs per SM then lasts as long as its fullest SM.  One CTA per SM and
+// fewer keep the gain.  Exact scores in a row, us (plain before there was an early start, early, by this rule): 20,000 rows by
+// 16 heads of 128 (625 CTAs) 9.1, 12.1, 8.7; 12,000 by 32 of 128 (375) 9.1, 11.4, 8.2; 4,096 by 16 of 64 (128) 3.6, 2.4, 2.4.
+// float32 attention, 24 tokens x 8 heads x 2,048 rows (1,056 CTAs) 161, 175, 155.
+inline bool one_cta_per_sm(dim3 grid) { return (int64_t)grid.x * grid.y * grid.z <= sm_count(); }
 
 // ---- element loads as float -------------------------------------------------
 template <int DT>

@@ -43,8 +43,6 @@ template <int D, int QT, int KT>
 __global__ void __launch_bounds__(128) indexer_exact_kernel(IndexerParams p) {
   extern __shared__ float q_s[];  // [t_tile][H][D]
   float* w_s = q_s + (size_t)p.t_tile * p.H * D;
-  ptx::grid_chain();
-  p.keys = ptx::behind_wait(p.keys);
   const int b = blockIdx.z;
   const int t0 = blockIdx.y * p.t_tile;
   const int64_t count = p.row_count ? (int64_t)p.row_count[b] : p.n_rows;
@@ -210,7 +208,8 @@ static int launch_exact_token(const IndexerParams& p, cudaStream_t st) {
   static_assert(8 * HPW <= D, "the dots take the keys' place");
   auto kern = indexer_exact_token_kernel<D, QT, KT, HPW, RPL>;
   if (smem > 48 * 1024) MXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  MXB_CUDA_OK(launch_early(kern, dim3((unsigned)ceil_div(p.n_rows, 32 * RPL), 1, (unsigned)p.B), 256, smem, st, p));
+  const dim3 grid((unsigned)ceil_div(p.n_rows, 32 * RPL), 1, (unsigned)p.B);
+  MXB_CUDA_OK(launch_early_if(one_cta_per_sm(grid), kern, grid, 256, smem, st, p));
   note_launch();
   return MXB_OK;
 }
@@ -249,8 +248,9 @@ static int launch_exact(IndexerParams& p, cudaStream_t st) {
   auto kern = indexer_exact_kernel<D, QT, KT>;
   if (smem > 48 * 1024) MXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((unsigned)ceil_div(p.n_rows, 128), (unsigned)ceil_div(p.T, t_tile), (unsigned)p.B);
-  MXB_CUDA_OK(launch_early(kern, grid, 128, smem, st, p));
+  kern<<<grid, 128, smem, st>>>(p);   // (many rows or tokens: see one_cta_per_sm)
   note_launch();
+  MXB_CUDA_OK(cudaGetLastError());
   return MXB_OK;
 }
 
