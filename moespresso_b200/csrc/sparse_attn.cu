@@ -535,7 +535,7 @@ static int launch_sparse(SparseParams& p, int out_dtype, size_t smem, dim3 grid,
   {                                                                                                        \
     auto kern = sparse_attn_kernel<KVT, QT, OT>;                                                           \
     MXB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));       \
-    MXB_CUDA_OK(launch_early_if(one_cta_per_sm(grid), kern, grid, 256, smem, st, p));                      \\
+    MXB_CUDA_OK(launch_early_if(one_cta_per_sm(grid), kern, grid, 256, smem, st, p));                      \
   }
   if (out_dtype == MXB_F32 || p.nsplit > 1 || p.partial_ml) MXB_SP(MXB_F32)
   else if (out_dtype == MXB_BF16) MXB_SP(MXB_BF16)
