@@ -211,3 +211,26 @@ def test_bins_of_values(rows, n, k):
     holes[:, : n - n // 4] = -np.inf                         # warps without a score
     for s in (base, few, many, crowd, wide, tiny, flat, holes, np.round(base), np.where(base > 0, 0.0, -0.0).astype(np.float32)):
         _check(s, min(k, n))
+
+
+@pytest.mark.parametrize("rows,n", [(1, 600), (2, 4096), (2, 8192), (150, 2500), (150, 8192)])
+def test_bins_that_fill_unevenly(rows, n):
+    """Long tails, where the row is seen to crowd and goes by the key's bits at once; a threshold's bin that turns out too full
+    although the row is not, in the middle and at either end."""
+    need_gpu()
+    rng = np.random.default_rng(n * 3 + rows)
+    x = rng.standard_normal((rows, n)).astype(np.float32)
+    tenth = rng.random((rows, n)) < 0.1
+
+    def at(level, spread):     # a tenth of an even row within `spread` of one level: too many for a bin, too few to be seen
+        u = rng.uniform(0, 2048, (rows, n))
+        return np.where(tenth, level + spread * np.abs(x), u).astype(np.float32)
+    tail = at(1000.25, 0.1)
+    tail[:, ::9] = 3e38 * rng.random((rows, len(range(0, n, 9))))
+    cases = [np.exp(4 * x), -np.exp(4 * x), np.exp(2 * x), np.exp(1.5 * x), x / rng.standard_normal((rows, n)).astype(np.float32),
+             at(1000.25, 0.1), at(1000.25, 1e-5), at(0.0, 0.1), at(2047.9, 0.1), at(2047.9, 1e-4), tail]
+    for s in cases:
+        order = np.sort(s[0])
+        inside = int((order > 1000.3).sum())
+        for k in {64, n // 2, n - n // 20, max(1, inside)}:
+            _check(s.astype(np.float32), k)
