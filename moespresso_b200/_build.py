@@ -20,7 +20,7 @@ NATIVE = os.path.join(HERE, "_native.so")
 STAMP = os.path.join(HERE, "build", "stamp.txt")
 NATIVE_STAMP = os.path.join(HERE, "build", "native_stamp.txt")
 HEADER = os.path.join(HERE, "..", "include", "moespresso_b200.h")
-SOURCES = ["runtime.cu", "indexer_scores.cu", "indexer_scores_fp8.cu", "indexer_decode.cu", "indexer_qat.cu", "kv_formats.cu", "qwen_q8.cu", "topk_select.cu", "topk_multi.cu", "topk_pivot.cu", "sparse_attn.cu", "decode_fused.cu", "sparse_attn_tc.cu", "sparse_attn_few.cu", "flash_prefill.cu"]
+SOURCES = ["runtime.cu", "indexer_scores.cu", "indexer_scores_fp8.cu", "indexer_decode.cu", "indexer_qat.cu", "kv_formats.cu", "qwen_q8.cu", "topk_select.cu", "topk_multi.cu", "topk_pivot.cu", "sparse_attn.cu", "decode_fused.cu", "sparse_attn_tc.cu", "sparse_attn_few.cu", "flash_prefill.cu", "flash_single.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-Xptxas", "-v",

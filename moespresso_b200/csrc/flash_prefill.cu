@@ -31,18 +31,12 @@
 // Drain: the gate tile arrives by TMA in the Q buffer during the last tile; each thread normalises its half row,
 // applies the sigmoid and writes the output chunks in place; TMA stores write the tile.
 // TMEM: S0 / P0 [0,128) S1 / P1 [128,256) O [256,512).
-#include "common.cuh"
-#include "ptx_sm100.cuh"
+#include "flash_common.cuh"
 
 namespace mxb {
 
-constexpr int FB_M = 128, FB_N = 128, FB_D = 256;
-constexpr int kMaxBins = 80;
+constexpr int FB_N = 128;
 constexpr int kStages = 5;
-#ifndef MXB_FLASH_POLY
-#define MXB_FLASH_POLY 1
-#endif
-constexpr int kPolyOf8 = MXB_FLASH_POLY;   // of every eight exponentials, this many (0 .. 4) run on the FMA pipe
 
 struct FlashSmem {
   static constexpr int stage_bytes = 32768;             // a CTA's half of a K or V tile
@@ -53,99 +47,6 @@ struct FlashSmem {
   static constexpr int rowsum_off = rowmax_off + 512;   // [2 groups][128 rows]
   static constexpr int total = rowsum_off + 1024;
 };
-
-struct FlashParams {
-  const void* gate;
-  int64_t g_ss, g_sh;
-  void* out;
-  int64_t o_ss, o_sh;
-  int32_t S, Skv, Hq, Hkv;
-  float scale_log2;  // scale * log2(e)
-  int32_t q_head_inner, k_head_inner;  // tensor-map dimension order: (D, head, row) instead of (D, row, head)
-  int32_t g_head_inner, o_head_inner, v_head_inner;
-  int32_t tma_drain;   // gate tile in and output tile out by TMA through the (then idle) Q buffer
-  int32_t pair_heads;  // the pair's query tiles: the same rows of two heads (one KV head), or 256 rows of one head
-  int32_t* status;
-  // Stretches of tiles, one per pair of CTAs (n_bins = 0: one item per pair).  Bin i covers the tiles from bin_start[i]
-  // up to bin_start[i + 1], both (item << 16 | tile of the item).
-  float4* part_o;      // [4 n_bins][64 groups of 4 features][128 rows]
-  float2* part_ml;     // [4 n_bins][128 rows]: reference maximum (log2 units), sum
-  int32_t n_bins;
-  uint32_t bin_start[kMaxBins + 1];
-};
-
-// An item: 128 query rows in each CTA of a pair.  Items are numbered longest first.
-struct FlashItems {
-  int n_qt, per_qt;   // query tiles (of 128 or 256 rows) and items of one
-};
-__host__ __device__ inline FlashItems flash_items(int S, int Hq, int pair_heads) {
-  FlashItems f;
-  f.n_qt = pair_heads ? (S + FB_M - 1) / FB_M : (S + 2 * FB_M - 1) / (2 * FB_M);
-  f.per_qt = pair_heads ? Hq / 2 : Hq;
-  return f;
-}
-// Where CTA `rank` of the pair that works on item `it` stands.
-__host__ __device__ inline void flash_item_at(const FlashItems& f, int it, int pair_heads, int rank, int& head, int& m0) {
-  const int qt = f.n_qt - 1 - it / f.per_qt, x = it % f.per_qt;
-  head = pair_heads ? 2 * x + rank : x;
-  m0 = pair_heads ? qt * FB_M : (2 * qt + rank) * FB_M;
-}
-// 128-key tiles that the rows of query tile qt see
-__host__ __device__ inline int flash_tiles(int qt, int S, int Skv, int pair_heads) {
-  const int rows = pair_heads ? FB_M : 2 * FB_M;
-  const int64_t end = (int64_t)qt * rows + rows + (Skv - S);
-  return (int)(((end < Skv ? end : (int64_t)Skv) + FB_N - 1) / FB_N);
-}
-// where a cut item's segment leaves its partial: a bin holds at most one segment that starts inside an item, and
-// one that starts an item and does not finish it
-__device__ __forceinline__ int part_slot(int bin, bool starts_inside, int rank) { return (2 * bin + (starts_inside ? 0 : 1)) * 2 + rank; }
-// The reference maximum a cut segment starts from: finite, so that a row that sees none of the segment's first tile
-// (the rows above the diagonal) gets weights of 0 and not of exp(-inf + inf).
-constexpr float kNoMax = -3e38f;
-constexpr float kGrow = 8.f;   // the reference moves when a logit exceeds it by this many powers of two
-
-template <bool BF16>
-__device__ __forceinline__ uint32_t pack2(float a, float b) {
-  if constexpr (BF16) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&v);
-  } else {
-    __half2 v = __floats2half2_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-}
-__device__ __forceinline__ float fast_ex2(float x) {   // 2^x, x <= 0 here; -inf -> 0
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// 2^x on the FMA pipe for x <= ~8: round-to-nearest split x = n + f with the 1.5 * 2^23 trick, a cubic for 2^f on
-// [-0.5, 0.5] (relative error 7.5e-5, below the rounding of a 16-bit P), n added into the exponent field.  One in
-// eight of a tile's exponentials goes this way.  (The special-function unit's 16 results per clock per SM no longer bound
-// the kernel: 0 / 1 / 2 / 3 in eight 433 / 437 / 439 / 447 us at 8,192 tokens.)  Inputs below -126 (masked keys) give 2^-126 instead of 0.
-__device__ __forceinline__ float poly_ex2(float x) {
-  x = fmaxf(x, -126.f);
-  const float kMagic = 12582912.f;
-  const float xr = x + kMagic;
-  const float f = x - (xr - kMagic);
-  float r = fmaf(0.0551716685295105f, f, 0.2426111251115799f);
-  r = fmaf(r, f, 0.6932609677314758f);
-  r = fmaf(r, f, 0.9999280571937561f);
-  return __int_as_float(__float_as_int(r) + (__float_as_int(xr) << 23));
-}
-
-__device__ __forceinline__ float fast_tanh(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-template <bool BF16>
-__device__ __forceinline__ float2 unpack2(uint32_t u) {
-  if constexpr (BF16) return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u));
-  else return __half22float2(*reinterpret_cast<__half2*>(&u));
-}
 
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
@@ -199,7 +100,7 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     Seg g;
     flash_item_at(items, it, p.pair_heads, rank, g.head, g.m0);
     g.kvh = g.head / (p.Hq / p.Hkv);
-    g.nt = flash_tiles(items.n_qt - 1 - it / items.per_qt, p.S, p.Skv, p.pair_heads);
+    g.nt = flash_tiles<FB_N>(items.n_qt - 1 - it / items.per_qt, p.pair_heads ? FB_M : 2 * FB_M, p.S, p.Skv);
     g.lo = BINS && it == it_first ? j_first : 0;
     g.hi = BINS && it == it_stop ? j_stop : g.nt;
     return g;
@@ -483,7 +384,7 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
       if (cut) {
         // partial: O as it stands, four features of the 128 rows side by side (a warp stores 512 bytes at a time)
-        const int slot = part_slot(pair, g.lo > 0, rank);
+        const int slot = part_slot(pair, g.lo > 0) * 2 + rank;
         float4* po = p.part_o + ((int64_t)slot * (FB_D / 4) + grp * (FB_D / 8)) * FB_M + row;
         ptx::mbar_wait(&pv_done[r_last & 1], (uint32_t)((r_last >> 1) & 1), abort_flag);
         ptx::tc_fence_after_sync();
@@ -598,11 +499,12 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 }
 
 // Joins the partials of the items that a bin boundary cut, and finishes them as the drain above would (division by
-// the sum, gate, rounding).  Block (bin - 1, 32 features, CTA of the pair): the block of the bin in which an item's second
+// the sum, gate, rounding).  Block (bin - 1, 32 features, CTA of the item): the block of the bin in which an item's second
 // piece lies does the item, the others leave.  Thread = (row, 16 features): the partials are read 512 bytes a warp, the output in
 // whole 32-byte sectors.
-template <bool BF16>
+template <bool BF16, bool SINGLE>
 __global__ void __launch_bounds__(256) flash_merge_kernel(const __grid_constant__ FlashParams p) {
+  constexpr int CTAS = SINGLE ? 1 : 2;
   const int bin = (int)blockIdx.x + 1, rank = (int)blockIdx.z;
   const uint32_t at = p.bin_start[bin], before = p.bin_start[bin - 1];
   const int it = (int)(at >> 16);
@@ -611,19 +513,24 @@ __global__ void __launch_bounds__(256) flash_merge_kernel(const __grid_constant_
   while (last + 1 < p.n_bins && (int)(p.bin_start[last + 1] >> 16) == it) ++last;
   const int row = threadIdx.x & (FB_M - 1), f16 = (int)blockIdx.y * 2 + (threadIdx.x >> 7);
   int head, m0;
-  flash_item_at(flash_items(p.S, p.Hq, p.pair_heads), it, p.pair_heads, rank, head, m0);
+  if constexpr (SINGLE) {
+    head = it % p.Hq;
+    m0 = ((p.S + FB_M - 1) / FB_M - 1 - it / p.Hq) * FB_M;
+  } else {
+    flash_item_at(flash_items(p.S, p.Hq, p.pair_heads), it, p.pair_heads, rank, head, m0);
+  }
   const int qi = m0 + row;
   if (qi >= p.S) return;
   float m = -INFINITY;
 #pragma unroll 8
-  for (int b = bin - 1; b <= last; ++b) m = fmaxf(m, __ldg(&p.part_ml[(int64_t)part_slot(b, b >= bin, rank) * FB_M + row].x));
+  for (int b = bin - 1; b <= last; ++b) m = fmaxf(m, __ldg(&p.part_ml[(int64_t)(part_slot(b, b >= bin) * CTAS + rank) * FB_M + row].x));
   float l = 0.f;
   float4 o[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) o[c] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
   for (int b = bin - 1; b <= last; ++b) {   // in the order of the keys
-    const int slot = part_slot(b, b >= bin, rank);
+    const int slot = part_slot(b, b >= bin) * CTAS + rank;
     const float2 ml = __ldg(p.part_ml + (int64_t)slot * FB_M + row);
     const float4* po = p.part_o + ((int64_t)slot * (FB_D / 4) + f16 * 4) * FB_M + row;
     float4 v[4];
@@ -670,12 +577,13 @@ __global__ void __launch_bounds__(256) flash_merge_kernel(const __grid_constant_
 
 using namespace mxb;
 
-// How the items are dealt out.  Costs are in tiles (1.3 to 1.6 us each on a B200): a segment costs its tiles and
-// kSegCost for its Q load, first scores and drain; cutting costs kCutCost (partials out, merge launch, partials in), and
-// the stretches must be kSaving percent shorter than the pair with the most whole items works.  That much, because tiles
+// How the items are dealt out.  Costs are in tiles (pairs: 128 keys, 1.3 to 1.6 us each on a B200; single CTAs: 64 keys, 0.9
+// to 1.05 us): a segment costs its tiles and `seg` for its Q load, first scores and drain; cutting costs `cut` (partials
+// out, merge launch, partials in), and the stretches must be kSaving percent shorter than the pair or CTA with the most whole
+// items works.  That much, because tiles
 // take longer when every SM streams K and V at once, and because a cut saves time and not energy: back to back, under
 // the power cap, the SMs that idle behind whole items leave the others a higher clock.  Stretches of less than
-// kMinShare are not worth a pair of their own.  Measured (16 query / 2 KV heads, bf16, gated; tokens over past, us, one
+// `share` are not worth SMs of their own.  Measured (16 query / 2 KV heads, bf16, gated; tokens over past, us, one
 // pair per item against equal stretches, 5 / 600 in a row):
 //   64 over 3,000 46.5 / 45.5 -> 29.3 / 28.7; 64 over 30,000 361 / 360 -> 68 / 64; 300 over 2,000 39.1 / 37.2 -> 31.9 / 30.7;
 //   500 over 30,000 369 / 369 -> 204 / 217; 1,200 over 4,000 126 / 123 -> 104 / 97; 1,200 over 30,000 746 / 747 -> 484 / 540;
@@ -686,38 +594,51 @@ using namespace mxb;
 //   3,000 over 0 88 / 83 -> 124 / 121.
 // A cut changes the results in the last bits (P is rounded to 16 bits against each segment's own reference; the error
 // against float64 stays the same, 2.31e-3 relative in bf16 on either side).  The partials take up to 39 MB (296 slots).
-constexpr int kSegCost = 2, kCutCost = 10, kMinShare = 6, kSaving = 15;
+struct FlashCosts {
+  int seg, cut, share;
+};
+constexpr FlashCosts kPairCosts = {2, 10, 6}, kSingleCosts = {4, 16, 12};
+constexpr int kSaving = 15;
 
-// Fills p.n_bins / p.bin_start (n_bins = 0: one CTA per item) and returns the bytes of partials the plan needs.
-static int64_t flash_plan(FlashParams& p, int sms) {
+// Fills p.n_bins and p.bin_start for pairs (ctas = 2) or single CTAs (n_bins = 0: an item each) and returns the bytes of
+// partials that the plan needs; *cost = how long it takes, in tiles.
+static int64_t flash_plan(FlashParams& p, int ctas, int sms, bool may_cut, int64_t* cost) {
   p.n_bins = 0;
-  int pairs = sms / 2;
-  if (pairs > kMaxBins) pairs = kMaxBins;
-  const FlashItems f = flash_items(p.S, p.Hq, p.pair_heads);
+  const FlashCosts c = ctas == 1 ? kSingleCosts : kPairCosts;
+  int workers = sms / ctas;
+  if (workers > kMaxBins) workers = kMaxBins;
+  if (workers < 1) workers = 1;
+  const FlashItems f = ctas == 1 ? FlashItems{(p.S + FB_M - 1) / FB_M, p.Hq} : flash_items(p.S, p.Hq, p.pair_heads);
   const int64_t items = (int64_t)f.n_qt * f.per_qt;
-  auto tiles = [&](int qt) { return flash_tiles(qt, p.S, p.Skv, p.pair_heads); };
-  // more than eight rounds of items even out by themselves; bin_start holds 16 bits of tile
-  if (pairs < 1 || items > 8 * pairs || tiles(f.n_qt - 1) > 0xFFFF) return 0;
-  // One pair per item: the hardware hands the next item to the pair of SMs that is done first.  Dealt back and forth over
-  // the pairs, longest first, that ends with the largest of these sums.
-  int load[kMaxBins] = {0}, longest = 0, k = 0, step = 1;
+  auto tiles = [&](int qt) {
+    return ctas == 1 ? flash_tiles<64>(qt, FB_M, p.S, p.Skv) : flash_tiles<FB_N>(qt, p.pair_heads ? FB_M : 2 * FB_M, p.S, p.Skv);
+  };
   int64_t total = 0;
+  for (int qt = 0; qt < f.n_qt; ++qt) total += (int64_t)(tiles(qt) + c.seg) * f.per_qt;
+  *cost = total / workers;
+  if (items > 8 * workers) return 0;   // more than eight rounds of items even out by themselves
+  // One pair or CTA per item: the hardware hands the next item to the SMs that are done first.  Dealt back and forth over
+  // the workers, longest first, that ends with the largest of these sums.
+  int load[kMaxBins] = {0}, longest = 0, k = 0, step = 1;
   for (int qt = f.n_qt - 1; qt >= 0; --qt) {
-    const int cost = tiles(qt) + kSegCost;
-    total += (int64_t)cost * f.per_qt;
+    const int x = tiles(qt) + c.seg;
     for (int h = 0; h < f.per_qt; ++h) {
-      load[k] += cost;
+      load[k] += x;
       if (load[k] > longest) longest = load[k];
       k += step;
-      if (k == pairs || k < 0) {
+      if (k == workers || k < 0) {
         step = -step;
         k += step;
       }
     }
   }
-  const int bins = (int)(total / kMinShare < pairs ? total / kMinShare : pairs);
-  if (bins < 2 || 100 * (int64_t)longest <= (100 + kSaving) * (total / bins) + 100 * kCutCost) return 0;
-  // Equal stretches of the items' costs.  A piece of fewer than kSegCost tiles is not worth a segment: the boundary
+  *cost = longest;
+  const int bins = (int)(total / c.share < workers ? total / c.share : workers);
+  // (bin_start holds 16 bits of tile)
+  if (!may_cut || sms < ctas || tiles(f.n_qt - 1) > 0xFFFF || bins < 2 ||
+      100 * (int64_t)longest <= (100 + kSaving) * (total / bins) + 100 * c.cut)
+    return 0;
+  // Equal stretches of the items' costs.  A piece of fewer than `seg` tiles is not worth a segment: the boundary
   // moves to the item's edge.
   uint32_t* start = p.bin_start;
   int n = 0, qt = f.n_qt - 1, h = 0, nt = tiles(qt);
@@ -726,25 +647,47 @@ static int64_t flash_plan(FlashParams& p, int sms) {
   start[n++] = 0;
   for (int b = 1; b < bins; ++b) {
     const int64_t x = total * b / bins;
-    while (x >= c0 + nt + kSegCost) {
-      c0 += nt + kSegCost;
+    while (x >= c0 + nt + c.seg) {
+      c0 += nt + c.seg;
       ++item;
       if (++h == f.per_qt) {
         h = 0;
         nt = tiles(--qt);
       }
     }
-    const int64_t j = x - c0 - kSegCost / 2;
-    const uint32_t at = j < kSegCost ? item << 16 : j > nt - kSegCost ? (item + 1) << 16 : item << 16 | (uint32_t)j;
+    const int64_t j = x - c0 - c.seg / 2;
+    const uint32_t at = j < c.seg ? item << 16 : j > nt - c.seg ? (item + 1) << 16 : item << 16 | (uint32_t)j;
     if (at > start[n - 1] && at < (uint32_t)items << 16) start[n++] = at;
   }
   start[n] = (uint32_t)items << 16;
   p.n_bins = n;
-  return (int64_t)4 * n * FB_M * (FB_D * 4 + 8);
+  *cost = total / bins + c.cut;
+  return (int64_t)2 * ctas * n * FB_M * (FB_D * 4 + 8);
 }
 
-// Two heads of one KV head share its tiles; heads that cannot be paired so take 256 rows at a time.
-static int flash_pair_heads(const mxb_flash_prefill_args* a) { return (a->Hq / a->Hkv) % 2 == 0 ? 1 : 0; }
+// Pairs of CTAs or single ones?  Two heads of one KV head share a pair; heads that cannot be paired so give it 256 rows at a
+// time, half of them empty in a sequence of up to 128.  By the two plans' times: 0.95 us per cost of a single CTA against 1.45 us
+// per cost of a pair and 2 us for its later start.  Over 356 shapes, 1/1 to 128/128 heads, 2 to 2,048 tokens over a past of 0 to
+// 30,000, that choice is 0.3 % behind the better of the two on average, and 1.17 times where 64 heads of keys and values bound
+// both (128 tokens over 4,000).  us, single against pairs: 16/2 heads, 2 tokens 8.2, 9.8, 128 tokens 10.0, 10.4,
+// 300 tokens 12.1, 12.9, 200 over 500 17.6, 17.2, 700 over 1,000 32.8, 29.6; 96/96 heads, 64 tokens 8.9, 19.8, 2,048 tokens 325,
+// 253; 48/16 heads, 300 over 1,000 28.3, 47.6, 1,000 over 1,000 93.4, 85.6.  Heads that pair up and more than 512 tokens were
+// never better off on single CTAs.
+// Fills p as flash_plan does; *ctas = what the choice is.
+static int64_t flash_choose(FlashParams& p, bool may_cut, int* ctas) {
+  p.pair_heads = (p.Hq / p.Hkv) % 2 == 0 ? 1 : 0;
+  const int sms = sm_count();
+  int64_t pair_cost, single_cost;
+  const int64_t pair_bytes = flash_plan(p, 2, sms, may_cut, &pair_cost);
+  *ctas = 2;
+  if (p.pair_heads && p.S > 4 * FB_M) return pair_bytes;
+  FlashParams single = p;
+  const int64_t single_bytes = flash_plan(single, 1, sms, may_cut, &single_cost);
+  if (95 * single_cost >= 145 * pair_cost + 200) return pair_bytes;
+  p = single;
+  *ctas = 1;
+  return single_bytes;
+}
 
 static int flash_validate(const mxb_flash_prefill_args* a) {
   MXB_REQUIRE(a != nullptr, MXB_ERR_INVALID, "flash prefill: null args");
@@ -761,9 +704,9 @@ static int flash_validate(const mxb_flash_prefill_args* a) {
 extern "C" int64_t mxb_flash_prefill_workspace_bytes(const mxb_flash_prefill_args* a) {
   if (flash_validate(a) != MXB_OK) return 0;
   FlashParams p{};
-  p.S = a->S; p.Skv = a->Skv; p.Hq = a->Hq;
-  p.pair_heads = flash_pair_heads(a);
-  return flash_plan(p, sm_count());
+  p.S = a->S; p.Skv = a->Skv; p.Hq = a->Hq; p.Hkv = a->Hkv;
+  int ctas;
+  return flash_choose(p, true, &ctas);
 }
 
 extern "C" int mxb_flash_prefill(const mxb_flash_prefill_args* a, void* stream) {
@@ -775,6 +718,15 @@ extern "C" int mxb_flash_prefill(const mxb_flash_prefill_args* a, void* stream) 
   MXB_REQUIRE(!a->gate || ((reinterpret_cast<uintptr_t>(a->gate) & 15) == 0 && a->gate_stride_s % 8 == 0 &&
                            a->gate_stride_h % 8 == 0),
               MXB_ERR_INVALID, "gate must be 16-byte aligned with strides that are multiples of 8 elements");
+  FlashParams p{};
+  p.S = a->S; p.Skv = a->Skv; p.Hq = a->Hq; p.Hkv = a->Hkv;
+  // the partials of cut items need the workspace; without it every item is one pair's, or one CTA's
+  const bool ws_ok = a->workspace && (reinterpret_cast<uintptr_t>(a->workspace) & 15) == 0;
+  int ctas;
+  const int64_t need = flash_choose(p, ws_ok, &ctas);
+  if (need > 0 && a->workspace_bytes < need) (void)flash_choose(p, false, &ctas);
+  // a CTA's share of a K and a V tile
+  const uint32_t k_box = ctas == 1 ? 64u : (uint32_t)FB_N / 2, v_box = ctas == 1 ? 64u : (uint32_t)FB_N;
   const CUtensorMapDataType dt = a->dtype == MXB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   CUtensorMap tq, tk, tv;
   // cuTensorMapEncodeTiled wants ascending strides: put the head axis before the row axis when its
@@ -792,7 +744,7 @@ extern "C" int mxb_flash_prefill(const mxb_flash_prefill_args* a, void* stream) 
     uint64_t dims[3] = {(uint64_t)a->D, (uint64_t)(k_hin ? a->Hkv : a->Skv), (uint64_t)(k_hin ? a->Skv : a->Hkv)};
     uint64_t str[2] = {(uint64_t)(k_hin ? a->k_stride_h : a->k_stride_s) * 2,
                        (uint64_t)(k_hin ? a->k_stride_s : a->k_stride_h) * 2};
-    uint32_t box[3] = {64, k_hin ? 1u : (uint32_t)FB_N / 2, k_hin ? (uint32_t)FB_N / 2 : 1u};   // a CTA's half of the keys
+    uint32_t box[3] = {64, k_hin ? 1u : k_box, k_hin ? k_box : 1u};
     rc = make_tensor_map(&tk, dt, 3, a->k, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != MXB_OK) return rc;
   }
@@ -801,7 +753,7 @@ extern "C" int mxb_flash_prefill(const mxb_flash_prefill_args* a, void* stream) 
     uint64_t dims[3] = {(uint64_t)a->D, (uint64_t)(v_hin ? a->Hkv : a->Skv), (uint64_t)(v_hin ? a->Skv : a->Hkv)};
     uint64_t str[2] = {(uint64_t)(v_hin ? a->v_stride_h : a->v_stride_s) * 2,
                        (uint64_t)(v_hin ? a->v_stride_s : a->v_stride_h) * 2};
-    uint32_t box[3] = {64, v_hin ? 1u : (uint32_t)FB_N, v_hin ? (uint32_t)FB_N : 1u};
+    uint32_t box[3] = {64, v_hin ? 1u : v_box, v_hin ? v_box : 1u};
     rc = make_tensor_map(&tv, dt, 3, a->v, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != MXB_OK) return rc;
   }
@@ -824,38 +776,37 @@ extern "C" int mxb_flash_prefill(const mxb_flash_prefill_args* a, void* stream) 
   if (tma_drain && a->gate) tma_drain = tile_map(&tg, a->gate, a->gate_stride_s, a->gate_stride_h, g_hin);
 
   MXB_REQUIRE(a->scale > 0.f, MXB_ERR_INVALID, "flash prefill: scale must be positive");
-  FlashParams p{};
   p.g_head_inner = g_hin ? 1 : 0; p.o_head_inner = o_hin ? 1 : 0; p.tma_drain = tma_drain ? 1 : 0;
   p.v_head_inner = v_hin ? 1 : 0;
   p.gate = a->gate; p.g_ss = a->gate_stride_s; p.g_sh = a->gate_stride_h;
   p.out = a->out; p.o_ss = a->out_stride_s; p.o_sh = a->out_stride_h;
-  p.S = a->S; p.Skv = a->Skv; p.Hq = a->Hq; p.Hkv = a->Hkv;
   p.scale_log2 = a->scale * 1.4426950408889634f;
   p.status = a->status;
   p.q_head_inner = q_hin ? 1 : 0;
   p.k_head_inner = k_hin ? 1 : 0;
-  p.pair_heads = flash_pair_heads(a);
-  const int smem = FlashSmem::total + 1024;
-  // the partials of cut items need the workspace; without it every item is one CTA's
-  const int64_t need = flash_plan(p, sm_count());
-  if (!a->workspace || a->workspace_bytes < need || (reinterpret_cast<uintptr_t>(a->workspace) & 15) != 0) p.n_bins = 0;
   p.part_o = reinterpret_cast<float4*>(a->workspace);
-  p.part_ml = reinterpret_cast<float2*>(p.part_o + (int64_t)4 * p.n_bins * (FB_D / 4) * FB_M);
+  p.part_ml = reinterpret_cast<float2*>(p.part_o + (int64_t)2 * ctas * p.n_bins * (FB_D / 4) * FB_M);
   const FlashItems items = flash_items(p.S, p.Hq, p.pair_heads);
-  const dim3 grid(2u * (p.n_bins > 0 ? (unsigned)p.n_bins : (unsigned)(items.n_qt * items.per_qt)));
-  const dim3 merge_grid((unsigned)(p.n_bins - 1), FB_D / 32, 2);
-  auto go = [&](auto* whole, auto* binned, auto* merge) -> int {
-    auto* kernel = p.n_bins > 0 ? binned : whole;
+  const int64_t whole = ctas == 1 ? ceil_div((int64_t)p.S, (int64_t)FB_M) * p.Hq : (int64_t)items.n_qt * items.per_qt;
+  const unsigned grid = (unsigned)(ctas * (p.n_bins > 0 ? p.n_bins : whole));
+  const bool bf16 = a->dtype == MXB_BF16;
+  if (ctas == 1) {
+    rc = launch_flash_single(tq, tk, tv, tg, to, p, bf16, grid, st);
+    if (rc != MXB_OK) return rc;
+  } else {
+    constexpr int smem = FlashSmem::total + 1024;
+    auto* kernel = bf16 ? (p.n_bins > 0 ? flash_prefill_kernel<true, true> : flash_prefill_kernel<true, false>)
+                        : (p.n_bins > 0 ? flash_prefill_kernel<false, true> : flash_prefill_kernel<false, false>);
     MXB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     kernel<<<grid, 384, smem, st>>>(tq, tk, tv, tg, to, p);
     note_launch();
-    if (p.n_bins > 1) {
-      merge<<<merge_grid, 256, 0, st>>>(p);
-      note_launch();
-    }
-    MXB_CUDA_OK(cudaGetLastError());
-    return MXB_OK;
-  };
-  return a->dtype == MXB_BF16 ? go(flash_prefill_kernel<true, false>, flash_prefill_kernel<true, true>, flash_merge_kernel<true>)
-                              : go(flash_prefill_kernel<false, false>, flash_prefill_kernel<false, true>, flash_merge_kernel<false>);
+  }
+  if (p.n_bins > 1) {
+    auto* merge = ctas == 1 ? (bf16 ? flash_merge_kernel<true, true> : flash_merge_kernel<false, true>)
+                            : (bf16 ? flash_merge_kernel<true, false> : flash_merge_kernel<false, false>);
+    merge<<<dim3((unsigned)(p.n_bins - 1), FB_D / 32, (unsigned)ctas), 256, 0, st>>>(p);
+    note_launch();
+  }
+  MXB_CUDA_OK(cudaGetLastError());
+  return MXB_OK;
 }

@@ -70,10 +70,18 @@ def test_items_cut_at_equal_stretches(S, past, Hq, Hkv, dt, gate):
     (300, 200, 3, 1),     # an odd number of query tiles
     (65, 3000, 3, 3),     # items cut between pairs that take 256 rows
     (257, 129, 6, 3),     # two heads of one KV head: three query tiles, a last key tile of two keys
+    (1, 1200, 2, 1),      # from here on long enough for pairs: one row of two heads
+    (64, 700, 7, 7),      # the pair's second query tile lies past the end
+    (129, 500, 3, 3),     # the second tile holds one row
+    (257, 700, 1, 1),     # 256 rows and one more
+    (300, 3000, 5, 5),    # items of 256 rows, cut
+    (64, 64, 96, 96),     # more heads than pairs of SMs: single CTAs
+    (300, 1000, 48, 16),  # 144 of them
 ])
 @pytest.mark.parametrize("dt", ["bf16", "f16"])
 def test_pairs_of_query_tiles(S, past, Hq, Hkv, dt):
-    """A pair of CTAs takes two heads of one KV head, or 256 rows of one head where the heads per KV head are odd."""
+    """A pair of CTAs takes two heads of one KV head, or 256 rows of one head where the heads per KV head are odd; short
+    sequences and heads that would leave pairs empty go to single CTAs."""
     need_gpu()
     rng = np.random.default_rng(S + past)
     tdt = torch.bfloat16 if dt == "bf16" else torch.float16
