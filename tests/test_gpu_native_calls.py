@@ -3,6 +3,8 @@ else (conversions, copies, errors) left to Python."""
 import numpy as np
 import pytest
 import torch
+from torch.overrides import TorchFunctionMode
+from torch.utils._python_dispatch import TorchDispatchMode
 
 from moespresso_b200 import _abi
 from moespresso_b200 import _torchabi as _t
@@ -166,3 +168,68 @@ def test_q8_token(taken):
     with pytest.raises(ValueError):
         sdpa_decode_q8(q, *narrow.state[0], *narrow.state[1], 0.0625)
     assert taken == [] and _abi.load().mxb_kernel_launches() == before
+
+
+class _Plain(torch.Tensor):
+    pass
+
+
+def test_modes_and_wrappers_are_left_to_python(taken):
+    """Function and dispatch modes, tensor subclasses and the wrappers of torch.func: the native calls see none of them."""
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    cache = _cache(torch.bfloat16, [1500], gen)
+    q, iq = (torch.randn(1, h, d, generator=gen, device="cuda").bfloat16() for h, d in ((64, 576), (16, 64)))
+    w = torch.randn(1, 16, generator=gen, device="cuda")
+    f = lambda x=q: sparse_decode_step(x, iq, w, cache, k=256, scale=0.05, d_v=512)
+    ref = f()
+    assert taken == ["decode_step"]
+    del taken[:]
+    seen = []
+
+    class Functions(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append("function")
+            return func(*args, **(kwargs or {}))
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append("dispatch")
+            return func(*args, **(kwargs or {}))
+    for mode, name in ((Functions, "function"), (Dispatch, "dispatch")):
+        del seen[:]
+        with mode():
+            out = f()
+        assert torch.equal(out, ref) and taken == [] and name in seen       # the operator's own tensor calls went through it
+    assert torch.equal(f(q.as_subclass(_Plain)).as_subclass(torch.Tensor), ref)
+    assert torch.equal(f(torch.nn.Parameter(q)), ref) and taken == ["decode_step"]       # (a parameter is a plain tensor)
+    args = lambda x: (x, iq, w, cache.kv, None, cache.idx_keys, cache.row_start, cache.row_count, cache.max_rows, 256, 0.05, 512, None,
+                      torch.float32, False)
+
+    def inside(x):
+        seen.append(_t.native("decode_step", *args(x)))
+        return x.float().sum()
+    del seen[:]
+    torch.func.vmap(inside)(torch.stack([q, q]))
+    torch.func.grad(inside)(q.float())
+    assert seen == [None, None] and _t.native("decode_step", *args(q)) is not None
+
+
+def test_native_calls_in_a_graph(taken):
+    """Under capture the outputs and scratch come from the graph's pool, and a replay computes from what the inputs hold then."""
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    cache = _cache(torch.float32, [1800], gen)
+    q, iq = (torch.randn(1, h, d, generator=gen, device="cuda") for h, d in ((64, 576), (16, 64)))
+    w = torch.randn(1, 16, generator=gen, device="cuda")
+    f = lambda: sparse_decode_step(q, iq, w, cache, k=256, scale=0.05, d_v=512, return_ids=True)
+    f()
+    graph = torch.cuda.CUDAGraph()
+    del taken[:]
+    with torch.cuda.graph(graph):
+        out, ids = f()
+    assert taken == ["decode_step"]
+    for _ in range(3):
+        q.copy_(torch.randn(q.shape, generator=gen, device="cuda"))
+        iq.copy_(torch.randn(iq.shape, generator=gen, device="cuda"))
+        graph.replay()
+        ref = f()
+        assert torch.equal(out, ref[0]) and torch.equal(ids, ref[1])
