@@ -25,17 +25,6 @@
 
 namespace mxb {
 
-#if defined(MXB_TRACE_MMA)
-#define TR(role, i)
-#define TRM(role, i) do { if (tr_on && (i) < 64) tr[(role) * 64 + (i)] = clock64(); } while (0)
-#elif defined(MXB_TRACE)
-#define TR(role, i) do { if (tr_on && (i) < 64) tr[(role) * 64 + (i)] = clock64(); } while (0)
-#define TRM(role, i)
-#else
-#define TR(role, i)
-#define TRM(role, i)
-#endif
-
 struct Fp8Params {
   const uint8_t* keys;
   int64_t rows_total;
@@ -134,11 +123,6 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
   const int ntiles = (int)((span + 127) / 128);
   const int nt = min(p.t_tile, p.T - t0);
   const int N = p.N, H = p.H, n_acc = p.n_acc;
-#if defined(MXB_TRACE) || defined(MXB_TRACE_MMA)
-  long long* tr = reinterpret_cast<long long*>(p.status);
-  const bool tr_on = p.status && blockIdx.x == 1 && blockIdx.z == 0 && lane == 0;
-  if (tr_on && tid == 0) tr[6 * 64] = clock64();
-#endif
 
   // 16 heads and eight tokens per tile: every group of drain warps keeps the weights of two tokens in registers and drains
   // those two of every tile, instead of all tokens of every fourth tile with the weights read again for each.  The reads
@@ -276,7 +260,6 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
           if (i >= S) ptx::mbar_wait(&raw_empty[s], (uint32_t)((i / S - 1) & 1), abort_flag);
         }
         const int64_t grow = rbase + row0 + (int64_t)i * 128;
-        TR(0, i);
         if constexpr (K16) {
           // 16-bit keys go straight into the swizzled operand ring
           constexpr int NAk = C::kNA;
@@ -333,11 +316,8 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
           ptx::mma_commit(&raw_empty[s]);
         } else {
           // descriptors differ from the precomputed bases only in their start-address field
-          TRM(0, i);
           ptx::mbar_wait(&a_full[ab], ab_ph, abort_flag);
-          TRM(1, i);
           if (i >= n_acc) ptx::mbar_wait(&acc_empty[a], a_ph, abort_flag);
-          TRM(2, i);
           ptx::tc_fence_after_sync();
           const uint64_t ad0 = ptx::desc_advance(a_desc0, (uint32_t)(ab * C::kA16));
 #pragma unroll
@@ -346,13 +326,9 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
             for (int ks = 0; ks < 4; ++ks)
               ptx::mma_f16_ss(d_tmem, ptx::desc_advance(ad0, kb * 16384 + ks * 32),
                               ptx::desc_advance(b_desc0, kb * N * 128 + ks * 32), idesc16, (kb | ks) ? 1u : 0u);
-          TRM(3, i);
           ptx::mma_commit(&a_empty[ab]);
-          TRM(4, i);
-          TR(3, i);
         }
         ptx::mma_commit(&acc_full[a]);
-        TRM(5, i);
         a += kMmaWarps;
         if (a >= n_acc) { a -= n_acc; a_ph ^= 1u; }
         if (NA > 0) {
@@ -371,7 +347,6 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
         const int s = i % S;
         ptx::mbar_wait(&raw_full[s], (uint32_t)((i / S) & 1), abort_flag);
         if (i >= NA) ptx::mbar_wait(&a_empty[cw], (uint32_t)((i / NA - 1) & 1), abort_flag);
-        TR(1, i);
         const uint8_t* raw = raw_buf + (size_t)s * C::kRaw;
 #pragma unroll 4
         for (int ci = lane; ci < 128 * CPR; ci += 32) {
@@ -392,7 +367,6 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
         ptx::fence_proxy_async_smem();
         ptx::mbar_arrive(&a_full[cw]);
         ptx::mbar_arrive(&raw_empty[s]);
-        TR(2, i);
       }
     }
   } else {
@@ -439,7 +413,6 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
       const int a = i % n_acc;
       ptx::mbar_wait(&acc_full[a], (uint32_t)((i / n_acc) & 1), abort_flag);
       ptx::tc_fence_after_sync();
-      if (quad == 0) TR(4, i);
       const int64_t r = row0 + (int64_t)i * 128 + rloc;
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * p.acc_stride);
       const bool r_ok = r < count;
@@ -495,15 +468,12 @@ indexer_fp8_kernel(const __grid_constant__ CUtensorMap tmap, Fp8Params p) {
       }
       ptx::tc_fence_before_sync();
       ptx::mbar_arrive(&acc_empty[a]);
-      if (quad == 0) TR(5, i);
     }
   }
 
   __syncthreads();
   if (warp == 0) ptx::tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
-#if !defined(MXB_TRACE) && !defined(MXB_TRACE_MMA)
   if (tid == 0 && *abort_flag && p.status) atomicExch(p.status, 1);
-#endif
 }
 
 // 16-bit keys, sequences of one length (all CTAs cost the same, one per SM): tokens per tile and row tiles per CTA, for the

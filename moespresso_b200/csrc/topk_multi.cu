@@ -68,12 +68,6 @@ __global__ void __launch_bounds__(kMThreads) topk_mhist_kernel(TopkMultiParams p
     if (hist[i]) atomicAdd(&g[i], hist[i]);
 }
 
-#ifdef MXB_TRACE_MF
-#define TRF(k) do { if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) reinterpret_cast<long long*>(p.cand_idx + p.n - 64)[k] = clock64(); } while (0)
-#else
-#define TRF(k)
-#endif
-
 __global__ void __launch_bounds__(kMThreads) topk_mfilter_kernel(TopkMultiParams p) {
   __shared__ uint32_t warp_sums[32];
   __shared__ uint32_t s_total, s_thr[4], s_base[2];
@@ -83,11 +77,9 @@ __global__ void __launch_bounds__(kMThreads) topk_mfilter_kernel(TopkMultiParams
   if (lo >= n) return;
   const int64_t hi = min(lo + p.part, n);
   const float* src = p.scores + (p.row_start ? p.row_start[row] : (int64_t)row * p.row_stride);
-  TRF(0);
   if (tid < 4) s_thr[tid] = 0;
   __syncthreads();
   row_threshold<kMThreads>(p.hist + (int64_t)row * kBigBins, p.k, warp_sums, &s_total, s_thr);
-  TRF(1);
   if (s_thr[0] == 0) return;
   const uint32_t bin = s_thr[1];
   uint32_t* cnt = p.counters + (int64_t)row * 4;
@@ -104,7 +96,6 @@ __global__ void __launch_bounds__(kMThreads) topk_mfilter_kernel(TopkMultiParams
       const int64_t i = i0 + tid + (int64_t)u * kMThreads;
       key[u] = i < hi ? score_key_full(__ldg(src + i)) : 0u;
     }
-    TRF(2);
     uint32_t na = 0, nc = 0;
 #pragma unroll
     for (int u = 0; u < kFilterRegs; ++u) {
@@ -112,7 +103,6 @@ __global__ void __launch_bounds__(kMThreads) topk_mfilter_kernel(TopkMultiParams
       na += (key[u] != 0 && kb > bin);
       nc += (key[u] != 0 && kb == bin);
     }
-    TRF(3);
     uint32_t pa = block_excl_scan(na, warp_sums, &s_total);
     if (tid == 0) s_base[0] = s_total ? atomicAdd(&cnt[0], s_total) : 0u;
     uint32_t pc = block_excl_scan(nc, warp_sums, &s_total);
@@ -120,7 +110,6 @@ __global__ void __launch_bounds__(kMThreads) topk_mfilter_kernel(TopkMultiParams
     __syncthreads();
     pa += s_base[0];
     pc += s_base[1];
-    TRF(4);
 #pragma unroll
     for (int u = 0; u < kFilterRegs; ++u) {
       const uint32_t kb = key[u] >> 21;
@@ -135,7 +124,6 @@ __global__ void __launch_bounds__(kMThreads) topk_mfilter_kernel(TopkMultiParams
       }
     }
     __syncthreads();
-    TRF(5);
   }
 }
 

@@ -43,12 +43,6 @@ struct TopkParams {
 constexpr int kCandSmem = 16384;
 constexpr int kStreamUnroll = 16;   // independent loads in flight per thread in the streaming passes
 
-#ifdef MXB_TRACE_TK
-#define TRK(k) do { if (threadIdx.x == 0 && blockIdx.x == MXB_TRACE_TK) reinterpret_cast<long long*>(p.cand_key)[k] = clock64(); } while (0)
-#else
-#define TRK(k)
-#endif
-
 __global__ void __launch_bounds__(1024) topk_stream_kernel(TopkParams p, int sort_n) {
   extern __shared__ uint32_t dyn[];
   int32_t* sel = reinterpret_cast<int32_t*>(dyn);                 // [sort_n]
@@ -68,7 +62,6 @@ __global__ void __launch_bounds__(1024) topk_stream_kernel(TopkParams p, int sor
   for (int i = tid; i < kBigBins; i += 1024) hist[i] = 0;
   if (tid == 0) { s_na = 0; s_nc = 0; s_keff = 0; s_bin = 0; s_above = 0; s_cnt_bin = 0; }
   __syncthreads();
-  TRK(0);
   // ---- pass 1
   for (int64_t i0 = 0; i0 < n; i0 += 1024 * kStreamUnroll) {   // trip count uniform over the CTA (warp-wide votes inside)
     const int64_t i = i0 + tid;
@@ -82,7 +75,6 @@ __global__ void __launch_bounds__(1024) topk_stream_kernel(TopkParams p, int sor
     }
   }
   __syncthreads();
-  TRK(1);
   // ---- threshold bin: thread t owns bins 2047-2t and 2046-2t (descending)
   {
     const uint32_t h0 = hist[2047 - 2 * tid], h1 = hist[2046 - 2 * tid];
@@ -104,7 +96,6 @@ __global__ void __launch_bounds__(1024) topk_stream_kernel(TopkParams p, int sor
   int32_t* ci = in_smem ? ci_s : p.cand_idx + (int64_t)row * p.n;
   for (int i = tid; i < sort_n; i += 1024) sel[i] = 0x7FFFFFFF;
   __syncthreads();
-  TRK(2);
   // ---- pass 2
   for (int64_t i0 = 0; i0 < n; i0 += 1024 * kStreamUnroll) {   // trip count uniform over the CTA (warp-wide votes inside)
     const int64_t i = i0 + tid;
@@ -136,7 +127,6 @@ __global__ void __launch_bounds__(1024) topk_stream_kernel(TopkParams p, int sor
   }
   __syncthreads();
 
-  TRK(3);
   // ---- the `want` largest among the C candidates on the low 21 bits (8 + 8 + 5)
   uint32_t want = k_eff - n_above;
   uint32_t prefix = bin << 21, prefix_mask = 0xFFE00000u;
@@ -159,7 +149,6 @@ __global__ void __launch_bounds__(1024) topk_stream_kernel(TopkParams p, int sor
   }
   const uint32_t thr = prefix;
   const uint32_t need = want;  // ties to take (lowest ids), >= 1
-  TRK(4);
   // ---- ties: the need-th smallest id among candidates with key == thr (ids are unique)
   if (tid == 0) s_total = 0;
   __syncthreads();
@@ -198,7 +187,6 @@ __global__ void __launch_bounds__(1024) topk_stream_kernel(TopkParams p, int sor
     if (key > thr || (key == thr && (uint32_t)id <= idx_thr)) sel[atomicAdd(&s_na, 1u)] = id;
   }
   __syncthreads();
-  TRK(5);
   // ---- bitonic sort ascending (padding = INT_MAX)
   for (int size = 2; size <= sort_n; size <<= 1) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
@@ -212,9 +200,7 @@ __global__ void __launch_bounds__(1024) topk_stream_kernel(TopkParams p, int sor
       __syncthreads();
     }
   }
-  TRK(6);
   for (uint32_t i = tid; i < k_eff; i += 1024) out[i] = sel[i];
-  TRK(7);
 }
 
 int64_t topk_multi_workspace(int32_t rows, int64_t n, int32_t k);   // topk_multi.cu
