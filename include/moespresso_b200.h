@@ -456,7 +456,7 @@ typedef struct {
   int32_t dtype;    /* BF16 | F16, all five tensors */
   int32_t S, Skv, Hq, Hkv, D;
   float scale;
-  void* workspace;            /* partials of the items that are cut between pairs of SMs; NULL or too small: none is cut */
+  void* workspace;            /* partials of the items that are cut between SMs; NULL or too small: none is cut */
   int64_t workspace_bytes;
   int32_t* status;
 } mxb_flash_prefill_args;

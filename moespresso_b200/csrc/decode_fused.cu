@@ -4,8 +4,9 @@
 // (src/moespresso/runtime/deepseek_v4/decode_attention_kernel.py:669-786).  A token is all latency: the arithmetic of
 // the small kernels is nothing, so what counts is how many of them there are.  decode_prep_kernel does everything that
 // precedes the score scan and decode_sdpa_prep_kernel everything that precedes the attention, whatever the row type;
-// the scan, the selection and the attention are the package's kernels.  At 2,500 rows a token takes 57 us (44 us of it
-// in eight kernels); as some twenty single operators it took 378 us, 104 of them in kernels.
+// the scan, the selection and the attention are the package's kernels.  At 2,500 rows a token takes 26.5 us: seven kernels, each
+// launched while the one before it runs (the attention of a few tokens needs no merge kernel); as some twenty single operators
+// it took 378 us, 104 of them in kernels.
 #include "decode_rows.cuh"
 #include "ptx_sm100.cuh"
 

@@ -26,9 +26,9 @@
 // consecutive bytes of a row.
 //
 // int8 rows: bytes become fp16 integers exactly (0x6400 | u = 1024 + u).  q is scaled per head by a power of two so that its
-// largest element lies in [2^14, 2^15): a 16-bit q is then an fp16 number exactly down to 2^-28 of that element.  The
-// row's scale is folded into the logit and into P, as in the kernel for many tokens: the references follow
-// logit + log2(scale), the denominator takes the rounded weights divided by the scale.
+// largest element lies in [2^14, 2^15), or by 2^126 if it is below 2^-112: a 16-bit q is then an fp16 number exactly, but for
+// elements below 2^-28 of the largest.  The row's scale is folded into the logit and into P, as in the kernel for many tokens:
+// the references follow logit + log2(scale), the denominator takes the rounded weights divided by the scale.
 //
 // What bounds it: latency, front to back (launch, list, rows, two contractions of one pass, cluster barrier, output); a
 // further 64 rows per CTA cost 2 us.  Both sides measured: at the rule in launch_sparse_few.

@@ -116,7 +116,8 @@ def fused_decode_sdpa(q, window, row, pooled, sel, sinks, inv_freq, params, *, s
     sel int32 ``[topk]``, sinks float16 ``[n_heads]``, inv_freq float32 ``[32]``, params int32
     ``[position, write_idx]``.  Every window row and every selected row is a key and a value; the sink joins the
     maximum and the denominator once.  Returns float16 ``[n_heads, 512]`` after the inverse rope.
-    Launches: the operands (rope, window, sinks), the attention (and its merge), the inverse rope."""
+    Launches: the operands (rope, window, sinks), the attention (and its merge, where its splits are not one cluster), the
+    inverse rope."""
     r = native("fused_decode_sdpa", q, window, row, pooled, sel, sinks, inv_freq, params, scale)
     if r is not None:
         return r
