@@ -78,7 +78,7 @@ def is_current() -> bool:
     return library_is_current() and native_is_current()
 
 
-def _native_command():
+def _native_command(out: str):
     """g++ over torch's headers; the symbols come from the torch libraries that the process has loaded."""
     import sysconfig
 
@@ -88,7 +88,7 @@ def _native_command():
     inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
            sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
     return ["g++", *GXX_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-            *(f"-I{d}" for d in inc), os.path.join(CSRC, "host_calls.cpp"), "-o", NATIVE, f"-L{os.path.join(root, 'lib')}",
+            *(f"-I{d}" for d in inc), os.path.join(CSRC, "host_calls.cpp"), "-o", out, f"-L{os.path.join(root, 'lib')}",
             "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
 
 
@@ -118,15 +118,19 @@ def _write(stamp: str, digest: str) -> None:
         f.write(digest)
 
 
+def _native_part() -> str:
+    """Where this process compiles to; moved into place when it is whole (another process may have the old one loaded)."""
+    return os.path.join(HERE, "build", f"native.{os.getpid()}.part")
+
+
 def _start_native():
     os.makedirs(os.path.join(HERE, "build"), exist_ok=True)
-    if os.path.exists(NATIVE_STAMP):
-        os.remove(NATIVE_STAMP)
-    return [("host_calls.cpp", _start(_native_command()))]
+    return [("host_calls.cpp", _start(_native_command(_native_part())))]
 
 
 def _finish_native(procs, verbose: bool) -> None:
     _finish(procs, "native.log", verbose)
+    os.replace(_native_part(), NATIVE)
     _write(NATIVE_STAMP, _native_digest())
 
 

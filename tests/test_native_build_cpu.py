@@ -59,3 +59,16 @@ def test_a_missing_extension_does_not_keep_the_library_from_loading(monkeypatch)
     monkeypatch.setattr(_build, "build_library", _broken_build)
     assert _build.library_is_current() and not _build.is_current()
     assert _abi.load().mxb_abi_version() == 1
+
+
+def test_a_rebuild_leaves_the_loaded_extension_alone():
+    """Ranks that start together may each build: the file is replaced whole, what another process has mapped stays."""
+    import os
+    _build.build()
+    before = os.stat(_build.NATIVE).st_ino
+    held = open(_build.NATIVE, "rb")
+    _build.build_native()
+    assert os.stat(_build.NATIVE).st_ino != before and os.fstat(held.fileno()).st_ino == before
+    assert held.read(4) == b"\x7fELF" and _build.is_current()
+    assert not [n for n in os.listdir(os.path.join(_build.HERE, "build")) if n.endswith(".part")]
+    held.close()
