@@ -92,6 +92,35 @@ def test_pairs_of_query_tiles(S, past, Hq, Hkv, dt):
     assert max_abs(out, ref) <= 2 * 2.0 ** -9 * float(np.abs(v).max())
 
 
+@pytest.mark.parametrize("S,past,Hq,Hkv", [
+    (64, 3001, 2, 1),     # pairs
+    (33, 3000, 45, 15),   # single CTAs, a stretch per SM
+    (128, 2000, 75, 25),  # more of them: stretches that end one item and start the next
+    (1, 4000, 51, 17),    # one row
+])
+@pytest.mark.parametrize("dt,gate", [("bf16", True), ("f16", False)])
+@pytest.mark.parametrize("scratch", ["whole", "short", "none"])
+def test_cut_items_of_pairs_and_single_ctas(S, past, Hq, Hkv, dt, gate, scratch, monkeypatch):
+    """Items cut at equal stretches and joined, and the same calls where the scratch for that is too small or missing."""
+    need_gpu()
+    rng = np.random.default_rng(S + past)
+    tdt = torch.bfloat16 if dt == "bf16" else torch.float16
+    q, k, v, g = _inputs(rng, S, past, Hq, Hkv, bf16_round if dt == "bf16" else f16_round)
+    q[-1] *= 8.0           # one peaked row: its maximum moves between the pieces
+    asked, whole = [], fa.workspace
+
+    def scratch_of(nbytes, device):
+        asked.append(nbytes)
+        return whole(nbytes, device) if scratch == "whole" else whole(nbytes - 4096, device) if scratch == "short" else None
+    monkeypatch.setattr(fa, "workspace", scratch_of)
+    out = fa.sdpa_fa_prefill(dev(q, tdt), dev(k, tdt), dev(v, tdt), 1.0 / 16.0, gate=dev(g, tdt) if gate else None,
+                             layout="lhd", check=True)
+    assert len(asked) == 1 and asked[0] > 0          # the plan cuts
+    ref = qwen.causal_gqa_prefill(q, k, v, g if gate else None, scale=1.0 / 16.0, past_len=past)
+    # half a unit of bf16 (2^-9) for P and for the result, relative to the largest |v| a row can average
+    assert max_abs(out, ref) <= 2 * 2.0 ** -9 * float(np.abs(v).max())
+
+
 def test_gate_layout_without_tensor_map():
     """A gate whose row stride is not a multiple of its head stride cannot be described by a tensor map: the drain
     then reads the gate and writes the output with per-thread accesses.  Same result as the tiled drain."""
